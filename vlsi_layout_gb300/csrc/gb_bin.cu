@@ -181,43 +181,75 @@ __device__ __forceinline__ void walk_raw_boxes(const int4* bx, const long long* 
   }
 }
 
-// Raw source: one thread per box; boxes of a warp can straddle cells, so the
-// warp reduces per cell only when all lanes agree, else atomics per lane.
-__global__ void k_bbox_raw(const DLayer* S, DLayer* O, int ncell, int E, int N, int W, int Sg,
-                           DStatus* st) {
+// Raw source.  A lane keeps the bounds of its boxes in registers while the
+// warp stays in one cell; the warp adds them to the cell's box when the cell
+// ends, the block at its end, so a large cell takes four atomics per block
+// and not four per 32 boxes (12M boxes of one cell: 1000 -> 40 us; four
+// same-address atomics per 32 boxes had bound it, HBM's share is 29 us).
+// Bounds that the cell's box already holds take no atomic.  A step whose
+// lanes straddle cells adds its boxes lane by lane.
+__device__ __forceinline__ void bbox_add(int4* dst, int4 b) {
+  const int4 cur = __ldcg(dst);  // bounds only widen, so an old value costs at most an atomic
+  if (b.x < cur.x) atomicMin(&dst->x, b.x);
+  if (b.y < cur.y) atomicMin(&dst->y, b.y);
+  if (b.z > cur.z) atomicMax(&dst->z, b.z);
+  if (b.w > cur.w) atomicMax(&dst->w, b.w);
+}
+__device__ __forceinline__ int4 bbox_none() { return make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN); }
+__device__ __forceinline__ int4 bbox_join(int4 a, int4 b) {
+  return make_int4(min(a.x, b.x), min(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
+}
+__device__ __forceinline__ int4 bbox_warp(int4 a) {
+  a.x = __reduce_min_sync(0xffffffffu, a.x);
+  a.y = __reduce_min_sync(0xffffffffu, a.y);
+  a.z = __reduce_max_sync(0xffffffffu, a.z);
+  a.w = __reduce_max_sync(0xffffffffu, a.w);
+  return a;
+}
+
+__global__ void __launch_bounds__(256) k_bbox_raw(const DLayer* S, DLayer* O, int ncell, int E, int N, int W, int Sg,
+                                                  DStatus* st) {
+  __shared__ int4 wb[8];
+  __shared__ int wk[8];
   if (st->err) return;
-  const long long n = S->nbox;
-  const int4* bx = S->boxes;
-  const long long* coff = S->coff;
-  walk_raw_boxes<BIN_LD>(bx, coff, ncell, n, [&](long long i, bool valid_i, int4 box, int kc) {
-    int x1 = INT32_MAX, y1 = INT32_MAX, x2 = INT32_MIN, y2 = INT32_MIN, k = -1;
-    if (valid_i) {
-      int4 g;
-      if (!grow_box(box, E, N, W, Sg, g)) {
-        gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, i);
-      } else {
-        x1 = g.x; y1 = g.y; x2 = g.z; y2 = g.w;
-        k = kc;
-      }
+  int4* const cb = O->cbox;
+  int kc = -1;  // the cell whose bounds the warp holds
+  int4 acc = bbox_none();
+  walk_raw_boxes<BIN_LD>(S->boxes, S->coff, ncell, S->nbox, [&](long long i, bool valid_i, int4 box, int k) {
+    int4 g = bbox_none();
+    if (valid_i && !grow_box(box, E, N, W, Sg, g)) {
+      gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, i);
+      g = bbox_none();
     }
     const int k0 = __shfl_sync(0xffffffffu, k, 0);
-    const bool same = __all_sync(0xffffffffu, k == k0 || k < 0);
-    if (same) {
-      if (k0 >= 0 || __any_sync(0xffffffffu, k >= 0)) {
-        int kk = k0;
-        if (kk < 0) {
-          unsigned m = __ballot_sync(0xffffffffu, k >= 0);
-          kk = __shfl_sync(0xffffffffu, k, __ffs(m) - 1);
-        }
-        warp_bbox_atomic(&O->cbox[kk], x1, y1, x2, y2);
-      }
-    } else if (k >= 0) {
-      atomicMin(&O->cbox[k].x, x1);
-      atomicMin(&O->cbox[k].y, y1);
-      atomicMax(&O->cbox[k].z, x2);
-      atomicMax(&O->cbox[k].w, y2);
+    const bool same = __all_sync(0xffffffffu, !valid_i || k == k0);
+    if (!same || k0 != kc) {
+      const int4 r = bbox_warp(acc);
+      if (gb_lane() == 0 && kc >= 0 && r.x <= r.z) bbox_add(&cb[kc], r);
+      acc = bbox_none();
+      kc = same ? k0 : -1;
     }
+    if (same) acc = bbox_join(acc, g);
+    else if (valid_i && g.x <= g.z) bbox_add(&cb[k], g);
   });
+  acc = bbox_warp(acc);
+  if (gb_lane() == 0) {
+    wb[gb_warp()] = acc;
+    wk[gb_warp()] = acc.x <= acc.z ? kc : -1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {  // the block's warps hold neighbouring chunks: nearly always one cell
+    for (int w = 0; w < 8; ++w) {
+      if (wk[w] < 0) continue;
+      int4 b = wb[w];
+      for (int v = w + 1; v < 8; ++v)
+        if (wk[v] == wk[w]) {
+          b = bbox_join(b, wb[v]);
+          wk[v] = -1;
+        }
+      bbox_add(&cb[wk[w]], b);
+    }
+  }
 }
 
 __device__ __forceinline__ void tile_of_index(const DLayer* L, long long t, int& k, int& tx, int& ty) {
@@ -398,18 +430,145 @@ __device__ __forceinline__ void emit_warp(DLayer* O, int k, int4 b, long long pa
   }
 }
 
+// Raw source, one contiguous chunk of boxes per block.  The tiles of the
+// chunk's cells are counted in shared memory (up to SPLIT_SM tiles; layers of
+// a few hundred tiles had been bound by global atomics on those few counters:
+// 1M boxes over 400 tiles, count 173 -> 15 us, scatter 178 -> 25 us).  Count:
+// the block adds its counts to the layer's once.  Scatter: the block counts
+// its chunk, reserves each tile's slots with one atomic, and places the
+// pieces on a second walk over the chunk.  A chunk over more tiles takes its
+// slots from the global counters, which many tiles spread.  A box over more
+// than SPLIT_WIDE tiles (the one-box frame of an erosion covers them all) is
+// left to the whole block after the walk: one lane had walked its tiles in
+// series (1200 tiles, 280 us).
+#define SPLIT_SM 8192
+#define SPLIT_SM_MIN 32768  // smaller layers: the counters see few atomics, and the second walk costs more
+#define SPLIT_WIDE 32
+#define SPLIT_NWIDE 64  // wide boxes of one chunk held for the block; more are walked by their lanes
+
+struct SplitBox {
+  int4 b;
+  long long idx;
+  int k;
+};
+
+// Tile ranges of a box in its cell: half-open extents (MODE 0) or closed.
+template <int MODE>
+__device__ __forceinline__ int4 box_tiles(int4 b, int g) {
+  return make_int4(gb_floor_shift(b.x, g), gb_floor_shift(b.y, g), gb_floor_shift(MODE ? b.z : b.z - 1, g),
+                   gb_floor_shift(MODE ? b.w : b.w - 1, g));
+}
+
+template <int MODE>
+__device__ __forceinline__ void put_piece(DLayer* O, long long pos, int4 b, long long idx, int tx, int ty, int g) {
+  if (MODE == 0) {
+    const int ox = tx << g, oy = ty << g;
+    const int x1 = max(b.x, ox) - ox, y1 = max(b.y, oy) - oy;
+    const int x2 = (int)(min((long long)b.z, (long long)ox + (1ll << g)) - ox);
+    const int y2 = (int)(min((long long)b.w, (long long)oy + (1ll << g)) - oy);
+    O->pcs[pos] = gb_pack(x1, y1, x2, y2);
+  } else {
+    ((int*)O->pcs)[pos] = (int)idx;
+  }
+}
+
 template <int MODE, bool SCATTER>
-__global__ void k_split_raw(const DLayer* S, DLayer* O, int ncell, int g, int E, int N, int W,
-                            int Sg, DStatus* st) {
+__global__ void __launch_bounds__(256) k_split_raw(const DLayer* S, DLayer* O, int ncell, int g, int E, int N, int W,
+                                                   int Sg, DStatus* st) {
+  __shared__ int hist[SPLIT_SM];
+  __shared__ SplitBox wide[SPLIT_NWIDE];
+  __shared__ int nwide;
   if (st->err) return;
-  walk_raw_boxes<SCATTER ? 2 : BIN_LD>(S->boxes, S->coff, ncell, S->nbox,
-                                       [&](long long i, bool valid_i, int4 box, int k) {
-    // raw boxes of one warp fall in scattered tiles of their cell, so a per-lane slot is cheaper
-    // here than grouping lanes by tile
-    int4 b;
-    if (!valid_i || !grow_box(box, E, N, W, Sg, b)) return;  // invalid: reported by k_bbox_raw
-    emit_box_tiles<MODE, SCATTER>(O, k, b, i, g);
-  });
+  const long long n = S->nbox;
+  const int4* const bx = S->boxes;
+  const long long* const coff = S->coff;
+  const int4* const win = O->win;
+  const long long* const tbase = O->tbase;
+  int* const tcount = O->tcount;
+  const long long* const tstart = O->tstart;
+  const int nt = blockDim.x, tid = threadIdx.x;
+  const long long ch = max((long long)nt * 2, (((n + gridDim.x - 1) / gridDim.x) + nt - 1) / nt * nt);
+  const long long c0 = (long long)blockIdx.x * ch, c1 = min(n, c0 + ch);
+  if (c0 >= n) return;
+  const int k0 = gb_find_cell(coff, ncell, c0), k1 = gb_find_cell(coff, ncell, c1 - 1);
+  const long long r0 = tbase[k0], nr = tbase[k1 + 1] - r0;
+  const bool sm = nr <= SPLIT_SM && n >= SPLIT_SM_MIN;
+  if (sm)
+    for (int i = tid; i < (int)nr; i += nt) hist[i] = 0;
+  // one tile of a box: count it (PLACE = 0) or take its slot and write the piece
+  auto visit = [&](bool place, int4 b, long long idx, int tx, int ty, long long t) {
+    if (!place) {
+      if (sm) atomicAdd(&hist[t - r0], 1);
+      else atomicAdd(&tcount[t], 1);
+    } else {
+      const int slot = sm ? atomicAdd(&hist[t - r0], 1) : atomicAdd(&tcount[t], 1);
+      put_piece<MODE>(O, tstart[t] + slot, b, idx, tx, ty, g);
+    }
+  };
+  auto walk = [&](bool place) {
+    if (tid == 0) nwide = 0;
+    __syncthreads();
+    int kc = -1;
+    int4 w = make_int4(0, 0, 0, 0);
+    long long tb = 0;
+    for (long long i0 = c0 + tid; i0 < c1; i0 += (long long)nt * BIN_LD) {
+      int4 ld[BIN_LD];
+#pragma unroll
+      for (int u = 0; u < BIN_LD; ++u)
+        if (i0 + (long long)u * nt < c1) ld[u] = bx[i0 + (long long)u * nt];
+#pragma unroll
+      for (int u = 0; u < BIN_LD; ++u) {
+        const long long i = i0 + (long long)u * nt;
+        if (i >= c1) break;
+        int4 b;
+        if (!grow_box(ld[u], E, N, W, Sg, b)) continue;  // invalid: reported by k_bbox_raw
+        if (kc < 0 || i >= coff[kc + 1]) {
+          kc = k0 == k1 ? k0 : k0 + gb_find_cell(coff + k0, k1 + 1 - k0, i);
+          w = win[kc];
+          tb = tbase[kc];
+        }
+        const int4 q = box_tiles<MODE>(b, g);
+        if ((long long)(q.z - q.x + 1) * (q.w - q.y + 1) > SPLIT_WIDE) {
+          const int at = atomicAdd(&nwide, 1);
+          if (at < SPLIT_NWIDE) {
+            wide[at].b = b;
+            wide[at].idx = i;
+            wide[at].k = kc;
+            continue;
+          }
+        }
+        for (int ty = q.y; ty <= q.w; ++ty)
+          for (int tx = q.x; tx <= q.z; ++tx)
+            visit(place, b, i, tx, ty, tb + (long long)(ty - w.y) * w.z + (tx - w.x));
+      }
+    }
+    __syncthreads();
+    const int nb = min(nwide, SPLIT_NWIDE);
+    for (int j = 0; j < nb; ++j) {
+      const SplitBox s = wide[j];
+      const int4 q = box_tiles<MODE>(s.b, g), ws = win[s.k];
+      const long long sx = q.z - q.x + 1, tot = sx * (q.w - q.y + 1);
+      for (long long v = tid; v < tot; v += nt) {
+        const int ty = q.y + (int)(v / sx), tx = q.x + (int)(v % sx);
+        visit(place, s.b, s.idx, tx, ty, tbase[s.k] + (long long)(ty - ws.y) * ws.z + (tx - ws.x));
+      }
+    }
+    __syncthreads();
+  };
+  if (!SCATTER) {
+    walk(false);
+    if (sm)
+      for (int i = tid; i < (int)nr; i += nt)
+        if (hist[i]) atomicAdd(&tcount[r0 + i], hist[i]);
+    return;
+  }
+  if (sm) {
+    walk(false);
+    for (int i = tid; i < (int)nr; i += nt)
+      if (hist[i]) hist[i] = atomicAdd(&tcount[r0 + i], hist[i]);
+    __syncthreads();
+  }
+  walk(true);
 }
 
 template <bool SCATTER>
