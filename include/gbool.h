@@ -403,8 +403,9 @@ long long gb_launch_count(gb_context* ctx);
  * pieces; then 16 per-warp counters of the sub-band steps (compress,
  * rasterise, scan, count, write, transpose cycles, members, columns); then
  * per sub-band-count bucket (1, 2-3, 4-7, 8-15, 16-31, 32+) the tiles and
- * their phase-C cycles; the sub-bands whose column words spilled to scratch
- * and their cycles, the others and theirs; all since gb_tile_timing(ctx, 1). */
+ * their phase-C cycles; the wide sub-bands (more columns or y ranks than one
+ * warp's buffer holds) and their cycles, the others and theirs; all since
+ * gb_tile_timing(ctx, 1). */
 int gb_tile_timing(gb_context* ctx, int on);
 /* Diagnostics: runs one radix pass whose only CTA waits for a predecessor
  * tile that never publishes; returns the status it reports (GB_ERR_TIMEOUT

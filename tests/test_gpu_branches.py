@@ -1,0 +1,79 @@
+"""The branches of the binning and scanline kernels at the sizes where they
+change over: shared or global tile counters, boxes over many tiles, sub-bands
+of a tile with more columns or y ranks than a warp's buffer holds at each
+level.  Everything bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from gen import random_layer
+
+pytestmark = pytest.mark.gpu
+
+
+def canon(b):
+    b = np.asarray(b, np.int32).reshape(-1, 4)
+    return b[np.lexsort((b[:, 3], b[:, 2], b[:, 1], b[:, 0]))] if len(b) else b
+
+
+def run(ctx, fn):
+    m = ctx.mark()
+    try:
+        return canon(fn().to_numpy())
+    finally:
+        ctx.release(m)
+
+
+# n around the shared-counter minimum (32768); dies of few tiles, of more tiles than shared counters (8192);
+# boxes over 33 tiles and more, fewer and more of them than a block holds (64)
+@pytest.mark.parametrize("n,die,nwide", [(32767, 400_000, 0), (32768, 400_000, 1), (33000, 6_100_000, 3),
+                                         (40001, 900_000, 65), (700, 3_000_000, 130), (1, 5_000_000, 1)])
+def test_binning(ctx, oracle, n, die, nwide):
+    A = random_layer(n, die=die, seed=n)
+    rng = np.random.default_rng(n)
+    y = rng.integers(-die // 2, die // 2, nwide)
+    wide = np.stack([np.full(nwide, -die // 2) + np.arange(nwide), y, np.full(nwide, die // 2), y + 9], 1).astype(np.int32)
+    A = np.concatenate([A, wide])[rng.permutation(n + nwide)]
+    assert np.array_equal(run(ctx, lambda: ctx.op(4, ctx.layer(A))), oracle.merge(A))
+    m = ctx.mark()
+    assert int(ctx.area(ctx.layer(A))[0]) == oracle.union_area(A)
+    ctx.release(m)
+    nc, lab = ctx.components(A)
+    en, elab = oracle.components(A)
+    assert nc == en and np.array_equal(lab, elab)
+
+
+def test_binning_cells(ctx, oracle):
+    """Cells of 0 .. 700 boxes: chunks that start and end inside cells, runs of empty cells."""
+    rng = np.random.default_rng(4)
+    counts = rng.choice([0, 1, 2, 31, 32, 33, 700], 400)
+    off = np.concatenate([[0], np.cumsum(counts)])
+    A = random_layer(int(off[-1]), die=150_000, seed=9, x0=-70_000, y0=-70_000)
+    m = ctx.mark()
+    area = ctx.area(ctx.layer(A, off))
+    ctx.release(m)
+    assert [int(a) for a in area] == [oracle.union_area(A[off[k]:off[k + 1]]) if counts[k] else 0 for k in range(len(counts))]
+
+
+# columns of a sub-band around the buffers of levels 0..3 (128, 288, 640, 1024)
+@pytest.mark.parametrize("wires", [64, 65, 144, 145, 320, 321, 512, 513, 700])
+def test_wide_subbands(ctx, oracle, wires):
+    i = np.arange(wires)
+    A = np.stack([50 + 3 * (i % 7), 7 * i, 60_000 - (i % 11), 7 * i + 3], 1).astype(np.int32)
+    B = random_layer(400, die=9000, wmin=3, wmax=400, seed=wires)
+    for op in (0, 2, 3, 4):
+        got = run(ctx, lambda: ctx.op(op, ctx.layer(A), ctx.layer(B) if op != 4 else None))
+        assert np.array_equal(got, oracle.boolean(A, B, op) if op != 4 else oracle.merge(A)), op
+    C = np.concatenate([A, B, A[::3]])
+    assert np.array_equal(run(ctx, lambda: ctx.op(7, ctx.layer(C))), oracle.boolean(C, C[:0], 7))
+
+
+# y ranks of a tile around the bitmaps of levels 0..3 (188, 320, 640, 2052 words)
+@pytest.mark.parametrize("n", [2900, 3300, 5500, 7000, 11000, 16000])
+def test_many_y_ranks(ctx, oracle, n):
+    rng = np.random.default_rng(n)
+    y = rng.permutation(32_000)[:n] * 2
+    x = rng.integers(0, 65_000, n)
+    A = np.stack([x, y, x + rng.integers(1, 500, n), y + 1], 1).astype(np.int32)
+    B = random_layer(500, die=65_000, wmin=20, wmax=3000, seed=n)
+    for op in (0, 3):
+        assert np.array_equal(run(ctx, lambda: ctx.op(op, ctx.layer(A), ctx.layer(B))), oracle.boolean(A, B, op)), op

@@ -33,6 +33,9 @@
 //     it again.  The pieces are dealt to the lanes 32 at a time in (column,
 //     row) order, so a column with many pieces does not hold up the warp; a
 //     piece's 16-byte record goes to the CTA's record region at its index.
+//     A sub-band with more columns or y ranks than a warp's buffer holds is
+//     wide: the tile's wide ones are swept afterwards by fewer warps with
+//     larger buffers.
 //  D. Stitch.  The records come into shared memory in one bulk copy.  Each
 //     continuation is linked to the open piece of the previous sub-band with
 //     the same y-interval; every chain head becomes one strip.  The output
@@ -55,12 +58,19 @@
 #define TK_SBS 256
 #define TK_MDS 128   // sub-bands whose metadata fits in the bitmap region after phase B
 #define TK_MD_INTS (TK_MDS * 4 + (TK_MDS + 2) * 2 + TK_MDS * 2 * 2)  // sbinfo, sbh, sbct, sbol, sbrec
-#define TK_LBW 128
-#define TK_LVN 256
+// Per-warp sweep buffers of phase C (6 KB a warp): bitmap words over the tile's y ranks, columns.  A sub-band
+// that needs more is wide; the wide ones of a tile are swept after the others by 4, 2 or 1 warps with 2, 4 or 8
+// times the buffer (levels 1..3), so their words stay in shared memory too.  Standard-cell tiles (2700 boxes of
+// each layer) have 160..290 columns in nearly every sub-band: with their words in the global scratch, and a walk
+// back over them for every piece, XOR of two 1M-box layers took 2337 us, now 1898 us.
+#define TK_LBW 188
+#define TK_LVN 132
 #define TK_LCN 128
+#define TK_WLEVELS 3
 #define TK_MC 128   // sub-band members kept in the per-warp member cache (8 bytes each)
 #define TK_MLD 2    // member records loaded per lane before the first is used (per 1024-cell deck: 4 -> 2
                     // records 30.88 -> 30.59 ms)
+#define TK_DU 2     // pieces per thread and step of phase D when the records stay in the scratch
 #define TK_LD 2     // independent global loads in flight per thread in the streaming loops
 #define TK_DIRECT 1 // columns of a member painted on its own lane; the rest are spread over the warp
                     // (measured per 1024-cell deck: 0 / 1 / 2 / 3 / 4 / 8 columns -> 35.16 / 34.78 /
@@ -116,6 +126,9 @@ struct TileSmem {
     int4 dbuf_align;  // the region starts on 16 bytes: bulk copies and int4 records land in it
   };
   int sbnext;                            // next sub-band to hand to a warp
+  int nwide[TK_WLEVELS + 1];             // wide sub-bands found at each level of phase C (listed in xyv)
+  int narrow;                            // sub-bands swept at level 1 that level 0 could have held
+  int hint;                              // the previous tile was mostly wide: start at level 1
   unsigned long long mbar;               // completion of phase D's bulk copies (one phase per tile)
   long long tmp64[33];
   long long tile;
@@ -140,9 +153,29 @@ struct TileSmem {
   int* sbc;      // per sub-band member counts / cursors (sbc_s or scratch)
   int** sbol;    // open list (then continuation list) per sub-band
   PieceRec** sbrec;  // strip pieces per sub-band (global piece index = sbinfo.x + local index)
-  unsigned* biglb;
   int* succ;
 };
+// Wide lists of phase C, alternating by level, behind the metadata and the hand-out order in xyv.
+#define TK_WLIST(s, level) ((s).xyv + TK_MD_INTS + TK_SBS + ((level) & 1) * (TK_NSBMAX + 2))
+static_assert(TK_MD_INTS + TK_SBS + 2 * (TK_NSBMAX + 2) <= 2 * TK_WMAX + 2 * (TK_WMAX / 2 + 1), "wide lists");
+
+// Sweep buffer of a warp at level 1..3: columns, bitmap words, cached members.
+__device__ __forceinline__ int wide_cols(int level) { return level == 1 ? 288 : level == 2 ? 640 : 1024; }
+__device__ __forceinline__ int wide_lbw(int level) { return level == 1 ? 320 : level == 2 ? 640 : 2052; }
+__device__ __forceinline__ int wide_mc(int level) { return level == 1 ? 176 : level == 2 ? 168 : 488; }
+constexpr int wide_bytes(int cols, int lbw, int mc) {
+  return cols * 16 + mc * 8 + lbw * 8 + (cols + 4) * 4 + 64 * (cols / 32) * 4;
+}
+constexpr int TK_WBUF = 6128;  // level 0's bytes per warp; 2, 4 or 8 warps' buffers together at the levels above
+static_assert(wide_bytes(288, 320, 176) <= 2 * TK_WBUF && wide_bytes(640, 640, 168) <= 4 * TK_WBUF &&
+                  wide_bytes(1024, 2052, 488) <= 8 * TK_WBUF,
+              "wide sweep buffers");
+static_assert(sizeof(((TileSmem*)0)->lb) + sizeof(((TileSmem*)0)->lp) + sizeof(((TileSmem*)0)->lv) +
+                      sizeof(((TileSmem*)0)->ca) + sizeof(((TileSmem*)0)->cb) + sizeof(((TileSmem*)0)->mc) +
+                      sizeof(((TileSmem*)0)->srow) ==
+                  TK_NW * TK_WBUF,
+              "sweep buffers");
+
 #include <cstddef>
 // Bulk asynchronous copies need 16-byte aligned shared-memory addresses, and
 // the staged ranks, piece records and sub-band metadata are read as int4.
@@ -269,9 +302,12 @@ __device__ __forceinline__ void tile_lookup(int op, const DLayer* A, const DLaye
 
 // TIMING: the phase counters of gb_tile_timing are compiled in (tctr non-null
 // then); the production instance has none of that code.
-template <bool TIMING>
-__device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int nA, char* base,
-                             unsigned long long scr, long long* tctr) {
+// WIDE: the level's larger buffers (level 1..3).  Returns false, with nothing
+// done, when the sub-band needs the next level's buffers; at the last level
+// columns beyond them spill to the scratch.
+template <bool TIMING, bool WIDE>
+__device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int nA, char* base,
+                             unsigned long long scr, int level, long long* tctr) {
   if (!TIMING) tctr = nullptr;
   const int lane = gb_lane(), wid = gb_warp();
   long long q0 = tctr ? clock64() : 0;
@@ -293,13 +329,34 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
       s.sbol[sb] = nullptr;
       s.sbrec[sb] = nullptr;
     }
-    return;
+    return true;
   }
   const int rowbase = 63 * sb - 1;
   const int nwy = ((Ny - 1) >> 5) + 1;
-  unsigned* lb = nwy <= TK_LBW ? s.lb[wid] : s.biglb + (size_t)wid * 2 * nwy;
-  unsigned* lp = nwy <= TK_LBW ? s.lp[wid] : lb + nwy;
-  const bool cache = m <= TK_MC;
+  const int lcn = WIDE ? wide_cols(level) : TK_LCN, mcn = WIDE ? wide_mc(level) : TK_MC;
+  if (nwy > (WIDE ? wide_lbw(level) : TK_LBW)) return false;  // the last level holds any tile's y ranks
+  unsigned long long *ca, *cb, *mc;
+  unsigned *lb, *lp, *srow;
+  int* lv;
+  const int srw = WIDE ? lcn >> 5 : TK_LCN / 32;  // words per row of srow
+  if (WIDE) {
+    ca = reinterpret_cast<unsigned long long*>(s.dbuf + (size_t)wid * (TK_WBUF << level));
+    cb = ca + lcn;
+    mc = cb + lcn;
+    lb = reinterpret_cast<unsigned*>(mc + mcn);
+    lp = lb + wide_lbw(level);
+    lv = reinterpret_cast<int*>(lp + wide_lbw(level));
+    srow = reinterpret_cast<unsigned*>(lv + lcn + 4);
+  } else {
+    ca = s.ca[wid];
+    cb = s.cb[wid];
+    mc = s.mc[wid];
+    lb = s.lb[wid];
+    lp = s.lp[wid];
+    lv = s.lv[wid];
+    srow = s.srow[wid][0];
+  }
+  const bool cache = m <= mcn;
   for (int w = lane; w < nwy; w += 32) lb[w] = 0;
   __syncwarp();
   for (int j0 = 0; j0 < m; j0 += 32 * TK_MLD) {
@@ -316,7 +373,7 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
         const int4 r = rr[u];
         if (cache) {
           const unsigned lo = (unsigned)max((r.x & 0x7fffffff) - rowbase, 0), hi = (unsigned)min(r.y - rowbase, 64);
-          s.mc[wid][j] = (unsigned long long)(lo | (hi << 7) | (((unsigned)r.x >> 31) << 14) | ((unsigned)r.z << 15)) |
+          mc[j] = (unsigned long long)(lo | (hi << 7) | (((unsigned)r.x >> 31) << 14) | ((unsigned)r.z << 15)) |
                          ((unsigned long long)(unsigned)r.w << 32);
         }
         atomicOr(&lb[r.z >> 5], 1u << (r.z & 31));
@@ -327,7 +384,7 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
   __syncwarp();
   int nl;
   {
-    const int per = (nwy + 31) >> 5, w0 = lane * per, w1 = min(nwy, w0 + per);
+    const int per = WIDE ? ((nwy + 31) >> 5) | 1 : (nwy + 31) >> 5, w0 = min(nwy, lane * per), w1 = min(nwy, w0 + per);
     int cnt = 0;
     for (int w = w0; w < w1; ++w) cnt += __popc(lb[w]);
     int tot;
@@ -341,23 +398,23 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
     atomicAdd((unsigned long long*)&tctr[6], (unsigned long long)m);
     atomicAdd((unsigned long long*)&tctr[7], (unsigned long long)L);
   }
-  int* lv = s.lv[wid];
-  unsigned long long* ca = s.ca[wid];
-  unsigned long long* cb = s.cb[wid];
-  if (nl > TK_LVN || L > TK_LCN) {
+  if (L > lcn) {
+    if (!WIDE || level < TK_WLEVELS) return false;
     unsigned long long pv = 0, pc = 0;
     if (lane == 0) {
-      if (nl > TK_LVN) pv = (unsigned long long)sc_up(s, base, half, (unsigned long long)nl * 4);
-      if (L > TK_LCN) pc = (unsigned long long)sc_up(s, base, half, (unsigned long long)L * 16);
+      pv = (unsigned long long)sc_up(s, base, half, (unsigned long long)nl * 4);
+      pc = (unsigned long long)sc_up(s, base, half, (unsigned long long)L * 16);
     }
     pv = __shfl_sync(0xffffffffu, pv, 0);
     pc = __shfl_sync(0xffffffffu, pc, 0);
-    if ((nl > TK_LVN && !pv) || (L > TK_LCN && !pc)) return;  // s.err is set
-    if (pv) lv = (int*)pv;
-    if (pc) { ca = (unsigned long long*)pc; cb = ca + L; }
+    if (!pv || !pc) return true;  // s.err is set
+    lv = (int*)pv;
+    ca = (unsigned long long*)pc;
+    cb = ca + L;
   }
+  if (WIDE && level == 1 && lane == 0 && L <= TK_LCN && nwy <= TK_LBW) atomicAdd(&s.narrow, 1);
   {
-    const int per = (nwy + 31) >> 5, w0 = lane * per, w1 = min(nwy, w0 + per);
+    const int per = WIDE ? ((nwy + 31) >> 5) | 1 : (nwy + 31) >> 5, w0 = min(nwy, lane * per), w1 = min(nwy, w0 + per);
     for (int w = w0; w < w1; ++w) {
       unsigned bits = lb[w];
       int k = lp[w];
@@ -370,7 +427,8 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
   }
   // ---- rasterise: one member per lane; each column word is updated as two
   // 32-bit halves with native shared-memory atomicOr
-  const int per = (L + 31) >> 5, c0 = min(L, lane * per), c1e = min(L, c0 + per);
+  // columns per lane; an odd count keeps the lanes' 8-byte words on different banks (wide ones have 5..33)
+  const int per = WIDE ? ((L + 31) >> 5) | 1 : (L + 31) >> 5, c0 = min(L, lane * per), c1e = min(L, c0 + per);
   for (int c = c0; c < c1e; ++c) { ca[c] = 0; cb[c] = 0; }
   __syncwarp();
   // 32 members at a time: the (member, column) pairs of the group are spread
@@ -384,7 +442,7 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
     if (j < m) {
       int lo, hi, yz, yw;
       if (cache) {
-        const unsigned long long e = s.mc[wid][j];
+        const unsigned long long e = mc[j];
         const unsigned e0 = (unsigned)e;
         lo = (int)(e0 & 127u);
         hi = (int)((e0 >> 7) & 127u);
@@ -473,12 +531,12 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
       s.sbrec[sb] = nullptr;
     }
     __syncwarp();
-    return;
+    return true;
   }
   __syncwarp();
   TSTEP(1)
   // ---- run starts S_c = R_c & ~R_{c-1}, transposed to one column bitmap per row
-  const bool tr = L <= TK_LCN;
+  const bool tr = !WIDE || L <= lcn;
   if (tr) {
     const int nb = (L + 31) >> 5;
     for (int b = 0; b < nb; ++b) {
@@ -501,8 +559,8 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
           hi = (hi & m0) | ((thi & m0) << j);
         }
       }
-      s.srow[wid][lane][b] = lo;
-      s.srow[wid][32 + lane][b] = hi;
+      srow[lane * srw + b] = lo;
+      srow[(32 + lane) * srw + b] = hi;
     }
     __syncwarp();
   }
@@ -537,7 +595,13 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
   TSTEP(2)
 
   // ---- count pieces / opens / heads
+  // Packed counts: pieces and heads (at most 64 x 512 each) in 16 bits, opens, continuations and row-0 ends (at
+  // most 512 each) in 10 bits.  pf[c] becomes the counts before column c; it lies in the member cache (and the
+  // bitmap words behind it in the wide buffers), dead after the raster.
+  const bool packed = !WIDE || L <= 512;
+  unsigned long long* const pf = mc;
   int np = 0, no = 0, nh = 0, ncn = 0, nz = 0;
+  unsigned long long pv = 0;
   {
     unsigned long long Rm1 = R(c0 - 1), fb = ~0ull;
     for (int c = c0; c < c1e; ++c) {
@@ -549,37 +613,35 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
       const unsigned long long Z = (Chg | 2ull) & Ec & ~1ull;
       cb[c] = Z | ((Chg >> 1) & 1ull);  // bit 0 of Z is always clear
       const int pc = __popcll(Z);
-      np += pc;
-      if (!last_sb && (Ec >> 63)) ++no;
+      const int open = !last_sb && (Ec >> 63);
       const int cont = (sb > 0) && ((Z >> 1) & 1ull) && !((Chg >> 1) & 1ull);
-      nh += pc - cont;
-      ncn += cont;
-      nz += (int)(Ec & 1ull);
+      if (packed) {
+        pf[c] = pv;
+        pv += ((unsigned long long)(unsigned)((int)(Ec & 1ull) << 20 | cont << 10 | open) << 32) |
+              (unsigned)(pc | (pc - cont) << 16);
+      } else {
+        np += pc;
+        no += open;
+        nh += pc - cont;
+        ncn += cont;
+        nz += (int)(Ec & 1ull);
+      }
       Rm1 = Rc;
     }
   }
   int totP, totO, totH, totC, totZ;
   // runs at row 0 are the runs at row 63 of the previous sub-band, both in y
   // order: a continuation's ordinal among them indexes that sub-band's open list
-  int posZ, posP, posO, posH, posC;
-  // one 64-bit scan when the fields cannot overflow: pieces and heads (at most 64 x 512 each) in 16 bits,
-  // opens, continuations and row-0 ends (at most 512 each) in 10 bits
-  if (L <= 512) {
-    const unsigned long long v = (unsigned long long)np | ((unsigned long long)nh << 16) |
-                                 ((unsigned long long)no << 32) | ((unsigned long long)ncn << 42) |
-                                 ((unsigned long long)nz << 52);
+  int posZ = 0, posP = 0, posO = 0, posH = 0, posC = 0;
+  if (packed) {
     unsigned long long t;
-    const unsigned long long e = gb_warp_excl(v, &t);
-    posP = (int)(e & 0xffffu);
-    posH = (int)((e >> 16) & 0xffffu);
-    posO = (int)((e >> 32) & 0x3ffu);
-    posC = (int)((e >> 42) & 0x3ffu);
-    posZ = (int)((e >> 52) & 0x3ffu);
+    const unsigned long long e = gb_warp_excl(pv, &t);
+    for (int c = c0; c < c1e; ++c) pf[c] += e;
     totP = (int)(t & 0xffffu);
     totH = (int)((t >> 16) & 0xffffu);
     totO = (int)((t >> 32) & 0x3ffu);
     totC = (int)((t >> 42) & 0x3ffu);
-    totZ = (int)((t >> 52) & 0x3ffu);
+    __syncwarp();
   } else {
     posZ = gb_warp_excl(nz, &totZ);
     posP = gb_warp_excl(np, &totP);
@@ -605,7 +667,7 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
       if (!p) pbase = -1;
     }
     if (totO + totC > 0 && pbase >= 0) {
-      void* p = sc_up(s, base, half, (unsigned long long)(totO + totC) * 4);
+      void* p = sc_up(s, base, half, (unsigned long long)(totO + 2 * totC) * 4);
       obase = (unsigned long long)p;
       if (!p) pbase = -1;
     }
@@ -613,30 +675,45 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
   pbase = __shfl_sync(0xffffffffu, pbase, 0);
   obase = __shfl_sync(0xffffffffu, obase, 0);
   rbase = __shfl_sync(0xffffffffu, rbase, 0);
-  if (pbase < 0) return;
+  if (pbase < 0) return true;
   PieceRec* recs = (PieceRec*)rbase;
-  int* olist = (int*)obase;  // open pieces, then continuation pieces, each in y order
+  int* olist = (int*)obase;  // open pieces, then continuation pieces, each in y order, then the latter's ordinals
   TSTEP(3)
 
-  // ---- write pieces, dealt to the lanes 32 at a time in (column, row) order: piece k's lane is found by a
-  // shuffle search over the lanes' piece counts, its column by a walk over that lane's columns, its row as
-  // its rank among the column's piece starts
+  // ---- write pieces, dealt to the lanes 32 at a time in (column, row) order: piece k's column is found by a
+  // binary search over the columns' packed counts (of more than 512 columns: by a shuffle search over the lanes'
+  // piece counts and a walk over that lane's columns), its row is its rank among the column's piece starts
   {
     const int inclP = posP + np;
     for (int k0 = 0; k0 < totP; k0 += 32) {  // warp-uniform trip count
       const int k = k0 + lane;
-      int ow = 0;  // owner lane: the first lane whose inclusive piece prefix exceeds k
+      int j = 0, o = 0, h = 0, q = 0, z = 0, c = 0;
+      if (packed) {
+        const unsigned* p32 = reinterpret_cast<const unsigned*>(pf);
 #pragma unroll
-      for (int st2 = 16; st2 > 0; st2 >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, inclP, ow + st2 - 1);
-        if (v <= k) ow += st2;
+        for (int st2 = WIDE ? 256 : TK_LCN / 2; st2 > 0; st2 >>= 1)
+          if (c + st2 < L && (int)(p32[2 * (c + st2)] & 0xffffu) <= k) c += st2;
+        const unsigned long long e = pf[c];
+        j = k - (int)(e & 0xffffu);
+        h = (int)((e >> 16) & 0xffffu);
+        o = (int)((e >> 32) & 0x3ffu);
+        q = (int)((e >> 42) & 0x3ffu);
+        z = (int)((e >> 52) & 0x3ffu);
+      } else {
+        int ow = 0;  // owner lane: the first lane whose inclusive piece prefix exceeds k
+#pragma unroll
+        for (int st2 = 16; st2 > 0; st2 >>= 1) {
+          const int v = __shfl_sync(0xffffffffu, inclP, ow + st2 - 1);
+          if (v <= k) ow += st2;
+        }
+        j = k - __shfl_sync(0xffffffffu, posP, ow);
+        o = __shfl_sync(0xffffffffu, posO, ow);
+        h = __shfl_sync(0xffffffffu, posH, ow);
+        q = __shfl_sync(0xffffffffu, posC, ow);
+        z = __shfl_sync(0xffffffffu, posZ, ow);
+        c = min(L, ow * per);
       }
-      const int oP = __shfl_sync(0xffffffffu, posP, ow), oO = __shfl_sync(0xffffffffu, posO, ow);
-      const int oH = __shfl_sync(0xffffffffu, posH, ow), oC = __shfl_sync(0xffffffffu, posC, ow);
-      const int oZ = __shfl_sync(0xffffffffu, posZ, ow);
       if (k < totP) {
-        int j = k - oP, o = oO, h = oH, q = oC, z = oZ;
-        int c = min(L, ow * per);
         unsigned long long zs, Z, Ec;
         int contc;
         for (;;) {  // the owner's columns before the piece's own: their pieces, opens, continuations, row-0 ends
@@ -644,6 +721,7 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
           Z = zs & ~1ull;
           Ec = ca[c] & ~R(c + 1);
           contc = (sb > 0) && ((Z >> 1) & 1ull) && !(zs & 1ull);
+          if (packed) break;
           const int pc = __popcll(Z);
           if (j < pc) break;
           j -= pc;
@@ -662,8 +740,8 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
         int cs = c;
         if (tr) {
           int b = c >> 5;
-          unsigned mk = s.srow[wid][r][b] & (0xFFFFFFFFu >> (31 - (c & 31)));
-          while (!mk && b > 0) mk = s.srow[wid][r][--b];
+          unsigned mk = srow[r * srw + b] & (0xFFFFFFFFu >> (31 - (c & 31)));
+          while (!mk && b > 0) mk = srow[r * srw + --b];
           cs = (b << 5) + 31 - __clz(mk);
         } else {
           while (cs > 0) {
@@ -676,22 +754,25 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
         const int open = (rend == 64) && !last_sb;
         const int p = pbase + k;
         PieceRec pr;
-        const unsigned hr = cont ? (unsigned)z : (unsigned)h;  // continuations keep their row-0 ordinal
+        const unsigned hr = (unsigned)h;
         pr.x = lv[cs] | (cont << 30) | (open << 31);
         pr.y = lv[c + 1] | (int)((hr & 0x7fffu) << 17);
         pr.z = (rowbase + r) | (int)((hr >> 15) << 17);
         pr.w = rowbase + rend;
         recs[k] = pr;
         if (open) olist[o] = p;
-        if (cont) olist[totO + q] = p;
+        if (cont) {
+          olist[totO + q] = p;
+          olist[totO + totC + q] = z;
+        }
       }
     }
   }
   TSTEP(4)
-  if (tctr && lane == 0) {  // sub-bands whose column words spilled to scratch: count and cycles
+  if (tctr && lane == 0) {  // wide sub-bands: count and cycles
     const long long q1 = clock64();
-    atomicAdd((unsigned long long*)&tctr[28 + (L > TK_LCN ? 0 : 2)], 1ull);
-    atomicAdd((unsigned long long*)&tctr[29 + (L > TK_LCN ? 0 : 2)], (unsigned long long)(q1 - qstart));
+    atomicAdd((unsigned long long*)&tctr[28 + (WIDE ? 0 : 2)], 1ull);
+    atomicAdd((unsigned long long*)&tctr[29 + (WIDE ? 0 : 2)], (unsigned long long)(q1 - qstart));
   }
   if (lane == 0) {
     s.sbinfo[sb] = make_int4(pbase, totP, totO, 0);
@@ -700,7 +781,92 @@ __device__ void tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int n
     s.sbh[sb] = totH;
     s.sbct[sb] = totC;
   }
+  return true;
 #undef TSTEP
+}
+
+// Phase D's emission for a tile whose piece records stay in the scratch: TK_DU pieces per thread and step, so
+// that the loads of one (record, table values) overlap those of the others.  A strip's chain runs through as many
+// sub-bands as the strip spans, so its links are what bounds the step: on chip (16 bits, sl16) a hop takes an L1
+// latency and not L2's.  Out of line: its registers stay out of the kernel's main path.  Returns the area.
+__device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* recs, int NP, int nsb, const int* Xv,
+                                                    const int* Yv, unsigned long long* outp, bool sl16) {
+  const PieceRec* rg = reinterpret_cast<const PieceRec*>(recs);
+  const unsigned short* s16 = reinterpret_cast<const unsigned short*>(s.dbuf);
+  const int* s32 = s.succ;
+  auto rec = [&](int q) -> PieceRec {
+    if (!s.rsplit) return rg[q];
+    int sb = 0;  // some records lie elsewhere: the sub-band that holds piece q
+    for (; sb < nsb - 1; ++sb) {
+      const int4 inf = s.sbinfo[sb];
+      if (q >= inf.x && q < inf.x + inf.y) break;
+    }
+    return s.sbrec[sb][q - s.sbinfo[sb].x];
+  };
+  auto next = [&](int q) -> int {
+    if (!sl16) return s32[q];
+    const int v = s16[q];
+    return v == 0xffff ? -1 : v;
+  };
+  long long area = 0;
+  for (int p0 = threadIdx.x; p0 < NP; p0 += TK_DU * TK_NT) {
+    PieceRec r[TK_DU];
+    int nx[TK_DU];
+#pragma unroll
+    for (int u = 0; u < TK_DU; ++u) {
+      const int p = p0 + u * TK_NT;
+      r[u].x = 1 << 30;  // past the end: as a continuation, skipped
+      nx[u] = -1;
+      if (p < NP) {
+        r[u] = rec(p);
+        nx[u] = next(p);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < TK_DU; ++u) {
+      if (pr_cont(r[u])) continue;
+      int q = -1, guard = 0;
+      while (nx[u] >= 0 && guard++ <= nsb) {
+        q = nx[u];
+        nx[u] = next(q);
+      }
+      if (q >= 0) r[u].w = rec(q).w;
+    }
+#pragma unroll
+    for (int u = 0; u < TK_DU; ++u) {
+      if (pr_cont(r[u])) continue;
+      const int slo = pr_slo(r[u]);
+      const int xs = Xv[slo], xe = Xv[pr_shi(r[u])], ylo = Yv[pr_ylo(r[u])], yhi = Yv[pr_yhi(r[u])];
+      if (outp) outp[s.sbh[slo / 63] + pr_hrank(r[u])] = gb_pack(xs, ylo, xe, yhi);
+      area += (long long)(xe - xs) * (long long)(yhi - ylo);
+    }
+  }
+  return area;
+}
+
+// Levels 1..3 of phase C: the wide sub-bands that the level below listed, by fewer warps with larger buffers.
+// Called by the whole CTA after level 0.  Out of line: its registers stay out of the kernel's narrow path.
+template <bool TIMING>
+__device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int nA, char* base,
+                                       unsigned long long scr, long long* tctr) {
+  for (int level = 1; level <= TK_WLEVELS; ++level) {
+    __syncthreads();
+    const int todo = s.err ? 0 : s.nwide[level - 1];
+    if (todo == 0) break;  // uniform: neither changes before the next barrier
+    if (threadIdx.x == 0) s.sbnext = 0;
+    __syncthreads();
+    if (gb_warp() >= (TK_NW >> level)) continue;
+    for (;;) {
+      int k = 0;
+      if (gb_lane() == 0) k = atomicAdd(&s.sbnext, 1);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      if (k >= todo) break;
+      const int sb = TK_WLIST(s, level - 1)[k];
+      if (!tile_subband<TIMING, true>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && gb_lane() == 0)
+        TK_WLIST(s, level)[atomicAdd(&s.nwide[level], 1)] = sb;
+      __syncwarp();
+    }
+  }
 }
 
 template <bool TIMING>
@@ -722,6 +888,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s.have_nx = 0;
+    s.hint = 0;
   }
   for (;;) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before this tile's bulk copies
@@ -914,7 +1081,6 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       M = (int)carry;
     }
     if (tid == 0) {
-      const int nwy = ((Ny - 1) >> 5) + 1;
       s.mem = (int4*)sc_up(s, base, half, (unsigned long long)M * 16);
       if (nsb <= TK_MDS) {  // the value bitmaps are dead now: keep the metadata on chip
         char* q = reinterpret_cast<char*>(s.xyv);
@@ -930,8 +1096,6 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         s.sbol = (int**)sc_up(s, base, half, (unsigned long long)nsb * 8 + 8);
         s.sbrec = (PieceRec**)sc_up(s, base, half, (unsigned long long)nsb * 8 + 8);
       }
-      s.biglb = nwy > TK_LBW ? (unsigned*)sc_up(s, base, half, (unsigned long long)TK_NW * 2 * nwy * 4)
-                             : nullptr;
     }
     __syncthreads();
     if (!s.err) {
@@ -975,17 +1139,36 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         ord[r] = q;
       }
     }
-    if (tid == 0) s.sbnext = 0;
+    if (tid <= TK_WLEVELS) s.nwide[tid] = 0;
+    if (tid == 0) {
+      s.sbnext = 0;
+      s.narrow = 0;
+    }
     __syncthreads();
+    // level 0: every warp with its own buffer.  Wide sub-bands are listed for level 1; once three of four have
+    // been wide (or when the previous tile's were), the rest are listed without a try.
+    const bool direct = s.hint != 0;
     if (!s.err) {
       for (;;) {
         int k = 0;
-        if (gb_lane() == 0) k = atomicAdd(&s.sbnext, 1);
+        bool list = direct;
+        if (gb_lane() == 0) {
+          k = atomicAdd(&s.sbnext, 1);
+          const int w = *(volatile int*)&s.nwide[0];
+          list |= w >= TK_NW && w * 4 >= k * 3;
+        }
         k = __shfl_sync(0xffffffffu, k, 0);
         if (k >= nsb) break;
-        tile_subband<TIMING>(s, op, lpt ? ord[k] : k, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
+        const int sb = lpt ? ord[k] : k;
+        if (__any_sync(0xffffffffu, list) ||
+            !tile_subband<TIMING, false>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
+          if (gb_lane() == 0) TK_WLIST(s, 0)[atomicAdd(&s.nwide[0], 1)] = sb;
+        }
       }
     }
+    __syncthreads();
+    if (s.nwide[0]) tile_wide<TIMING>(s, op, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
+    if (tid == 0 && !s.err) s.hint = direct ? s.narrow * 4 <= nsb : s.nwide[0] * 4 >= nsb * 3;
     // the bulk copies of phase D (async proxy) read the records written above and overwrite shared
     // memory written in phases A-C (generic proxy)
     asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -1010,7 +1193,9 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     const int xyoff = nsb <= TK_MDS ? TK_MD_INTS : 0;  // metadata occupies the front of the region
     const int nx4 = (Nx + 3) & ~3, ny4 = (Ny + 3) & ~3;  // tables start on 16-byte boundaries
     const bool xys = nx4 + ny4 + xyoff <= 2 * TK_WMAX + 2 * (TK_WMAX / 2 + 1);
-    if (tid == 0 && !s.err && !prs) s.succ = (int*)sc_up(s, base, half, (unsigned long long)NP * 4 + 4);
+    // chain links of a tile whose records stay in the scratch: 16 bits each on chip when they fit
+    const bool sl16 = !prs && NP * 2 <= DBYTES;
+    if (tid == 0 && !s.err && !prs && !sl16) s.succ = (int*)sc_up(s, base, half, (unsigned long long)NP * 4 + 4);
     __syncthreads();
     if (s.err) {
       if (tid == 0) {
@@ -1030,8 +1215,6 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     int* succ = prs ? reinterpret_cast<int*>(s.dbuf + (size_t)NP * 16) : s.succ;
     const int* Xv = xys ? s.xyv + xyoff : s.Xt;
     const int* Yv = xys ? s.xyv + xyoff + nx4 : s.Yt;
-    // record of global piece q, which belongs to sub-band sb
-    auto REC = [&](int sb, int q) -> PieceRec { return prs ? PR[q] : s.sbrec[sb][q - s.sbinfo[sb].x]; };
     const int wid = gb_warp(), lane = gb_lane();
     // piece records of every sub-band and the x / y value tables into shared memory by bulk copies
     // (all 16-byte aligned: records are 16 bytes, scratch allocations are rounded to 16 bytes)
@@ -1062,7 +1245,11 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         return;
       }
     }
-    for (int p = tid; p < NP; p += TK_NT) succ[p] = -1;
+    unsigned short* const succ16 = reinterpret_cast<unsigned short*>(s.dbuf);
+    if (sl16)
+      for (int p = tid; p < NP; p += TK_NT) succ16[p] = 0xffffu;
+    else
+      for (int p = tid; p < NP; p += TK_NT) succ[p] = -1;
     int H = 0;
     {
       long long carry = 0;
@@ -1100,10 +1287,11 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       const int4 pinf = s.sbinfo[sb - 1];
       const int* ol = s.sbol[sb - 1];
       for (int k = lane; k < nc; k += 32) {
-        const int p = cl[k];
-        const int ord = pr_hrank(REC(sb, p));
-        if (ord < pinf.z) succ[ol[ord]] = p;
-        else gb_set_error(st, GB_ERR_INTERNAL, KID_TILE, t);
+        const int p = cl[k], ord = cl[nc + k];
+        if (ord < pinf.z) {
+          if (sl16) succ16[ol[ord]] = (unsigned short)p;
+          else succ[ol[ord]] = p;
+        } else gb_set_error(st, GB_ERR_INTERNAL, KID_TILE, t);
       }
     }
     __syncthreads();
@@ -1126,22 +1314,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         area += (long long)(xe - xs) * (long long)(yhi - ylo);
       }
     } else {
-      for (int sb = wid; sb < nsb; sb += TK_NW) {
-        const int4 inf = s.sbinfo[sb];
-        for (int j = lane; j < inf.y; j += 32) {
-          const int p = inf.x + j;
-          const PieceRec pr = REC(sb, p);
-          if (pr_cont(pr)) continue;
-          int q = p, sq = sb, guard = 0;
-          while (succ[q] >= 0 && guard++ <= nsb) { q = succ[q]; ++sq; }
-          const int shi = q == p ? pr_shi(pr) : pr_shi(REC(sq, q));
-          const int slo = pr_slo(pr);
-          const int xs = Xv[slo], xe = Xv[shi], ylo = Yv[pr_ylo(pr)], yhi = Yv[pr_yhi(pr)];
-          const int pos = s.sbh[sb] + pr_hrank(pr);
-          if (outp) outp[pos] = gb_pack(xs, ylo, xe, yhi);
-          area += (long long)(xe - xs) * (long long)(yhi - ylo);
-        }
-      }
+      area = tile_emit_scratch(s, base + (half & ~15ull), NP, nsb, Xv, Yv, outp, sl16);
     }
     area = gb_block_sum(area, s.tmp64);
     if (tid == 0) {
