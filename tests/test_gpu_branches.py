@@ -77,3 +77,31 @@ def test_many_y_ranks(ctx, oracle, n):
     B = random_layer(500, die=65_000, wmin=20, wmax=3000, seed=n)
     for op in (0, 3):
         assert np.array_equal(run(ctx, lambda: ctx.op(op, ctx.layer(A), ctx.layer(B))), oracle.boolean(A, B, op)), op
+
+
+def _snap_cases():
+    rng = np.random.default_rng(5)
+    out = {}
+    for n in (1, 1023, 1024, 1025, 2049, 65535, 65536, 65537, 70001):
+        out["random %d" % n] = random_layer(n, die=300_000, seed=n, x0=-150_000, y0=-150_000)
+    i = np.arange(70_000)
+    # one-byte records; records whose bytes also parse out of step (20 a0 20 ...)
+    out["equal boxes"] = np.tile(np.array([[5, 6, 15, 16]], np.int32), (70_000, 1))
+    out["out of step"] = np.stack([2064 * i, 0 * i, 2064 * i + 10, 0 * i + 10], 1).astype(np.int32)
+    x = rng.integers(-2**31, 2**31 - 1, (5000, 4), dtype=np.int64)  # longest records
+    out["long records"] = np.stack([np.minimum(x[:, 0], x[:, 2]), np.minimum(x[:, 1], x[:, 3]),
+                                    np.maximum(x[:, 0], x[:, 2]) + 1, np.maximum(x[:, 1], x[:, 3]) + 1], 1).astype(np.int32)
+    sq = random_layer(70_000, die=300_000, seed=3)  # squares with a rare other box: far back to the last height
+    sq[:, 2:] = sq[:, :2] + (sq[:, 2:3] - sq[:, 0:1])
+    sq[[0, 30_000, 64_000], 3] += 3
+    out["squares"] = sq
+    return out
+
+
+@pytest.mark.parametrize("case", list(_snap_cases()))
+@pytest.mark.parametrize("method", [0, 1])
+def test_snap_sizes(ctx, oracle, case, method):
+    b = _snap_cases()[case]
+    chunks = ctx.compress_boxes_to_stream(b, method)
+    assert [c[3] for c in chunks] == [c[3] for c in oracle.stream_encode(b, method)]
+    assert np.array_equal(ctx.decompress_stream_to_boxes(chunks, method), b)

@@ -27,12 +27,15 @@
 // chunk's length preamble.  Decoding takes one warp per chunk through the
 // elements (all element forms of the format are accepted), with the last
 // 32 KB of output in a shared-memory ring for the copies.
-// Decoding the codec: one CTA per chunk finds the record boundaries (seven
-// warps compute, per 4 KB window, the lengths of the next four records from
-// every byte; one thread walks the chain four records per load, overlapped
-// with the next window's computation), then one CTA per chunk parses the
-// records 1024 at a time, rebuilds the anchors and dictionary indices with
-// block scans and gathers widths and heights from per-chunk dictionaries.
+// Decoding the codec.  Record boundaries: a record's length follows from its
+// bytes, so a chain started anywhere falls in with the true one after a few
+// records.  Every 256-byte segment guesses its first record by a chain from
+// 128 bytes before it and walks to its end; one CTA per chunk then redoes the
+// segments whose guess is not where the segment before them ended, until all
+// agree, and the record counts give every segment its first record's number.
+// Boxes: blocks of 1024 records sum their anchor deltas and dictionary
+// entries, then every block adds up the blocks before it and rebuilds its
+// boxes, with the dictionary entries looked up by block.
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -45,7 +48,6 @@
 #define SN_FCAP (SN_FRAG + SN_FRAG / 6 + 64)
 #define SN_T 1024       // threads of the per-chunk CTAs
 #define SN_REC_MAX 31   // longest record of a valid box (1 + 5 + 5 + 10 + 10)
-#define SN_WPAD 64      // look-ahead behind the window
 #define SN_MIN_MATCH 8  // shortest copy the compressor emits
 #define SN_CODEC_VERSION 1
 #define SN_LAYER_STATE_PNUM 4
@@ -401,250 +403,439 @@ k_enc_emit(const int4* __restrict__ boxes, long long n, const unsigned* __restri
 }
 
 // ---------------------------------------------------------------- codec decoder
-// One 256-thread CTA per chunk: rec[c * SN_CHUNK + r] = offset of record r in
-// the chunk.  The chunk is taken in 4 KB windows.  For a window, warps 1..7
-// load its bytes (and the look-ahead), mark the varint continuation bits
-// with ballots, compute at every byte the length a record starting there
-// would have (each varint's length is one find-first-zero in the continuation
-// bits) and then, per byte, the lengths of the four records of the chain
-// starting there (one word).  Meanwhile lane 0 of warp 0 walks the previous
-// window's chain four records per shared-memory load.
-#define SN_BT 256
-#define SN_BWIN 4096
-#define SN_BPAD 256  // lengths are needed up to three records (3 * 41 bytes) past the window
-#define SN_BBUF (SN_BWIN + SN_BPAD + 64)
-__device__ __forceinline__ int sn_vl(const unsigned* cont, int q) {  // varint length at q (0: longer than 10)
-  const unsigned long long w = ((unsigned long long)cont[(q >> 5) + 1] << 32) | cont[q >> 5];
-  const int k = __ffsll(~(w >> (q & 31)));  // first byte without the continuation bit, 1-based
-  return k <= 10 ? k : 0;
-}
+// Record boundaries by guessed segments (see the top).  The walk of a chunk
+// is a serial chain of 65536 lengths (one CTA per chunk with one walking
+// thread: 1774 us for 184 chunks); segments make it 2100 chains of about 30
+// records per chunk, and the guesses cost 14 more each.  A block stages 128
+// segments (32 KB) with the continuation bits of their bytes, so a length is
+// one byte and three words from shared memory and then register work.
+#define SN_SEG 256
+#define SN_WARM 128       // a guess starts this many bytes before its segment
+#define SN_SEGT 128       // segments (threads) per block
+#define SN_SEGB (SN_SEG * SN_SEGT)
+#define SN_LOOK 64        // bytes staged past the block (more than a record's length)
+#define SN_STG (SN_WARM + SN_SEGB + SN_LOOK)
+#define SN_LMAX 41           // longest record the decoder accepts (1 + 4 x 10)
+#define SN_DEAD 0xffffffffu  // no chain reaches the segment (a malformed record lies before)
 
-// Branch-free: every field's varint length is looked up and selected by the
-// infobyte's bits, so the lanes of a warp (at different bytes) do not diverge.
-__device__ __forceinline__ int sn_rec_len_bits(const unsigned char* buf, const unsigned* cont, int b) {
-  const unsigned info = buf[b];
+// Length of the record whose infobyte is `info`, from the continuation bits
+// of the bytes behind it; 0 when a varint is longer than 10 bytes.
+__device__ __forceinline__ int sn_len(unsigned info, unsigned long long cont) {
   int l = 1;
   bool bad = false;
-  int k = sn_vl(cont, b + l);
-  bad |= (info & 32) && !k;
-  l += (info & 32) ? k : 0;
-  k = sn_vl(cont, b + l);
-  bad |= (info & 64) && !k;
-  l += (info & 64) ? k : 0;
-  k = sn_vl(cont, b + l);
-  bad |= (info & 3) == 3 && !k;
-  l += (info & 1) ? ((info & 2) ? k : 2) : 0;
-  k = sn_vl(cont, b + l);
+  auto varint = [&](bool on) {
+    const int k = __ffsll((long long)~cont);
+    const bool ok = k >= 1 && k <= 10;
+    bad |= on && !ok;
+    const int u = on && ok ? k : 0;
+    cont >>= u;
+    l += u;
+  };
+  varint(info & 32);
+  varint(info & 64);
+  varint((info & 3) == 3);
+  if ((info & 3) == 1) {
+    cont >>= 2;
+    l += 2;
+  }
   const bool hf = (info & 20) == 4;
-  bad |= hf && (info & 8) && !k;
-  l += hf ? ((info & 8) ? k : 2) : 0;
+  varint(hf && (info & 8));
+  if (hf && !(info & 8)) l += 2;
   return bad ? 0 : l;
 }
 
-__global__ void __launch_bounds__(SN_BT)
-k_codec_bounds(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
-               const long long* __restrict__ raw_len, long long n, long long nchunks, unsigned* __restrict__ rec,
-               DStatus* st) {
-  __shared__ unsigned char buf[SN_BBUF];
-  __shared__ unsigned cont[SN_BBUF / 32 + 2];
-  __shared__ unsigned char lenb[SN_BWIN + SN_BPAD];
-  __shared__ unsigned quad[2][SN_BWIN];
-  __shared__ int s_pos, s_r, s_bad, s_skip;  // s_pos: offset into the next window
-  const int t = threadIdx.x, wid = t >> 5;
-  const long long c = blockIdx.x;
-  if (t == 0) {
-    s_skip = *(volatile int*)&st->err;  // the Snappy layer was malformed: one read for the whole CTA
-    s_pos = 0;
-    s_r = 0;
-    s_bad = 0;
+struct SegStage {  // a block's bytes; byte pos of the chunk is at buf[pos - pos0]
+  __align__(16) unsigned char buf[SN_STG + 32];
+  unsigned cont[SN_STG / 32 + 4];
+};
+
+// Bytes [first, first + SN_STG) of the chunk (zeros outside [0, L)) and their
+// continuation bits.  Returns the chunk position of buf[0].
+__device__ __forceinline__ long long seg_stage(SegStage& s, const unsigned char* base, long long L, long long first) {
+  // 16-byte groups of the source, so buf[0] lies up to 15 bytes before `first`
+  const int sh = (int)((uintptr_t)(base + first) & 15);
+  const long long p0 = first - sh;
+  for (int i = threadIdx.x * 16; i < SN_STG + 32; i += SN_SEGT * 16) {
+    const long long p = p0 + i;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (p >= 0 && p + 16 <= L) {
+      v = *reinterpret_cast<const uint4*>(base + p);
+    } else if (p + 16 > 0 && p < L) {
+      unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (p + j >= 0 && p + j < L) w[j >> 2] |= (unsigned)base[p + j] << (8 * (j & 3));
+      v = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    *reinterpret_cast<uint4*>(s.buf + i) = v;
   }
   __syncthreads();
-  if (s_skip) return;
-  const int nb = (int)min((long long)SN_CHUNK, n - c * SN_CHUNK);
-  const long long L = raw_len[c];
-  const unsigned char* base = raw + raw_off[c];
-  unsigned* out = rec + c * SN_CHUNK;
-  auto sync = [&](int bar, int nt) {
-    if (bar)
-      asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory");
-    else
-      __syncthreads();
-  };
-  // quads of window w into quad[w & 1]; run by threads [t0, t0 + nt) (whole warps), barrier id bar
-  auto build = [&](long long w, int t0, int nt, int bar) {
-    const long long ws = w * SN_BWIN;
-    const int u = t - t0;
-#pragma unroll 8
-    for (int b = u; b < SN_BBUF; b += nt) buf[b] = ws + b < L ? base[ws + b] : 0;  // independent loads in flight
-    sync(bar, nt);
-    for (int b = u; b < SN_BBUF; b += nt) {
-      const unsigned m = __ballot_sync(0xffffffffu, buf[b] & 128u);
-      if ((b & 31) == 0) cont[b >> 5] = m;
+  for (int w = threadIdx.x; w < SN_STG / 32 + 4; w += SN_SEGT) {
+    unsigned m = 0;
+    if (w < SN_STG / 32 + 1) {
+      const unsigned* q = reinterpret_cast<const unsigned*>(s.buf) + w * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m |= ((((q[j] >> 7) & 0x01010101u) * 0x10204080u) >> 28) << (4 * j);  // 4 top bits
     }
-    if (u < 2) cont[SN_BBUF / 32 + u] = 0xffffffffu;  // past the buffer: a varint there is too long
-    sync(bar, nt);
-    for (int b = u; b < SN_BWIN + SN_BPAD; b += nt) lenb[b] = (unsigned char)sn_rec_len_bits(buf, cont, b);
-    sync(bar, nt);
-    unsigned* qd = quad[w & 1];
-    for (int b = u; b < SN_BWIN; b += nt) {
-      const unsigned l0 = lenb[b];
-      const unsigned l1 = l0 ? lenb[b + l0] : 0u;
-      const unsigned l2 = l1 ? lenb[b + l0 + l1] : 0u;
-      const unsigned l3 = l2 ? lenb[b + l0 + l1 + l2] : 0u;
-      qd[b] = l0 | (l1 << 8) | (l2 << 16) | (l3 << 24);
-    }
-  };
-  const long long nwin = (L + SN_BWIN - 1) / SN_BWIN;
-  if (nwin > 0) build(0, 0, SN_BT, 0);
-  __syncthreads();
-  for (long long w = 0;; ++w) {
-    // every thread reads the walk's state before the barrier; lane 0 of warp 0 changes it only after
-    const int done = (s_r >= nb || s_bad) ? 1 : (w >= nwin ? 2 : 0);
-    __syncthreads();
-    if (done) {
-      if (done == 2 && t == 0) s_bad = 1;  // the stream ends before the chunk's last record
-      break;
-    }
-    if (t == 0) {
-      const unsigned ws = (unsigned)(w * SN_BWIN);
-      const unsigned* qd = quad[w & 1];
-      const int lim = (int)min((long long)SN_BWIN, L - (long long)ws);  // starts inside window and stream
-      int pos = s_pos, r = s_r, bad = 0;
-      while (r < nb && pos < SN_BWIN) {
-        const unsigned q = qd[pos];
-        const int l0 = q & 255u, l1 = (q >> 8) & 255u, l2 = (q >> 16) & 255u, l3 = q >> 24;
-        const int p1 = pos + l0, p2 = p1 + l1, p3 = p2 + l2;
-        if (l3 && p3 < lim && r + 4 <= nb) {  // four whole records (l3 != 0 implies l0..l2 != 0)
-          out[r] = ws + pos;
-          out[r + 1] = ws + p1;
-          out[r + 2] = ws + p2;
-          out[r + 3] = ws + p3;
-          r += 4;
-          pos = p3 + l3;
-          continue;
-        }
-        if (pos >= lim || !l0) {  // the stream ends early, or a malformed record
-          bad = 1;
-          break;
-        }
-        out[r++] = ws + pos;
-        pos = p1;
-      }
-      if (!bad && r >= nb && (long long)ws + pos > L) bad = 1;  // the last record runs past the stream
-      s_pos = pos - SN_BWIN;
-      s_r = r;
-      s_bad = bad;
-    } else if (wid > 0 && w + 1 < nwin) {
-      build(w + 1, 32, SN_BT - 32, 1);
-    }
-    __syncthreads();
+    s.cont[w] = m;
   }
-  if (t == 0 && s_bad) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAP_BOUNDS, c);
+  __syncthreads();
+  return p0;
 }
 
-// One CTA per chunk: records -> boxes.  dict: per chunk 2 * SN_CHUNK ints.
-__global__ void __launch_bounds__(SN_T, 1)
-k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
-               const unsigned* __restrict__ rec, long long n, int* dict, int4* __restrict__ out, DStatus* st) {
-  __shared__ Sum4 bufA[2][32];
-  __shared__ Last2 bufB[2][32];
-  __shared__ int s_skip;
-  const long long c = blockIdx.x;
-  const int t = threadIdx.x;
-  if (t == 0) s_skip = *(volatile int*)&st->err;  // the boundaries (or the Snappy layer) were malformed
+__device__ __forceinline__ int seg_len(const SegStage& s, int b) {
+  const int w = (b + 1) >> 5, sh = (b + 1) & 31;
+  const unsigned c0 = s.cont[w], c1 = s.cont[w + 1], c2 = s.cont[w + 2];
+  const unsigned long long cont =
+      ((unsigned long long)__funnelshift_r(c1, c2, sh) << 32) | __funnelshift_r(c0, c1, sh);
+  return sn_len(s.buf[b], cont);
+}
+
+// The chunk of a block: blk[c] is the first block of chunk c.
+__device__ __forceinline__ int seg_chunk(const long long* blk, int nchunks) {
+  return gb_find_cell(blk, nchunks, blockIdx.x);
+}
+
+__global__ void __launch_bounds__(SN_SEGT)
+k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
+            const long long* __restrict__ raw_len, const long long* __restrict__ blk, int nchunks,
+            unsigned* __restrict__ entry, unsigned* __restrict__ exit_, unsigned* __restrict__ cnt) {
+  __shared__ SegStage s;
+  const int c = seg_chunk(blk, nchunks);
+  const long long L = raw_len[c];
+  const long long start = (blockIdx.x - blk[c]) * SN_SEGB;
+  const long long p0 = seg_stage(s, raw + raw_off[c], L, start - SN_WARM);
+  const int s0 = (int)(start - p0) + (int)threadIdx.x * SN_SEG, s1 = s0 + SN_SEG;
+  const int lim = (int)min((long long)s1, L - p0);
+  int b = s0;
+  if (start + threadIdx.x > 0) {
+    b = s0 - SN_WARM;
+    while (b < s0) b += max(1, seg_len(s, b));
+  }
+  const size_t g = (size_t)blockIdx.x * SN_SEGT + threadIdx.x;
+  entry[g] = (unsigned)(p0 + b);
+  unsigned n = 0;
+  bool bad = false;
+  while (b < lim) {
+    const int l = seg_len(s, b);
+    if (!l) {
+      bad = true;
+      break;
+    }
+    b += l;
+    ++n;
+  }
+  exit_[g] = bad ? SN_DEAD : (unsigned)(p0 + b);
+  cnt[g] = n;
+}
+
+// One CTA per chunk: segments whose guess does not follow from the segment
+// before them are walked again until all agree (segment k is right after at
+// most k rounds, so the loop ends), then cnt becomes the number of the
+// segment's first record.  The chunk is malformed when the chain holds fewer
+// records than it has boxes.
+__global__ void __launch_bounds__(SN_T)
+k_seg_settle(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
+             const long long* __restrict__ raw_len, const long long* __restrict__ blk, long long n, unsigned* entry,
+             unsigned* exit_, unsigned* cnt, DStatus* st) {
+  __shared__ SumS buf[2][32];
+  const int c = blockIdx.x;
+  const int nb = (int)min((long long)SN_CHUNK, n - (long long)c * SN_CHUNK);
+  const long long L = raw_len[c];
+  const unsigned char* base = raw + raw_off[c];
+  // segments that start inside the stream (records lie in its first SN_CHUNK * SN_LMAX bytes)
+  const int nseg = (int)((min(L, (long long)SN_CHUNK * SN_LMAX) + SN_SEG - 1) / SN_SEG);
+  entry += blk[c] * SN_SEGT;
+  exit_ += blk[c] * SN_SEGT;
+  cnt += blk[c] * SN_SEGT;
+  for (int round = 0; round <= nseg; ++round) {
+    int changed = 0;
+    for (int k = threadIdx.x; k < nseg; k += SN_T) {
+      const unsigned e = k ? *(volatile unsigned*)&exit_[k - 1] : 0u;
+      if (entry[k] == e) continue;
+      changed = 1;
+      entry[k] = e;
+      unsigned m = 0, x = e;
+      if (e != SN_DEAD) {
+        long long p = e;
+        const long long lim = min(L, (long long)(k + 1) * SN_SEG);
+        while (p < lim) {
+          unsigned long long cont = 0;
+          for (int j = 0; j < SN_LMAX; ++j) {  // as many continuation bits as a record can use
+            const long long q = p + 1 + j;
+            if (q < L) cont |= (unsigned long long)(base[q] >> 7) << j;
+          }
+          const int l = sn_len(base[p], cont);
+          if (!l) break;
+          p += l;
+          ++m;
+        }
+        x = p < lim ? SN_DEAD : (unsigned)p;
+      }
+      cnt[k] = m;
+      *(volatile unsigned*)&exit_[k] = x;
+    }
+    if (!__syncthreads_or(changed)) break;
+  }
+  unsigned carry = 0;
+  for (int k0 = 0, it = 0; k0 < nseg; k0 += SN_T, ++it) {
+    const int k = k0 + (int)threadIdx.x;
+    SumS tot;
+    const SumS ex = block_excl(SumS{k < nseg ? cnt[k] : 0u}, SumS{0}, buf[it & 1], &tot);
+    if (k < nseg) cnt[k] = carry + ex.a;
+    carry += tot.a;
+  }
+  if (threadIdx.x == 0 && carry < (unsigned)nb) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAP_BOUNDS, c);
+}
+
+// rec[c * SN_CHUNK + r] = offset of record r in the chunk: every segment marks
+// its records' bytes, the block writes the marked offsets in order.
+__global__ void __launch_bounds__(SN_SEGT)
+k_seg_records(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
+              const long long* __restrict__ raw_len, const long long* __restrict__ blk, int nchunks, long long n,
+              const unsigned* __restrict__ entry, const unsigned* __restrict__ first, unsigned* __restrict__ rec,
+              DStatus* st) {
+  __shared__ SegStage s;
+  __shared__ unsigned mark[SN_SEGB / 32];
+  __shared__ SumS buf[32];
+  const int c = seg_chunk(blk, nchunks);
+  const int nb = (int)min((long long)SN_CHUNK, n - (long long)c * SN_CHUNK);
+  const long long L = raw_len[c];
+  const long long start = (blockIdx.x - blk[c]) * SN_SEGB;
+  const size_t g0 = (size_t)blockIdx.x * SN_SEGT, g = g0 + threadIdx.x;
+  if (first[g0] >= (unsigned)nb) return;  // uniform: the chunk's records end before this block
+  for (int i = threadIdx.x; i < SN_SEGB / 32; i += SN_SEGT) mark[i] = 0;
+  const long long p0 = seg_stage(s, raw + raw_off[c], L, start - SN_WARM);
+  const int o = (int)(start - p0);  // buf index of the block's first byte
+  const unsigned e = entry[g];
+  if (e != SN_DEAD) {
+    int b = (int)((long long)e - p0);
+    const int lim = (int)min((long long)(o + ((int)threadIdx.x + 1) * SN_SEG), L - p0);
+    unsigned r = first[g];
+    while (b < lim && r < (unsigned)nb) {
+      const int l = seg_len(s, b);
+      if (!l) break;
+      atomicOr(&mark[(b - o) >> 5], 1u << ((b - o) & 31));
+      b += l;
+      if (++r == (unsigned)nb && p0 + b > L) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAP_BOUNDS, c);  // past the stream
+    }
+  }
   __syncthreads();
-  if (s_skip) return;
+  // words of mark in order: SN_SEGB / 32 / SN_SEGT per thread
+  constexpr int WPT = SN_SEGB / 32 / SN_SEGT;
+  unsigned m = 0;
+#pragma unroll
+  for (int j = 0; j < WPT; ++j) m += __popc(mark[threadIdx.x * WPT + j]);
+  SumS tot;
+  const SumS ex = block_excl(SumS{m}, SumS{0}, buf, &tot);
+  unsigned* out = rec + (long long)c * SN_CHUNK + first[g0] + ex.a;
+#pragma unroll
+  for (int j = 0; j < WPT; ++j) {
+    const int w = threadIdx.x * WPT + j;
+    for (unsigned v = mark[w]; v; v &= v - 1) *out++ = (unsigned)(start + w * 32 + __ffs(v) - 1);
+  }
+}
+
+// Records to boxes, SN_RB records per block, four consecutive ones per thread.
+// Pass 0 leaves the block's sums (anchor deltas, dictionary entries, last
+// width and height set) and its dictionary entries, in the block's own part of
+// the dictionary; pass 1 adds up the blocks of the chunk before it and writes
+// the boxes.  The chunk's 64 steps in one CTA, each behind the scans of the
+// one before, took 459 us for 184 chunks.
+#define SN_RB 1024
+#define SN_RT 256
+#define SN_REL (1 << 30)  // a "last set" code: the block's own entry, 1-based; else SN_ABS | index, 0 = none
+#define SN_ABS (1 << 29)
+struct RecBlock {
+  unsigned dx, dy, nw, nh;
+  int lw, lh, pad0, pad1;
+};
+
+struct RecFields {
+  unsigned info;
+  int dx, dy, wv, hv;
+  __device__ __forceinline__ int wsel() const { return (info & 1) ? ((info & 2) ? 1 : 2) : 0; }
+  __device__ __forceinline__ int hsel() const { return (info & 20) == 4 ? ((info & 8) ? 1 : 2) : 0; }
+};
+
+__device__ __forceinline__ RecFields rec_parse(const unsigned char* p) {
+  RecFields f{p[0], 0, 0, 0, 0};
+  int i = 1, k;
+  if (f.info & 32) {
+    f.dx = sn_unzigzag(sn_get_varint(p + i, &k));
+    i += k;
+  }
+  if (f.info & 64) {
+    f.dy = sn_unzigzag(sn_get_varint(p + i, &k));
+    i += k;
+  }
+  if (f.info & 1) {
+    if (f.info & 2) {
+      f.wv = (int)(unsigned)sn_get_varint(p + i, &k);
+      i += k;
+    } else {
+      f.wv = (short)(unsigned short)(p[i] | (p[i + 1] << 8));
+      i += 2;
+    }
+  }
+  if ((f.info & 20) == 4) {
+    if (f.info & 8)
+      f.hv = (int)(unsigned)sn_get_varint(p + i, &k);
+    else
+      f.hv = (short)(unsigned short)(p[i] | (p[i + 1] << 8));
+  }
+  return f;
+}
+
+template <bool WRITE>
+__global__ void __launch_bounds__(SN_RT)
+k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
+               const unsigned* __restrict__ rec, long long n, int* dict, RecBlock* blocks, int4* __restrict__ out,
+               DStatus* st) {
+  __shared__ Sum4 bufA[32];
+  __shared__ Last2 bufB[32];
+  __shared__ unsigned pnw[64], pnh[64];  // entries of the chunk's blocks before block j
+  __shared__ RecBlock pre;               // sums of the blocks before this one, last codes made absolute
+  __shared__ int s_skip;
+  constexpr int BPC = SN_CHUNK / SN_RB;  // 64
+  const long long c = blockIdx.x / BPC;
+  const int kb = blockIdx.x % BPC, t = threadIdx.x;
   const long long b0 = c * SN_CHUNK;
   const int nb = (int)min((long long)SN_CHUNK, n - b0);
+  const int j0 = kb * SN_RB;
+  if (j0 >= nb) return;
+  if (t == 0) s_skip = *(volatile int*)&st->err;  // the boundaries (or the Snappy layer) were malformed
+  if (WRITE && t < 32) {
+    unsigned dx = 0, dy = 0, nw = 0, nh = 0;
+    int lw = 0, lh = 0;
+    for (int h = 0; h < 2; ++h) {  // blocks 0..31, then 32..63
+      const int j = h * 32 + t;
+      RecBlock q{0, 0, 0, 0, 0, 0, 0, 0};
+      if (j < kb) q = blocks[c * BPC + j];
+      SumS e[4] = {{q.dx}, {q.dy}, {q.nw}, {q.nh}};
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const SumS o = shup(e[x], d);
+          if (t >= d) e[x].a += o.a;
+        }
+      pnw[j] = nw + e[2].a - q.nw;
+      pnh[j] = nh + e[3].a - q.nh;
+      const unsigned mw = __ballot_sync(0xffffffffu, q.lw != 0), mh = __ballot_sync(0xffffffffu, q.lh != 0);
+      // the last block that sets a width (height), its own entries counted from the blocks before it
+      const int aw = q.lw & SN_REL ? (int)pnw[j] + (q.lw & ~SN_REL) : (short)(q.lw & 0xffff);
+      const int ah = q.lh & SN_REL ? (int)pnh[j] + (q.lh & ~SN_REL) : (short)(q.lh & 0xffff);
+      const int sw = __shfl_sync(0xffffffffu, aw, mw ? 31 - __clz(mw) : 0);
+      const int sh = __shfl_sync(0xffffffffu, ah, mh ? 31 - __clz(mh) : 0);
+      if (mw) lw = sw;
+      if (mh) lh = sh;
+      dx += __shfl_sync(0xffffffffu, e[0].a, 31);
+      dy += __shfl_sync(0xffffffffu, e[1].a, 31);
+      nw += __shfl_sync(0xffffffffu, e[2].a, 31);
+      nh += __shfl_sync(0xffffffffu, e[3].a, 31);
+    }
+    if (t == 0) pre = RecBlock{dx, dy, nw, nh, lw, lh, 0, 0};
+  }
+  __syncthreads();
+  if (s_skip) return;
   const unsigned char* base = raw + raw_off[c];
-  int* dw = dict + c * 2 * SN_CHUNK;
-  int* dh = dw + SN_CHUNK;
-  Sum4 cA{0, 0, 0, 0};
-  Last2 cB{0, 0};
-  for (int k = 0; k * SN_T < nb; ++k) {
-    const int j = k * SN_T + t;
-    const bool valid = j < nb;
-    unsigned info = 0;
-    int dx = 0, dy = 0, wv = 0, hv = 0, wsel = 0, hsel = 0, bad = 0;
-    if (valid) {
-      const unsigned char* p = base + rec[b0 + j];
-      info = p[0];
-      int i = 1, kk;
-      if (info & 32) {
-        dx = sn_unzigzag(sn_get_varint(p + i, &kk));
-        i += kk;
-      }
-      if (info & 64) {
-        dy = sn_unzigzag(sn_get_varint(p + i, &kk));
-        i += kk;
-      }
-      if (info & 1) {
-        if (info & 2) {
-          wv = (int)(unsigned)sn_get_varint(p + i, &kk);
-          i += kk;
-          wsel = 1;
-        } else {
-          wv = (short)(unsigned short)(p[i] | (p[i + 1] << 8));
-          i += 2;
-          wsel = 2;
-        }
-      }
-      if (!(info & 16) && (info & 4)) {
-        if (info & 8) {
-          hv = (int)(unsigned)sn_get_varint(p + i, &kk);
-          i += kk;
-          hsel = 1;
-        } else {
-          hv = (short)(unsigned short)(p[i] | (p[i + 1] << 8));
-          i += 2;
-          hsel = 2;
-        }
-      }
+  int* const dw = dict + c * 2 * SN_CHUNK;
+  int* const dh = dw + SN_CHUNK;
+  RecFields f[4];
+  Sum4 sum{0, 0, 0, 0};
+  {
+    unsigned at[4];
+    const int j = j0 + 4 * t;
+    if (j + 4 <= nb) {
+      const uint4 q = *reinterpret_cast<const uint4*>(rec + b0 + j);
+      at[0] = q.x;
+      at[1] = q.y;
+      at[2] = q.z;
+      at[3] = q.w;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) at[u] = j + u < nb ? rec[b0 + j + u] : 0;
     }
-    Sum4 tA;
-    Sum4 ea = block_excl(Sum4{(unsigned)dx, (unsigned)dy, wsel == 1 ? 1u : 0u, hsel == 1 ? 1u : 0u},
-                         Sum4{0, 0, 0, 0}, bufA[k & 1], &tA);
-    ea = op(cA, ea);
-    int wself = 0, hself = 0;
-    if (wsel == 1) {
-      wself = (int)ea.nw + 1;
-      dw[wself - 1] = wv;
-    } else if (wsel == 2) {
-      if (wv < 1 || wv > (int)ea.nw) bad = 1;
-      wself = bad ? 0 : wv;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      f[u] = RecFields{0, 0, 0, 0, 0};
+      if (j + u < nb) f[u] = rec_parse(base + at[u]);
+      sum = op(sum, Sum4{(unsigned)f[u].dx, (unsigned)f[u].dy, f[u].wsel() == 1 ? 1u : 0u, f[u].hsel() == 1 ? 1u : 0u});
     }
-    if (hsel == 1) {
-      hself = (int)ea.nh + 1;
-      dh[hself - 1] = hv;
-    } else if (hsel == 2) {
-      if (hv < 1 || hv > (int)ea.nh) bad = 1;
-      hself = bad ? 0 : hv;
+  }
+  Sum4 tA;
+  Sum4 ea = block_excl(sum, Sum4{0, 0, 0, 0}, bufA, &tA);
+  if (!WRITE) {
+    Last2 last{0, 0};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (f[u].wsel() == 1) {
+        dw[j0 + ea.nw] = f[u].wv;
+        last.w = SN_REL | (int)++ea.nw;
+      } else if (f[u].wsel() == 2) {
+        last.w = SN_ABS | (f[u].wv & 0xffff);
+      }
+      if (f[u].hsel() == 1) {
+        dh[j0 + ea.nh] = f[u].hv;
+        last.h = SN_REL | (int)++ea.nh;
+      } else if (f[u].hsel() == 2) {
+        last.h = SN_ABS | (f[u].hv & 0xffff);
+      }
     }
     Last2 tB;
-    Last2 eb = block_excl(Last2{wself, hself}, Last2{0, 0}, bufB[k & 1], &tB);
-    eb = op(cB, eb);
-    if (valid) {
-      const int cw = wself ? wself : eb.w;
-      const int x = (int)(ea.x + (unsigned)dx), y = (int)(ea.y + (unsigned)dy);
-      int w = 0, h = 0;
-      if (cw < 1)
-        bad = 1;
-      else
-        w = dw[cw - 1];
-      if (info & 16) {
-        h = w;
-      } else {
-        const int ch = hself ? hself : eb.h;
-        if (ch < 1)
-          bad = 1;
-        else
-          h = dh[ch - 1];
+    block_excl(last, Last2{0, 0}, bufB, &tB);
+    if (t == 0) blocks[c * BPC + kb] = RecBlock{tA.x, tA.y, tA.nw, tA.nh, tB.w, tB.h, 0, 0};
+    return;
+  }
+  ea = op(Sum4{pre.dx, pre.dy, pre.nw, pre.nh}, ea);
+  // the dictionary index every record sets (0: none); an index outside the entries so far is malformed
+  int wi[4], hi[4], bad = 0;
+  Last2 last{0, 0};
+  {
+    Sum4 e = ea;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      wi[u] = hi[u] = 0;
+      if (f[u].wsel() == 1) {
+        wi[u] = (int)++e.nw;
+      } else if (f[u].wsel() == 2) {
+        if (f[u].wv < 1 || f[u].wv > (int)e.nw) bad |= 1 << u;
+        else wi[u] = f[u].wv;
       }
-      if (bad) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAP_DEC, b0 + j);
-      out[b0 + j] = make_int4(x, y, (int)((unsigned)x + (unsigned)w), (int)((unsigned)y + (unsigned)h));
+      if (f[u].hsel() == 1) {
+        hi[u] = (int)++e.nh;
+      } else if (f[u].hsel() == 2) {
+        if (f[u].hv < 1 || f[u].hv > (int)e.nh) bad |= 1 << u;
+        else hi[u] = f[u].hv;
+      }
+      last = op(last, Last2{wi[u], hi[u]});
     }
-    cA = op(cA, tA);
-    cB = op(cB, tB);
+  }
+  Last2 tB;
+  Last2 cur = op(Last2{pre.lw, pre.lh}, block_excl(last, Last2{0, 0}, bufB, &tB));
+  auto entry_at = [&](const int* d, const unsigned* p, int idx) {  // entry idx (1-based) of the chunk's dictionary
+    int j = 0;
+#pragma unroll
+    for (int s2 = 32; s2 > 0; s2 >>= 1)
+      if (j + s2 <= kb && (int)p[j + s2] < idx) j += s2;
+    return d[j * SN_RB + idx - 1 - (int)p[j]];
+  };
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int j = j0 + 4 * t + u;
+    ea.x += (unsigned)f[u].dx;
+    ea.y += (unsigned)f[u].dy;
+    cur = op(cur, Last2{wi[u], hi[u]});
+    if (j >= nb) break;
+    int w = 0, h = 0;
+    if (cur.w < 1) bad |= 1 << u;
+    else w = entry_at(dw, pnw, cur.w);
+    if (f[u].info & 16) h = w;
+    else if (cur.h < 1) bad |= 1 << u;
+    else h = entry_at(dh, pnh, cur.h);
+    if ((bad >> u) & 1) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAP_DEC, b0 + j);
+    out[b0 + j] = make_int4((int)ea.x, (int)ea.y, (int)(ea.x + (unsigned)w), (int)(ea.y + (unsigned)h));
   }
 }
 
@@ -795,45 +986,68 @@ __global__ void k_snappy_gather(const unsigned char* __restrict__ fout, const in
     for (long long c = threadIdx.x; c < nchunks; c += blockDim.x) sn_put_varint(dst + pre_at[c], (unsigned long long)pre_val[c]);
 }
 
-// One single-warp CTA per chunk: Snappy raw stream -> codec bytes.  The
-// element tags are read from a 4 KB staging copy of the input, literals are
-// copied with four loads in flight per lane, and copies whose source lies in
-// the last 32 KB of output are read from a shared-memory ring of it (older
-// sources from global memory).
+// One CTA per chunk: Snappy raw stream -> codec bytes.  Warp 0 takes the
+// elements; a literal of SN_LONG bytes or more is copied by the whole CTA, 16
+// bytes per thread and step (a chunk of 65536-byte literals, as a stream
+// without repeats has them, had one warp copy 1 byte per lane: 1892 us for
+// 184 chunks).  Element tags are read from a 4 KB staging copy of the input;
+// copies whose source lies in the last 32 KB of output are read from a
+// shared-memory ring of it (older sources from global memory).
 #define SN_RING 32768
 #define SN_STAGE 4096
-__global__ void __launch_bounds__(32)
+#define SN_LONG 1024
+#define SN_DT 256
+__global__ void __launch_bounds__(SN_DT)
 k_snappy_decompress(const unsigned char* __restrict__ in_all, const long long* __restrict__ in_off,
                     const long long* __restrict__ in_len, unsigned char* out_all, const long long* __restrict__ out_off,
                     const long long* __restrict__ out_len, long long nchunks, DStatus* st) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  unsigned char* ring = dsm;           // output byte x at ring[x % SN_RING] for the last SN_RING bytes
+  unsigned char* ring = dsm;           // output byte x at ring[(x + ra) % SN_RING] for the last SN_RING bytes
   unsigned char* stg = dsm + SN_RING;  // input bytes [sb, sb + SN_STAGE)
-  const int lane = threadIdx.x;
+  __shared__ long long s_lit[3];       // a long literal: input position, output position, length (0: done)
+  const int lane = threadIdx.x & 31;
   const long long c = blockIdx.x;
   if (c >= nchunks) return;
   const unsigned char* in = in_all + in_off[c];
   const long long len = in_len[c];
   unsigned char* out = out_all + out_off[c];
   const long long want = out_len[c];
+  const int ra = (int)((uintptr_t)out & 15);  // ring and output agree modulo 16 bytes
   long long sb = -(long long)SN_STAGE - 8;
-  auto stage = [&](long long p) {  // bytes p .. p + 7 staged
+  auto stage = [&](long long p) {  // bytes p .. p + 7 staged (warp 0)
     if (p < sb || p + 8 > sb + SN_STAGE) {
-      sb = p;
+      sb = p - (long long)((uintptr_t)(in + p) & 15);
       __syncwarp();
-#pragma unroll 16
-      for (int i = lane; i < SN_STAGE; i += 32) stg[i] = sb + i < len ? in[sb + i] : 0;  // 16 loads in flight
+      for (int i0 = 0; i0 < SN_STAGE; i0 += 32 * 16 * 4) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const long long q = sb + i0 + u * 512 + lane * 16;
+          v[u] = make_uint4(0, 0, 0, 0);
+          if (q >= 0 && q + 16 <= len) {
+            v[u] = *reinterpret_cast<const uint4*>(in + q);
+          } else if (q + 16 > 0 && q < len) {
+            unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (q + j >= 0 && q + j < len) w[j >> 2] |= (unsigned)in[q + j] << (8 * (j & 3));
+            v[u] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(stg + i0 + u * 512 + lane * 16) = v[u];
+      }
       __syncwarp();
     }
   };
   int bad = 0;
   long long p = 0, o = 0;
-  stage(0);
-  {
+  if (threadIdx.x < 32) {
+    stage(0);
     unsigned long long v = 0;
     int k = 0;
     for (int i = 0; i < 5 && i < len; ++i) {
-      const unsigned b = stg[i];
+      const unsigned b = stg[i - sb];
       v |= (unsigned long long)(b & 127u) << (7 * i);
       if (!(b & 128u)) {
         k = i + 1;
@@ -843,97 +1057,145 @@ k_snappy_decompress(const unsigned char* __restrict__ in_all, const long long* _
     if (!k || (long long)v != want) bad = 1;
     p = k;
   }
-  while (!bad && p < len) {
-    stage(p);
-    const unsigned tag = stg[p - sb];
-    const unsigned char* tb = stg + (p - sb) + 1;  // up to 4 bytes after the tag
-    ++p;
-    const unsigned tt = tag & 3u;
-    if (tt == 0) {
-      long long m = tag >> 2;
-      if (m >= 60) {
-        const int nb = (int)m - 59;
-        if (p + nb > len) {
-          bad = 1;
-          break;
-        }
-        m = 0;
-        for (int i = 0; i < nb; ++i) m |= (long long)tb[i] << (8 * i);
-        p += nb;
-      }
-      const long long L = m + 1;
-      if (p + L > len || o + L > want) {
-        bad = 1;
-        break;
-      }
-      for (long long i0 = 0; i0 < L; i0 += 128) {
-        unsigned char v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const long long i = i0 + u * 32 + lane;
-          v[u] = i < L ? in[p + i] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const long long i = i0 + u * 32 + lane;
-          if (i < L) {
-            out[o + i] = v[u];
-            ring[(o + i) & (SN_RING - 1)] = v[u];
+  for (;;) {
+    if (threadIdx.x < 32) {
+      long long lit = 0;
+      while (!bad && p < len) {
+        stage(p);
+        const unsigned tag = stg[p - sb];
+        const unsigned char* tb = stg + (p - sb) + 1;  // up to 4 bytes after the tag
+        ++p;
+        const unsigned tt = tag & 3u;
+        if (tt == 0) {
+          long long m = tag >> 2;
+          if (m >= 60) {
+            const int nb = (int)m - 59;
+            if (p + nb > len) {
+              bad = 1;
+              break;
+            }
+            m = 0;
+            for (int i = 0; i < nb; ++i) m |= (long long)tb[i] << (8 * i);
+            p += nb;
           }
+          const long long L = m + 1;
+          if (p + L > len || o + L > want) {
+            bad = 1;
+            break;
+          }
+          if (L >= SN_LONG) {
+            lit = L;
+            break;
+          }
+          for (long long i0 = 0; i0 < L; i0 += 128) {
+            unsigned char v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const long long i = i0 + u * 32 + lane;
+              v[u] = i < L ? in[p + i] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const long long i = i0 + u * 32 + lane;
+              if (i < L) {
+                out[o + i] = v[u];
+                ring[(o + i + ra) & (SN_RING - 1)] = v[u];
+              }
+            }
+          }
+          p += L;
+          o += L;
+        } else {
+          long long L, off;
+          if (tt == 1) {
+            if (p + 1 > len) {
+              bad = 1;
+              break;
+            }
+            L = 4 + ((tag >> 2) & 7u);
+            off = ((long long)(tag >> 5) << 8) | tb[0];
+            p += 1;
+          } else if (tt == 2) {
+            if (p + 2 > len) {
+              bad = 1;
+              break;
+            }
+            L = 1 + (tag >> 2);
+            off = (long long)tb[0] | ((long long)tb[1] << 8);
+            p += 2;
+          } else {
+            if (p + 4 > len) {
+              bad = 1;
+              break;
+            }
+            L = 1 + (tag >> 2);
+            off = (long long)tb[0] | ((long long)tb[1] << 8) | ((long long)tb[2] << 16) | ((long long)tb[3] << 24);
+            p += 4;
+          }
+          if (off == 0 || off > o || o + L > want) {
+            bad = 1;
+            break;
+          }
+          // byte o + i repeats the period [o - off, o): every source precedes this element
+          if (off + L <= SN_RING) {
+            for (long long i = lane; i < L; i += 32) {
+              const unsigned char v = ring[(o - off + (i < off ? i : i % off) + ra) & (SN_RING - 1)];
+              out[o + i] = v;
+              ring[(o + i + ra) & (SN_RING - 1)] = v;
+            }
+          } else {
+            for (long long i = lane; i < L; i += 32) {
+              const unsigned char v = out[o - off + (i < off ? i : i % off)];
+              out[o + i] = v;
+              ring[(o + i + ra) & (SN_RING - 1)] = v;
+            }
+          }
+          o += L;
         }
+        __syncwarp();
       }
-      p += L;
-      o += L;
-    } else {
-      long long L, off;
-      if (tt == 1) {
-        if (p + 1 > len) {
-          bad = 1;
-          break;
-        }
-        L = 4 + ((tag >> 2) & 7u);
-        off = ((long long)(tag >> 5) << 8) | tb[0];
-        p += 1;
-      } else if (tt == 2) {
-        if (p + 2 > len) {
-          bad = 1;
-          break;
-        }
-        L = 1 + (tag >> 2);
-        off = (long long)tb[0] | ((long long)tb[1] << 8);
-        p += 2;
-      } else {
-        if (p + 4 > len) {
-          bad = 1;
-          break;
-        }
-        L = 1 + (tag >> 2);
-        off = (long long)tb[0] | ((long long)tb[1] << 8) | ((long long)tb[2] << 16) | ((long long)tb[3] << 24);
-        p += 4;
+      if (lane == 0) {
+        s_lit[0] = p;
+        s_lit[1] = o;
+        s_lit[2] = lit;
       }
-      if (off == 0 || off > o || o + L > want) {
-        bad = 1;
-        break;
-      }
-      // byte o + i repeats the period [o - off, o): every source precedes this element
-      if (off + L <= SN_RING) {
-        for (long long i = lane; i < L; i += 32) {
-          const unsigned char v = ring[(o - off + (i < off ? i : i % off)) & (SN_RING - 1)];
-          out[o + i] = v;
-          ring[(o + i) & (SN_RING - 1)] = v;
-        }
-      } else {
-        for (long long i = lane; i < L; i += 32) {
-          const unsigned char v = out[o - off + (i < off ? i : i % off)];
-          out[o + i] = v;
-          ring[(o + i) & (SN_RING - 1)] = v;
-        }
-      }
-      o += L;
     }
-    __syncwarp();
+    __syncthreads();
+    const long long lp = s_lit[0], lo = s_lit[1], L = s_lit[2];
+    if (L == 0) break;
+    const long long keep = L - SN_RING;  // only the last SN_RING bytes stay in the ring
+    auto put = [&](long long i) {
+      const unsigned char v = in[lp + i];
+      out[lo + i] = v;
+      if (i >= keep) ring[(lo + i + ra) & (SN_RING - 1)] = v;
+    };
+    // body: 16-byte groups of the output, each from five aligned source words inside the literal
+    const long long i0 = 3 + ((16 - ((uintptr_t)(out + lo + 3) & 15)) & 15);
+    const long long ng = L >= i0 + 20 ? (L - i0 - 20) / 16 + 1 : 0;
+    const unsigned char* src = in + lp + i0;
+    const int sh = 8 * (int)((uintptr_t)src & 3);
+    const unsigned* s32 = reinterpret_cast<const unsigned*>(src - ((uintptr_t)src & 3));
+#pragma unroll 4
+    for (long long g = threadIdx.x; g < ng; g += SN_DT) {
+      unsigned w[5];
+#pragma unroll
+      for (int j = 0; j < 5; ++j) w[j] = s32[4 * g + j];
+      const uint4 v = make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh),
+                                 __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+      const long long i = i0 + 16 * g;
+      *reinterpret_cast<uint4*>(out + lo + i) = v;
+      if (i >= keep) *reinterpret_cast<uint4*>(ring + ((lo + i + ra) & (SN_RING - 1))) = v;
+      else if (i + 16 > keep)
+        for (int j = 0; j < 16; ++j) put(i + j);
+    }
+    for (long long i = threadIdx.x; i < (ng ? i0 : L); i += SN_DT) put(i);
+    if (ng)
+      for (long long i = i0 + 16 * ng + threadIdx.x; i < L; i += SN_DT) put(i);
+    __syncthreads();
+    p = lp + L;
+    o = lo + L;
   }
-  if (lane == 0 && (bad || o != want)) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAPPY_D, c);
+  if (threadIdx.x == 0 && (bad || o != want)) gb_set_error(st, GB_ERR_CORRUPT, KID_SNAPPY_D, c);
 }
 
 // ---------------------------------------------------------------- host side
@@ -1092,33 +1354,54 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
     for (long long i = 0; i < nch; ++i)
       if (rlen[i] != clen[i]) return gbi::set_err(ctx, GB_ERR_CORRUPT, "snap chunk sizes");
   DevMem M(c.stream);
-  long long* d_tab = M.get<long long>(4 * (nch + 1));
+  std::vector<long long> sblk(nch + 1, 0);  // blocks of segments before each chunk
+  for (long long i = 0; i < nch; ++i)
+    sblk[i + 1] = sblk[i] + (std::min(rlen[i], (long long)SN_CHUNK * SN_LMAX) + SN_SEGB - 1) / SN_SEGB;
+  const size_t nseg = (size_t)std::max(sblk[nch], 1ll) * SN_SEGT;
+  long long* d_tab = M.get<long long>(5 * (nch + 1));
   unsigned* d_rec = M.get<unsigned>((size_t)nch * SN_CHUNK);
   int* d_dict = M.get<int>((size_t)nch * 2 * SN_CHUNK);
+  unsigned* d_seg = M.get<unsigned>(3 * nseg);  // entries, exits, counts
+  RecBlock* d_blk = M.get<RecBlock>((size_t)nch * (SN_CHUNK / SN_RB));
   unsigned char* d_raw = method == 0 ? nullptr : M.get<unsigned char>((size_t)roff[nch] + 16);
-  if (!d_tab || !d_rec || !d_dict || (method != 0 && !d_raw)) return gbi::set_err(ctx, GB_ERR_OOM, "snap decode scratch");
-  std::vector<long long> tab(4 * (nch + 1));
+  if (!d_tab || !d_rec || !d_dict || !d_seg || !d_blk || (method != 0 && !d_raw)) return gbi::set_err(ctx, GB_ERR_OOM, "snap decode scratch");
+  std::vector<long long> tab(5 * (nch + 1));
   std::copy(roff.begin(), roff.end(), tab.begin());
   std::copy(coff.begin(), coff.end(), tab.begin() + (nch + 1));
   std::copy(rlen.begin(), rlen.end(), tab.begin() + 2 * (nch + 1));
   std::copy(clen.begin(), clen.end(), tab.begin() + 3 * (nch + 1));
+  std::copy(sblk.begin(), sblk.end(), tab.begin() + 4 * (nch + 1));
   cudaMemcpyAsync(d_tab, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice, c.stream);
   const long long* d_roff = d_tab;
   const long long* d_coff = d_tab + (nch + 1);
   const long long* d_rlen = d_tab + 2 * (nch + 1);
   const long long* d_clen = d_tab + 3 * (nch + 1);
+  const long long* d_sblk = d_tab + 4 * (nch + 1);
   const unsigned char* raw = d_data;
   if (method != 0) {
     cudaFuncSetAttribute((const void*)k_snappy_decompress, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          SN_RING + SN_STAGE);
-    k_snappy_decompress<<<(unsigned)nch, 32, SN_RING + SN_STAGE, c.stream>>>(d_data, d_coff, d_clen, d_raw, d_roff,
+    k_snappy_decompress<<<(unsigned)nch, SN_DT, SN_RING + SN_STAGE, c.stream>>>(d_data, d_coff, d_clen, d_raw, d_roff,
                                                                              d_rlen, nch, c.st);
     ++c.launches;
     raw = d_raw;
   }
-  k_codec_bounds<<<(unsigned)nch, SN_BT, 0, c.stream>>>(raw, d_roff, d_rlen, n, nch, d_rec, c.st);
-  k_codec_decode<<<(unsigned)nch, SN_T, 0, c.stream>>>(raw, d_roff, d_rec, n, d_dict, d_boxes, c.st);
-  c.launches += 2;
+  if (sblk[nch]) {
+    k_seg_guess<<<(unsigned)sblk[nch], SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, (int)nch, d_seg, d_seg + nseg,
+                                                               d_seg + 2 * nseg);
+    ++c.launches;
+  }
+  k_seg_settle<<<(unsigned)nch, SN_T, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, n, d_seg, d_seg + nseg, d_seg + 2 * nseg,
+                                                     c.st);
+  if (sblk[nch]) {
+    k_seg_records<<<(unsigned)sblk[nch], SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, (int)nch, n, d_seg,
+                                                                 d_seg + 2 * nseg, d_rec, c.st);
+    ++c.launches;
+  }
+  const unsigned rb = (unsigned)(nch * (SN_CHUNK / SN_RB));
+  k_codec_decode<false><<<rb, SN_RT, 0, c.stream>>>(raw, d_roff, d_rec, n, d_dict, d_blk, d_boxes, c.st);
+  k_codec_decode<true><<<rb, SN_RT, 0, c.stream>>>(raw, d_roff, d_rec, n, d_dict, d_blk, d_boxes, c.st);
+  c.launches += 3;
   return gb_sync(ctx, nullptr);
 }
 
