@@ -12,21 +12,23 @@
 //     that keeps each value's first position; a bitmap of first positions
 //     with prefix popcounts gives each value its 1-based order of first
 //     appearance, the codec's dictionary index, stored per box;
-//   * boxes are then taken in order, 1024 at a time: a box's record (infobyte,
-//     zigzag varint anchor deltas, the width / height as a varint when new or
-//     an int16 index when seen before) depends only on the previous box, the
-//     previous non-square box (a block scan) and the two ranks, and lands at
-//     the exclusive sum of the record sizes.  One launch sizes the chunks, a
-//     second writes them.
+//   * blocks of 1024 boxes then size and write their records: a box's record
+//     (infobyte, zigzag varint anchor deltas, the width / height as a varint
+//     when new or an int16 index when seen before) depends only on the
+//     previous box, the previous non-square box and the two ranks, and lands
+//     at the sum of the sizes of the blocks and boxes before it.  One launch
+//     sizes the blocks, a second writes them through shared memory.
 // Snappy: each 65536-byte fragment of a chunk's codec bytes is compressed by
-// one warp, 32 positions at a time: a position's candidate is the latest
-// earlier position with the same 11-bit hash of its 4 bytes (warp match for
-// the batch, a 2048-slot table across batches); the greedy parse jumps to
-// the next verified candidate, extends the match 32 bytes per step and, when
-// it is at least 8 bytes long, emits Snappy literal / copy elements.  Fragments are concatenated behind the
-// chunk's length preamble.  Decoding takes one warp per chunk through the
-// elements (all element forms of the format are accepted), with the last
-// 32 KB of output in a shared-memory ring for the copies.
+// one CTA with the fragment in shared memory.  A position's candidate is the
+// latest earlier position with the same 11-bit hash of its 4 bytes; 32 warps
+// find the candidates of 8192 positions (each warp's last positions per hash,
+// a scan of these over the warps, then every warp through its positions), and
+// mark those whose first 8 bytes match.  One warp takes the greedy parse from
+// mark to mark, extends a match 32 bytes per step and emits Snappy literal /
+// copy elements.  Fragments are concatenated behind the chunk's length
+// preamble.  Decoding takes one CTA per chunk through the elements (all
+// element forms of the format are accepted), with the last 32 KB of output in
+// a shared-memory ring for the copies and long literals copied by the CTA.
 // Decoding the codec.  Record boundaries: a record's length follows from its
 // bytes, so a chain started anywhere falls in with the true one after a few
 // records.  Every 256-byte segment guesses its first record by a chain from
@@ -45,7 +47,7 @@
 
 #define SN_CHUNK 65536  // boxes per chunk (box_codec.f90:227)
 #define SN_FRAG 65536   // Snappy fragment (bytes)
-#define SN_FCAP (SN_FRAG + SN_FRAG / 6 + 64)
+#define SN_FCAP ((SN_FRAG + SN_FRAG / 6 + 64 + 15) / 16 * 16)
 #define SN_T 1024       // threads of the per-chunk CTAs
 #define SN_REC_MAX 31   // longest record of a valid box (1 + 5 + 5 + 10 + 10)
 #define SN_MIN_MATCH 8  // shortest copy the compressor emits
@@ -95,6 +97,27 @@ __device__ __forceinline__ unsigned long long sn_get_varint(const unsigned char*
   }
   *k = 0;
   return 0;
+}
+
+// len bytes from src to dst, thread t of nt: 16-byte groups of the destination, each from five aligned source words
+// that lie inside [src, src + len); the ends byte by byte.
+__device__ __forceinline__ void sn_copy(unsigned char* dst, const unsigned char* src, long long len, int t, int nt) {
+  const long long i0 = 3 + ((16 - ((uintptr_t)(dst + 3) & 15)) & 15);
+  const long long ng = len >= i0 + 20 ? (len - i0 - 20) / 16 + 1 : 0;
+  const int sh = 8 * (int)((uintptr_t)(src + i0) & 3);
+  const unsigned* s32 = reinterpret_cast<const unsigned*>(src + i0 - ((uintptr_t)(src + i0) & 3));
+#pragma unroll 4
+  for (long long g = t; g < ng; g += nt) {
+    unsigned w[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) w[j] = s32[4 * g + j];
+    *reinterpret_cast<uint4*>(dst + i0 + 16 * g) =
+        make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh),
+                   __funnelshift_r(w[3], w[4], sh));
+  }
+  for (long long i = t; i < (ng ? i0 : len); i += nt) dst[i] = src[i];
+  if (ng)
+    for (long long i = i0 + 16 * ng + t; i < len; i += nt) dst[i] = src[i];
 }
 
 // ---------------------------------------------------------------- block scans
@@ -208,12 +231,15 @@ __device__ __forceinline__ unsigned sn_rank(const unsigned* bits, const unsigned
   return pre[p >> 5] + __popc(bits[p >> 5] & ((1u << (p & 31)) - 1u)) + 1u;
 }
 
-// Dictionary ranks of one chunk per CTA: ranks[b] (widths) and ranks[n + b]
-// (heights of non-square boxes) = order of first appearance | first << 31.
-// The width table is built and read, then the height table in the same
-// storage.  GT: 131072-slot tables in global memory for the chunks in list
+// Dictionary ranks of one chunk's widths (blockIdx.y 0: ranks[b]) or of its
+// non-square boxes' heights (1: ranks[n + b]) per CTA = order of first
+// appearance | first << 31.  A CTA takes most of an SM's shared memory, so
+// chunks fill the chip in waves; half a chunk per CTA leaves less of the last
+// one idle, and SN_RLD boxes are loaded ahead of their inserts (184 chunks:
+// 388 -> 173 us).  GT: 131072-slot tables in global memory for the chunks in list
 // (one table per CTA), else 16384-slot shared tables (chunk = block index);
 // a chunk with more values than a shared table holds goes to ovf_list.
+#define SN_RLD 4
 template <bool GT>
 __global__ void __launch_bounds__(SN_T, 1)
 k_enc_rank(const int4* __restrict__ boxes, long long n, const int* __restrict__ list, int nlist,
@@ -225,7 +251,7 @@ k_enc_rank(const int4* __restrict__ boxes, long long n, const int* __restrict__ 
   unsigned char* q = sm;
   unsigned long long* tab;
   if (GT) {
-    tab = gtab + (size_t)blockIdx.x * SLOTS;
+    tab = gtab + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * SLOTS;
   } else {
     tab = (unsigned long long*)q;
     q += SLOTS * 8;
@@ -237,28 +263,40 @@ k_enc_rank(const int4* __restrict__ boxes, long long n, const int* __restrict__ 
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
   const long long nchunks = (n + SN_CHUNK - 1) / SN_CHUNK;
   const long long nitems = GT ? nlist : nchunks;
+  const int which = blockIdx.y;
   for (long long li = blockIdx.x; li < nitems; li += gridDim.x) {
-    const long long c = GT ? list[li] : li;
+    if (GT && li >= list[which - 2]) break;  // the widths' and the heights' lists alternate behind their counts
+    const long long c = GT ? list[2 * li + which] : li;
     const long long b0 = c * SN_CHUNK;
     const int nb = (int)min((long long)SN_CHUNK, n - b0);
     bool ovf = false;
-    for (int which = 0; which < 2 && !ovf; ++which) {
+    {
       for (unsigned i = t; i < SLOTS; i += SN_T) tab[i] = SN_EMPTY;
       for (int i = t; i < 2048; i += SN_T) bits[i] = 0;
       if (t < 2) flags[t] = 0;
       __syncthreads();
-      for (int j = t; j < nb; j += SN_T) {
-        const int4 b = boxes[b0 + j];
-        const int w = (int)((unsigned)b.z - (unsigned)b.x), h = (int)((unsigned)b.w - (unsigned)b.y);
-        if (which && w == h) continue;
-        if (!tab_insert(tab, MASK, which ? h : w, (unsigned)j, &flags[0], LIMIT)) {
-          flags[1] = 1;
-          break;
+      bool full = false;
+      for (int j0 = t; j0 < nb && !full; j0 += SN_RLD * SN_T) {
+        int4 ld[SN_RLD];
+#pragma unroll
+        for (int u = 0; u < SN_RLD; ++u)
+          if (j0 + u * SN_T < nb) ld[u] = boxes[b0 + j0 + u * SN_T];
+#pragma unroll
+        for (int u = 0; u < SN_RLD; ++u) {
+          const int j = j0 + u * SN_T;
+          const int4 b = ld[u];
+          const int w = (int)((unsigned)b.z - (unsigned)b.x), h = (int)((unsigned)b.w - (unsigned)b.y);
+          if (full || j >= nb || (which && w == h)) continue;
+          if (!tab_insert(tab, MASK, which ? h : w, (unsigned)j, &flags[0], LIMIT)) {
+            flags[1] = 1;
+            full = true;
+          }
         }
       }
       __syncthreads();
       ovf = *(volatile unsigned*)&flags[1] != 0;
-      if (ovf) break;  // uniform
+    }
+    if (!ovf) {  // uniform
       for (unsigned i = t; i < SLOTS; i += SN_T) {
         const unsigned long long cur = *(volatile unsigned long long*)&tab[i];
         if (cur != SN_EMPTY) {
@@ -293,16 +331,24 @@ k_enc_rank(const int4* __restrict__ boxes, long long n, const int* __restrict__ 
       }
       __syncthreads();
       unsigned* out = ranks + (which ? n : 0) + b0;
-      for (int j = t; j < nb; j += SN_T) {
-        const int4 b = boxes[b0 + j];
-        const int w = (int)((unsigned)b.z - (unsigned)b.x), h = (int)((unsigned)b.w - (unsigned)b.y);
-        if (which && w == h) continue;
-        const unsigned p = tab_first(tab, MASK, which ? h : w);
-        if (p >= SN_CHUNK) {
-          gb_set_error(st, GB_ERR_INTERNAL, KID_SNAP_ENC, b0 + j);
-          continue;
+      for (int j0 = t; j0 < nb; j0 += SN_RLD * SN_T) {
+        int4 ld[SN_RLD];
+#pragma unroll
+        for (int u = 0; u < SN_RLD; ++u)
+          if (j0 + u * SN_T < nb) ld[u] = boxes[b0 + j0 + u * SN_T];
+#pragma unroll
+        for (int u = 0; u < SN_RLD; ++u) {
+          const int j = j0 + u * SN_T;
+          const int4 b = ld[u];
+          const int w = (int)((unsigned)b.z - (unsigned)b.x), h = (int)((unsigned)b.w - (unsigned)b.y);
+          if (j >= nb || (which && w == h)) continue;
+          const unsigned p = tab_first(tab, MASK, which ? h : w);
+          if (p >= SN_CHUNK) {
+            gb_set_error(st, GB_ERR_INTERNAL, KID_SNAP_ENC, b0 + j);
+            continue;
+          }
+          out[j] = sn_rank(bits, pre, p) | ((p == (unsigned)j) ? 0x80000000u : 0u);
         }
-        out[j] = sn_rank(bits, pre, p) | ((p == (unsigned)j) ? 0x80000000u : 0u);
       }
       __syncthreads();
     }
@@ -310,96 +356,163 @@ k_enc_rank(const int4* __restrict__ boxes, long long n, const int* __restrict__ 
       if (GT)
         gb_set_error(st, GB_ERR_INTERNAL, KID_SNAP_ENC, c);
       else
-        ovf_list[atomicAdd(ovf_count, 1)] = (int)c;
+        ovf_list[2 * atomicAdd(&ovf_count[which], 1) + which] = (int)c;
     }
     __syncthreads();
   }
 }
 
-// Codec records of one chunk per CTA from the ranks: WRITE emits the bytes
-// at raw + raw_off[c], else raw_size[c] receives the chunk's byte count.
+// Codec records from the ranks, SN_RB boxes per block, four consecutive ones
+// per thread.  WRITE: the block's records are put together in shared memory
+// and copied to raw at the chunk's offset plus the sizes of the blocks before
+// it; else bsize[block] receives the block's byte count.  (One CTA per chunk,
+// 64 steps behind one another, took 369 us for the sizes and 606 us for the
+// records of 184 chunks, written byte by byte.)
+#define SN_RB 1024
+#define SN_RT 256
+#define SN_BPC (SN_CHUNK / SN_RB)  // blocks per chunk: 64
 template <bool WRITE>
-__global__ void __launch_bounds__(SN_T, 1)
-k_enc_emit(const int4* __restrict__ boxes, long long n, const unsigned* __restrict__ ranks,
-           long long* raw_size, const long long* __restrict__ raw_off, unsigned char* __restrict__ raw, DStatus* st) {
-  __shared__ SumS bufS[2][32];
-  __shared__ LastS bufL[2][32];
-  const long long c = blockIdx.x;
-  const int t = threadIdx.x;
+__global__ void __launch_bounds__(SN_RT)
+k_enc_emit(const int4* __restrict__ boxes, long long n, const unsigned* __restrict__ ranks, int* __restrict__ bsize,
+           const long long* __restrict__ raw_off, unsigned char* __restrict__ raw, DStatus* st) {
+  __shared__ SumS bufS[32];
+  __shared__ LastS bufL[32];
+  __shared__ int s_back, s_off;
+  extern __shared__ __align__(16) unsigned char sm[];  // WRITE: SN_RB * SN_REC_MAX bytes
+  const long long c = blockIdx.x / SN_BPC;
+  const int kb = blockIdx.x % SN_BPC, t = threadIdx.x;
   const long long b0 = c * SN_CHUNK;
   const int nb = (int)min((long long)SN_CHUNK, n - b0);
-  unsigned long long cbytes = 0;  // bytes of the records so far
-  LastS chl{0, 0};                // last non-square box's height so far
-  unsigned char* out = WRITE ? raw + raw_off[c] : nullptr;
-  for (int k = 0; k * SN_T < nb; ++k) {
-    const int j = k * SN_T + t;
-    const bool valid = j < nb;
-    int4 b = make_int4(0, 0, 0, 0), pb = make_int4(0, 0, 0, 0);
-    if (valid) {
-      b = boxes[b0 + j];
-      if (j) pb = boxes[b0 + j - 1];
-    }
-    const int w = (int)((unsigned)b.z - (unsigned)b.x), h = (int)((unsigned)b.w - (unsigned)b.y);
-    const bool sq = w == h;
-    LastS tl;
-    LastS ph = block_excl(LastS{valid && !sq, h}, LastS{0, 0}, bufL[k & 1], &tl);
-    ph = op(chl, ph);
-    unsigned info = 0, size = 0, wr = 0, hr = 0;
-    int dx = 0, dy = 0;
-    if (valid) {
-      const int pw = j ? (int)((unsigned)pb.z - (unsigned)pb.x) : 0;
-      dx = (int)((unsigned)b.x - (unsigned)pb.x);  // the anchor cursor starts at 0 and follows x1
-      dy = (int)((unsigned)b.y - (unsigned)pb.y);
-      if (sq) info |= 16;
-      if (dx) info |= 32;
-      if (dy) info |= 64;
-      const unsigned rw = ranks[b0 + j];
-      wr = rw & 0x7fffffffu;
-      if (j == 0 || w != pw) info |= (rw >> 31) ? 3u : 1u;
-      if (!sq) {
-        const unsigned rh = ranks[n + b0 + j];
-        hr = rh & 0x7fffffffu;
-        if (!ph.has || ph.val != h) info |= (rh >> 31) ? 12u : 4u;
-      }
-      size = 1;
-      if (info & 32) size += sn_vlen(sn_zigzag(dx));
-      if (info & 64) size += sn_vlen(sn_zigzag(dy));
-      if (info & 1) size += (info & 2) ? sn_vlen((unsigned long long)(long long)w) : 2;
-      if (info & 4) size += (info & 8) ? sn_vlen((unsigned long long)(long long)h) : 2;
-    }
-    SumS ts;
-    const SumS ex = block_excl(SumS{size}, SumS{0}, bufS[k & 1], &ts);
-    if (WRITE && valid) {
-      unsigned char* o = out + cbytes + ex.a;
-      *o++ = (unsigned char)info;
-      if (info & 32) o = sn_put_varint(o, sn_zigzag(dx));
-      if (info & 64) o = sn_put_varint(o, sn_zigzag(dy));
-      if (info & 1) {
-        if (info & 2) {
-          o = sn_put_varint(o, (unsigned long long)(long long)w);
-        } else {  // int16 index, little-endian (wraps above 32767 as the reference's int16 does)
-          *o++ = (unsigned char)wr;
-          *o++ = (unsigned char)(wr >> 8);
-        }
-      }
-      if (info & 4) {
-        if (info & 8) {
-          o = sn_put_varint(o, (unsigned long long)(long long)h);
-        } else {
-          *o++ = (unsigned char)hr;
-          *o++ = (unsigned char)(hr >> 8);
-        }
-      }
-    }
-    cbytes += ts.a;
-    chl = op(chl, tl);
+  const int j0 = kb * SN_RB;
+  if (j0 >= nb) {
+    if (!WRITE && t == 0) bsize[blockIdx.x] = 0;
+    return;
   }
-  if (t == 0) {
-    if (!WRITE)
-      raw_size[c] = (long long)cbytes;
-    else if ((long long)cbytes != raw_off[c + 1] - raw_off[c])
-      gb_set_error(st, GB_ERR_INTERNAL, KID_SNAP_ENC, c);
+  const int4* bx = boxes + b0;
+  int4 b[5];  // the box before the thread's four, then these
+  LastS lh{0, 0};
+#pragma unroll
+  for (int u = 0; u < 5; ++u) {
+    const int j = j0 + 4 * t + u - 1;
+    b[u] = j >= 0 && j < nb ? bx[j] : make_int4(0, 0, 0, 0);
   }
+  int w[4], h[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    w[u] = (int)((unsigned)b[u + 1].z - (unsigned)b[u + 1].x);
+    h[u] = (int)((unsigned)b[u + 1].w - (unsigned)b[u + 1].y);
+    lh = op(lh, LastS{j0 + 4 * t + u < nb && w[u] != h[u], h[u]});
+  }
+  // the last non-square box of the chunk before this block, searched backwards when the block needs it
+  LastS before{0, 0};
+  if (t == 0) s_back = -1;
+  if (__syncthreads_or(lh.has) && j0 > 0) {
+    for (int e = j0; e > 0; e -= SN_RT) {
+      const int j = e - 1 - t;
+      if (j >= 0) {
+        const int4 q = bx[j];
+        if ((unsigned)q.z - (unsigned)q.x != (unsigned)q.w - (unsigned)q.y) atomicMax(&s_back, j);
+      }
+      __syncthreads();
+      const int found = s_back;
+      __syncthreads();
+      if (found >= 0) break;
+    }
+    if (s_back >= 0) {
+      const int4 q = bx[s_back];
+      before = LastS{1, (int)((unsigned)q.w - (unsigned)q.y)};
+    }
+  }
+  LastS tl;
+  LastS ph = op(before, block_excl(lh, LastS{0, 0}, bufL, &tl));
+  unsigned info[4], wr[4], hr[4], size = 0;
+  int dx[4], dy[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int j = j0 + 4 * t + u;
+    info[u] = wr[u] = hr[u] = 0;
+    dx[u] = dy[u] = 0;
+    if (j >= nb) continue;
+    const int4 q = b[u + 1], pb = b[u];  // the anchor cursor starts at 0 and follows x1 (b[0] is 0 at the chunk's start)
+    const bool sq = w[u] == h[u];
+    const int pw = (int)((unsigned)pb.z - (unsigned)pb.x);
+    dx[u] = (int)((unsigned)q.x - (unsigned)pb.x);
+    dy[u] = (int)((unsigned)q.y - (unsigned)pb.y);
+    if (sq) info[u] |= 16;
+    if (dx[u]) info[u] |= 32;
+    if (dy[u]) info[u] |= 64;
+    const unsigned rw = ranks[b0 + j];
+    wr[u] = rw & 0x7fffffffu;
+    if (j == 0 || w[u] != pw) info[u] |= (rw >> 31) ? 3u : 1u;
+    if (!sq) {
+      const unsigned rh = ranks[n + b0 + j];
+      hr[u] = rh & 0x7fffffffu;
+      if (!ph.has || ph.val != h[u]) info[u] |= (rh >> 31) ? 12u : 4u;
+      ph = LastS{1, h[u]};
+    }
+    size += 1;
+    if (info[u] & 32) size += sn_vlen(sn_zigzag(dx[u]));
+    if (info[u] & 64) size += sn_vlen(sn_zigzag(dy[u]));
+    if (info[u] & 1) size += (info[u] & 2) ? sn_vlen((unsigned long long)(long long)w[u]) : 2;
+    if (info[u] & 4) size += (info[u] & 8) ? sn_vlen((unsigned long long)(long long)h[u]) : 2;
+  }
+  SumS ts;
+  const SumS ex = block_excl(SumS{size}, SumS{0}, bufS, &ts);
+  if (!WRITE) {
+    if (t == 0) bsize[blockIdx.x] = (int)ts.a;
+    return;
+  }
+  if (t < 32) {  // sizes of the chunk's blocks before this one, and of all (checked by its last block)
+    int v = 0, all = 0;
+    for (int j = t; j < SN_BPC; j += 32) {
+      const int x = bsize[c * SN_BPC + j];
+      v += j < kb ? x : 0;
+      all += x;
+    }
+    v = __reduce_add_sync(0xffffffffu, v);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if (t == 0) {
+      s_off = v;
+      if (j0 + SN_RB >= nb && ((long long)v + ts.a != all || all != raw_off[c + 1] - raw_off[c]))
+        gb_set_error(st, GB_ERR_INTERNAL, KID_SNAP_ENC, c);
+    }
+  }
+  unsigned char* o = sm + ex.a;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    if (j0 + 4 * t + u >= nb) break;
+    *o++ = (unsigned char)info[u];
+    if (info[u] & 32) o = sn_put_varint(o, sn_zigzag(dx[u]));
+    if (info[u] & 64) o = sn_put_varint(o, sn_zigzag(dy[u]));
+    if (info[u] & 1) {
+      if (info[u] & 2) {
+        o = sn_put_varint(o, (unsigned long long)(long long)w[u]);
+      } else {  // int16 index, little-endian (wraps above 32767 as the reference's int16 does)
+        *o++ = (unsigned char)wr[u];
+        *o++ = (unsigned char)(wr[u] >> 8);
+      }
+    }
+    if (info[u] & 4) {
+      if (info[u] & 8) {
+        o = sn_put_varint(o, (unsigned long long)(long long)h[u]);
+      } else {
+        *o++ = (unsigned char)hr[u];
+        *o++ = (unsigned char)(hr[u] >> 8);
+      }
+    }
+  }
+  __syncthreads();
+  sn_copy(raw + raw_off[c] + s_off, sm, ts.a, t, SN_RT);
+}
+
+// Chunk sizes from the block sizes (one warp per chunk).
+__global__ void k_enc_sizes(const int* __restrict__ bsize, long long nchunks, long long* __restrict__ raw_size) {
+  const long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nchunks) return;
+  int v = 0;
+  for (int j = threadIdx.x & 31; j < SN_BPC; j += 32) v += bsize[c * SN_BPC + j];
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) raw_size[c] = v;
 }
 
 // ---------------------------------------------------------------- codec decoder
@@ -642,8 +755,6 @@ k_seg_records(const unsigned char* __restrict__ raw, const long long* __restrict
 // the dictionary; pass 1 adds up the blocks of the chunk before it and writes
 // the boxes.  The chunk's 64 steps in one CTA, each behind the scans of the
 // one before, took 459 us for 184 chunks.
-#define SN_RB 1024
-#define SN_RT 256
 #define SN_REL (1 << 30)  // a "last set" code: the block's own entry, 1-based; else SN_ABS | index, 0 = none
 #define SN_ABS (1 << 29)
 struct RecBlock {
@@ -697,9 +808,8 @@ k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restric
   __shared__ unsigned pnw[64], pnh[64];  // entries of the chunk's blocks before block j
   __shared__ RecBlock pre;               // sums of the blocks before this one, last codes made absolute
   __shared__ int s_skip;
-  constexpr int BPC = SN_CHUNK / SN_RB;  // 64
-  const long long c = blockIdx.x / BPC;
-  const int kb = blockIdx.x % BPC, t = threadIdx.x;
+  const long long c = blockIdx.x / SN_BPC;
+  const int kb = blockIdx.x % SN_BPC, t = threadIdx.x;
   const long long b0 = c * SN_CHUNK;
   const int nb = (int)min((long long)SN_CHUNK, n - b0);
   const int j0 = kb * SN_RB;
@@ -711,7 +821,7 @@ k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restric
     for (int h = 0; h < 2; ++h) {  // blocks 0..31, then 32..63
       const int j = h * 32 + t;
       RecBlock q{0, 0, 0, 0, 0, 0, 0, 0};
-      if (j < kb) q = blocks[c * BPC + j];
+      if (j < kb) q = blocks[c * SN_BPC + j];
       SumS e[4] = {{q.dx}, {q.dy}, {q.nw}, {q.nh}};
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1)
@@ -785,7 +895,7 @@ k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restric
     }
     Last2 tB;
     block_excl(last, Last2{0, 0}, bufB, &tB);
-    if (t == 0) blocks[c * BPC + kb] = RecBlock{tA.x, tA.y, tA.nw, tA.nh, tB.w, tB.h, 0, 0};
+    if (t == 0) blocks[c * SN_BPC + kb] = RecBlock{tA.x, tA.y, tA.nw, tA.nh, tB.w, tB.h, 0, 0};
     return;
   }
   ea = op(Sum4{pre.dx, pre.dy, pre.nw, pre.nh}, ea);
@@ -840,10 +950,6 @@ k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restric
 }
 
 // ---------------------------------------------------------------- Snappy
-__device__ __forceinline__ unsigned sn_ld32(const unsigned char* p) {
-  return (unsigned)p[0] | ((unsigned)p[1] << 8) | ((unsigned)p[2] << 16) | ((unsigned)p[3] << 24);
-}
-
 // Writes one Snappy copy element of 4..64 bytes (lane 0 only); returns its size.
 __device__ __forceinline__ int sn_copy_piece(unsigned char* o, unsigned off, int len, bool write) {
   if (len <= 11 && off < 2048u) {
@@ -861,112 +967,209 @@ __device__ __forceinline__ int sn_copy_piece(unsigned char* o, unsigned off, int
   return 3;
 }
 
-// One warp per fragment (8 per CTA).  fsrc / flen: the fragment's bytes in
-// raw; the compressed elements go to fout + f * SN_FCAP, their count to flout.
-__global__ void __launch_bounds__(256)
+// One CTA per fragment (see the top; one warp per fragment, 2048 steps of 32
+// positions behind one another and bytes copied singly, took 1950 us for 1600
+// fragments, this 706 us: bound by shared memory, 74% of its wavefronts, the
+// hash tables' random 2-byte accesses most of them; match_any in every step
+// cost 1097 us, the scan one hash at a time 838 us).  fsrc / flen: the fragment's bytes in raw; the compressed
+// elements go to fout + f * SN_FCAP, their count to flout.
+#define SN_CT 1024
+#define SN_CW (SN_CT / 32)
+#define SN_SUB 8192  // positions whose candidates are held at once
+struct SnapFrag {
+  __align__(16) unsigned char buf[SN_FRAG + 32];  // the fragment at buf[sh], sh = its address modulo 16
+  __align__(16) unsigned short tab[SN_CW][2048];  // latest position + 1 per hash (positions with 4 bytes left are < 65533)
+  unsigned short last[2048];        // the same before the current SN_SUB positions
+  unsigned short cand[SN_SUB];     // candidates of the marked positions
+  unsigned mark[SN_SUB / 32];      // positions whose candidate matches SN_MIN_MATCH bytes
+  int o, lit, fail;
+};
+
+__global__ void __launch_bounds__(SN_CT, 1)
 k_snappy_compress(const unsigned char* __restrict__ raw, const long long* __restrict__ fsrc,
-                  const int* __restrict__ flen, long long nfrag, unsigned char* __restrict__ fout,
-                  int* __restrict__ flout, DStatus* st) {
-  extern __shared__ unsigned short table[];  // [8][2048]: latest position + 1 (positions with 4 bytes left are < 65533)
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long f = (long long)blockIdx.x * 8 + wid;
-  if (f >= nfrag) return;
-  unsigned short* tab = table + wid * 2048;
-  for (int i = lane; i < 2048; i += 32) tab[i] = 0;
-  __syncwarp();
+                  const int* __restrict__ flen, unsigned char* __restrict__ fout, int* __restrict__ flout,
+                  DStatus* st) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  SnapFrag& s = *reinterpret_cast<SnapFrag*>(sm);
+  const int t = threadIdx.x, wid = t >> 5, lane = t & 31;
+  const long long f = blockIdx.x;
   const unsigned char* src = raw + fsrc[f];
   const int fl = flen[f];
   unsigned char* out = fout + f * SN_FCAP;
-  int o = 0, p = 0, lit = 0;
-  for (int bb = 0; bb + 4 <= fl; bb += 32) {
-    const int q = bb + lane;
-    const bool has = q + 4 <= fl;
-    const unsigned v = has ? sn_ld32(src + q) : 0u;
-    const unsigned h = (v * 0x9E3779B1u) >> 21;
-    const unsigned peers = __match_any_sync(0xffffffffu, has ? h : 0x10000u + lane);
-    const unsigned lower = peers & ((1u << lane) - 1u);
-    unsigned cand = 0;  // 1-based
-    if (has) cand = lower ? (unsigned)(bb + 31 - __clz(lower)) + 1u : tab[h];
-    __syncwarp();
-    if (has && (peers >> lane) == 1u) tab[h] = (unsigned short)(q + 1);
-    __syncwarp();
-    // a candidate counts when its first 8 bytes match (shorter copies are not emitted)
-    const bool has8 = q + SN_MIN_MATCH <= fl;
-    const bool ok = has8 && cand && sn_ld32(src + cand - 1) == v && sn_ld32(src + cand + 3) == sn_ld32(src + q + 4);
-    const unsigned okm = __ballot_sync(0xffffffffu, ok);
-    while (p < bb + 32 && p + 4 <= fl) {
-      const unsigned m = okm & (0xffffffffu << (p - bb));
-      if (!m) {
-        p = bb + 32;
-        break;
-      }
-      const int ln = __ffs(m) - 1;
-      p = bb + ln;
-      const int qs = (int)__shfl_sync(0xffffffffu, cand, ln) - 1;
-      int L = SN_MIN_MATCH;
-      for (;;) {
-        const int a = p + L + lane;
-        const bool eq = a < fl && src[qs + L + lane] == src[a];
-        const unsigned ne = __ballot_sync(0xffffffffu, !eq);
-        if (ne) {
-          L += __ffs(ne) - 1;
-          break;
-        }
-        L += 32;
-      }
-      // pending literal
-      if (p > lit) {
-        const int len = p - lit;
-        const unsigned mm = (unsigned)len - 1u;
-        const int nb = mm < 60u ? 0 : mm < 256u ? 1 : 2;
-        if (o + 1 + nb + len + 3 * ((L + 59) / 60) > SN_FCAP) {
-          if (lane == 0) gb_set_error(st, GB_ERR_INTERNAL, KID_SNAPPY_C, f);
-          if (lane == 0) flout[f] = 0;
-          return;
-        }
-        if (lane == 0) {
-          out[o] = (unsigned char)(nb ? (59 + nb) << 2 : mm << 2);
-          for (int i = 0; i < nb; ++i) out[o + 1 + i] = (unsigned char)(mm >> (8 * i));
-        }
+  const int sh = (int)((uintptr_t)src & 15);
 #pragma unroll 4
-        for (int i = lane; i < len; i += 32) out[o + 1 + nb + i] = src[lit + i];
-        o += 1 + nb + len;
-      }
-      {
-        const unsigned off = (unsigned)(p - qs);
-        int rem = L;
-        while (rem >= 68) {
-          o += sn_copy_piece(out + o, off, 64, lane == 0);
-          rem -= 64;
-        }
-        if (rem > 64) {
-          o += sn_copy_piece(out + o, off, 60, lane == 0);
-          rem -= 60;
-        }
-        o += sn_copy_piece(out + o, off, rem, lane == 0);
-      }
-      p += L;
-      lit = p;
+  for (int i = t * 16; i < SN_FRAG + 32; i += SN_CT * 16) {
+    const int q = i - sh;  // fragment position of the group
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (q >= 0 && q + 16 <= fl) {
+      v = *reinterpret_cast<const uint4*>(src + q);
+    } else if (q + 16 > 0 && q < fl) {
+      unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (q + j >= 0 && q + j < fl) w[j >> 2] |= (unsigned)src[q + j] << (8 * (j & 3));
+      v = make_uint4(w[0], w[1], w[2], w[3]);
     }
+    *reinterpret_cast<uint4*>(s.buf + i) = v;
   }
-  if (fl > lit) {
+  for (int i = t; i < 2048; i += SN_CT) s.last[i] = 0;
+  if (t == 0) s.fail = 0;
+  __syncthreads();
+  const unsigned* b32 = reinterpret_cast<const unsigned*>(s.buf);
+  const unsigned char* by = s.buf + sh;
+  auto ld32 = [&](int q) -> unsigned {  // the 4 bytes from position q (staged: q + 8 <= fl + 16)
+    const int i = q + sh;
+    return __funnelshift_r(b32[i >> 2], b32[(i >> 2) + 1], 8 * (i & 3));
+  };
+  unsigned short* tab = s.tab[wid];
+  int o = 0, p = 0, lit = 0;  // the parse (warp 0)
+  for (int h0 = 0; h0 + 4 <= fl; h0 += SN_SUB) {
+    const int q0 = h0 + wid * (SN_SUB / SN_CW);
+    const int q1 = min(q0 + SN_SUB / SN_CW, fl - 3);  // positions with 4 bytes left
+    for (int i = lane; i < 1024; i += 32) reinterpret_cast<unsigned*>(tab)[i] = 0;
+    for (int i = t; i < SN_SUB / 32; i += SN_CT) s.mark[i] = 0;
+    __syncwarp();
+    for (int b = q0; b < q1; b += 32) {  // the warp's latest position per hash
+      const int q = b + lane;
+      const bool has = q < q1;
+      const unsigned h = has ? (ld32(q) * 0x9E3779B1u) >> 21 : 0u;
+      bool again = has;
+      while (__any_sync(0xffffffffu, again)) {  // lanes of one hash: the highest position stays
+        if (again) tab[h] = (unsigned short)(q + 1);
+        __syncwarp();
+        again = has && tab[h] < (unsigned short)(q + 1);
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    {  // before each warp's positions: a running maximum over the warps, two hashes per thread
+      static_assert(SN_CT == 1024, "one word of two hashes per thread");
+      unsigned run = reinterpret_cast<unsigned*>(s.last)[t];
+#pragma unroll 8
+      for (int w = 0; w < SN_CW; ++w) {
+        unsigned* e = reinterpret_cast<unsigned*>(s.tab[w]) + t;
+        const unsigned x = *e;
+        *e = run;
+        run = __vmaxu2(run, x);
+      }
+      reinterpret_cast<unsigned*>(s.last)[t] = run;
+    }
+    __syncthreads();
+    for (int b = q0; b < q1; b += 32) {
+      const int q = b + lane;
+      const bool has = q < q1;
+      const unsigned v = ld32(min(q, fl - 4));
+      const unsigned h = (v * 0x9E3779B1u) >> 21;
+      unsigned cand = has ? tab[h] : 0u;  // 1-based
+      __syncwarp();
+      if (has) tab[h] = (unsigned short)(q + 1);
+      __syncwarp();
+      // lanes of one hash (one step in five): the latest lower lane is the candidate, the highest lane stays
+      if (__any_sync(0xffffffffu, has && tab[h] != (unsigned short)(q + 1))) {
+        const unsigned peers = __match_any_sync(0xffffffffu, has ? h : 0x10000u + lane);
+        const unsigned lower = peers & ((1u << lane) - 1u);
+        if (lower) cand = (unsigned)(b + 31 - __clz(lower)) + 1u;
+        if (has && (peers >> lane) == 1u) tab[h] = (unsigned short)(q + 1);
+        __syncwarp();
+      }
+      // a candidate counts when its first 8 bytes match (shorter copies are not emitted)
+      const bool ok = has && q + SN_MIN_MATCH <= fl && cand && ld32((int)cand - 1) == v &&
+                      ld32((int)cand + 3) == ld32(q + 4);
+      const unsigned okm = __ballot_sync(0xffffffffu, ok);
+      if (ok) s.cand[q - h0] = (unsigned short)(cand - 1);
+      if (lane == 0 && okm) s.mark[(b - h0) >> 5] = okm;
+    }
+    __syncthreads();
+    if (wid == 0) {
+      const int hend = min(h0 + SN_SUB, fl - 3);
+      while (p < hend && !s.fail) {
+        // the next marked position at or after p, 32 words of marks at a time
+        const int w0 = (p - h0) >> 5, w = w0 + lane;
+        unsigned m = w < SN_SUB / 32 ? s.mark[w] : 0u;
+        if (lane == 0) m &= 0xffffffffu << (p & 31);
+        const unsigned any = __ballot_sync(0xffffffffu, m != 0);
+        if (!any) {
+          p = min(hend, h0 + ((w0 + 32) << 5));
+          continue;
+        }
+        const int l0 = __ffs(any) - 1;
+        p = h0 + ((w0 + l0) << 5) + __ffs(__shfl_sync(0xffffffffu, m, l0)) - 1;
+        const int qs = s.cand[p - h0];
+        int L = SN_MIN_MATCH;
+        for (;;) {
+          const int a = p + L + lane;
+          const bool eq = a < fl && by[qs + L + lane] == by[a];
+          const unsigned ne = __ballot_sync(0xffffffffu, !eq);
+          if (ne) {
+            L += __ffs(ne) - 1;
+            break;
+          }
+          L += 32;
+        }
+        // pending literal
+        if (p > lit) {
+          const int len = p - lit;
+          const unsigned mm = (unsigned)len - 1u;
+          const int nb = mm < 60u ? 0 : mm < 256u ? 1 : 2;
+          if (o + 1 + nb + len + 3 * ((L + 59) / 60) > SN_FCAP) {
+            if (lane == 0) s.fail = 1;
+            __syncwarp();
+            break;
+          }
+          if (lane == 0) {
+            out[o] = (unsigned char)(nb ? (59 + nb) << 2 : mm << 2);
+            for (int i = 0; i < nb; ++i) out[o + 1 + i] = (unsigned char)(mm >> (8 * i));
+          }
+          sn_copy(out + o + 1 + nb, by + lit, len, lane, 32);
+          o += 1 + nb + len;
+        }
+        {
+          const unsigned off = (unsigned)(p - qs);
+          int rem = L;
+          while (rem >= 68) {
+            o += sn_copy_piece(out + o, off, 64, lane == 0);
+            rem -= 64;
+          }
+          if (rem > 64) {
+            o += sn_copy_piece(out + o, off, 60, lane == 0);
+            rem -= 60;
+          }
+          o += sn_copy_piece(out + o, off, rem, lane == 0);
+        }
+        p += L;
+        lit = p;
+      }
+    }
+    __syncthreads();  // the next positions overwrite marks, candidates and tables
+    if (s.fail) break;
+  }
+  if (t == 0) {
+    s.o = o;
+    s.lit = lit;
+  }
+  __syncthreads();
+  o = s.o;
+  lit = s.lit;
+  int bad = s.fail;
+  if (!bad && fl > lit) {  // the last literal, by the whole CTA
     const int len = fl - lit;
     const unsigned mm = (unsigned)len - 1u;
     const int nb = mm < 60u ? 0 : mm < 256u ? 1 : 2;
     if (o + 1 + nb + len > SN_FCAP) {
-      if (lane == 0) gb_set_error(st, GB_ERR_INTERNAL, KID_SNAPPY_C, f);
-      if (lane == 0) flout[f] = 0;
-      return;
+      bad = 1;
+    } else {
+      if (t == 0) {
+        out[o] = (unsigned char)(nb ? (59 + nb) << 2 : mm << 2);
+        for (int i = 0; i < nb; ++i) out[o + 1 + i] = (unsigned char)(mm >> (8 * i));
+      }
+      sn_copy(out + o + 1 + nb, by + lit, len, t, SN_CT);
+      o += 1 + nb + len;
     }
-    if (lane == 0) {
-      out[o] = (unsigned char)(nb ? (59 + nb) << 2 : mm << 2);
-      for (int i = 0; i < nb; ++i) out[o + 1 + i] = (unsigned char)(mm >> (8 * i));
-    }
-#pragma unroll 4
-    for (int i = lane; i < len; i += 32) out[o + 1 + nb + i] = src[lit + i];
-    o += 1 + nb + len;
   }
-  if (lane == 0) flout[f] = o;
+  if (t == 0) {
+    if (bad) gb_set_error(st, GB_ERR_INTERNAL, KID_SNAPPY_C, f);
+    flout[f] = bad ? 0 : o;
+  }
 }
 
 // Chunk preambles and fragment copies into the final stream.  One CTA per
@@ -978,9 +1181,7 @@ __global__ void k_snappy_gather(const unsigned char* __restrict__ fout, const in
                                 long long nchunks, unsigned char* __restrict__ dst) {
   const long long f = blockIdx.x;
   if (f < nfrag) {
-    const unsigned char* s = fout + f * SN_FCAP;
-    unsigned char* d = dst + fdst[f];
-    for (int i = threadIdx.x; i < flout[f]; i += blockDim.x) d[i] = s[i];
+    sn_copy(dst + fdst[f], fout + f * SN_FCAP, flout[f], threadIdx.x, blockDim.x);
   }
   if (blockIdx.x == 0)
     for (long long c = threadIdx.x; c < nchunks; c += blockDim.x) sn_put_varint(dst + pre_at[c], (unsigned long long)pre_val[c]);
@@ -1230,31 +1431,37 @@ int snap_encode(gb_context* ctx, const int4* d_boxes, long long n, int method, u
   DevMem M(c.stream);
   long long* d_rsize = M.get<long long>(nch);
   long long* d_roff = M.get<long long>(nch + 1);
-  int* d_ovf = M.get<int>(nch + 1);  // count, then the chunks that need global tables
+  int* d_ovf = M.get<int>(2 * nch + 2);  // the widths' and heights' counts of chunks that need global tables, then these
   unsigned* d_rank = M.get<unsigned>((size_t)2 * n);
-  if (!d_rsize || !d_roff || !d_ovf || !d_rank) return gbi::set_err(ctx, GB_ERR_OOM, "snap encode scratch");
-  cudaMemsetAsync(d_ovf, 0, (nch + 1) * sizeof(int), c.stream);
-  const size_t sm_s = rank_smem(false), sm_g = rank_smem(true);
-  cudaFuncSetAttribute((const void*)k_enc_rank<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s);
-  k_enc_rank<false><<<(unsigned)nch, SN_T, sm_s, c.stream>>>(d_boxes, n, nullptr, 0, nullptr, d_rank, d_ovf + 1, d_ovf,
-                                                             c.st);
-  ++c.launches;
-  int novf = 0;
-  cudaMemcpyAsync(&novf, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
-  if (cudaStreamSynchronize(c.stream) != cudaSuccess) return gbi::set_err(ctx, GB_ERR_CUDA, "snap encode (ranks)");
-  if (novf) {
-    const int gblocks = std::min(novf, std::max(1, c.nsm));
-    unsigned long long* gtab = M.get<unsigned long long>((size_t)gblocks * SN_GTAB_SLOTS);
-    if (!gtab) return gbi::set_err(ctx, GB_ERR_OOM, "snap encode tables");
-    k_enc_rank<true><<<gblocks, SN_T, sm_g, c.stream>>>(d_boxes, n, d_ovf + 1, novf, gtab, d_rank, nullptr, nullptr,
-                                                        c.st);
-    ++c.launches;
-  }
-  k_enc_emit<false><<<(unsigned)nch, SN_T, 0, c.stream>>>(d_boxes, n, d_rank, d_rsize, nullptr, nullptr, c.st);
-  ++c.launches;
+  int* d_bsize = M.get<int>((size_t)nch * SN_BPC);
+  if (!d_rsize || !d_roff || !d_ovf || !d_rank || !d_bsize) return gbi::set_err(ctx, GB_ERR_OOM, "snap encode scratch");
+  cudaMemsetAsync(d_ovf, 0, 2 * sizeof(int), c.stream);
+  const size_t sm_s = rank_smem(false), sm_g = rank_smem(true), sm_e = (size_t)SN_RB * SN_REC_MAX;
+  const unsigned eb = (unsigned)(nch * SN_BPC);
   std::vector<long long> rsize(nch), roff(nch + 1, 0);
-  cudaMemcpyAsync(rsize.data(), d_rsize, nch * 8, cudaMemcpyDeviceToHost, c.stream);
-  if (cudaStreamSynchronize(c.stream) != cudaSuccess) return gbi::set_err(ctx, GB_ERR_CUDA, "snap encode (size)");
+  int novf[2] = {0, 0};
+  auto sizes = [&]() -> bool {  // block and chunk sizes from the ranks; the chunks' to the host
+    k_enc_emit<false><<<eb, SN_RT, 0, c.stream>>>(d_boxes, n, d_rank, d_bsize, nullptr, nullptr, c.st);
+    k_enc_sizes<<<(unsigned)((nch + 7) / 8), 256, 0, c.stream>>>(d_bsize, nch, d_rsize);
+    c.launches += 2;
+    cudaMemcpyAsync(rsize.data(), d_rsize, nch * 8, cudaMemcpyDeviceToHost, c.stream);
+    return cudaStreamSynchronize(c.stream) == cudaSuccess;
+  };
+  cudaFuncSetAttribute((const void*)k_enc_rank<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s);
+  k_enc_rank<false><<<dim3((unsigned)nch, 2), SN_T, sm_s, c.stream>>>(d_boxes, n, nullptr, 0, nullptr, d_rank, d_ovf + 2,
+                                                                      d_ovf, c.st);
+  ++c.launches;
+  cudaMemcpyAsync(novf, d_ovf, sizeof(novf), cudaMemcpyDeviceToHost, c.stream);
+  if (!sizes()) return gbi::set_err(ctx, GB_ERR_CUDA, "snap encode (sizes)");
+  if (novf[0] || novf[1]) {  // the listed chunks again with global tables
+    const int gblocks = std::min(std::max(novf[0], novf[1]), std::max(1, c.nsm));
+    unsigned long long* gtab = M.get<unsigned long long>((size_t)2 * gblocks * SN_GTAB_SLOTS);
+    if (!gtab) return gbi::set_err(ctx, GB_ERR_OOM, "snap encode tables");
+    k_enc_rank<true><<<dim3(gblocks, 2), SN_T, sm_g, c.stream>>>(d_boxes, n, d_ovf + 2, (int)nch, gtab, d_rank, nullptr,
+                                                                 nullptr, c.st);
+    ++c.launches;
+    if (!sizes()) return gbi::set_err(ctx, GB_ERR_CUDA, "snap encode (sizes)");
+  }
   {
     int e = gb_sync(ctx, nullptr);
     if (e) return e;
@@ -1266,7 +1473,7 @@ int snap_encode(gb_context* ctx, const int4* d_boxes, long long n, int method, u
   if (method != 0 && !d_raw) return gbi::set_err(ctx, GB_ERR_OOM, "snap raw buffer");
   unsigned char* rawbuf = method == 0 ? d_out : d_raw;
   cudaMemcpyAsync(d_roff, roff.data(), (nch + 1) * 8, cudaMemcpyHostToDevice, c.stream);
-  k_enc_emit<true><<<(unsigned)nch, SN_T, 0, c.stream>>>(d_boxes, n, d_rank, nullptr, d_roff, rawbuf, c.st);
+  k_enc_emit<true><<<eb, SN_RT, sm_e, c.stream>>>(d_boxes, n, d_rank, d_bsize, d_roff, rawbuf, c.st);
   ++c.launches;
   if (method == 0) {
     for (long long i = 0; i < nch; ++i) {
@@ -1297,9 +1504,9 @@ int snap_encode(gb_context* ctx, const int4* d_boxes, long long n, int method, u
   if (nfrag) {
     cudaMemcpyAsync(d_fsrc, fsrc.data(), nfrag * 8, cudaMemcpyHostToDevice, c.stream);
     cudaMemcpyAsync(d_flen, flen.data(), nfrag * 4, cudaMemcpyHostToDevice, c.stream);
-    cudaFuncSetAttribute((const void*)k_snappy_compress, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 2);
-    k_snappy_compress<<<(unsigned)((nfrag + 7) / 8), 256, 8 * 2048 * 2, c.stream>>>(d_raw, d_fsrc, d_flen, nfrag, d_fout,
-                                                                                    d_flout, c.st);
+    cudaFuncSetAttribute((const void*)k_snappy_compress, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(SnapFrag));
+    k_snappy_compress<<<(unsigned)nfrag, SN_CT, sizeof(SnapFrag), c.stream>>>(d_raw, d_fsrc, d_flen, d_fout, d_flout, c.st);
     ++c.launches;
   }
   std::vector<int> flout(nfrag);
@@ -1362,7 +1569,7 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
   unsigned* d_rec = M.get<unsigned>((size_t)nch * SN_CHUNK);
   int* d_dict = M.get<int>((size_t)nch * 2 * SN_CHUNK);
   unsigned* d_seg = M.get<unsigned>(3 * nseg);  // entries, exits, counts
-  RecBlock* d_blk = M.get<RecBlock>((size_t)nch * (SN_CHUNK / SN_RB));
+  RecBlock* d_blk = M.get<RecBlock>((size_t)nch * SN_BPC);
   unsigned char* d_raw = method == 0 ? nullptr : M.get<unsigned char>((size_t)roff[nch] + 16);
   if (!d_tab || !d_rec || !d_dict || !d_seg || !d_blk || (method != 0 && !d_raw)) return gbi::set_err(ctx, GB_ERR_OOM, "snap decode scratch");
   std::vector<long long> tab(5 * (nch + 1));
@@ -1398,7 +1605,7 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
                                                                  d_seg + 2 * nseg, d_rec, c.st);
     ++c.launches;
   }
-  const unsigned rb = (unsigned)(nch * (SN_CHUNK / SN_RB));
+  const unsigned rb = (unsigned)(nch * SN_BPC);
   k_codec_decode<false><<<rb, SN_RT, 0, c.stream>>>(raw, d_roff, d_rec, n, d_dict, d_blk, d_boxes, c.st);
   k_codec_decode<true><<<rb, SN_RT, 0, c.stream>>>(raw, d_roff, d_rec, n, d_dict, d_blk, d_boxes, c.st);
   c.launches += 3;
