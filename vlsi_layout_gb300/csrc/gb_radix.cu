@@ -7,13 +7,13 @@
 //     atomics; two adjacent narrow passes share a joint table, so a shared
 //     atomic counts a key for both).
 //  2. Each pass is one kernel: a CTA takes the next tile from an atomic
-//     counter (so tiles start in order) and pulls the tile's keys and values
-//     into shared memory with two bulk asynchronous copies completing on an
-//     mbarrier.  Warps rank the keys stably (peers by shared lane masks, or
-//     warp match and per-bit ballots for wide digits), the CTA
-//     publishes its per-digit counts, and obtains the exclusive prefix of all
-//     earlier tiles by a decoupled look-back over a status array.  Keys and
-//     values are then permuted in place in shared memory by digit and
+//     counter (so tiles start in order) and pulls the tile's keys into shared
+//     memory with a bulk asynchronous copy completing on an mbarrier.  Warps
+//     rank the keys stably (peers by shared lane masks, or warp match and
+//     per-bit ballots for 10-bit digits), the CTA publishes its per-digit
+//     counts, and obtains the exclusive prefix of all earlier tiles by a
+//     decoupled look-back over a status array, under which the tile's values
+//     arrive.  Keys and values are permuted by digit in shared memory and
 //     written out in runs.
 // Digits are 1..10 bits wide; the passes split the significant key bits as
 // evenly as possible (e.g. 52 bits in 6 passes: 9,9,9,9,8,8), so the pass
@@ -168,6 +168,10 @@ __device__ __forceinline__ void rs_bulk_load(unsigned dst, const void* src, unsi
                : "memory");
 }
 
+__device__ __forceinline__ void rs_bulk_prefetch(const void* src, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ bool rs_mbar_try(unsigned a, unsigned parity) {
   unsigned ok;
   asm volatile(
@@ -178,24 +182,33 @@ __device__ __forceinline__ bool rs_mbar_try(unsigned a, unsigned parity) {
   return ok != 0;
 }
 
-// bounded wait for phase 0 of the mbarrier; false after `limit` polls
-__device__ __forceinline__ bool rs_mbar_wait(unsigned a, int limit) {
+// bounded wait for a phase of the mbarrier; false after `limit` polls
+__device__ __forceinline__ bool rs_mbar_wait(unsigned a, unsigned parity, int limit) {
   for (int i = 0; i < limit; ++i)
-    if (rs_mbar_try(a, 0)) return true;
+    if (rs_mbar_try(a, parity)) return true;
   return false;
 }
 
 // ---------------------------------------------------------------- one pass
 // Radices up to RS_AO_RADIX find a key's peers through per-warp lane masks in
 // shared memory (one word per digit); larger ones by warp match / ballots.
-#define RS_AO_RADIX 128
+#define RS_AO_RADIX 512
 
 // Shared memory of a pass with NT threads, tile T = NT * IT keys and radix R:
-//   keys T*8 | vals T*4 | wh[NT/32][R] u16 | bstart[R] u32 | gpos[R] u32 | mbarrier, tile, scan scratch
-//   | lane masks [NT/32][R] u32 when R <= RS_AO_RADIX
+//   keys T*8 | vals T*4 | gpos[R] u32 | mbarrier, tile, scan scratch
+// A warp's lane masks lie in its own part of the keys (32 * IT * 8 bytes),
+// which are in registers by then, and the warp counters wh[NT/32][R] u16 in
+// the values, which are loaded after the counters' last use: two CTAs of 8192
+// keys fit an SM for digits of up to 9 bits.  Masks and counters beside the
+// tile had kept such digits to one, so 52-bit keys took 8 passes of 7 and 6
+// bits (60M keys: 3070 us) and now take 6 of 9 and 8 (2517 us; 64-bit
+// keys 3775 -> 3080 us).
+// Counters that do not fit the values (10-bit digits of 12-key threads)
+// follow the scan scratch.
+__host__ __device__ constexpr bool rs_wh_inside(int it, int radix) { return radix <= 64 * it; }
 __host__ __device__ constexpr size_t rs_smem_bytes(int nt, int it, int radix) {
-  return (size_t)nt * it * 12 + (size_t)(nt / 32) * radix * 2 + (size_t)radix * 8 + 16 + 33 * 8 +
-         (radix <= RS_AO_RADIX ? (size_t)(nt / 32) * radix * 4 : 0);
+  return (size_t)nt * it * 12 + (size_t)radix * 4 + 16 + 33 * 8 +
+         (rs_wh_inside(it, radix) ? 0 : (size_t)(nt / 32) * radix * 2);
 }
 
 // The digit [shift, shift + dbits) of a key, taken from its two 32-bit words
@@ -211,44 +224,52 @@ struct RsDigit {
   }
 };
 
-// The work on a tile resident in shared memory: rank, prefix, permutation,
-// look-back and write-out.  FULL: the tile holds TILE keys (no bounds tests).
-template <int NT, int IT, int MAXB, bool FULL>
-__device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, unsigned short* wh, unsigned* bstart,
-                                        unsigned* gpos, long long* tmp, unsigned* mbuf, const RsDigit& digit,
-                                        int radix, int cnt,
-                                        long long tile, long long ntile, const unsigned* __restrict__ gofs,
-                                        unsigned long long* status, unsigned long long epoch, DStatus* st,
-                                        int spin_limit, unsigned long long* __restrict__ kout,
-                                        unsigned* __restrict__ vout) {
+// The work on a tile whose keys are in shared memory: rank, prefix,
+// permutation, look-back and write-out.  vin: the tile's values in global
+// memory.  FULL: the tile holds TILE keys (no bounds tests).
+template <int NT, int IT, bool AO, bool FULL>
+__device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, unsigned short* wh, unsigned* gpos,
+                                        long long* tmp, const RsDigit& digit, int radix, int cnt,
+                                        const unsigned* __restrict__ vin, unsigned mb, int bulk, long long tile,
+                                        const unsigned* __restrict__ gofs, unsigned long long* status,
+                                        unsigned long long epoch, DStatus* st, int spin_limit,
+                                        unsigned long long* __restrict__ kout, unsigned* __restrict__ vout) {
   constexpr int TILE = NT * IT;
   constexpr int NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  // ---- rank: warp w owns keys [w*32*IT, (w+1)*32*IT) in order.  Peers with
-  // the same digit are found through shared lane masks (radix <= RS_AO_RADIX)
-  // or by a warp match (every third item) and one ballot per digit bit (the
-  // others), so the match unit and the integer pipe share the work; the lowest peer adds the group to the warp's counter (two 16-bit counters share a 32-bit
-  // word; a count never exceeds 32*IT, so no carry crosses halves) and
-  // broadcasts the old value.  Keys stay in registers; ranks are packed two
-  // to a register.
+  // ---- rank: warp w owns keys [w*32*IT, (w+1)*32*IT) in order, all loaded into registers first.  Peers with
+  // the same digit are found through shared lane masks (AO; in the place of the warp's own keys) or by a warp match
+  // (every third item) and one ballot per digit bit (the others), so the match unit and the integer pipe share the
+  // work; the lowest peer adds the group to the warp's counter (two 16-bit counters share a 32-bit word; a count
+  // never exceeds 32*IT, so no carry crosses halves) and broadcasts the old value.  Ranks are packed two to a
+  // register.
   const unsigned lt = (1u << lane) - 1u;
   const int wbase = wid * 32 * IT;
   unsigned short* mywh = wh + wid * radix;
   unsigned* mywh32 = reinterpret_cast<unsigned*>(mywh);
+  unsigned* mm = reinterpret_cast<unsigned*>(sk + wbase);
   unsigned long long kk[IT];
   unsigned rd[(IT + 1) / 2];
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     const int idx = wbase + it * 32 + lane;
+    kk[it] = FULL || idx < cnt ? sk[idx] : 0ull;
+  }
+  if (AO) {
+    __syncwarp();
+    for (int i = lane; i < radix; i += 32) mm[i] = 0u;
+    __syncwarp();
+  }
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int idx = wbase + it * 32 + lane;
     const bool ok = FULL || idx < cnt;
-    kk[it] = ok ? sk[idx] : 0ull;
     const unsigned d = digit(kk[it]);
     unsigned peers;
-    if (radix <= RS_AO_RADIX) {
+    if (AO) {
       // lane masks: each lane ORs its bit into its warp's word for its digit
       // and reads the word back (shared-memory pipe, no votes); the peers
       // then clear it for the next item
-      unsigned* mm = mbuf + wid * radix;
       if (ok) atomicOr(&mm[d], 1u << lane);
       __syncwarp();
       peers = ok ? mm[d] : 0u;
@@ -270,7 +291,7 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
         peers = ok ? vm : ~vm;
       }
 #pragma unroll
-      for (int b = 0; b < MAXB; ++b) {
+      for (int b = 0; b < 10; ++b) {
         const unsigned bit = (d >> b) & 1u;
         const unsigned bb = __ballot_sync(0xffffffffu, bit);
         peers &= bit ? bb : ~bb;
@@ -288,17 +309,18 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
 
   // ---- per digit: tile total (published as the tile's aggregate), the
   // tile's bucket start, and each warp's first slot of the digit, folded
-  // into the warp counters (loops over a thread's digits run to the
-  // compile-time bound 4 so the per-digit arrays stay in registers)
-  const int dpt = radix > NT ? radix / NT : 1;  // digits per thread (1..4)
+  // into the warp counters (loops over a thread's digits run to a
+  // compile-time bound so the per-digit arrays stay in registers)
+  constexpr int DPT = (AO ? RS_AO_RADIX : 1024) / NT;  // digits per thread at most: 1, 2 or 4
+  const int dpt = DPT > 1 && radix > NT ? radix / NT : 1;  // digits per thread
   const int d0 = tid * dpt;
   const bool own = d0 < radix;
-  unsigned tots[4] = {0u, 0u, 0u, 0u};
-  long long tsum = 0;
+  unsigned tots[DPT];
+  int tsum = 0;
   const unsigned long long etag = (epoch & 0xFFFFull) << 48;
   if (own) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < DPT; ++j) {
       if (j < dpt) {
         const int d = d0 + j;
         unsigned tot = 0;
@@ -306,21 +328,20 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
         for (int w = 0; w < NW; ++w) tot += wh[w * radix + d];
         tots[j] = tot;
         tsum += tot;
-        gpos[d] = tot;  // kept for the look-back, which replaces it
         const unsigned long long flag = tile == 0 ? RS_FLAG_PRE : RS_FLAG_AGG;
         *(volatile unsigned long long*)(status + (size_t)tile * radix + d) = etag | (flag << 46) | tot;
       }
     }
   }
   {
-    long long tt;
-    long long ex = gb_block_excl(tsum, tmp, &tt);
+    int tt;
+    int ex = gb_block_excl(tsum, reinterpret_cast<int*>(tmp), &tt);
     if (own) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < DPT; ++j) {
         if (j < dpt) {
           const int d = d0 + j;
-          bstart[d] = (unsigned)ex;
+          gpos[d] = (unsigned)ex;  // the bucket's start in the tile, until the look-back replaces it
           unsigned run = (unsigned)ex;
 #pragma unroll
           for (int w = 0; w < NW; ++w) {
@@ -337,7 +358,8 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
 
   // ---- permute in place: every read of the key array happened before the
   // last barrier, so keys go straight from registers to their slots; rd
-  // becomes the slot pair.  Values: all reads, a barrier, then the writes.
+  // becomes the slot pair.  Then the warp counters are dead and the values
+  // come into their place, under the look-back.
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     if (FULL || wbase + it * 32 + lane < cnt) {
@@ -348,17 +370,18 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
       rd[it >> 1] = (it & 1) ? ((rd[it >> 1] & 0xFFFFu) | (p << 16)) : ((rd[it >> 1] & 0xFFFF0000u) | p);
     }
   }
-  {
-    unsigned vv[IT];
-#pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      const int idx = wbase + it * 32 + lane;
-      if (FULL || idx < cnt) vv[it] = sv[idx];
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the counters' accesses before the copy over them
+  __syncthreads();
+  if (bulk) {
+    const int cb = cnt & ~3;
+    if (tid == 0) {
+      rs_mbar_expect(mb, (unsigned)cb * 4u);
+      if (cb > 0) rs_bulk_load(rs_smem(sv), vin, (unsigned)cb * 4u, mb);
     }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < IT; ++it)
-      if (FULL || wbase + it * 32 + lane < cnt) sv[(it & 1) ? (rd[it >> 1] >> 16) : (rd[it >> 1] & 0xFFFFu)] = vv[it];
+    if (!FULL)
+      for (int i = cb + tid; i < cnt; i += NT) sv[i] = vin[i];
+  } else {
+    for (int i = tid; i < cnt; i += NT) sv[i] = vin[i];
   }
 
   // ---- decoupled look-back: the thread of digit d polls the status words of
@@ -368,7 +391,7 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
   if (own) {
     constexpr int DEPTH = RS_LBDEPTH;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < DPT; ++j) {
       if (j < dpt) {
         const int d = d0 + j;
         unsigned excl = 0;
@@ -403,9 +426,27 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
           *(volatile unsigned long long*)(status + (size_t)tile * radix + d) =
               etag | (RS_FLAG_PRE << 46) | (unsigned long long)(excl + tots[j]);
         }
-        gpos[d] = gofs[d] + excl - bstart[d];  // modulo 2^32: slot + gpos < n < 2^32
+        gpos[d] = gofs[d] + excl - gpos[d];  // modulo 2^32: slot + gpos < n < 2^32
       }
     }
+  }
+  // ---- the values: all reads, a barrier, then the writes to their slots
+  if (bulk && !rs_mbar_wait(mb, 1, spin_limit)) {
+    gb_set_error(st, GB_ERR_TIMEOUT, KID_RADIX_COPY, tile);
+    rs_mbar_wait(mb, 1, RS_SPIN_LIMIT);  // let the copy land before its place is used
+  }
+  if (!FULL || !bulk) __syncthreads();  // values stored by other threads
+  {
+    unsigned vv[IT];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int idx = wbase + it * 32 + lane;
+      if (FULL || idx < cnt) vv[it] = sv[idx];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < IT; ++it)
+      if (FULL || wbase + it * 32 + lane < cnt) sv[(it & 1) ? (rd[it >> 1] >> 16) : (rd[it >> 1] & 0xFFFFu)] = vv[it];
   }
   __syncthreads();
   // ---- write runs: consecutive threads write consecutive slots of a digit's run
@@ -417,8 +458,8 @@ __device__ __forceinline__ void rs_tile(unsigned long long* sk, unsigned* sv, un
   }
 }
 
-// NT threads, IT keys per thread; digits of at most MAXB bits; n < 2^32.
-template <int NT, int IT, int MAXB>
+// NT threads, IT keys per thread; AO: radix <= RS_AO_RADIX; n < 2^32.
+template <int NT, int IT, bool AO>
 __global__ void __launch_bounds__(NT, NT == 512 ? 2 : (IT <= 12 ? 4 : 3))
 k_rs_pass(const unsigned long long* __restrict__ kin, const unsigned* __restrict__ vin,
           unsigned long long* __restrict__ kout, unsigned* __restrict__ vout, long long n, int shift, int dbits,
@@ -431,13 +472,11 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const unsigned* __restrict
   const RsDigit digit(shift, (unsigned)radix - 1u);
   unsigned long long* sk = reinterpret_cast<unsigned long long*>(smraw);
   unsigned* sv = reinterpret_cast<unsigned*>(sk + TILE);
-  unsigned short* wh = reinterpret_cast<unsigned short*>(sv + TILE);  // [NW][radix]
-  unsigned* bstart = reinterpret_cast<unsigned*>(wh + NW * radix);
-  unsigned* gpos = bstart + radix;
+  unsigned* gpos = sv + TILE;
   unsigned long long* mbar = reinterpret_cast<unsigned long long*>(gpos + radix);
   long long* stile = reinterpret_cast<long long*>(mbar + 1);
   long long* tmp = stile + 1;  // [33]
-  unsigned* mbuf = reinterpret_cast<unsigned*>(tmp + 33);  // [NW][radix] lane masks (radix <= RS_AO_RADIX)
+  unsigned short* wh = reinterpret_cast<unsigned short*>(rs_wh_inside(IT, radix) ? (void*)sv : (void*)(tmp + 33));  // [NW][radix]
   const int tid = threadIdx.x;
   const long long ntile = (n + TILE - 1) / TILE;
   const unsigned mb = rs_smem(mbar);
@@ -449,46 +488,38 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const unsigned* __restrict
       const long long tb = t * TILE;
       const int cb = (int)min((long long)TILE, n - tb) & ~3;  // bulk part: whole 16-byte groups
       rs_mbar_init(mb);
-      rs_mbar_expect(mb, (unsigned)cb * 12u);
+      rs_mbar_expect(mb, (unsigned)cb * 8u);
       if (cb > 0) {
         rs_bulk_load(rs_smem(sk), kin + tb, (unsigned)cb * 8u, mb);
-        rs_bulk_load(rs_smem(sv), vin + tb, (unsigned)cb * 4u, mb);
+        rs_bulk_prefetch(vin + tb, (unsigned)cb * 4u);  // the values are read after the ranking
       }
     }
   }
   for (int i = tid; i < NW * radix / 2; i += NT) reinterpret_cast<unsigned*>(wh)[i] = 0u;
-  if (radix <= RS_AO_RADIX)
-    for (int i = tid; i < NW * radix; i += NT) mbuf[i] = 0u;
   __syncthreads();
   const long long tile = *stile;
   if (tile >= ntile) return;
   const long long tb = tile * TILE;
   const int cnt = (int)min((long long)TILE, n - tb);
   if (bulk) {
-    for (int i = (cnt & ~3) + tid; i < cnt; i += NT) {
-      sk[i] = kin[tb + i];
-      sv[i] = vin[tb + i];
-    }
-    const bool ok = rs_mbar_wait(mb, spin_limit);
+    for (int i = (cnt & ~3) + tid; i < cnt; i += NT) sk[i] = kin[tb + i];
+    const bool ok = rs_mbar_wait(mb, 0, spin_limit);
     if (__syncthreads_or(!ok)) {
       if (tid == 0) gb_set_error(st, GB_ERR_TIMEOUT, KID_RADIX_COPY, tile);
-      rs_mbar_wait(mb, spin_limit);  // let copies in flight land before the CTA exits
+      rs_mbar_wait(mb, 0, RS_SPIN_LIMIT);  // let copies in flight land before the CTA exits
       return;
     }
   } else {
-    for (int i = tid; i < cnt; i += NT) {
-      sk[i] = kin[tb + i];
-      sv[i] = vin[tb + i];
-    }
+    for (int i = tid; i < cnt; i += NT) sk[i] = kin[tb + i];
     __syncthreads();
   }
 
   if (cnt == TILE)
-    rs_tile<NT, IT, MAXB, true>(sk, sv, wh, bstart, gpos, tmp, mbuf, digit, radix, cnt, tile, ntile, gofs, status, epoch, st,
-                            spin_limit, kout, vout);
+    rs_tile<NT, IT, AO, true>(sk, sv, wh, gpos, tmp, digit, radix, cnt, vin + tb, mb, bulk, tile, gofs, status, epoch, st,
+                              spin_limit, kout, vout);
   else
-    rs_tile<NT, IT, MAXB, false>(sk, sv, wh, bstart, gpos, tmp, mbuf, digit, radix, cnt, tile, ntile, gofs, status, epoch, st,
-                             spin_limit, kout, vout);
+    rs_tile<NT, IT, AO, false>(sk, sv, wh, gpos, tmp, digit, radix, cnt, vin + tb, mb, bulk, tile, gofs, status, epoch, st,
+                               spin_limit, kout, vout);
 }
 
 __global__ void k_rs_zero(unsigned* p, int n, long long* ctrs, int nc) {
@@ -513,16 +544,12 @@ using PassFn = void (*)(const unsigned long long*, const unsigned*, unsigned lon
 
 struct RsKernel {
   int nt, it;
-  PassFn fn[4];  // digits of at most 6, 7, 8, 10 bits
+  PassFn fn[2];  // digits of at most 9 bits, 10 bits
   int tile() const { return nt * it; }
 };
-const RsKernel kKernels[] = {
-    {256, 12, {k_rs_pass<256, 12, 6>, k_rs_pass<256, 12, 7>, k_rs_pass<256, 12, 8>, k_rs_pass<256, 12, 10>}},
-    {256, 16, {k_rs_pass<256, 16, 6>, k_rs_pass<256, 16, 7>, k_rs_pass<256, 16, 8>, k_rs_pass<256, 16, 10>}},
-    {256, 20, {k_rs_pass<256, 20, 6>, k_rs_pass<256, 20, 7>, k_rs_pass<256, 20, 8>, k_rs_pass<256, 20, 10>}},
-    {512, 12, {k_rs_pass<512, 12, 6>, k_rs_pass<512, 12, 7>, k_rs_pass<512, 12, 8>, k_rs_pass<512, 12, 10>}},
-    {512, 16, {k_rs_pass<512, 16, 6>, k_rs_pass<512, 16, 7>, k_rs_pass<512, 16, 8>, k_rs_pass<512, 16, 10>}},
-};
+#define RS_KERNEL(NT, IT) {NT, IT, {k_rs_pass<NT, IT, true>, k_rs_pass<NT, IT, false>}}
+const RsKernel kKernels[] = {RS_KERNEL(256, 12), RS_KERNEL(256, 16), RS_KERNEL(256, 20), RS_KERNEL(512, 12),
+                             RS_KERNEL(512, 16)};
 
 // the kernel whose tile holds `tile` keys
 const RsKernel* kernel_for(int tile) {
@@ -531,7 +558,7 @@ const RsKernel* kernel_for(int tile) {
   return nullptr;
 }
 
-PassFn pass_fn(const RsKernel* K, int dbits) { return K->fn[dbits <= 6 ? 0 : dbits == 7 ? 1 : dbits == 8 ? 2 : 3]; }
+PassFn pass_fn(const RsKernel* K, int dbits) { return K->fn[(1 << dbits) <= RS_AO_RADIX ? 0 : 1]; }
 
 RsState* state_of(GbCtx& c) {
   if (!c.rs) c.rs = new RsState();
@@ -603,10 +630,6 @@ void gb_radix_free(GbCtx& c) {
   c.rs = nullptr;
 }
 
-// Default configuration for a sort of `bits` significant bits: the fewest
-// passes with digits of at most 7 bits (radix <= RS_AO_RADIX ranks through
-// shared lane masks), one more when that makes the count even (it moves as
-// many bytes as the final copy it saves), tiles of 8192 keys.
 // The plan gb_radix_sort_pairs takes for `bits` significant bits and n keys
 // on `device`: the tuned one for that bit width and size class, else the
 // default.
@@ -627,8 +650,13 @@ extern "C" int gb_radix_plan(int device, int bits, long long n, int* passes, int
   return GB_OK;
 }
 
+// Default configuration for a sort of `bits` significant bits: the fewest
+// passes with digits of at most 9 bits (ranked through shared lane masks, two
+// CTAs of 8192 keys per SM), one more when that makes the count even (it
+// moves as many bytes as the final copy it saves).  60M keys: 398 us for a
+// pass of 8 or 9 bits, 330 us for one of 6 or 7, so fewer passes win.
 void gb_radix_default(int bits, int* passes, int* tile) {
-  int p = (bits + 6) / 7;
+  int p = (bits + 8) / 9;
   if ((p & 1) && p + 1 <= bits) ++p;
   *passes = std::max(1, p);
   *tile = 8192;
@@ -678,11 +706,11 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
     cudaMemsetAsync(S->status, 0, want * 8, c.stream);
     S->status_words = want;
   }
-  // passes of different digit widths lay shared memory out differently (the
-  // lane masks exist only for radix <= RS_AO_RADIX): size for the largest
+  // passes of different digit widths lay shared memory out differently: size
+  // for the largest
   size_t smem = 0;
   for (int p = 0; p < passes; ++p) smem = std::max(smem, rs_smem_bytes(K->nt, K->it, 1 << plan.bits[p]));
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 2; ++i) {
     cudaFuncSetAttribute((const void*)K->fn[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute((const void*)K->fn[i], cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   }
@@ -693,7 +721,8 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
   {
     const size_t hsm = (size_t)hplan.words * sizeof(unsigned);
     const long long want_blocks = (n / RS_HIST_KPT + 1023) / 1024;
-    const unsigned hb = (unsigned)std::max(1ll, std::min<long long>(c.nsm, want_blocks));
+    // one CTA per SM with joint tables, two when the counters leave the room
+    const unsigned hb = (unsigned)std::max(1ll, std::min<long long>(hsm <= 96 * 1024 ? 2 * c.nsm : c.nsm, want_blocks));
     const void* hf = !((uintptr_t)keys & 15u) ? (const void*)k_rs_hist<true> : (const void*)k_rs_hist<false>;
     cudaFuncSetAttribute(hf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
     if (!((uintptr_t)keys & 15u))
@@ -814,8 +843,8 @@ int gb_radix_lookback_timeout_probe(GbCtx& c, int spin_limit) {
   cudaMemsetAsync(gofs, 0, 256 * 4, c.stream);
   k_rs_set_counter<<<1, 1, 0, c.stream>>>(ctr, 1);
   const size_t smem = rs_smem_bytes(NT, IT, 256);
-  cudaFuncSetAttribute((const void*)k_rs_pass<NT, IT, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_rs_pass<NT, IT, 8><<<1, NT, smem, c.stream>>>(k, v, k2, v2, n, 0, 8, gofs, status, 7, ctr, c.st, spin_limit,
+  cudaFuncSetAttribute((const void*)k_rs_pass<NT, IT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_rs_pass<NT, IT, true><<<1, NT, smem, c.stream>>>(k, v, k2, v2, n, 0, 8, gofs, status, 7, ctr, c.st, spin_limit,
                                                    1);
   const cudaError_t e = cudaStreamSynchronize(c.stream);
   cudaFree(k); cudaFree(k2); cudaFree(v); cudaFree(v2); cudaFree(status); cudaFree(gofs); cudaFree(ctr);
