@@ -200,7 +200,8 @@ int gb_morton_sort(gb_context* ctx, c_box* boxes, long long n, int sort_boxes,
  * in d_keys / d_vals.  The pass count and keys per thread come from the
  * autotuner's table when it holds this device, bit width and size class,
  * else from the default (digits of at most 9 bits, an even pass count when
- * that costs no extra pass of bytes, tiles of 8192 keys).  n < 2^32.  Returns the number
+ * that costs no extra pass of bytes, tiles of 4096, 6144 or 8192 keys by n;
+ * up to 8192 keys are sorted by one CTA).  n < 2^32.  Returns the number
  * of passes (>= 0) or minus a GB_ERR_* status.  Asynchronous on the context stream.
  * Replaces the Thrust radix sorts of gpu_morton.cu:149-187 and
  * event_sorter.cu:64-81 on device-resident data. */
@@ -225,7 +226,7 @@ void gb_radix_tuning_reset(void);
 /* The plan (pass count, keys per tile) the device sort takes for `bits`
  * significant key bits and n keys on `device`: the tuned one for that bit
  * width and size class, else the default (fewest passes of at most 9 bits,
- * rounded up to an even count; 8192-key tiles).  For byte accounting. */
+ * rounded up to an even count; tiles by n).  For byte accounting. */
 int gb_radix_plan(int device, int bits, long long n, int* passes, int* tile);
 /* Morton keys of device boxes (gpu_morton.cu:113-144) and the identity
  * permutation, on the device. */

@@ -105,3 +105,35 @@ def test_snap_sizes(ctx, oracle, case, method):
     chunks = ctx.compress_boxes_to_stream(b, method)
     assert [c[3] for c in chunks] == [c[3] for c in oracle.stream_encode(b, method)]
     assert np.array_equal(ctx.decompress_stream_to_boxes(chunks, method), b)
+
+
+# one CTA up to 8192 keys, tiles of 4096, 6144 and 8192 above; digits of 1 to 9 bits
+@pytest.mark.parametrize("n", [2, 31, 512, 513, 8191, 8192, 8193, 65535, 65536, (1 << 21) - 1, 1 << 21])
+@pytest.mark.parametrize("bits", [1, 9, 10, 19, 52, 64])
+def test_radix_sizes(ctx, n, bits):
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n + bits)
+    k = rng.integers(0, 1 << 63, n, dtype=np.uint64) << np.uint64(1) | rng.integers(0, 2, n, dtype=np.uint64)
+    v = rng.permutation(n).astype(np.uint32)
+    order = np.argsort(k & np.uint64((1 << bits) - 1), kind="stable")
+    dk, dv = torch.from_numpy(k.view(np.int64)).cuda(), torch.from_numpy(v.view(np.int32)).cuda()
+    tk, tv = torch.empty_like(dk), torch.empty_like(dv)
+    torch.cuda.synchronize()
+    ctx.radix_sort_device(dk.data_ptr(), dv.data_ptr(), n, bits, tk.data_ptr(), tv.data_ptr())
+    ctx.sync()
+    assert np.array_equal(dk.cpu().numpy().view(np.uint64), k[order])
+    assert np.array_equal(dv.cpu().numpy().view(np.uint32), v[order])
+
+
+@pytest.mark.parametrize("n", [2, 8192, 100_003])
+@pytest.mark.parametrize("lo,hi", [((0, 0), (40_000_000, 40_000_000)), ((-2**31, -2**31), (2**31 - 1, 2**31 - 1)),
+                                   ((-5, 7), (-4, 8)), ((-70_000, 3), (80_000, 4)), ((9, -300), (10, 300))])
+def test_event_ranges(n, lo, hi):
+    from vlsi_layout_gb300 import engine
+    rng = np.random.default_rng(n)
+    t = np.zeros(n, engine.TRACKER_DTYPE)
+    t["X"], t["Y"] = rng.integers(lo[0], hi[0], n), rng.integers(lo[1], hi[1], n)
+    t["polygonNumber"] = rng.integers(-128, 128, n)
+    t["pad"] = rng.integers(-128, 128, (n, 3))
+    exp = t[np.lexsort((t["Y"], t["X"]))]
+    assert engine.event_sort(t).tobytes() == exp.tobytes()

@@ -157,7 +157,7 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
                         unsigned long long* keys_tmp, unsigned* vals_tmp, int passes = 0, int items = 0);
 int gb_radix_tune(GbCtx& c, const unsigned long long* keys, const unsigned* vals, long long n, int bits,
                       int* best_passes, int* best_items, float* best_ms);
-void gb_radix_default(int bits, int* passes, int* items);
+void gb_radix_default(int bits, long long n, int* passes, int* tile);
 void gb_radix_forget_tuning();
 void gb_radix_free(GbCtx& c);
 

@@ -70,8 +70,9 @@ struct RsHistPlan {
 template <bool VEC>
 __global__ void __launch_bounds__(1024, 1)
 k_rs_hist(const unsigned long long* __restrict__ keys, long long n, RsPlan plan, RsHistPlan hp,
-          unsigned* __restrict__ ghist) {
+          unsigned* __restrict__ ghist, unsigned long long* ticket) {
   extern __shared__ unsigned hj[];
+  __shared__ bool last;
   const int ng = hp.ng;
   for (int i = threadIdx.x; i < hp.words; i += blockDim.x) hj[i] = 0;
   __syncthreads();
@@ -133,18 +134,25 @@ k_rs_hist(const unsigned long long* __restrict__ keys, long long n, RsPlan plan,
       if (lane == 0 && v) atomicAdd(&ghist[plan.off[p + 1] + e], v);
     }
   }
-}
-
-// one block of 1024 threads per pass: exclusive scan of the pass's digit counts
-__global__ void __launch_bounds__(1024) k_rs_hist_scan(unsigned* ghist, RsPlan plan) {
-  __shared__ long long tmp[33];
-  const int p = blockIdx.x;
+  // the last block to finish turns the counts into exclusive prefixes, a warp per pass
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
+  __syncthreads();
+  const int p = threadIdx.x >> 5;
+  if (!last || p >= plan.np) return;
+  __threadfence();
   const int radix = 1 << plan.bits[p];
   unsigned* g = ghist + plan.off[p];
-  const long long v = threadIdx.x < radix ? g[threadIdx.x] : 0;
-  long long tot;
-  const long long ex = gb_block_excl(v, tmp, &tot);
-  if (threadIdx.x < radix) g[threadIdx.x] = (unsigned)ex;
+  unsigned carry = 0;
+  for (int d0 = 0; d0 < radix; d0 += 32) {
+    const int d = d0 + lane;
+    const unsigned v = d < radix ? __ldcg(&g[d]) : 0u;
+    unsigned tot;
+    const unsigned ex = gb_warp_excl(v, &tot);
+    if (d < radix) g[d] = carry + ex;
+    carry += tot;
+  }
 }
 
 // ---------------------------------------------------------------- async copy helpers
@@ -522,6 +530,100 @@ k_rs_pass(const unsigned long long* __restrict__ kin, const unsigned* __restrict
                                spin_limit, kout, vout);
 }
 
+// A sort of at most RS_ONE keys in one CTA: all passes in shared memory, one
+// launch (the zeroing, the histogram and a launch per pass, each a few
+// microseconds of latency, took 73 us for 1000 keys of 52 bits and 81 us for
+// 8192, this 22 and 44 us).
+// Ranking as in rs_tile; digits of at most 9 bits.
+#define RS_ONE 8192
+#define RS_ONE_NT 512
+#define RS_ONE_SMEM (RS_ONE * 12 + RS_ONE_NT / 32 * RS_AO_RADIX * 2)
+__global__ void __launch_bounds__(RS_ONE_NT, 1)
+k_rs_one(unsigned long long* __restrict__ keys, unsigned* __restrict__ vals, int n, RsPlan plan) {
+  constexpr int NT = RS_ONE_NT, IT = RS_ONE / RS_ONE_NT, NW = NT / 32;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  __shared__ int tmp[33];
+  unsigned long long* sk = reinterpret_cast<unsigned long long*>(smraw);
+  unsigned* sv = reinterpret_cast<unsigned*>(sk + RS_ONE);
+  unsigned short* wh = reinterpret_cast<unsigned short*>(sv + RS_ONE);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  // the warps share the keys evenly, in order: items per lane, first key of the warp
+  const int items = (n + NT - 1) / NT, wbase = wid * 32 * items;
+  for (int i = tid; i < n; i += NT) {
+    sk[i] = keys[i];
+    sv[i] = vals[i];
+  }
+  __syncthreads();
+  for (int p = 0; p < plan.np; ++p) {
+    const int radix = 1 << plan.bits[p];
+    const RsDigit digit(plan.shift[p], (unsigned)radix - 1u);
+    unsigned short* mywh = wh + wid * radix;
+    unsigned* mywh32 = reinterpret_cast<unsigned*>(mywh);
+    unsigned* mm = reinterpret_cast<unsigned*>(sk + wid * 32 * IT);  // lane masks, in the place of keys held in registers
+    unsigned long long kk[IT];
+    unsigned vv[IT], rd[IT];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int idx = wbase + it * 32 + lane;
+      if (it < items && idx < n) {
+        kk[it] = sk[idx];
+        vv[it] = sv[idx];
+      }
+    }
+    __syncthreads();  // masks may lie in other warps' keys
+    for (int i = lane; i < radix; i += 32) mm[i] = 0u;
+    for (int i = lane; i < radix / 2; i += 32) mywh32[i] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      if (it >= items) break;
+      const bool ok = wbase + it * 32 + lane < n;
+      const unsigned d = ok ? digit(kk[it]) : 0u;
+      if (ok) atomicOr(&mm[d], 1u << lane);
+      __syncwarp();
+      unsigned peers = ok ? mm[d] : 0u;
+      const unsigned vm = __ballot_sync(0xffffffffu, ok);
+      if (!ok) peers = ~vm;
+      __syncwarp();
+      if (ok) mm[d] = 0u;
+      __syncwarp();
+      const int leader = __ffs(peers) - 1;
+      unsigned old = 0;
+      if (ok && lane == leader) old = atomicAdd(&mywh32[d >> 1], (unsigned)__popc(peers) << ((d & 1u) * 16));
+      old = __shfl_sync(0xffffffffu, old, leader);
+      rd[it] = ((old >> ((d & 1u) * 16)) & 0xFFFFu) + __popc(peers & lt);
+    }
+    __syncthreads();
+    int tot = 0, all;
+    if (tid < radix)
+#pragma unroll
+      for (int w = 0; w < NW; ++w) tot += wh[w * radix + tid];
+    int run = gb_block_excl(tot, tmp, &all);
+    if (tid < radix)
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const int c = wh[w * radix + tid];
+        wh[w * radix + tid] = (unsigned short)run;
+        run += c;
+      }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      if (it < items && wbase + it * 32 + lane < n) {
+        const unsigned q = mywh[digit(kk[it])] + rd[it];
+        sk[q] = kk[it];
+        sv[q] = vv[it];
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < n; i += NT) {
+    keys[i] = sk[i];
+    vals[i] = sv[i];
+  }
+}
+
 __global__ void k_rs_zero(unsigned* p, int n, long long* ctrs, int nc) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = 0;
   if (threadIdx.x < nc) ctrs[threadIdx.x] = 0;
@@ -644,7 +746,7 @@ extern "C" int gb_radix_plan(int device, int bits, long long n, int* passes, int
       ti = f->second.second;
     }
   }
-  if (!tp) gb_radix_default(bits, &tp, &ti);
+  if (!tp) gb_radix_default(bits, n, &tp, &ti);
   *passes = std::min(tp, bits);
   *tile = ti;
   return GB_OK;
@@ -655,11 +757,13 @@ extern "C" int gb_radix_plan(int device, int bits, long long n, int* passes, int
 // CTAs of 8192 keys per SM), one more when that makes the count even (it
 // moves as many bytes as the final copy it saves).  60M keys: 398 us for a
 // pass of 8 or 9 bits, 330 us for one of 6 or 7, so fewer passes win.
-void gb_radix_default(int bits, int* passes, int* tile) {
+// Smaller tiles where 8192 keys leave SMs idle (52 bits: 30000 keys 94 us with
+// 8192-key tiles, 79 with 4096; 700000 keys 120 us, 111 with 6144; 3M equal).
+void gb_radix_default(int bits, long long n, int* passes, int* tile) {
   int p = (bits + 8) / 9;
   if ((p & 1) && p + 1 <= bits) ++p;
   *passes = std::max(1, p);
-  *tile = 8192;
+  *tile = n < 65536 ? 4096 : n < (1 << 21) ? 6144 : 8192;
 }
 
 int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long long n, int bits,
@@ -668,6 +772,7 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
   if (n >= (1ll << 32)) return -1;  // slots and values are 32-bit
   if (bits < 1) bits = 1;
   if (bits > 64) bits = 64;
+  const bool given = passes > 0 || tile > 0;  // an explicit configuration runs as it is
   if (passes <= 0 || tile <= 0) {
     int tp = 0, ti = 0;
     {
@@ -678,7 +783,7 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
         ti = f->second.second;
       }
     }
-    if (!tp) gb_radix_default(bits, &tp, &ti);
+    if (!tp) gb_radix_default(bits, n, &tp, &ti);
     if (passes <= 0) passes = tp;
     if (tile <= 0) tile = ti;
   }
@@ -688,13 +793,19 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
   if (!K) return -1;
   RsPlan plan;
   make_plan(bits, passes, plan);
+  if (n <= RS_ONE && !given && (1 << plan.bits[0]) <= RS_AO_RADIX) {
+    cudaFuncSetAttribute((const void*)k_rs_one, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_ONE_SMEM);
+    k_rs_one<<<1, RS_ONE_NT, RS_ONE_SMEM, c.stream>>>(keys, vals, (int)n, plan);
+    ++c.launches;
+    return passes;
+  }
   const int maxradix = 1 << plan.bits[0];
   const int TILE = K->tile();
   const long long ntile = (n + TILE - 1) / TILE;
   RsState* S = state_of(c);
   if (!S->ghist) {
     if (cudaMalloc(&S->ghist, RS_HIST_SLOTS * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&S->ctrs, RS_MAXPASS * sizeof(long long)) != cudaSuccess)
+        cudaMalloc(&S->ctrs, (RS_MAXPASS + 1) * sizeof(long long)) != cudaSuccess)
       return -2;
   }
   const size_t want = (size_t)(ntile + 1024) * maxradix;
@@ -715,7 +826,7 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
     cudaFuncSetAttribute((const void*)K->fn[i], cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   }
   const bool al = !(((uintptr_t)keys | (uintptr_t)vals | (uintptr_t)keys_tmp | (uintptr_t)vals_tmp) & 15u);
-  k_rs_zero<<<1, 1024, 0, c.stream>>>(S->ghist, RS_HIST_SLOTS, S->ctrs, RS_MAXPASS);
+  k_rs_zero<<<1, 1024, 0, c.stream>>>(S->ghist, RS_HIST_SLOTS, S->ctrs, RS_MAXPASS + 1);
   RsHistPlan hplan;
   make_hist_plan(plan, hplan);
   {
@@ -726,12 +837,13 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
     const void* hf = !((uintptr_t)keys & 15u) ? (const void*)k_rs_hist<true> : (const void*)k_rs_hist<false>;
     cudaFuncSetAttribute(hf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
     if (!((uintptr_t)keys & 15u))
-      k_rs_hist<true><<<hb, 1024, hsm, c.stream>>>(keys, n, plan, hplan, S->ghist);
+      k_rs_hist<true><<<hb, 1024, hsm, c.stream>>>(keys, n, plan, hplan, S->ghist,
+                                                   (unsigned long long*)S->ctrs + RS_MAXPASS);
     else
-      k_rs_hist<false><<<hb, 1024, hsm, c.stream>>>(keys, n, plan, hplan, S->ghist);
+      k_rs_hist<false><<<hb, 1024, hsm, c.stream>>>(keys, n, plan, hplan, S->ghist,
+                                                    (unsigned long long*)S->ctrs + RS_MAXPASS);
   }
-  k_rs_hist_scan<<<passes, 1024, 0, c.stream>>>(S->ghist, plan);
-  c.launches += 3;
+  c.launches += 2;
   unsigned long long* ka = keys;
   unsigned* va = vals;
   unsigned long long* kb = keys_tmp;
