@@ -10,16 +10,20 @@
 // Candidate pairs come from a closed-range tile binning (every box is listed
 // in each tile its closed extent touches, so two touching boxes share at
 // least one tile).  Tiles of up to UF_WARP_BOXES boxes (nearly all: the grid
-// is sized for about 32 boxes per tile) are taken one per warp, with the
-// tile's boxes staged in the warp's shared memory; larger tiles are taken one
-// per CTA.  Every pair that meets is hooked with atomicCAS, the larger root
+// is sized for about 32 boxes per tile) are taken one per warp; larger tiles
+// are taken one per CTA.  A lane keeps its boxes in registers and meets the
+// tile's boxes one after the other, each read from shared memory by all lanes
+// at once.  Pairs that meet are united in shared memory first, so a tile adds
+// to the global forest one edge per box that is not its local root, and not
+// one per pair.  Global edges are hooked with atomicCAS, the larger root
 // under the smaller, so the surviving root is the component minimum whatever
 // the order of the hooks.  Pointer jumping then flattens the forest.
 #include "gb_internal.h"
 #include "gb_scan.cuh"
 
 #define UF_SMEM_BOXES 1024
-#define UF_WARP_BOXES 64   // tiles up to this size go one per warp
+#define UF_WARP_BOXES 128  // tiles up to this size go one per warp, four boxes per lane
+#define UF_LB (UF_WARP_BOXES / 32)
 #define UF_WARPS 8         // warps per CTA of the per-warp kernels
 #define KID_UF 30
 
@@ -60,85 +64,202 @@ __device__ __forceinline__ bool closed_overlap(int4 a, int4 b) {
   return max(a.x, b.x) <= min(a.z, b.z) && max(a.y, b.y) <= min(a.w, b.w);
 }
 
-// The tile's pairs, one warp per tile of at most UF_WARP_BOXES boxes (tiles
-// are taken in a grid stride over all warps; larger tiles are skipped and left
-// to the per-CTA kernel).  act(ia, ba, ib, bb, t) handles one pair that meets.
-template <typename Act>
-__device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin, int4 (*sb)[UF_WARP_BOXES],
-                                           int (*si)[UF_WARP_BOXES], Act act) {
+// Shared-memory union-find over a tile's boxes (indices into the tile).
+__device__ __forceinline__ int sm_find(const int* sp, int x) {
+  for (int guard = 0; guard <= UF_SMEM_BOXES; ++guard) {
+    const int p = *(volatile const int*)&sp[x];
+    if (p == x) break;
+    x = p;
+  }
+  return x;
+}
+__device__ __forceinline__ void sm_unite(int* sp, int a, int b) {
+  for (int it = 0; it < (1 << 16); ++it) {  // a failed hook means another one succeeded
+    a = sm_find(sp, a);
+    b = sm_find(sp, b);
+    if (a == b) return;
+    if (a > b) { const int t = a; a = b; b = t; }
+    if (atomicCAS(&sp[b], b, a) == b) return;
+  }
+}
+
+// Boxes of a tile in shared memory, for the warp or the CTA that has it.
+template <int N>
+struct TileBoxes {
+  int4 box[N];
+  int idx[N];
+};
+
+// One warp's tiles of at most UF_WARP_BOXES boxes (in a grid stride over all
+// warps; larger tiles are left to the per-CTA kernels): the boxes go to
+// shared memory and, four per lane, to registers, then pair(a, u, ba) is
+// called by the lanes whose box u * 32 + lane > a meets box a, and finally
+// done(k, hit) with the lane's boxes that met any (bit u).
+template <typename Begin, typename Pair, typename Done>
+__device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin, TileBoxes<UF_WARP_BOXES>* tb, Begin begin,
+                                           Pair pair, Done done) {
   const int4* boxes = raw->boxes;
   const int* idx = (const int*)bin->pcs;
-  const int w = gb_warp(), lane = gb_lane();
+  TileBoxes<UF_WARP_BOXES>& s = tb[gb_warp()];
+  const int lane = gb_lane();
   const long long nt = bin->ntiles;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + w; t < nt; t += nwarps) {
+  for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + gb_warp(); t < nt; t += nwarps) {
     const int k = bin->tcount[t];
     if (k < 2 || k > UF_WARP_BOXES) continue;
     const int* ti = idx + bin->tstart[t];
-    for (int j = lane; j < k; j += 32) {
-      const int i = ti[j];
-      si[w][j] = i;
-      sb[w][j] = boxes[i];
-    }
-    __syncwarp();
-    for (int a = 0; a + 1 < k; ++a) {
-      const int ia = si[w][a];
-      const int4 ba = sb[w][a];
-      for (int b = a + 1 + lane; b < k; b += 32) {
-        const int4 bb = sb[w][b];
-        if (closed_overlap(ba, bb)) act(ia, ba, si[w][b], bb, t);
+    int4 bb[UF_LB];
+#pragma unroll
+    for (int u = 0; u < UF_LB; ++u) {
+      const int j = u * 32 + lane;
+      // an inverted box meets nothing
+      bb[u] = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
+      if (j < k) {
+        const int i = ti[j];
+        bb[u] = boxes[i];
+        s.idx[j] = i;
+        s.box[j] = bb[u];
       }
     }
+    begin(k, t);
+    __syncwarp();
+    unsigned hit = 0;
+    for (int a = 0; a + 1 < k; ++a) {
+      const int4 ba = s.box[a];
+      bool any = false;
+#pragma unroll
+      for (int u = 0; u < UF_LB; ++u) {
+        if (u * 32 + 31 <= a || u * 32 >= k) continue;  // warp-uniform
+        const bool ok = u * 32 + lane > a && closed_overlap(ba, bb[u]);
+        if (ok) {
+          hit |= 1u << u;
+          pair(a, u, ba, bb[u]);
+        }
+        any |= ok;
+      }
+      if (__any_sync(0xffffffffu, any) && lane == (a & 31)) hit |= 1u << (a >> 5);
+    }
+    __syncwarp();
+    done(k, hit);
     __syncwarp();  // the next tile overwrites the warp's boxes
   }
 }
 
 __global__ void __launch_bounds__(UF_WARPS * 32) k_uf_tile_warp(const DLayer* raw, const DLayer* bin, int* parent,
                                                               unsigned char* touched, DStatus* st) {
-  __shared__ int4 sb[UF_WARPS][UF_WARP_BOXES];
-  __shared__ int si[UF_WARPS][UF_WARP_BOXES];
+  __shared__ TileBoxes<UF_WARP_BOXES> tb[UF_WARPS];
+  __shared__ int sparent[UF_WARPS][UF_WARP_BOXES];
   if (st->err) return;
-  warp_tiles(raw, bin, sb, si, [&](int ia, int4, int ib, int4, long long) {
-    touched[ia] = 1;
-    touched[ib] = 1;
-    uf_unite(parent, ia, ib, st);
-  });
+  int* sp = sparent[gb_warp()];
+  const TileBoxes<UF_WARP_BOXES>& s = tb[gb_warp()];
+  const int lane = gb_lane();
+  warp_tiles(
+      raw, bin, tb,
+      [&](int k, long long) {
+        for (int j = lane; j < k; j += 32) sp[j] = j;
+      },
+      [&](int a, int u, int4, int4) { sm_unite(sp, a, u * 32 + lane); },
+      [&](int k, unsigned hit) {
+#pragma unroll
+        for (int u = 0; u < UF_LB; ++u) {
+          if (!((hit >> u) & 1)) continue;
+          const int j = u * 32 + lane, r = sm_find(sp, j);
+          touched[s.idx[j]] = 1;
+          if (r != j) uf_unite(parent, s.idx[j], s.idx[r], st);
+        }
+      });
 }
 
-// Tiles of more than UF_WARP_BOXES boxes, one per CTA (a grid stride over
-// the tiles; the others are skipped without a barrier).
-__global__ void __launch_bounds__(256) k_uf_tile(const DLayer* raw, const DLayer* bin, int* parent,
-                                                 unsigned char* touched, DStatus* st) {
-  __shared__ int4 sb[UF_SMEM_BOXES];
-  __shared__ int si[UF_SMEM_BOXES];
+// Tiles of more than UF_WARP_BOXES boxes, one per CTA (a grid stride over the
+// tiles; the others are skipped without a barrier).  Up to UF_SMEM_BOXES boxes
+// the CTA keeps four per thread in registers, as a warp does; the boxes of
+// larger tiles are read from global memory for every pair, and
+// pair(ia, ba, ib, bb) then has no place in shared memory (j = -1).
+template <typename Begin, typename Pair, typename Done>
+__device__ __forceinline__ void cta_tiles(const DLayer* raw, const DLayer* bin, TileBoxes<UF_SMEM_BOXES>& s, Begin begin,
+                                          Pair pair, Done done) {
+  constexpr int NT = 256, LB = UF_SMEM_BOXES / NT;
   const int4* boxes = raw->boxes;
   const int* idx = (const int*)bin->pcs;
-  if (st->err) return;
   for (long long t = blockIdx.x; t < bin->ntiles; t += gridDim.x) {
     const int k = bin->tcount[t];
     if (k <= UF_WARP_BOXES) continue;
     const int* ti = idx + bin->tstart[t];
-    const bool in_smem = k <= UF_SMEM_BOXES;
     __syncthreads();  // the previous tile's boxes are no longer read
-    if (in_smem) {
-      for (int j = threadIdx.x; j < k; j += blockDim.x) { si[j] = ti[j]; sb[j] = boxes[si[j]]; }
-      __syncthreads();
+    begin(k, t);
+    if (k > UF_SMEM_BOXES) {
+      const int nw = NT >> 5;
+      for (int a = gb_warp(); a < k; a += nw) {
+        const int ia = ti[a];
+        const int4 ba = boxes[ia];
+        for (int b = a + 1 + gb_lane(); b < k; b += 32) {
+          const int ib = ti[b];
+          const int4 bb = boxes[ib];
+          if (closed_overlap(ba, bb)) pair(-1, -1, ia, ba, ib, bb);
+        }
+      }
+      continue;
     }
-    const int nw = blockDim.x >> 5;
-    for (int a = gb_warp(); a < k; a += nw) {
-      const int ia = in_smem ? si[a] : ti[a];
-      const int4 ba = in_smem ? sb[a] : boxes[ia];
-      for (int b = a + 1 + gb_lane(); b < k; b += 32) {
-        const int ib = in_smem ? si[b] : ti[b];
-        const int4 bb = in_smem ? sb[b] : boxes[ib];
-        if (closed_overlap(ba, bb)) {
+    int4 bb[LB];
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      const int j = u * NT + threadIdx.x;
+      bb[u] = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
+      if (j < k) {
+        const int i = ti[j];
+        bb[u] = boxes[i];
+        s.idx[j] = i;
+        s.box[j] = bb[u];
+      }
+    }
+    __syncthreads();
+    for (int a = 0; a + 1 < k; ++a) {
+      const int4 ba = s.box[a];
+#pragma unroll
+      for (int u = 0; u < LB; ++u) {
+        if (u * NT + NT - 1 <= a || u * NT >= k) continue;  // uniform
+        const int j = u * NT + threadIdx.x;
+        if (j > a && closed_overlap(ba, bb[u])) pair(a, j, s.idx[a], ba, s.idx[j], bb[u]);
+      }
+    }
+    __syncthreads();
+    done(k);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_uf_tile(const DLayer* raw, const DLayer* bin, int* parent,
+                                                 unsigned char* touched, DStatus* st) {
+  __shared__ TileBoxes<UF_SMEM_BOXES> s;
+  __shared__ int sp[UF_SMEM_BOXES];
+  __shared__ unsigned char met[UF_SMEM_BOXES];
+  if (st->err) return;
+  cta_tiles(
+      raw, bin, s,
+      [&](int k, long long) {
+        for (int j = threadIdx.x; j < min(k, UF_SMEM_BOXES); j += blockDim.x) {
+          sp[j] = j;
+          met[j] = 0;
+        }
+      },
+      [&](int a, int b, int ia, int4, int ib, int4) {
+        if (a < 0) {
           touched[ia] = 1;
           touched[ib] = 1;
           uf_unite(parent, ia, ib, st);
+        } else {
+          met[a] = 1;
+          met[b] = 1;
+          sm_unite(sp, a, b);
         }
-      }
-    }
-  }
+      },
+      [&](int k) {
+        for (int j = threadIdx.x; j < k; j += blockDim.x) {
+          if (!met[j]) continue;
+          const int r = sm_find(sp, j);
+          touched[s.idx[j]] = 1;
+          if (r != j) uf_unite(parent, s.idx[j], s.idx[r], st);
+        }
+      });
 }
 
 // Overlap statistics (ComputeInteractionsCPU, pnummerge.f90:483-562, and
@@ -149,29 +270,34 @@ __global__ void __launch_bounds__(256) k_uf_tile(const DLayer* raw, const DLayer
 __device__ __forceinline__ bool strict_overlap(int4 a, int4 b) {
   return max(a.x, b.x) < min(a.z, b.z) && max(a.y, b.y) < min(a.w, b.w);
 }
-
-// A strict pair is counted in the tile holding the lower-left corner of its
-// intersection.
-__device__ __forceinline__ bool counted_here(int4 ba, int4 bb, int g, const DLayer* bin, long long t) {
-  if (!strict_overlap(ba, bb)) return false;
+__device__ __forceinline__ bool counted_here(int4 ba, int4 bb, int g, int tx, int ty) {
+  return strict_overlap(ba, bb) && (max(ba.x, bb.x) >> g) == tx && (max(ba.y, bb.y) >> g) == ty;
+}
+__device__ __forceinline__ void tile_xy(const DLayer* bin, long long t, int* tx, int* ty) {
   const int4 w = bin->win[0];
   const long long li = t - bin->tbase[0];
-  const int tx = w.x + (int)(li % w.z), ty = w.y + (int)(li / w.z);
-  return (max(ba.x, bb.x) >> g) == tx && (max(ba.y, bb.y) >> g) == ty;
+  *tx = w.x + (int)(li % w.z);
+  *ty = w.y + (int)(li / w.z);
 }
 
 __global__ void __launch_bounds__(UF_WARPS * 32) k_pair_stats_warp(const DLayer* raw, const DLayer* bin, int g,
                                                                  unsigned char* touched,
                                                                  unsigned long long* strict, DStatus* st) {
-  __shared__ int4 sb[UF_WARPS][UF_WARP_BOXES];
-  __shared__ int si[UF_WARPS][UF_WARP_BOXES];
+  __shared__ TileBoxes<UF_WARP_BOXES> tb[UF_WARPS];
   if (st->err) return;
+  const TileBoxes<UF_WARP_BOXES>& s = tb[gb_warp()];
+  int tx = 0, ty = 0;
   unsigned long long cnt = 0;
-  warp_tiles(raw, bin, sb, si, [&](int ia, int4 ba, int ib, int4 bb, long long t) {
-    touched[ia] = 1;
-    touched[ib] = 1;
-    if (counted_here(ba, bb, g, bin, t)) ++cnt;
-  });
+  warp_tiles(
+      raw, bin, tb, [&](int, long long t) { tile_xy(bin, t, &tx, &ty); },
+      [&](int, int, int4 ba, int4 bb) {
+        if (counted_here(ba, bb, g, tx, ty)) ++cnt;
+      },
+      [&](int, unsigned hit) {
+#pragma unroll
+        for (int u = 0; u < UF_LB; ++u)
+          if ((hit >> u) & 1) touched[s.idx[u * 32 + gb_lane()]] = 1;
+      });
   cnt = gb_warp_sum(cnt);
   if (gb_lane() == 0 && cnt) atomicAdd(strict, cnt);
 }
@@ -180,37 +306,31 @@ __global__ void __launch_bounds__(UF_WARPS * 32) k_pair_stats_warp(const DLayer*
 __global__ void __launch_bounds__(256) k_pair_stats(const DLayer* raw, const DLayer* bin, int g,
                                                     unsigned char* touched, unsigned long long* strict,
                                                     DStatus* st) {
-  __shared__ int4 sb[UF_SMEM_BOXES];
-  __shared__ int si[UF_SMEM_BOXES];
-  const int4* boxes = raw->boxes;
-  const int* idx = (const int*)bin->pcs;
+  __shared__ TileBoxes<UF_SMEM_BOXES> s;
+  __shared__ unsigned char met[UF_SMEM_BOXES];
   if (st->err) return;
+  int tx = 0, ty = 0;
   unsigned long long cnt = 0;
-  for (long long t = blockIdx.x; t < bin->ntiles; t += gridDim.x) {
-    const int k = bin->tcount[t];
-    if (k <= UF_WARP_BOXES) continue;
-    const int* ti = idx + bin->tstart[t];
-    const bool in_smem = k <= UF_SMEM_BOXES;
-    __syncthreads();  // the previous tile's boxes are no longer read
-    if (in_smem) {
-      for (int j = threadIdx.x; j < k; j += blockDim.x) { si[j] = ti[j]; sb[j] = boxes[si[j]]; }
-      __syncthreads();
-    }
-    const int nw = blockDim.x >> 5;
-    for (int a = gb_warp(); a < k; a += nw) {
-      const int ia = in_smem ? si[a] : ti[a];
-      const int4 ba = in_smem ? sb[a] : boxes[ia];
-      for (int b = a + 1 + gb_lane(); b < k; b += 32) {
-        const int ib = in_smem ? si[b] : ti[b];
-        const int4 bb = in_smem ? sb[b] : boxes[ib];
-        if (closed_overlap(ba, bb)) {
+  cta_tiles(
+      raw, bin, s,
+      [&](int k, long long t) {
+        tile_xy(bin, t, &tx, &ty);
+        for (int j = threadIdx.x; j < min(k, UF_SMEM_BOXES); j += blockDim.x) met[j] = 0;
+      },
+      [&](int a, int b, int ia, int4 ba, int ib, int4 bb) {
+        if (a < 0) {
           touched[ia] = 1;
           touched[ib] = 1;
-          if (counted_here(ba, bb, g, bin, t)) ++cnt;
+        } else {
+          met[a] = 1;
+          met[b] = 1;
         }
-      }
-    }
-  }
+        if (counted_here(ba, bb, g, tx, ty)) ++cnt;
+      },
+      [&](int k) {
+        for (int j = threadIdx.x; j < k; j += blockDim.x)
+          if (met[j]) touched[s.idx[j]] = 1;
+      });
   cnt = gb_warp_sum(cnt);
   if (gb_lane() == 0 && cnt) atomicAdd(strict, cnt);
 }
