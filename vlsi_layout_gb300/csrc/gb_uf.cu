@@ -61,7 +61,7 @@ __global__ void k_uf_init(int* parent, unsigned char* touched, long long n) {
 }
 
 __device__ __forceinline__ bool closed_overlap(int4 a, int4 b) {
-  return max(a.x, b.x) <= min(a.z, b.z) && max(a.y, b.y) <= min(a.w, b.w);
+  return a.x <= b.z && b.x <= a.z && a.y <= b.w && b.y <= a.w;  // both boxes are valid
 }
 
 // Shared-memory union-find over a tile's boxes (indices into the tile).
@@ -83,6 +83,18 @@ __device__ __forceinline__ void sm_unite(int* sp, int a, int b) {
   }
 }
 
+// Box i of a tile's component whose smallest box index is m: touched, and
+// joined to m.  A box that lies in this tile alone is seen by no other tile,
+// and nothing is ever hooked under it (it is not its component's smallest
+// box), so it takes m as its parent with a plain store; only boxes over
+// several tiles walk and hook the forest.
+__device__ __forceinline__ void tile_edge(int* parent, unsigned char* touched, int i, int4 b, int m, int g, DStatus* st) {
+  touched[i] = 1;
+  if (i == m) return;
+  if ((b.x >> g) == (b.z >> g) && (b.y >> g) == (b.w >> g)) parent[i] = m;
+  else uf_unite(parent, i, m, st);
+}
+
 // Boxes of a tile in shared memory, for the warp or the CTA that has it.
 template <int N>
 struct TileBoxes {
@@ -92,12 +104,16 @@ struct TileBoxes {
 
 // One warp's tiles of at most UF_WARP_BOXES boxes (in a grid stride over all
 // warps; larger tiles are left to the per-CTA kernels): the boxes go to
-// shared memory and, four per lane, to registers, then pair(a, u, ba) is
-// called by the lanes whose box u * 32 + lane > a meets box a, and finally
-// done(k, hit) with the lane's boxes that met any (bit u).
-template <typename Begin, typename Pair, typename Done>
+// shared memory and, four per lane, to registers.  32 boxes of the tile at a
+// time are read by all lanes at once and tested against the lanes' own, the
+// outcomes kept as bits; then met(j, a0, m) is called with the pairs of the
+// lane's box j (bit i of m: it meets box a0 + i < j), so that the work per
+// pair runs on all lanes together and not lane by lane as pairs turn up
+// (5500 -> 2900 instructions a tile).  Finally done(k, hit): the lane's boxes
+// that met any (bit u: box u * 32 + lane).
+template <typename Begin, typename Met, typename Done>
 __device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin, TileBoxes<UF_WARP_BOXES>* tb, Begin begin,
-                                           Pair pair, Done done) {
+                                           Met met, Done done) {
   const int4* boxes = raw->boxes;
   const int* idx = (const int*)bin->pcs;
   TileBoxes<UF_WARP_BOXES>& s = tb[gb_warp()];
@@ -124,20 +140,31 @@ __device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin,
     begin(k, t);
     __syncwarp();
     unsigned hit = 0;
-    for (int a = 0; a + 1 < k; ++a) {
-      const int4 ba = s.box[a];
-      bool any = false;
 #pragma unroll
-      for (int u = 0; u < UF_LB; ++u) {
-        if (u * 32 + 31 <= a || u * 32 >= k) continue;  // warp-uniform
-        const bool ok = u * 32 + lane > a && closed_overlap(ba, bb[u]);
-        if (ok) {
-          hit |= 1u << u;
-          pair(a, u, ba, bb[u]);
-        }
-        any |= ok;
+    for (int w = 0; w < UF_LB; ++w) {
+      if (w * 32 + 1 >= k) break;  // warp-uniform, as the tests on k below
+      unsigned m[UF_LB];
+#pragma unroll
+      for (int u = 0; u < UF_LB; ++u) m[u] = 0;
+      const int na = min(32, k - w * 32);
+      for (int i = 0; i < na; ++i) {
+        const int4 ba = s.box[w * 32 + i];
+#pragma unroll
+        for (int u = w; u < UF_LB; ++u)
+          if (u * 32 < k && closed_overlap(ba, bb[u])) m[u] |= 1u << i;
       }
-      if (__any_sync(0xffffffffu, any) && lane == (a & 31)) hit |= 1u << (a >> 5);
+      m[w] &= (1u << lane) - 1u;  // earlier boxes only
+      unsigned all = 0;
+#pragma unroll
+      for (int u = w; u < UF_LB; ++u) {
+        if (u * 32 >= k) break;
+        if (m[u]) {
+          hit |= 1u << u;
+          met(u * 32 + lane, w * 32, m[u]);
+        }
+        all |= m[u];
+      }
+      hit |= ((__reduce_or_sync(0xffffffffu, all) >> lane) & 1u) << w;
     }
     __syncwarp();
     done(k, hit);
@@ -149,24 +176,35 @@ __global__ void __launch_bounds__(UF_WARPS * 32) k_uf_tile_warp(const DLayer* ra
                                                               unsigned char* touched, DStatus* st) {
   __shared__ TileBoxes<UF_WARP_BOXES> tb[UF_WARPS];
   __shared__ int sparent[UF_WARPS][UF_WARP_BOXES];
+  __shared__ int least[UF_WARPS][UF_WARP_BOXES];  // smallest box index per component
   if (st->err) return;
-  int* sp = sparent[gb_warp()];
   const TileBoxes<UF_WARP_BOXES>& s = tb[gb_warp()];
-  const int lane = gb_lane();
+  int* const sp = sparent[gb_warp()];
+  int* const lm = least[gb_warp()];
+  const int lane = gb_lane(), g = bin->g;
   warp_tiles(
       raw, bin, tb,
       [&](int k, long long) {
-        for (int j = lane; j < k; j += 32) sp[j] = j;
-      },
-      [&](int a, int u, int4, int4) { sm_unite(sp, a, u * 32 + lane); },
-      [&](int k, unsigned hit) {
-#pragma unroll
-        for (int u = 0; u < UF_LB; ++u) {
-          if (!((hit >> u) & 1)) continue;
-          const int j = u * 32 + lane, r = sm_find(sp, j);
-          touched[s.idx[j]] = 1;
-          if (r != j) uf_unite(parent, s.idx[j], s.idx[r], st);
+        for (int j = lane; j < k; j += 32) {
+          sp[j] = j;
+          lm[j] = INT32_MAX;
         }
+      },
+      [&](int j, int a0, unsigned m) {
+        for (; m; m &= m - 1) sm_unite(sp, a0 + __ffs(m) - 1, j);
+      },
+      [&](int, unsigned hit) {
+        int r[UF_LB];
+#pragma unroll
+        for (int u = 0; u < UF_LB; ++u)
+          if ((hit >> u) & 1) {
+            r[u] = sm_find(sp, u * 32 + lane);
+            atomicMin(&lm[r[u]], s.idx[u * 32 + lane]);
+          }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < UF_LB; ++u)
+          if ((hit >> u) & 1) tile_edge(parent, touched, s.idx[u * 32 + lane], s.box[u * 32 + lane], lm[r[u]], g, st);
       });
 }
 
@@ -231,13 +269,16 @@ __global__ void __launch_bounds__(256) k_uf_tile(const DLayer* raw, const DLayer
                                                  unsigned char* touched, DStatus* st) {
   __shared__ TileBoxes<UF_SMEM_BOXES> s;
   __shared__ int sp[UF_SMEM_BOXES];
+  __shared__ int least[UF_SMEM_BOXES];
   __shared__ unsigned char met[UF_SMEM_BOXES];
   if (st->err) return;
+  const int g = bin->g;
   cta_tiles(
       raw, bin, s,
       [&](int k, long long) {
         for (int j = threadIdx.x; j < min(k, UF_SMEM_BOXES); j += blockDim.x) {
           sp[j] = j;
+          least[j] = INT32_MAX;
           met[j] = 0;
         }
       },
@@ -253,12 +294,11 @@ __global__ void __launch_bounds__(256) k_uf_tile(const DLayer* raw, const DLayer
         }
       },
       [&](int k) {
-        for (int j = threadIdx.x; j < k; j += blockDim.x) {
-          if (!met[j]) continue;
-          const int r = sm_find(sp, j);
-          touched[s.idx[j]] = 1;
-          if (r != j) uf_unite(parent, s.idx[j], s.idx[r], st);
-        }
+        for (int j = threadIdx.x; j < k; j += blockDim.x)
+          if (met[j]) atomicMin(&least[sm_find(sp, j)], s.idx[j]);
+        __syncthreads();
+        for (int j = threadIdx.x; j < k; j += blockDim.x)
+          if (met[j]) tile_edge(parent, touched, s.idx[j], s.box[j], least[sm_find(sp, j)], g, st);
       });
 }
 
@@ -290,8 +330,10 @@ __global__ void __launch_bounds__(UF_WARPS * 32) k_pair_stats_warp(const DLayer*
   unsigned long long cnt = 0;
   warp_tiles(
       raw, bin, tb, [&](int, long long t) { tile_xy(bin, t, &tx, &ty); },
-      [&](int, int, int4 ba, int4 bb) {
-        if (counted_here(ba, bb, g, tx, ty)) ++cnt;
+      [&](int j, int a0, unsigned m) {
+        const int4 b = s.box[j];
+        for (; m; m &= m - 1)
+          if (counted_here(s.box[a0 + __ffs(m) - 1], b, g, tx, ty)) ++cnt;
       },
       [&](int, unsigned hit) {
 #pragma unroll
