@@ -60,10 +60,11 @@ void drop_layer(gb_context* ctx, gb_layer* L) {
   if (!L) return;
   if (L->slot >= 0) ctx->c.desc_free.push_back(L->slot);
   L->slot = -1;
-  if (L->own_boxes) cudaFree(L->own_boxes);
-  if (L->own_coff) cudaFree(L->own_coff);
-  if (L->own_cell) cudaFree(L->own_cell);
-  L->own_boxes = L->own_coff = L->own_cell = nullptr;
+  if (L->own_cell) {
+    if (!L->internal) cudaDeviceSynchronize();  // other contexts' streams may still read the layer
+    gb_tmp_free(ctx->c, L->own_cell);
+  }
+  L->own_boxes = L->own_cell = nullptr;
 }
 
 // The binned form of L on grid g: L itself, the cached binning of a raw
@@ -78,11 +79,21 @@ gb_layer* binned_of(gb_context* ctx, gb_layer* L, int g) {
   return B;
 }
 
+// The status and nwords words from `words` (device), in one synchronisation.
+static cudaError_t read_back(gb_context* ctx, HostBack* out, const void* words = nullptr, int nwords = 0) {
+  GbCtx& c = ctx->c;
+  std::lock_guard<std::mutex> lk(ctx->hb_mu);
+  cudaMemcpyAsync(&c.hb->st, c.st, sizeof(DStatus), cudaMemcpyDeviceToHost, c.stream);
+  if (nwords) cudaMemcpyAsync(c.hb->w, words, (size_t)nwords * 8, cudaMemcpyDeviceToHost, c.stream);
+  const cudaError_t e = cudaStreamSynchronize(c.stream);
+  *out = *c.hb;
+  return e;
+}
+
 DStatus read_status(gb_context* ctx) {
-  DStatus s;
-  cudaStreamSynchronize(ctx->c.stream);
-  cudaMemcpy(&s, ctx->c.st, sizeof(DStatus), cudaMemcpyDeviceToHost);
-  return s;
+  HostBack h;
+  read_back(ctx, &h);
+  return h.st;
 }
 
 __global__ void k_clear_status(DStatus* st) {
@@ -396,6 +407,16 @@ extern "C" int gb_context_create(int device, unsigned long long arena_bytes, gb_
   if (cudaMalloc(&c.desc, GB_NDESC * sizeof(DLayer)) != cudaSuccess) return GB_ERR_OOM;
   cudaMemset(c.desc, 0, GB_NDESC * sizeof(DLayer));
   for (int i = GB_NDESC - 1; i >= 0; --i) c.desc_free.push_back(i);
+  if (cudaMalloc(&c.dmarks, GB_DMARKS * 8) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMallocHost(&c.hb, sizeof(HostBack)) != cudaSuccess) return GB_ERR_OOM;
+  cudaMemPoolProps pp;
+  memset(&pp, 0, sizeof(pp));
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = device;
+  if (cudaMemPoolCreate(&c.pool, &pp) != cudaSuccess) return GB_ERR_CUDA;
+  unsigned long long keep = GB_POOL_KEEP;
+  cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &keep);
   gb_tile_setup(c);
   if (realloc_scratch(ctx.get(), 8ull << 20) != GB_OK) return GB_ERR_OOM;
   cudaDeviceSynchronize();
@@ -417,6 +438,9 @@ extern "C" int gb_context_destroy(gb_context* ctx) {
   cudaFree(c.tile_counter);
   cudaFree(c.desc);
   cudaFree(c.tile_scratch);
+  cudaFree(c.dmarks);
+  if (c.hb) cudaFreeHost(c.hb);
+  if (c.pool) cudaMemPoolDestroy(c.pool);
   if (c.io_buf) cudaFree(c.io_buf);
   if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
   gb_radix_free(c);
@@ -443,14 +467,24 @@ extern "C" int gb_set_stream(gb_context* ctx, void* stream) {
 
 extern "C" const char* gb_last_error(gb_context* ctx) { return ctx ? ctx->c.last_error.c_str() : ""; }
 
+static int sync_words(gb_context* ctx, HostBack* h, const void* words, int nwords);
+
 extern "C" int gb_sync(gb_context* ctx, long long* need) {
   if (!ctx) return GB_ERR_ARG;
-  cudaError_t e = cudaStreamSynchronize(ctx->c.stream);
+  HostBack h;
+  h.st.need = 0;
+  const int e = sync_words(ctx, &h, nullptr, 0);
+  if (need && e != GB_ERR_CUDA) *need = h.st.need;
+  return e;
+}
+
+// gb_sync that also brings nwords device words along.
+static int sync_words(gb_context* ctx, HostBack* h, const void* words, int nwords) {
+  cudaError_t e = read_back(ctx, h, words, nwords);
   if (e != cudaSuccess) return set_err(ctx, GB_ERR_CUDA, cudaGetErrorString(e));
   e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(ctx, GB_ERR_CUDA, cudaGetErrorString(e));
-  DStatus s = read_status(ctx);
-  if (need) *need = s.need;
+  const DStatus& s = h->st;
   if (s.err) {
     char buf[160];
     snprintf(buf, sizeof buf, "device status %d raised by kernel %d (need %lld)", s.err, s.where, s.need);
@@ -460,9 +494,11 @@ extern "C" int gb_sync(gb_context* ctx, long long* need) {
 }
 
 int sync_where(gb_context* ctx, int* where, long long* need) {
-  int e = gb_sync(ctx, need);
-  DStatus s = read_status(ctx);
-  if (where) *where = s.where;
+  HostBack h;
+  memset(&h, 0, sizeof(h));
+  const int e = sync_words(ctx, &h, nullptr, 0);
+  if (need) *need = h.st.need;
+  if (where) *where = h.st.where;
   return e;
 }
 
@@ -470,18 +506,32 @@ extern "C" void gb_clear_status(gb_context* ctx) {
   if (ctx) k_clear_status<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st);
 }
 
+// The mark stays on the device, in the stream's order (GB_DMARKS deep; deeper
+// ones, and marks taken during a capture, are read back as numbers).
+#define MARK_ON_DEVICE (~0ull)
+__global__ void k_arena_mark(const DStatus* st, unsigned long long* slot) { *slot = st->arena_off; }
+__global__ void k_arena_release(DStatus* st, const unsigned long long* slot) { st->arena_off = *slot; }
+
 extern "C" unsigned long long gb_arena_mark(gb_context* ctx) {
   if (!ctx) return 0;
-  DStatus s = read_status(ctx);
-  ctx->marks.push_back({s.arena_off, ctx->seq});
-  return (unsigned long long)(ctx->marks.size() - 1);
+  GbCtx& c = ctx->c;
+  const size_t i = ctx->marks.size();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (i < GB_DMARKS && cudaStreamIsCapturing(c.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+    k_arena_mark<<<1, 1, 0, c.stream>>>(c.st, c.dmarks + i);
+    ctx->marks.push_back({MARK_ON_DEVICE, ctx->seq});
+  } else {
+    ctx->marks.push_back({read_status(ctx).arena_off, ctx->seq});
+  }
+  return (unsigned long long)i;
 }
 
 extern "C" int gb_arena_release(gb_context* ctx, unsigned long long mark) {
   if (!ctx || mark >= ctx->marks.size()) return GB_ERR_ARG;
   const auto m = ctx->marks[mark];
   ctx->marks.resize(mark);
-  gb_launch_arena_reset(ctx->c, m.first);
+  if (m.first == MARK_ON_DEVICE) k_arena_release<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st, ctx->c.dmarks + mark);
+  else gb_launch_arena_reset(ctx->c, m.first);
   std::vector<gb_layer*> keep;
   for (gb_layer* L : ctx->arena_layers) {
     if (L->seq > m.second) {
@@ -517,6 +567,15 @@ extern "C" int gb_set_tile_scratch(gb_context* ctx, unsigned long long bytes) {
 }
 
 // ======================================================================= layers
+// A raw layer's descriptor; one_cell: its offsets too.
+__global__ void k_raw_desc(DLayer* d, DLayer v, bool one_cell) {
+  *d = v;
+  if (one_cell) {
+    v.coff[0] = 0;
+    v.coff[1] = v.nbox;
+  }
+}
+
 // borrow: boxes is a device pointer used in place (coff then a host pointer).
 static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long long n,
                           const long long* coff, int ncell, bool device_src, gb_layer** out, bool borrow = false) {
@@ -531,43 +590,37 @@ static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long lon
   L->ncell = ncell;
   L->binned = 0;
   L->nbox_host = (long long)n;
-  void *pb = borrow ? (void*)boxes : nullptr, *pc = nullptr, *pcell = nullptr;
-  if ((!borrow && cudaMalloc(&pb, std::max<size_t>(16, n * 16)) != cudaSuccess) ||
-      cudaMalloc(&pc, (size_t)(ncell + 1) * 8) != cudaSuccess ||
-      cudaMalloc(&pcell, (size_t)ncell * (16 + 8 + 8 + 16) + (size_t)(ncell + 1) * 8) != cudaSuccess) {
-    if (pb && !borrow) cudaFree(pb);
-    if (pc) cudaFree(pc);
+  // one allocation: boxes (unless borrowed), cell offsets, per-cell arrays
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t nb = borrow ? 0 : up(std::max<size_t>(16, n * 16)), no = up((size_t)(ncell + 1) * 8);
+  char* q = (char*)gb_tmp_alloc(c, nb + no + (size_t)ncell * (16 + 8 + 8 + 16) + (size_t)(ncell + 1) * 8);
+  if (!q) {
     c.desc_free.push_back(s);
     delete L;
-    return set_err(ctx, GB_ERR_OOM, "cudaMalloc failed for a layer");
+    return set_err(ctx, GB_ERR_OOM, "no device memory for a layer");
   }
+  L->own_cell = q;
+  void* pb = borrow ? (void*)boxes : (void*)q;
   L->own_boxes = borrow ? nullptr : pb;
-  L->own_coff = pc;
-  L->own_cell = pcell;
-  const cudaMemcpyKind kind = device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (n && !borrow) cudaMemcpyAsync(pb, boxes, n * 16, kind, c.stream);
-  if (coff) {
-    cudaMemcpyAsync(pc, coff, (size_t)(ncell + 1) * 8, borrow ? cudaMemcpyHostToDevice : kind, c.stream);
-  } else {
-    long long h[2] = {0, (long long)n};
-    cudaMemcpyAsync(pc, h, 16, cudaMemcpyHostToDevice, c.stream);
-    cudaStreamSynchronize(c.stream);
-  }
+  q += nb;
   DLayer d;
   memset(&d, 0, sizeof(d));
   d.ncell = ncell;
   d.binned = 0;
   d.boxes = (int4*)pb;
-  d.coff = (long long*)pc;
+  d.coff = (long long*)q; q += no;
   d.nbox = (long long)n;
-  char* q = (char*)pcell;
   d.cbox = (int4*)q; q += (size_t)ncell * 16;
+  d.win = (int4*)q; q += (size_t)ncell * 16;
   d.cell_count = (long long*)q; q += (size_t)ncell * 8;
   d.cell_area = (long long*)q; q += (size_t)ncell * 8;
-  d.win = (int4*)q; q += (size_t)ncell * 16;
   d.tbase = (long long*)q;
-  cudaMemcpyAsync(L->d, &d, sizeof(d), cudaMemcpyHostToDevice, c.stream);
-  cudaStreamSynchronize(c.stream);
+  L->cbox = d.cbox;
+  const cudaMemcpyKind kind = device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  k_raw_desc<<<1, 1, 0, c.stream>>>(L->d, d, coff == nullptr);
+  if (n && !borrow) cudaMemcpyAsync(pb, boxes, n * 16, kind, c.stream);
+  if (coff) cudaMemcpyAsync(d.coff, coff, (size_t)(ncell + 1) * 8, borrow ? cudaMemcpyHostToDevice : kind, c.stream);
+  cudaStreamSynchronize(c.stream);  // the caller's arrays are its own again
   gb_launch_cell_bbox_fill(c, L->d, ncell);
   *out = L;
   return GB_OK;
@@ -600,13 +653,13 @@ extern "C" int gb_layer_ncell(gb_layer* L) { return L ? L->ncell : 0; }
 extern "C" int gb_layer_digest(gb_context* ctx, gb_layer* L, unsigned long long* out) {
   if (!ctx || !L || L->dead || !out || !L->binned) return GB_ERR_ARG;
   GbCtx& c = ctx->c;
-  unsigned long long* d = nullptr;
-  if (cudaMalloc(&d, (size_t)L->ncell * 8) != cudaSuccess) return set_err(ctx, GB_ERR_OOM, "digest buffer");
+  unsigned long long* d = (unsigned long long*)gb_tmp_alloc(c, (size_t)L->ncell * 8);
+  if (!d) return set_err(ctx, GB_ERR_OOM, "digest buffer");
   cudaMemsetAsync(d, 0, (size_t)L->ncell * 8, c.stream);
   gb_launch_digest(c, L->d, d, 1);
   cudaStreamSynchronize(c.stream);
   const cudaError_t ce = cudaMemcpy(out, d, (size_t)L->ncell * 8, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  gb_tmp_free(c, d);
   if (ce != cudaSuccess) return set_err(ctx, GB_ERR_CUDA, "digest copy");
   return gb_sync(ctx, nullptr);
 }
@@ -623,19 +676,46 @@ extern "C" int gb_layer_count(gb_context* ctx, gb_layer* L, long long* total, lo
   } else if (L->counted) {
     if (d.cell_count) cudaMemcpy(pc.data(), d.cell_count, pc.size() * 8, cudaMemcpyDeviceToHost);
   } else {
-    long long* tmp = nullptr;
-    cudaMalloc(&tmp, pc.size() * 8);
+    long long* tmp = (long long*)gb_tmp_alloc(c, pc.size() * 8);
+    if (!tmp) return set_err(ctx, GB_ERR_OOM, "count buffer");
     cudaMemsetAsync(tmp, 0, pc.size() * 8, c.stream);
     k_count_tiles<<<c.work_blocks, 256, 0, c.stream>>>(L->d, tmp, L->ncell, c.st);
     cudaStreamSynchronize(c.stream);
     cudaMemcpy(pc.data(), tmp, pc.size() * 8, cudaMemcpyDeviceToHost);
-    cudaFree(tmp);
+    gb_tmp_free(c, tmp);
   }
   long long t = 0;
   for (long long v : pc) t += v;
   if (total) *total = t;
   if (per_cell) memcpy(per_cell, pc.data(), pc.size() * 8);
   return gb_sync(ctx, nullptr);
+}
+
+// Exports a binned layer and copies its boxes to where(count) (null: nowhere);
+// GB_ERR_CAPACITY when there are more than cap.
+template <typename Where>
+static int export_to_host(gb_context* ctx, gb_layer* L, unsigned long long* n, long long* cell_offsets, Where where,
+                          unsigned long long cap) {
+  GbCtx& c = ctx->c;
+  gb_launch_export(c, L->d, nullptr, nullptr);
+  HostBack h;
+  int e = sync_words(ctx, &h, c.dscal, 4);
+  if (e) return e;
+  const long long* sc = h.w;
+  *n = (unsigned long long)sc[2];
+  if (cell_offsets) {
+    DLayer d = read_desc(ctx, L);
+    std::vector<long long> tb(L->ncell + 1);
+    cudaMemcpy(tb.data(), d.tbase, tb.size() * 8, cudaMemcpyDeviceToHost);
+    std::vector<long long> off(d.ntiles + 1);
+    cudaMemcpy(off.data(), (void*)sc[1], (size_t)(d.ntiles + 1) * 8, cudaMemcpyDeviceToHost);
+    off[d.ntiles] = sc[2];
+    for (int k = 0; k <= L->ncell; ++k) cell_offsets[k] = off[std::min<long long>(tb[k], d.ntiles)];
+  }
+  c_box* out = where(*n);
+  if (*n > cap) return set_err(ctx, GB_ERR_CAPACITY, "output buffer too small");
+  if (*n && out) cudaMemcpy(out, (void*)sc[0], (size_t)*n * 16, cudaMemcpyDeviceToHost);
+  return GB_OK;
 }
 
 extern "C" int gb_layer_to_host(gb_context* ctx, gb_layer* L, c_box* out, unsigned long long cap,
@@ -650,24 +730,16 @@ extern "C" int gb_layer_to_host(gb_context* ctx, gb_layer* L, c_box* out, unsign
     if (d.nbox && out) cudaMemcpy(out, d.boxes, (size_t)d.nbox * 16, cudaMemcpyDeviceToHost);
     return GB_OK;
   }
-  gb_launch_export(c, L->d, nullptr, nullptr);
-  int e = gb_sync(ctx, nullptr);
-  if (e) return e;
-  long long sc[4];
-  cudaMemcpy(sc, c.dscal, sizeof(sc), cudaMemcpyDeviceToHost);
-  *n = (unsigned long long)sc[2];
-  if (cell_offsets) {
-    DLayer d = read_desc(ctx, L);
-    std::vector<long long> tb(L->ncell + 1);
-    cudaMemcpy(tb.data(), d.tbase, tb.size() * 8, cudaMemcpyDeviceToHost);
-    std::vector<long long> off(d.ntiles + 1);
-    cudaMemcpy(off.data(), (void*)sc[1], (size_t)(d.ntiles + 1) * 8, cudaMemcpyDeviceToHost);
-    off[d.ntiles] = sc[2];
-    for (int k = 0; k <= L->ncell; ++k) cell_offsets[k] = off[std::min<long long>(tb[k], d.ntiles)];
+  if (cap == 0 && !out && !cell_offsets) {  // the count alone: nothing is exported
+    HostBack h;
+    int e = sync_words(ctx, &h, &L->d->ntot, 1);
+    if (e) return e;
+    *n = (unsigned long long)h.w[0];
+    return *n ? set_err(ctx, GB_ERR_CAPACITY, "output buffer too small") : GB_OK;
   }
-  if ((unsigned long long)sc[2] > cap) return set_err(ctx, GB_ERR_CAPACITY, "output buffer too small");
-  if (sc[2] && out) cudaMemcpy(out, (void*)sc[0], (size_t)sc[2] * 16, cudaMemcpyDeviceToHost);
-  return GB_OK;
+  return export_to_host(ctx, L, n, cell_offsets, [&](unsigned long long k) -> c_box* {
+    return k <= cap ? out : nullptr;
+  }, cap);
 }
 
 namespace gbi {
@@ -684,19 +756,18 @@ int layer_device_boxes(gb_context* ctx, gb_layer* L, const c_box** d_boxes, long
     return GB_OK;
   }
   gb_launch_export(c, L->d, nullptr, nullptr);
-  int e = gb_sync(ctx, nullptr);
+  HostBack h;
+  int e = sync_words(ctx, &h, c.dscal, 4);
   if (e) return e;
-  long long sc[4];
-  cudaMemcpy(sc, c.dscal, sizeof(sc), cudaMemcpyDeviceToHost);
-  *d_boxes = (const c_box*)sc[0];
-  *n = sc[2];
+  *d_boxes = (const c_box*)h.w[0];
+  *n = h.w[2];
   return GB_OK;
 }
 }  // namespace gbi
 
 extern "C" void gb_layer_free(gb_context* ctx, gb_layer* L) {
   if (!ctx || !L) return;
-  cudaStreamSynchronize(ctx->c.stream);
+  if (!L->internal) cudaStreamSynchronize(ctx->c.stream);
   if (L->arena_owned) {
     // arena layers are reclaimed by gb_arena_release; only the handle goes
     drop_layer(ctx, L);
@@ -826,15 +897,20 @@ int gb_run_retry(gb_context* ctx, const std::function<int()>& body) { return run
 
 // ======================================================================= connectivity
 // Grid for candidate pairs of a one-cell raw layer: about 32 boxes per tile.
-static int pair_grid(gb_context* ctx, gb_layer* L, long long n) {
-  DLayer d = read_desc(ctx, L);
+// Synchronises and returns the context's status (a layer's invalid boxes).
+static int pair_grid(gb_context* ctx, gb_layer* L, long long n, int* grid) {
+  // the one cell's bounding box follows its offsets in the layer's allocation
+  HostBack h;
+  const int e = sync_words(ctx, &h, L->cbox, 2);
+  if (e) return e;
   int4 bb;
-  cudaMemcpy(&bb, d.cbox, 16, cudaMemcpyDeviceToHost);
+  memcpy(&bb, h.w, 16);
   const double W = (double)bb.z - bb.x + 1, H = (double)bb.w - bb.y + 1;
   const double cell = std::sqrt(W * H * 32.0 / (double)(n > 0 ? n : 1));
   int g = 4;
   while (g < 30 && (double)(1ll << g) < cell) ++g;
-  return g;
+  *grid = g;
+  return GB_OK;
 }
 
 extern "C" int gb_components(gb_context* ctx, const c_box* boxes, unsigned long long n,
@@ -846,37 +922,31 @@ extern "C" int gb_components(gb_context* ctx, const c_box* boxes, unsigned long 
   gb_layer* L = nullptr;
   int e = gb_layer_from_host(ctx, boxes, n, nullptr, 1, &L);
   if (e) return e;
-  e = gb_sync(ctx, nullptr);
+  L->internal = true;
+  int g = 0;
+  e = pair_grid(ctx, L, (long long)n, &g);
   if (e) { gb_layer_free(ctx, L); return e; }
-  const int g = pair_grid(ctx, L, (long long)n);
-  int* parent = nullptr;
-  unsigned char* touched = nullptr;
-  long long* lab = nullptr;
-  long long* map = nullptr;
-  int* flag = nullptr;
-  long long* nc = nullptr;
-  cudaMalloc(&parent, n * 4);
-  cudaMalloc(&touched, n);
-  cudaMalloc(&lab, n * 8);
-  cudaMalloc(&map, n * 8);
-  cudaMalloc(&flag, n * 4);
-  cudaMalloc(&nc, 8);
-  if (!parent || !touched || !lab || !map || !flag || !nc) {
-    e = set_err(ctx, GB_ERR_OOM, "cudaMalloc failed in gb_components");
-  } else {
-    e = run_retry(ctx, [&]() -> int {
-      gb_layer* B = new_arena_layer(ctx, 1, g);
-      if (!B) return GB_ERR_CAPACITY;
-      gb_launch_bin_index(c, L->d, B->d, 1, g);
-      gb_launch_components(c, L->d, B->d, parent, touched, lab, (long long)n, nc, flag, map);
-      return GB_OK;
-    });
-    if (e == GB_OK) {
-      cudaMemcpy(ncomp, nc, 8, cudaMemcpyDeviceToHost);
-      if (labels) cudaMemcpy(labels, lab, n * 8, cudaMemcpyDeviceToHost);
+  {
+    GbTmp M(c);
+    const size_t parent = M.add(n * 4), touched = M.add(n), lab = M.add(n * 8), map = M.add(n * 8), flag = M.add(n * 4),
+                 nc = M.add(8);
+    if (!M.get()) {
+      e = set_err(ctx, GB_ERR_OOM, "no device memory in gb_components");
+    } else {
+      e = run_retry(ctx, [&]() -> int {
+        gb_layer* B = new_arena_layer(ctx, 1, g);
+        if (!B) return GB_ERR_CAPACITY;
+        gb_launch_bin_index(c, L->d, B->d, 1, g);
+        gb_launch_components(c, L->d, B->d, M.ptr<int>(parent), M.ptr<unsigned char>(touched), M.ptr<long long>(lab),
+                             (long long)n, M.ptr<long long>(nc), M.ptr<int>(flag), M.ptr<long long>(map));
+        return GB_OK;
+      });
+      if (e == GB_OK) {
+        cudaMemcpy(ncomp, M.ptr<char>(nc), 8, cudaMemcpyDeviceToHost);
+        if (labels) cudaMemcpy(labels, M.ptr<char>(lab), n * 8, cudaMemcpyDeviceToHost);
+      }
     }
   }
-  cudaFree(parent); cudaFree(touched); cudaFree(lab); cudaFree(map); cudaFree(flag); cudaFree(nc);
   gb_layer_free(ctx, L);
   return e;
 }
@@ -896,34 +966,34 @@ extern "C" int gb_interactions(gb_context* ctx, const c_box* boxes, unsigned lon
   gb_layer* L = nullptr;
   int e = gb_layer_from_host(ctx, boxes, n, nullptr, 1, &L);
   if (e) return e;
-  e = gb_sync(ctx, nullptr);
+  L->internal = true;
+  int g = 0;
+  e = pair_grid(ctx, L, (long long)n, &g);
   if (e) { gb_layer_free(ctx, L); return e; }
-  const int g = pair_grid(ctx, L, (long long)n);
-  unsigned char* touched = nullptr;
-  unsigned char* mask = nullptr;
-  unsigned long long* cnt = nullptr;
-  cudaMalloc(&touched, n);
-  cudaMalloc(&cnt, 16);
-  if (is_singleton) cudaMalloc(&mask, n);
-  if (!touched || !cnt || (is_singleton && !mask)) {
-    e = set_err(ctx, GB_ERR_OOM, "cudaMalloc failed in gb_interactions");
-  } else {
-    e = run_retry(ctx, [&]() -> int {
-      gb_layer* B = new_arena_layer(ctx, 1, g);
-      if (!B) return GB_ERR_CAPACITY;
-      gb_launch_bin_index(c, L->d, B->d, 1, g);
-      gb_launch_pair_stats(c, L->d, B->d, g, touched, (long long)n, cnt, cnt + 1, mask);
-      return GB_OK;
-    });
-    if (e == GB_OK) {
-      unsigned long long h[2];
-      cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
-      if (strict_pairs) *strict_pairs = (long long)h[0];
-      if (singletons) *singletons = (long long)h[1];
-      if (is_singleton) cudaMemcpy(is_singleton, mask, n, cudaMemcpyDeviceToHost);
+  {
+    GbTmp M(c);
+    const size_t touched = M.add(n), cnt = M.add(16), mask = M.add(is_singleton ? n : 0);
+    if (!M.get()) {
+      e = set_err(ctx, GB_ERR_OOM, "no device memory in gb_interactions");
+    } else {
+      unsigned long long* dc = M.ptr<unsigned long long>(cnt);
+      e = run_retry(ctx, [&]() -> int {
+        gb_layer* B = new_arena_layer(ctx, 1, g);
+        if (!B) return GB_ERR_CAPACITY;
+        gb_launch_bin_index(c, L->d, B->d, 1, g);
+        gb_launch_pair_stats(c, L->d, B->d, g, M.ptr<unsigned char>(touched), (long long)n, dc, dc + 1,
+                             is_singleton ? M.ptr<unsigned char>(mask) : nullptr);
+        return GB_OK;
+      });
+      if (e == GB_OK) {
+        unsigned long long h[2];
+        cudaMemcpy(h, dc, 16, cudaMemcpyDeviceToHost);
+        if (strict_pairs) *strict_pairs = (long long)h[0];
+        if (singletons) *singletons = (long long)h[1];
+        if (is_singleton) cudaMemcpy(is_singleton, M.ptr<char>(mask), n, cudaMemcpyDeviceToHost);
+      }
     }
   }
-  cudaFree(touched); cudaFree(mask); cudaFree(cnt);
   gb_layer_free(ctx, L);
   return e;
 }
@@ -975,36 +1045,35 @@ extern "C" int gb_component_areas(gb_context* ctx, const c_box* boxes, unsigned 
   gb_layer* L = nullptr;
   int e = gb_layer_from_host(ctx, boxes, n, nullptr, 1, &L);
   if (e) return e;
-  e = gb_sync(ctx, nullptr);
+  L->internal = true;
+  int g = 0;
+  e = pair_grid(ctx, L, (long long)n, &g);
   if (e) { gb_layer_free(ctx, L); return e; }
-  const int g = pair_grid(ctx, L, (long long)n);
-  int* parent = nullptr;
-  unsigned char* touched = nullptr;
-  long long *lab = nullptr, *map = nullptr, *nc = nullptr, *off = nullptr;
-  int* flag = nullptr;
+  GbTmp M(c);
+  const size_t o_parent = M.add(n * 4), o_touched = M.add(n), o_lab = M.add(n * 8), o_map = M.add(n * 8),
+               o_flag = M.add(n * 4), o_nc = M.add(8), o_keys = M.add(n * 8), o_kt = M.add(n * 8), o_vals = M.add(n * 4),
+               o_vt = M.add(n * 4), o_sorted = M.add(n * 16);
+  long long *lab = nullptr, *nc = nullptr, *off = nullptr;
   unsigned long long *keys = nullptr, *kt = nullptr;
   unsigned *vals = nullptr, *vt = nullptr;
   int4* sorted = nullptr;
-  cudaMalloc(&parent, n * 4);
-  cudaMalloc(&touched, n);
-  cudaMalloc(&lab, n * 8);
-  cudaMalloc(&map, n * 8);
-  cudaMalloc(&flag, n * 4);
-  cudaMalloc(&nc, 8);
-  cudaMalloc(&keys, n * 8);
-  cudaMalloc(&kt, n * 8);
-  cudaMalloc(&vals, n * 4);
-  cudaMalloc(&vt, n * 4);
-  cudaMalloc(&sorted, n * 16);
   gb_layer* G = nullptr;
-  if (!parent || !touched || !lab || !map || !flag || !nc || !keys || !kt || !vals || !vt || !sorted) {
-    e = set_err(ctx, GB_ERR_OOM, "cudaMalloc failed in gb_component_areas");
+  if (!M.get()) {
+    e = set_err(ctx, GB_ERR_OOM, "no device memory in gb_component_areas");
   } else {
+    lab = M.ptr<long long>(o_lab);
+    nc = M.ptr<long long>(o_nc);
+    keys = M.ptr<unsigned long long>(o_keys);
+    kt = M.ptr<unsigned long long>(o_kt);
+    vals = M.ptr<unsigned>(o_vals);
+    vt = M.ptr<unsigned>(o_vt);
+    sorted = M.ptr<int4>(o_sorted);
     e = run_retry(ctx, [&]() -> int {
       gb_layer* B = new_arena_layer(ctx, 1, g);
       if (!B) return GB_ERR_CAPACITY;
       gb_launch_bin_index(c, L->d, B->d, 1, g);
-      gb_launch_components(c, L->d, B->d, parent, touched, lab, (long long)n, nc, flag, map);
+      gb_launch_components(c, L->d, B->d, M.ptr<int>(o_parent), M.ptr<unsigned char>(o_touched), lab, (long long)n, nc,
+                           M.ptr<int>(o_flag), M.ptr<long long>(o_map));
       return GB_OK;
     });
   }
@@ -1018,8 +1087,8 @@ extern "C" int gb_component_areas(gb_context* ctx, const c_box* boxes, unsigned 
     if (cap < (unsigned long long)(R + 1)) e = GB_ERR_CAPACITY;
   }
   if (e == GB_OK) {
-    cudaMalloc(&off, (size_t)(R + 2) * 8);
-    if (!off) e = set_err(ctx, GB_ERR_OOM, "cudaMalloc failed in gb_component_areas");
+    off = (long long*)gb_tmp_alloc(c, (size_t)(R + 2) * 8);
+    if (!off) e = set_err(ctx, GB_ERR_OOM, "no device memory in gb_component_areas");
   }
   if (e == GB_OK) {
     int bits = 1;
@@ -1037,8 +1106,7 @@ extern "C" int gb_component_areas(gb_context* ctx, const c_box* boxes, unsigned 
     if (!e) e = areas ? gb_op_area(ctx, G, areas) : GB_OK;
   }
   if (G) gb_layer_free(ctx, G);
-  cudaFree(parent); cudaFree(touched); cudaFree(lab); cudaFree(map); cudaFree(flag); cudaFree(nc);
-  cudaFree(keys); cudaFree(kt); cudaFree(vals); cudaFree(vt); cudaFree(sorted); cudaFree(off);
+  gb_tmp_free(c, off);
   gb_layer_free(ctx, L);
   return e;
 }
@@ -1052,27 +1120,22 @@ static int sort_keys_perm(gb_context* ctx, unsigned long long* dkeys, unsigned* 
   GbCtx& c = ctx->c;
   unsigned long long* orx = d_span;
   if (!orx) {
-    cudaMalloc(&orx, 8);
+    orx = (unsigned long long*)gb_tmp_alloc(c, 8);
+    if (!orx) return set_err(ctx, GB_ERR_OOM, "no device memory in sort");
     cudaMemsetAsync(orx, 0, 8, c.stream);
     k_key_span<<<c.work_blocks, 256, 0, c.stream>>>(dkeys, n, orx);
   }
   unsigned long long span = 0;
   cudaMemcpyAsync(&span, orx, 8, cudaMemcpyDeviceToHost, c.stream);
   cudaStreamSynchronize(c.stream);
-  if (!d_span) cudaFree(orx);
+  if (!d_span) gb_tmp_free(c, orx);
   int bits = 0;
   while (bits < 64 && (span >> bits)) ++bits;
   if (bits == 0) return GB_OK;
-  unsigned long long* kt = nullptr;
-  unsigned* vt = nullptr;
-  if (cudaMalloc(&kt, (size_t)n * 8) != cudaSuccess || cudaMalloc(&vt, (size_t)n * 4) != cudaSuccess) {
-    if (kt) cudaFree(kt);
-    return set_err(ctx, GB_ERR_OOM, "cudaMalloc failed in sort");
-  }
-  int p = gb_radix_sort_pairs(c, dkeys, dvals, n, bits, kt, vt);
-  cudaStreamSynchronize(c.stream);
-  cudaFree(kt);
-  cudaFree(vt);
+  GbTmp M(c);
+  const size_t kt = M.add((size_t)n * 8), vt = M.add((size_t)n * 4);
+  if (!M.get()) return set_err(ctx, GB_ERR_OOM, "no device memory in sort");
+  const int p = gb_radix_sort_pairs(c, dkeys, dvals, n, bits, M.ptr<unsigned long long>(kt), M.ptr<unsigned>(vt));
   return p < 0 ? set_err(ctx, GB_ERR_INTERNAL, "radix sort setup failed") : gb_sync(ctx, nullptr);
 }
 
@@ -1090,48 +1153,36 @@ static int morton_sort_impl(gb_context* ctx, c_box* boxes, long long n, int sort
                             bool dev_io) {
   GbCtx& c = ctx->c;
   if (n <= 0) return GB_OK;
-  int4* db = nullptr;
-  int4* db2 = nullptr;
-  unsigned long long* dk = nullptr;
-  unsigned* dv = nullptr;
-  int e = GB_OK;
-  if (dev_io) db = (int4*)boxes;
-  else if (cudaMalloc(&db, (size_t)n * 16) != cudaSuccess) return GB_ERR_OOM;
+  GbTmp M(c);
   // keys, then one word for their span
-  if (cudaMalloc(&dk, (size_t)(n + 1) * 8) != cudaSuccess || cudaMalloc(&dv, (size_t)n * 4) != cudaSuccess) {
-    e = GB_ERR_OOM;
-    goto done;
-  }
+  const size_t o_k = M.add((size_t)(n + 1) * 8), o_v = M.add((size_t)n * 4), o_b = M.add(dev_io ? 0 : (size_t)n * 16),
+               o_b2 = M.add(sort_boxes ? (size_t)n * 16 : 0), o_p = M.add(perm_out && !dev_io ? (size_t)n * 8 : 0);
+  if (!M.get()) return GB_ERR_OOM;
+  int4* db = dev_io ? (int4*)boxes : M.ptr<int4>(o_b);
+  unsigned long long* dk = M.ptr<unsigned long long>(o_k);
+  unsigned* dv = M.ptr<unsigned>(o_v);
   if (!dev_io) cudaMemcpyAsync(db, boxes, (size_t)n * 16, cudaMemcpyHostToDevice, c.stream);
   cudaMemsetAsync(dk + n, 0, 8, c.stream);
   k_morton_keys<<<c.work_blocks, 256, 0, c.stream>>>(db, n, dk, dv, dk + n);
-  e = sort_keys_perm(ctx, dk, dv, n, dk + n);
-  if (e) goto done;
+  const int e = sort_keys_perm(ctx, dk, dv, n, dk + n);
+  if (e) return e;
   if (keys_out) cudaMemcpy(keys_out, dk, (size_t)n * 8, dev_io ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost);
   if (perm_out) {
-    long long* dp = nullptr;
-    if (dev_io) dp = perm_out;
-    else if (cudaMalloc(&dp, (size_t)n * 8) != cudaSuccess) { e = GB_ERR_OOM; goto done; }
+    long long* dp = dev_io ? perm_out : M.ptr<long long>(o_p);
     k_perm_out<<<c.work_blocks, 256, 0, c.stream>>>(dv, dp, n, perm_add);
     if (!dev_io) {
       cudaMemcpyAsync(perm_out, dp, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream);
       cudaStreamSynchronize(c.stream);
-      cudaFree(dp);
     }
   }
   if (sort_boxes) {
-    if (cudaMalloc(&db2, (size_t)n * 16) != cudaSuccess) { e = GB_ERR_OOM; goto done; }
+    int4* db2 = M.ptr<int4>(o_b2);
     k_gather_boxes<<<c.work_blocks, 256, 0, c.stream>>>(db, dv, db2, n);
     cudaMemcpyAsync(boxes, db2, (size_t)n * 16, dev_io ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                     c.stream);
   }
   cudaStreamSynchronize(c.stream);
-done:
-  if (!dev_io && db) cudaFree(db);
-  if (db2) cudaFree(db2);
-  if (dk) cudaFree(dk);
-  if (dv) cudaFree(dv);
-  return e;
+  return GB_OK;
 }
 
 extern "C" int gb_morton_sort(gb_context* ctx, c_box* boxes, long long n, int sort_boxes,
@@ -1146,14 +1197,16 @@ extern "C" int gb_canonical_sort(gb_context* ctx, c_box* boxes, long long n) {
   if (!ctx || (n > 0 && !boxes)) return GB_ERR_ARG;
   if (n <= 1) return GB_OK;
   GbCtx& c = ctx->c;
-  int4 *db = nullptr, *db2 = nullptr;
-  unsigned long long* dk = nullptr;
-  unsigned* dv = nullptr;
+  GbTmp M(c);
+  const size_t o_b = M.add((size_t)n * 16), o_b2 = M.add((size_t)n * 16), o_k = M.add((size_t)n * 8),
+               o_v = M.add((size_t)n * 4);
   int e = GB_OK;
-  if (cudaMalloc(&db, (size_t)n * 16) || cudaMalloc(&db2, (size_t)n * 16) || cudaMalloc(&dk, (size_t)n * 8) ||
-      cudaMalloc(&dv, (size_t)n * 4)) {
+  if (!M.get()) {
     e = GB_ERR_OOM;
   } else {
+    int4 *db = M.ptr<int4>(o_b), *db2 = M.ptr<int4>(o_b2);
+    unsigned long long* dk = M.ptr<unsigned long long>(o_k);
+    unsigned* dv = M.ptr<unsigned>(o_v);
     cudaMemcpyAsync(db, boxes, (size_t)n * 16, cudaMemcpyHostToDevice, c.stream);
     // LSD over the two 64-bit halves: first (x2, y2), then (x1, y1), both stable.
     k_canon_keys<<<c.work_blocks, 256, 0, c.stream>>>(db, n, dk, 1);
@@ -1169,7 +1222,6 @@ extern "C" int gb_canonical_sort(gb_context* ctx, c_box* boxes, long long n) {
       cudaStreamSynchronize(c.stream);
     }
   }
-  cudaFree(db); cudaFree(db2); cudaFree(dk); cudaFree(dv);
   return e;
 }
 
@@ -1223,6 +1275,7 @@ static int host_bool(gb_context* ctx, int control, long value, const c_box* A, u
     if (LA) gb_layer_free(ctx, LA);
     return e;
   }
+  LA->internal = LB->internal = true;
   e = run_retry(ctx, [&]() -> int {
     gb_layer* O = nullptr;
     int r;
@@ -1231,10 +1284,10 @@ static int host_bool(gb_context* ctx, int control, long value, const c_box* A, u
     else r = gb_op_bool(ctx, (int)control, LA, LB, &O);
     if (r) return r;
     unsigned long long n = 0;
-    r = gb_layer_to_host(ctx, O, nullptr, 0, &n, nullptr);
-    if (r && r != GB_ERR_CAPACITY) return r;
-    res.resize(n);
-    return gb_layer_to_host(ctx, O, res.data(), n, &n, nullptr);
+    return export_to_host(ctx, O, &n, nullptr, [&](unsigned long long k) {
+      res.resize(k);
+      return res.data();
+    }, ~0ull);
   });
   gb_layer_free(ctx, LA);
   gb_layer_free(ctx, LB);
@@ -1321,24 +1374,21 @@ extern "C" void device_event_sort(struct XYTracker* arr, int64_t n) {
   if (!ctx) return;
   GbCtx& c = ctx->c;
   const bool dev = is_device_ptr(arr);
-  TrackerWords* dt = nullptr;
-  unsigned long long *dk = nullptr, *kt = nullptr;
-  unsigned *dv = nullptr, *vt = nullptr, *range = nullptr;
-  if (dev) dt = (TrackerWords*)arr;
-  else cudaMalloc(&dt, (size_t)n * sizeof(XYTracker));
-  cudaMalloc(&dk, (size_t)n * 8);
-  cudaMalloc(&kt, (size_t)n * 8);
-  cudaMalloc(&dv, (size_t)n * 4);
-  cudaMalloc(&vt, (size_t)n * 4);
-  cudaMalloc(&range, 16);
-  if (dt && dk && kt && dv && vt && range) {
+  GbTmp M(c);
+  const size_t o_k = M.add((size_t)n * 8), o_kt = M.add((size_t)n * 8), o_v = M.add((size_t)n * 4),
+               o_vt = M.add((size_t)n * 4), o_r = M.add(16), o_t = M.add(dev ? 0 : (size_t)n * sizeof(XYTracker));
+  if (M.get()) {
+    TrackerWords* dt = dev ? (TrackerWords*)arr : M.ptr<TrackerWords>(o_t);
+    unsigned long long *dk = M.ptr<unsigned long long>(o_k), *kt = M.ptr<unsigned long long>(o_kt);
+    unsigned *dv = M.ptr<unsigned>(o_v), *vt = M.ptr<unsigned>(o_vt), *range = M.ptr<unsigned>(o_r);
     if (!dev) cudaMemcpyAsync(dt, arr, (size_t)n * sizeof(XYTracker), cudaMemcpyHostToDevice, c.stream);
     cudaMemsetAsync(range, 0xff, 8, c.stream);
     cudaMemsetAsync(range + 2, 0, 8, c.stream);
     k_tracker_range<<<c.work_blocks, 256, 0, c.stream>>>(dt, n, range);
-    unsigned r[4] = {0, 0, 0, 0};
-    cudaMemcpyAsync(r, range, 16, cudaMemcpyDeviceToHost, c.stream);
-    cudaStreamSynchronize(c.stream);
+    HostBack h;
+    read_back(ctx, &h, range, 2);
+    unsigned r[4];
+    memcpy(r, h.w, 16);
     auto width = [](unsigned v) {
       int b = 0;
       while (b < 32 && (v >> b)) ++b;
@@ -1358,12 +1408,6 @@ extern "C" void device_event_sort(struct XYTracker* arr, int64_t n) {
     }
     if (e) fprintf(stderr, "device_event_sort: sort failed (%s)\n", gb_last_error(ctx));
   } else {
-    fprintf(stderr, "device_event_sort: cudaMalloc failed\n");
+    fprintf(stderr, "device_event_sort: no device memory\n");
   }
-  if (!dev && dt) cudaFree(dt);
-  if (dk) cudaFree(dk);
-  if (kt) cudaFree(kt);
-  if (dv) cudaFree(dv);
-  if (vt) cudaFree(vt);
-  if (range) cudaFree(range);
 }

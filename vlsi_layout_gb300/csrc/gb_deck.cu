@@ -276,15 +276,14 @@ static int op1_host_impl(gb_context* ctx, const c_box* boxes, unsigned long long
       cudaMemcpyAsync(dbox + b0 * 16, boxes + b0, (size_t)(b1 - b0) * 16, cudaMemcpyHostToDevice, c.copy_stream);
     cudaEventRecord(ev[g], c.copy_stream);
   }
-  long long* dcounts = nullptr;
-  long long* darea = nullptr;
-  unsigned long long* ddig = nullptr;
-  DLayer** dl = nullptr;
-  int e = GB_OK;
-  if (cudaMalloc(&dcounts, (size_t)ncell * 6 * 8) != cudaSuccess || cudaMalloc(&darea, (size_t)ncell * 8) != cudaSuccess ||
-      cudaMalloc(&dl, 8 * sizeof(DLayer*)) != cudaSuccess ||
-      (digests && cudaMalloc(&ddig, (size_t)ncell * 6 * 8) != cudaSuccess))
-    e = set_err(ctx, GB_ERR_OOM, "deck result buffers");
+  GbTmp M(c);
+  const size_t o_counts = M.add((size_t)ncell * 6 * 8), o_area = M.add((size_t)ncell * 8), o_dl = M.add(8 * sizeof(DLayer*)),
+               o_dig = M.add(digests ? (size_t)ncell * 6 * 8 : 0);
+  int e = M.get() ? GB_OK : set_err(ctx, GB_ERR_OOM, "deck result buffers");
+  long long* dcounts = M.ptr<long long>(o_counts);
+  long long* darea = M.ptr<long long>(o_area);
+  unsigned long long* ddig = digests ? M.ptr<unsigned long long>(o_dig) : nullptr;
+  DLayer** dl = M.ptr<DLayer*>(o_dl);
   for (int g = 0; g < ng && !e; ++g) {
     const int k0 = cut[g], k1 = cut[g + 1];
     const long long b0 = off[k0];
@@ -294,6 +293,7 @@ static int op1_host_impl(gb_context* ctx, const c_box* boxes, unsigned long long
     gb_layer* P = nullptr;
     e = gbi::layer_over_device(ctx, dbox + b0 * 16, off[k1] - b0, goff.data(), k1 - k0, &P);
     if (e) break;
+    P->internal = true;
     const int gn = k1 - k0;
     e = gb_run_retry(ctx, [&]() -> int {
       gb_layer* outs[6];
@@ -326,10 +326,6 @@ static int op1_host_impl(gb_context* ctx, const c_box* boxes, unsigned long long
   }
   for (cudaEvent_t x : ev) cudaEventDestroy(x);
   cudaEventDestroy(ready);
-  if (dcounts) cudaFree(dcounts);
-  if (darea) cudaFree(darea);
-  if (ddig) cudaFree(ddig);
-  if (dl) cudaFree(dl);
   return e;
 }
 

@@ -48,6 +48,55 @@ struct GbCtx {
   void* io_buf = nullptr;            // device staging of host inputs (gb_op1_host), grow-only
   size_t io_cap = 0;
   cudaStream_t copy_stream = nullptr;  // host-to-device copies that overlap the compute stream
+  cudaMemPool_t pool = nullptr;      // layers and call temporaries (gb_tmp_alloc), in the order of the stream
+  unsigned long long* dmarks = nullptr;  // arena marks kept on the device [GB_DMARKS]
+  struct HostBack* hb = nullptr;     // pinned: where read_back's copies land
+};
+
+// What one synchronisation brings back: the status and up to 8 words.
+struct HostBack {
+  DStatus st;
+  long long w[8];
+};
+#define GB_DMARKS 64
+// The pool keeps at most this much memory that is not in use (the rest goes
+// back at the next synchronisation, all of it with the context): cudaMalloc
+// and cudaFree of the temporaries of a call cost more than its kernels (sort
+// of 20M trackers: 900 of 2000 us).
+#define GB_POOL_KEEP (4ull << 30)
+
+// Temporary device memory of one call or layer, in the order of the context's
+// stream; freed with gb_tmp_free.  Null when there is no memory, or (as
+// cudaMalloc) while the stream is being captured.
+inline void* gb_tmp_alloc(GbCtx& c, size_t bytes) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
+  void* p = nullptr;
+  if (cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, c.pool, c.stream) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+inline void gb_tmp_free(GbCtx& c, void* p) {
+  if (p) cudaFreeAsync(p, c.stream);
+}
+// Several arrays in one allocation, each on 256 bytes.
+struct GbTmp {
+  GbCtx& c;
+  char* base = nullptr;
+  size_t size = 0, at = 0;
+  explicit GbTmp(GbCtx& ctx) : c(ctx) {}
+  GbTmp(const GbTmp&) = delete;
+  ~GbTmp() { gb_tmp_free(c, base); }
+  size_t add(size_t bytes) {
+    const size_t o = size;
+    size += (bytes + 255) & ~(size_t)255;
+    return o;
+  }
+  bool get() { return (base = (char*)gb_tmp_alloc(c, size)) != nullptr; }
+  template <typename T>
+  T* ptr(size_t off) const { return reinterpret_cast<T*>(base + off); }
 };
 
 struct gb_layer {
@@ -60,9 +109,10 @@ struct gb_layer {
   int arena_owned = 0;  // arrays live in the work arena
   unsigned long long seq = 0;  // creation sequence (arena layers)
   bool dead = false;
-  void* own_boxes = nullptr;  // raw layers: cudaMalloc'd arrays
-  void* own_coff = nullptr;
-  void* own_cell = nullptr;
+  bool internal = false;  // made and freed within one call, on the context's stream alone
+  void* own_boxes = nullptr;  // raw layers: the boxes (unless borrowed), in
+  void* own_cell = nullptr;   // their one allocation
+  int4* cbox = nullptr;       // raw layers: the cells' bounding boxes (device)
   gb_layer* bin_cache = nullptr;
   long long nbox_host = 0;
 };
@@ -70,6 +120,7 @@ struct gb_layer {
 struct gb_context {
   GbCtx c;
   std::mutex mu;
+  std::mutex hb_mu;  // c.hb, for the time of one read_back
   unsigned long long seq = 0;
   std::vector<gb_layer*> arena_layers;
   std::vector<std::pair<unsigned long long, unsigned long long>> marks;  // (device off, seq)

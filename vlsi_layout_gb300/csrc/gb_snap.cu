@@ -1400,18 +1400,17 @@ k_snappy_decompress(const unsigned char* __restrict__ in_all, const long long* _
 }
 
 // ---------------------------------------------------------------- host side
-struct DevMem {  // stream-ordered scratch, freed on scope exit
-  cudaStream_t s;
+struct DevMem {  // scratch from the context's pool, freed on scope exit
+  GbCtx& c;
   std::vector<void*> ptrs;
-  explicit DevMem(cudaStream_t st) : s(st) {}
+  explicit DevMem(GbCtx& ctx) : c(ctx) {}
   ~DevMem() {
-    for (void* p : ptrs) cudaFreeAsync(p, s);
+    for (void* p : ptrs) gb_tmp_free(c, p);
   }
   template <class T>
   T* get(size_t count) {
-    void* p = nullptr;
-    if (cudaMallocAsync(&p, std::max<size_t>(count * sizeof(T), 16), s) != cudaSuccess) return nullptr;
-    ptrs.push_back(p);
+    void* p = gb_tmp_alloc(c, std::max<size_t>(count * sizeof(T), 16));
+    if (p) ptrs.push_back(p);
     return (T*)p;
   }
 };
@@ -1428,7 +1427,7 @@ int snap_encode(gb_context* ctx, const int4* d_boxes, long long n, int method, u
   const long long nch = nchunks_of(n);
   *total = 0;
   if (nch == 0) return GB_OK;
-  DevMem M(c.stream);
+  DevMem M(c);
   long long* d_rsize = M.get<long long>(nch);
   long long* d_roff = M.get<long long>(nch + 1);
   int* d_ovf = M.get<int>(2 * nch + 2);  // the widths' and heights' counts of chunks that need global tables, then these
@@ -1560,7 +1559,7 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
   if (method == 0)
     for (long long i = 0; i < nch; ++i)
       if (rlen[i] != clen[i]) return gbi::set_err(ctx, GB_ERR_CORRUPT, "snap chunk sizes");
-  DevMem M(c.stream);
+  DevMem M(c);
   std::vector<long long> sblk(nch + 1, 0);  // blocks of segments before each chunk
   for (long long i = 0; i < nch; ++i)
     sblk[i + 1] = sblk[i] + (std::min(rlen[i], (long long)SN_CHUNK * SN_LMAX) + SN_SEGB - 1) / SN_SEGB;
