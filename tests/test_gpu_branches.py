@@ -137,3 +137,35 @@ def test_event_ranges(n, lo, hi):
     t["pad"] = rng.integers(-128, 128, (n, 3))
     exp = t[np.lexsort((t["Y"], t["X"]))]
     assert engine.event_sort(t).tobytes() == exp.tobytes()
+
+
+# tiles shared by 8, 4, 2 and 1 CTAs; wires that run through every share of a tile, and a tile with one sub-band
+@pytest.mark.parametrize("side", [1, 2, 6, 7, 9, 10, 13, 14, 15, 20])
+def test_shared_tiles(ctx, oracle, side):
+    die, rng = side * 65536, np.random.default_rng(side)
+    n = 120 * side * side
+    A = random_layer(n, die=die, wmin=20, wmax=2500, seed=side)
+    y = np.sort(rng.integers(0, die - 40, 60 * side))
+    wires = np.stack([rng.integers(0, 3000, len(y)), y, die - rng.integers(0, 3000, len(y)), y + rng.integers(1, 30, len(y))],
+                     1).astype(np.int32)
+    A = np.concatenate([A, wires, [[5, 5, 9, 9]]]).astype(np.int32)
+    B = random_layer(n // 2 + 1, die=die, seed=side + 100)
+    for op in (0, 1, 2, 3, 4):
+        got = run(ctx, lambda: ctx.op(op, ctx.layer(A), ctx.layer(B) if op != 4 else None))
+        assert np.array_equal(got, oracle.boolean(A, B, op) if op != 4 else oracle.merge(A)), op
+    assert np.array_equal(run(ctx, lambda: ctx.op(7, ctx.layer(A))), oracle.boolean(A, A[:0], 7))
+    assert np.array_equal(run(ctx, lambda: ctx.size(ctx.layer(A), -6)), oracle.size(A, -6))
+    m = ctx.mark()
+    assert int(ctx.area(ctx.layer(A))[0]) == oracle.union_area(A)
+    ctx.release(m)
+
+
+def test_shared_tile_capacity(oracle):
+    """A scratch that one CTA's share outgrows: the op is retried or spills, and stays exact."""
+    from vlsi_layout_gb300 import engine
+    A = random_layer(6000, die=60_000, wmin=20, wmax=9000, seed=1)
+    B = random_layer(6000, die=60_000, wmin=20, wmax=9000, seed=2)
+    with engine.Context(0, 1 << 30) as ctx:
+        ctx._chk(engine.lib().gb_set_tile_scratch(ctx.h, 64 << 10))
+        got = run(ctx, lambda: ctx.op(0, ctx.layer(A), ctx.layer(B)))
+    assert np.array_equal(got, oracle.boolean(A, B, 0))

@@ -24,6 +24,7 @@ struct GbCtx {
   int work_blocks = 0;     // persistent grid of streaming kernels
   int tile_blocks = 0;     // persistent grid of the tile kernel (1 CTA / SM)
   size_t tile_smem = 0;
+  int split_ctas = 0;      // grid of the tile kernel whose CTAs share tiles (clusters of 8; 0: none)
   DStatus* st = nullptr;   // device
   char* arena = nullptr;   // work arena (device bump allocation)
   unsigned long long arena_cap = 0;

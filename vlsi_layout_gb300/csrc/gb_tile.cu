@@ -42,9 +42,15 @@
 //     slots are reserved while the links are made.  Strips are written in
 //     (sub-band, column, row) order, so the output of a tile is
 //     deterministic.
-// No CTA ever waits on another CTA.  The only waits are on the CTA's own
-// mbarrier for the bulk copies of phases A and D; each is bounded (a poll
+// Layers of few tiles: one tile per CTA would leave most of the chip idle, so a
+// cluster's CTAs then share tiles (k_tile<false, true>): each ranks the whole
+// tile, takes a contiguous share of the sub-bands through phases B to D, and
+// chains that run on into the next CTA's share are followed through a table of
+// that CTA's continuations.  These CTAs meet at two hardware cluster barriers.
+// Otherwise no CTA ever waits on another CTA.  The only other waits are on the
+// CTA's own mbarrier for the bulk copies of phases A and D; each is bounded (a poll
 // limit, then GB_ERR_TIMEOUT and the CTA leaves after its copies land).
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
@@ -154,7 +160,46 @@ struct TileSmem {
   int** sbol;    // open list (then continuation list) per sub-band
   PieceRec** sbrec;  // strip pieces per sub-band (global piece index = sbinfo.x + local index)
   int* succ;
+  int q0, nsbg;  // a shared tile: the CTA's first sub-band, the tile's sub-bands
+  int2* cont;    // a shared tile: the CTA's continuations from the CTA before it (ordinal, end)
 };
+
+// A tile shared by several CTAs: what a CTA tells the others, at the start of its scratch.
+struct SplitPub {
+  int err;          // 1 until the CTA's strips are known
+  int H;            // strips that start in its share
+  int nc;           // continuations: (ordinal among the open pieces of the CTA before, end), in order
+  int pad;
+  int2* cont;       // end >= 0: end slab; else -1 - (ordinal among its own open pieces)
+  long long obase;  // first CTA of the tile: the output slots (-1: none)
+};
+#define TK_PUB_BYTES 64
+static_assert(sizeof(SplitPub) <= TK_PUB_BYTES, "published words");
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Where a chain that is open at the end of CTA `me`'s share ends: open ordinal
+// o is looked up among the continuations of the CTAs after it.  pub(j) is CTA
+// j's words, ka the tile's CTAs, nsbg its sub-bands.
+__device__ __forceinline__ int split_end(const char* pub0, unsigned long long scr, int me, int ka, int nsbg, int o) {
+  for (int j = me + 1; j < ka; ++j) {
+    const SplitPub* p = reinterpret_cast<const SplitPub*>(pub0 + (size_t)j * scr);
+    const int2* c = (const int2*)__ldcg((const unsigned long long*)&p->cont);
+    int lo = 0, hi = __ldcg(&p->nc);
+    while (lo < hi) {  // first continuation of ordinal >= o
+      const int mid = (lo + hi) >> 1;
+      if (__ldcg(&c[mid].x) < o) lo = mid + 1;
+      else hi = mid;
+    }
+    const bool found = lo < __ldcg(&p->nc) && __ldcg(&c[lo].x) == o;
+    if (!found) return 63 * (int)((long long)nsbg * j / ka);  // it ends where that share starts
+    const int e = __ldcg(&c[lo].y);
+    if (e >= 0) return e;
+    o = -1 - e;
+  }
+  return 0;  // not reached: the last share has no open pieces
+}
 // Wide lists of phase C, alternating by level, behind the metadata and the hand-out order in xyv.
 #define TK_WLIST(s, level) ((s).xyv + TK_MD_INTS + TK_SBS + ((level) & 1) * (TK_NSBMAX + 2))
 static_assert(TK_MD_INTS + TK_SBS + 2 * (TK_NSBMAX + 2) <= 2 * TK_WMAX + 2 * (TK_WMAX / 2 + 1), "wide lists");
@@ -305,7 +350,7 @@ __device__ __forceinline__ void tile_lookup(int op, const DLayer* A, const DLaye
 // WIDE: the level's larger buffers (level 1..3).  Returns false, with nothing
 // done, when the sub-band needs the next level's buffers; at the last level
 // columns beyond them spill to the scratch.
-template <bool TIMING, bool WIDE>
+template <bool TIMING, bool WIDE, bool SPLIT>
 __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int nA, char* base,
                              unsigned long long scr, int level, long long* tctr) {
   if (!TIMING) tctr = nullptr;
@@ -331,7 +376,8 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     }
     return true;
   }
-  const int rowbase = 63 * sb - 1;
+  const int gsb = SPLIT ? s.q0 + sb : sb;  // of the tile; sb and nsb count the CTA's share
+  const int rowbase = 63 * gsb - 1;
   const int nwy = ((Ny - 1) >> 5) + 1;
   const int lcn = WIDE ? wide_cols(level) : TK_LCN, mcn = WIDE ? wide_mc(level) : TK_MC;
   if (nwy > (WIDE ? wide_lbw(level) : TK_LBW)) return false;  // the last level holds any tile's y ranks
@@ -591,7 +637,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   }
   unsigned long long Fin = __shfl_up_sync(0xffffffffu, IA, 1);
   if (lane == 0) Fin = 0ull;
-  const bool last_sb = (sb == nsb - 1);
+  const bool last_sb = gsb == (SPLIT ? s.nsbg : nsb) - 1;
   TSTEP(2)
 
   // ---- count pieces / opens / heads
@@ -614,7 +660,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       cb[c] = Z | ((Chg >> 1) & 1ull);  // bit 0 of Z is always clear
       const int pc = __popcll(Z);
       const int open = !last_sb && (Ec >> 63);
-      const int cont = (sb > 0) && ((Z >> 1) & 1ull) && !((Chg >> 1) & 1ull);
+      const int cont = (gsb > 0) && ((Z >> 1) & 1ull) && !((Chg >> 1) & 1ull);
       if (packed) {
         pf[c] = pv;
         pv += ((unsigned long long)(unsigned)((int)(Ec & 1ull) << 20 | cont << 10 | open) << 32) |
@@ -720,7 +766,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
           zs = cb[c];
           Z = zs & ~1ull;
           Ec = ca[c] & ~R(c + 1);
-          contc = (sb > 0) && ((Z >> 1) & 1ull) && !(zs & 1ull);
+          contc = (gsb > 0) && ((Z >> 1) & 1ull) && !(zs & 1ull);
           if (packed) break;
           const int pc = __popcll(Z);
           if (j < pc) break;
@@ -789,8 +835,10 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
 // that the loads of one (record, table values) overlap those of the others.  A strip's chain runs through as many
 // sub-bands as the strip spans, so its links are what bounds the step: on chip (16 bits, sl16) a hop takes an L1
 // latency and not L2's.  Out of line: its registers stay out of the kernel's main path.  Returns the area.
+template <bool SPLIT>
 __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* recs, int NP, int nsb, const int* Xv,
-                                                    const int* Yv, unsigned long long* outp, bool sl16) {
+                                                    const int* Yv, unsigned long long* outp, bool sl16,
+                                                    const char* pub0, unsigned long long scr, int me, int ka) {
   const PieceRec* rg = reinterpret_cast<const PieceRec*>(recs);
   const unsigned short* s16 = reinterpret_cast<const unsigned short*>(s.dbuf);
   const int* s32 = s.succ;
@@ -831,13 +879,14 @@ __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* rec
         nx[u] = next(q);
       }
       if (q >= 0) r[u].w = rec(q).w;
+      if (SPLIT && nx[u] <= -2) r[u].w = split_end(pub0, scr, me, ka, s.nsbg, -2 - nx[u]);
     }
 #pragma unroll
     for (int u = 0; u < TK_DU; ++u) {
       if (pr_cont(r[u])) continue;
       const int slo = pr_slo(r[u]);
       const int xs = Xv[slo], xe = Xv[pr_shi(r[u])], ylo = Yv[pr_ylo(r[u])], yhi = Yv[pr_yhi(r[u])];
-      if (outp) outp[s.sbh[slo / 63] + pr_hrank(r[u])] = gb_pack(xs, ylo, xe, yhi);
+      if (outp) outp[s.sbh[slo / 63 - (SPLIT ? s.q0 : 0)] + pr_hrank(r[u])] = gb_pack(xs, ylo, xe, yhi);
       area += (long long)(xe - xs) * (long long)(yhi - ylo);
     }
   }
@@ -846,7 +895,7 @@ __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* rec
 
 // Levels 1..3 of phase C: the wide sub-bands that the level below listed, by fewer warps with larger buffers.
 // Called by the whole CTA after level 0.  Out of line: its registers stay out of the kernel's narrow path.
-template <bool TIMING>
+template <bool TIMING, bool SPLIT>
 __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int nA, char* base,
                                        unsigned long long scr, long long* tctr) {
   for (int level = 1; level <= TK_WLEVELS; ++level) {
@@ -862,17 +911,29 @@ __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int
       k = __shfl_sync(0xffffffffu, k, 0);
       if (k >= todo) break;
       const int sb = TK_WLIST(s, level - 1)[k];
-      if (!tile_subband<TIMING, true>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && gb_lane() == 0)
+      if (!tile_subband<TIMING, true, SPLIT>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && gb_lane() == 0)
         TK_WLIST(s, level)[atomicAdd(&s.nwide[level], 1)] = sb;
       __syncwarp();
     }
   }
 }
 
-template <bool TIMING>
+// CTAs per tile for a layer of nt tiles when `ctas` CTAs can share (a multiple
+// of 8; 0: never): as many as the chip holds, at least two, else 1.  Sharing
+// repeats the ranking (a quarter of a small tile's time), so it pays while it
+// fills idle CTAs and not beyond.  XOR of two standard-cell layers, one CTA per
+// tile and shared: 9 tiles 1350 -> 541 us, 25 tiles 1400 -> 553 us, 81 tiles
+// 1485 -> 776 us; area of 144 tiles (50000 boxes) 198 -> 161 us.
+__device__ __forceinline__ int tile_share(long long nt, int ctas) {
+  return nt * 8 <= ctas ? (ctas ? 8 : 1) : nt * 4 <= ctas ? 4 : nt * 2 <= ctas ? 2 : 1;
+}
+
+// SPLIT: clusters of 8 CTAs, groups of `ka` of them share a tile each; every
+// CTA passes two cluster barriers and takes one tile at most.
+template <bool TIMING, bool SPLIT>
 __global__ void __launch_bounds__(TK_NT, 3)
 k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, char* scratch,
-       unsigned long long scr, long long* counter, DStatus* st) {
+       unsigned long long scr, long long* counter, DStatus* st, int split_ctas) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TileSmem& s = *reinterpret_cast<TileSmem*>(smraw);
   const int tid = threadIdx.x;
@@ -882,6 +943,17 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
   const bool timing = TIMING && (mode & 4) != 0;
   mode &= 3;
   long long tA = 0, tB = 0, tC = 0, tD = 0, t0 = 0;
+  const int share = tile_share(O->ntiles, split_ctas);
+  if ((share > 1) != SPLIT) return;  // the other launch takes the layer (the same on every CTA)
+  // a shared tile: the CTA's place among the tile's CTAs, the first one's scratch
+  const int me = SPLIT ? (int)blockIdx.x % share : 0;
+  const char* const pub0 = scratch + (size_t)(blockIdx.x - me) * scr;
+  SplitPub* const pub = reinterpret_cast<SplitPub*>(base);
+  int ka = 1;  // CTAs that have a part of the tile
+  if (SPLIT && tid == 0) {
+    pub->err = 1;  // until the CTA has its strips
+    __threadfence();
+  }
   const unsigned mbar = tk_smem(&s.mbar);
   unsigned mph = 0;  // parity of the mbarrier phase the next bulk copies complete
   if (tid == 0) {
@@ -897,24 +969,31 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       s.st = st;
       TileRef r;
       if (s.have_nx) r = s.nx;
+      else if (SPLIT) tile_lookup(op, A, B, O, blockIdx.x / share, r);
       else tile_lookup(op, A, B, O, st->err ? (1ll << 62) : (long long)atomicAdd((unsigned long long*)counter, 1ull), r);
       s.have_nx = 0;
-      if (st->err) r.tile = 1ll << 62;  // an error stops the CTA, a reserved tile too
+      if (st->err && !SPLIT) r.tile = 1ll << 62;  // an error stops the CTA, a reserved tile too
       s.tile = r.tile;
       s.nA = r.nA;
       s.nB = r.nB;
       s.pa = r.pa;
       s.pb = r.pb;
       s.cell = r.cell;
-      s.up = 0;
+      s.up = SPLIT ? TK_PUB_BYTES : 0;
       s.down = 0;
-      s.err = 0;
+      s.err = SPLIT && st->err;
       s.rsplit = 0;
     }
     __syncthreads();
     const long long t = s.tile;
-    if (t >= O->ntiles) break;
+    if (!SPLIT && t >= O->ntiles) break;
     const int nA = s.nA, nB = s.nB, P = nA + nB;
+    if (SPLIT && (t >= O->ntiles || P == 0 || s.err)) {  // the same for the tile's CTAs, but for s.err: published
+      if (tid == 0 && me == 0 && t < O->ntiles) { O->tcount[t] = 0; O->tstart[t] = 0; }
+      cluster_sync();
+      cluster_sync();
+      break;
+    }
     if (P == 0) {
       if (tid == 0) { O->tcount[t] = 0; O->tstart[t] = 0; }
       continue;
@@ -1032,7 +1111,18 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       }
     }
     const int nslab = Nx - 1;
-    const int nsb = (nslab + 62) / 63;
+    const int nsbg = (nslab + 62) / 63;
+    int q0 = 0, q1 = nsbg;  // the CTA's sub-bands
+    if (SPLIT) {
+      ka = min(share, nsbg);
+      q0 = (int)((long long)nsbg * min(me, ka) / ka);
+      q1 = (int)((long long)nsbg * min(me + 1, ka) / ka);
+      if (tid == 0) {
+        s.q0 = q0;
+        s.nsbg = nsbg;
+      }
+    }
+    const int nsb = q1 - q0;
     if (timing) { __syncthreads(); const long long t1 = clock64(); tA += t1 - t0; t0 = t1; }
     // ---- B: sub-band membership (counting sort in shared memory)
     if (tid == 0) s.sbc = nsb <= TK_SBS ? s.sbc_s : (int*)sc_up(s, base, half, (unsigned long long)(nsb + 2) * 4);
@@ -1057,10 +1147,14 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
             int x1, y1, x2, y2;
             gb_unpack(pk[u], x1, y1, x2, y2);
             const int r1 = bm_rank2(s.xb, s.xp, x1), r2 = bm_rank2(s.xb, s.xp, x2);
-            const int c1 = bm_rank2(s.yb, s.yp, y1), c2 = bm_rank2(s.yb, s.yp, y2);
+            const int lo = max(r1 / 63, q0), hi = min(q1 - 1, r2 / 63);
+            int c1 = 0, c2 = 0;
+            if (!SPLIT || lo <= hi) {
+              c1 = bm_rank2(s.yb, s.yp, y1);
+              c2 = bm_rank2(s.yb, s.yp, y2);
+            }
             s.rk[i] = make_int4(r1, r2, c1, c2);
-            const int lo = r1 / 63, hi = min(nsb - 1, r2 / 63);
-            for (int q = lo; q <= hi; ++q) atomicAdd(&s.sbc[q], 1);
+            for (int q = lo; q <= hi; ++q) atomicAdd(&s.sbc[q - q0], 1);
           }
         }
       }
@@ -1114,9 +1208,9 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
           const int i = i0 + u * TK_NT;
           if (i < P) {
             const int4 r = rr[u];
-            const int lo = r.x / 63, hi = min(nsb - 1, r.y / 63);
+            const int lo = max(r.x / 63, q0), hi = min(q1 - 1, r.y / 63);
             const int4 rec = make_int4(r.x | (i >= nA ? (int)0x80000000 : 0), r.y, r.z, r.w);
-            for (int q = lo; q <= hi; ++q) memp[atomicAdd(&s.sbc[q], 1)] = rec;
+            for (int q = lo; q <= hi; ++q) memp[atomicAdd(&s.sbc[q - q0], 1)] = rec;
           }
         }
       }
@@ -1161,13 +1255,13 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         if (k >= nsb) break;
         const int sb = lpt ? ord[k] : k;
         if (__any_sync(0xffffffffu, list) ||
-            !tile_subband<TIMING, false>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
+            !tile_subband<TIMING, false, SPLIT>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
           if (gb_lane() == 0) TK_WLIST(s, 0)[atomicAdd(&s.nwide[0], 1)] = sb;
         }
       }
     }
     __syncthreads();
-    if (s.nwide[0]) tile_wide<TIMING>(s, op, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
+    if (s.nwide[0]) tile_wide<TIMING, SPLIT>(s, op, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
     if (tid == 0 && !s.err) s.hint = direct ? s.narrow * 4 <= nsb : s.nwide[0] * 4 >= nsb * 3;
     // the bulk copies of phase D (async proxy) read the records written above and overwrite shared
     // memory written in phases A-C (generic proxy)
@@ -1194,20 +1288,29 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     const int nx4 = (Nx + 3) & ~3, ny4 = (Ny + 3) & ~3;  // tables start on 16-byte boundaries
     const bool xys = nx4 + ny4 + xyoff <= 2 * TK_WMAX + 2 * (TK_WMAX / 2 + 1);
     // chain links of a tile whose records stay in the scratch: 16 bits each on chip when they fit
-    const bool sl16 = !prs && NP * 2 <= DBYTES;
+    const bool sl16 = !SPLIT && !prs && NP * 2 <= DBYTES;
     if (tid == 0 && !s.err && !prs && !sl16) s.succ = (int*)sc_up(s, base, half, (unsigned long long)NP * 4 + 4);
+    const int nc0 = SPLIT && me > 0 && nsb > 0 && !s.err ? s.sbct[0] : 0;  // continuations from the CTA before
+    if (SPLIT && tid == 0 && nc0) s.cont = (int2*)sc_up(s, base, half, (unsigned long long)nc0 * 8);
     __syncthreads();
     if (s.err) {
       if (tid == 0) {
-        O->tcount[t] = 0;
-        O->tstart[t] = 0;
+        if (me == 0) {
+          O->tcount[t] = 0;
+          O->tstart[t] = 0;
+        }
         gb_set_error(st, GB_ERR_CAPACITY, KID_TILE, (long long)scr * 2);
+      }
+      if (SPLIT) {
+        cluster_sync();
+        cluster_sync();
+        break;
       }
       continue;
     }
     // the next tile's reservation (the work counter) and its descriptor load run on the last thread while
     // the bulk copies below land
-    if (tid == TK_NT - 1 && !st->err) {
+    if (!SPLIT && tid == TK_NT - 1 && !st->err) {
       tile_lookup(op, A, B, O, (long long)atomicAdd((unsigned long long*)counter, 1ull), s.nx);
       s.have_nx = 1;
     }
@@ -1264,7 +1367,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       H = (int)carry;
     }
     __syncthreads();
-    if (tid == TK_NT - 32) {  // read after the links' barrier
+    if (!SPLIT && tid == TK_NT - 32) {  // read after the links' barrier
       s.obase = -1;
       if (mode == 0 && H > 0) {
         atomicAdd((unsigned long long*)&O->ntot, (unsigned long long)H);
@@ -1294,7 +1397,75 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         } else gb_set_error(st, GB_ERR_INTERNAL, KID_TILE, t);
       }
     }
+    if (SPLIT && me < ka - 1 && nsb > 0) {  // open at the end of the share: -2 - ordinal
+      const int no = s.sbinfo[nsb - 1].z;
+      const int* ol = s.sbol[nsb - 1];
+      for (int k = tid; k < no; k += TK_NT) succ[ol[k]] = -2 - k;
+    }
     __syncthreads();
+    if (SPLIT) {
+      if (nc0) {  // where the chains that come in end
+        const int* cl = s.sbol[0] + s.sbinfo[0].z;
+        const PieceRec* rg = reinterpret_cast<const PieceRec*>(base + (half & ~15ull));
+        for (int k = tid; k < nc0; k += TK_NT) {
+          int q = cl[k], e, guard = 0;
+          while ((e = succ[q]) >= 0 && guard++ <= nsb) q = e;
+          if (e > -2) {
+            if (prs) e = pr_shi(PR[q]);
+            else if (!s.rsplit) e = pr_shi(rg[q]);
+            else {
+              int sb = 0;
+              for (; sb < nsb - 1; ++sb)
+                if (q >= s.sbinfo[sb].x && q < s.sbinfo[sb].x + s.sbinfo[sb].y) break;
+              e = pr_shi(s.sbrec[sb][q - s.sbinfo[sb].x]);
+            }
+          } else {
+            e += 1;  // -1 - ordinal
+          }
+          s.cont[k] = make_int2(cl[nc0 + k], e);
+        }
+      }
+      if (tid == 0) {
+        pub->H = H;
+        pub->nc = nc0;
+        pub->cont = s.cont;
+        pub->err = 0;
+      }
+      cluster_sync();
+      int before = 0, total = 0, bad = 0;
+      for (int j = 0; j < ka; ++j) {
+        const SplitPub* pj = reinterpret_cast<const SplitPub*>(pub0 + (size_t)j * scr);
+        const int h = __ldcg(&pj->H);
+        bad |= __ldcg(&pj->err);
+        if (j < me) before += h;
+        total += h;
+      }
+      if (me == 0 && tid == 0) {
+        long long o = -1;
+        if (mode == 0 && total > 0 && !bad) {
+          atomicAdd((unsigned long long*)&O->ntot, (unsigned long long)total);
+          o = (long long)atomicAdd((unsigned long long*)&O->nused, (unsigned long long)total);
+          if (o + total > O->npcs) {
+            unsigned long long* p =
+                (unsigned long long*)gb_arena_alloc_atomic(st, (unsigned long long)total * 8ull, KID_TILE + 1);
+            o = p ? (long long)(p - O->pcs) : -1;
+          }
+        }
+        pub->obase = o;
+      }
+      cluster_sync();
+      if (bad) {  // a CTA of the tile failed and said so
+        if (tid == 0 && me == 0) {
+          O->tcount[t] = 0;
+          O->tstart[t] = 0;
+        }
+        break;
+      }
+      H = total;
+      if (tid == 0) s.obase = __ldcg(&reinterpret_cast<const SplitPub*>(pub0)->obase);
+      for (int q = tid; q < nsb; q += TK_NT) s.sbh[q] += before;
+      __syncthreads();
+    }
     const long long obase = s.obase;
     unsigned long long* outp = obase >= 0 ? O->pcs + obase : nullptr;
     long long area = 0;
@@ -1306,18 +1477,20 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         if (pr_cont(pr)) continue;
         int q = p, guard = 0;
         while (succ[q] >= 0 && guard++ <= nsb) q = succ[q];
-        const int shi = q == p ? pr_shi(pr) : pr_shi(PR[q]);
+        int shi = q == p ? pr_shi(pr) : pr_shi(PR[q]);
+        if (SPLIT && succ[q] <= -2) shi = split_end(pub0, scr, me, ka, nsbg, -2 - succ[q]);
         const int slo = pr_slo(pr);
         const int xs = Xv[slo], xe = Xv[shi], ylo = Yv[pr_ylo(pr)], yhi = Yv[pr_yhi(pr)];
-        const int pos = s.sbh[slo / 63] + pr_hrank(pr);
+        const int pos = s.sbh[slo / 63 - q0] + pr_hrank(pr);
         if (outp) outp[pos] = gb_pack(xs, ylo, xe, yhi);
         area += (long long)(xe - xs) * (long long)(yhi - ylo);
       }
     } else {
-      area = tile_emit_scratch(s, base + (half & ~15ull), NP, nsb, Xv, Yv, outp, sl16);
+      area = tile_emit_scratch<SPLIT>(s, base + (half & ~15ull), NP, nsb, Xv, Yv, outp, sl16, pub0, scr, me, ka);
     }
     area = gb_block_sum(area, s.tmp64);
-    if (tid == 0) {
+    if (SPLIT && tid == 0 && me > 0) atomicAdd((unsigned long long*)&O->cell_area[s.cell], (unsigned long long)area);
+    if (tid == 0 && me == 0) {
       if (mode == 0) {
         O->tcount[t] = obase >= 0 ? H : 0;
         O->tstart[t] = obase >= 0 ? obase : 0;
@@ -1337,6 +1510,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       atomicAdd((unsigned long long*)&counter[8], (unsigned long long)P * 8ull);
       atomicAdd((unsigned long long*)&counter[9], (unsigned long long)(mode == 0 ? H : 0) * 8ull);
     }
+    if (SPLIT) break;
   }
   if (timing && threadIdx.x == 0) {
     atomicAdd((unsigned long long*)&counter[16], (unsigned long long)tA);
@@ -1346,13 +1520,37 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
   }
 }
 
+static cudaLaunchConfig_t split_config(GbCtx& c, cudaLaunchAttribute* at, int ctas) {
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = 8;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(TK_NT);
+  cfg.dynamicSmemBytes = c.tile_smem;
+  cfg.stream = c.stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 void gb_tile_setup(GbCtx& c) {
   c.tile_smem = sizeof(TileSmem);
-  cudaFuncSetAttribute(k_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
-  cudaFuncSetAttribute(k_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<false>, TK_NT, c.tile_smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<false, false>, TK_NT, c.tile_smem);
   c.tile_blocks = c.nsm * (per_sm > 0 ? per_sm : 1);
+  // clusters of 8 CTAs that the chip holds at once
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t cfg = split_config(c, &at, c.tile_blocks / 8 * 8);
+  int ncl = 0;
+  if (cudaOccupancyMaxActiveClusters(&ncl, k_tile<false, true>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    ncl = 0;
+  }
+  c.split_ctas = std::min(ncl, c.tile_blocks / 8) * 8;
 }
 
 __global__ void k_zero_counter(long long* ctr) { *ctr = 0; }
@@ -1390,12 +1588,21 @@ void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLa
     c.prof_flags = cs == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0;
     cudaEventRecordWithFlags(e0, c.stream, c.prof_flags);
   }
-  if (c.timing)
-    k_tile<true><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(op, A, B, O, g, mode | 4, c.tile_scratch,
-                                                                c.tile_scr_bytes, c.tile_counter, c.st);
-  else
-    k_tile<false><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(op, A, B, O, g, mode, c.tile_scratch,
-                                                                 c.tile_scr_bytes, c.tile_counter, c.st);
+  // which of the two launches takes the layer depends on its tiles, which the device knows
+  if (c.timing) {
+    k_tile<true, false><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
+        op, A, B, O, g, mode | 4, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, 0);
+  } else {
+    if (c.split_ctas) {
+      cudaLaunchAttribute at;
+      const cudaLaunchConfig_t cfg = split_config(c, &at, c.split_ctas);
+      cudaLaunchKernelEx(&cfg, k_tile<false, true>, op, A, B, O, g, mode, c.tile_scratch,
+                         (unsigned long long)c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
+      ++c.launches;
+    }
+    k_tile<false, false><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
+        op, A, B, O, g, mode, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
+  }
   if (c.prof) cudaEventRecordWithFlags(e1, c.stream, c.prof_flags);
   c.launches += 2;
   if (mode == 0) {
@@ -1592,7 +1799,7 @@ extern "C" int gb_bool_tile_noalloc(int op, const int4* d_A, int nA, const int4*
         fprintf(stderr, "gb_bool_tile_noalloc: cudaGetSymbolAddress failed on device %d\n", dev);
         return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
       }
-      if (cudaFuncSetAttribute(k_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)) !=
+      if (cudaFuncSetAttribute(k_tile<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)) !=
           cudaSuccess)
         return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
       g_na_state_ptr[dev] = (NoAllocState*)a;
@@ -1616,8 +1823,9 @@ extern "C" int gb_bool_tile_noalloc(int op, const int4* d_A, int nA, const int4*
     unsigned long long scr_bytes = GB_NA_SCRATCH;
     long long* ctr = S->ctr;
     DStatus* st = &S->res.st;
-    void* args[] = {&op, &la, &lb, &lo, &gg, &mode, &scr, &scr_bytes, &ctr, &st};
-    if (cudaLaunchKernel((const void*)k_tile<false>, dim3(1), dim3(TK_NT), args, sizeof(TileSmem), s) != cudaSuccess)
+    int split = 0;
+    void* args[] = {&op, &la, &lb, &lo, &gg, &mode, &scr, &scr_bytes, &ctr, &st, &split};
+    if (cudaLaunchKernel((const void*)k_tile<false, false>, dim3(1), dim3(TK_NT), args, sizeof(TileSmem), s) != cudaSuccess)
       return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
   }
   {
