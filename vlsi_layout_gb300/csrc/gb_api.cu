@@ -14,7 +14,6 @@
 #include "gb_internal.h"
 #include "gb_scan.cuh"
 
-#define KID_FRAME 50
 #define KID_KEYS 51
 
 namespace gbi {
@@ -24,15 +23,6 @@ int set_err(gb_context* ctx, int code, const char* msg) {
   return code;
 }
 
-__global__ void k_desc_init(DLayer* d, int ncell, int g, int binned) {
-  DLayer z;
-  memset(&z, 0, sizeof(z));
-  z.ncell = ncell;
-  z.g = g;
-  z.binned = binned;
-  *d = z;
-}
-
 int alloc_slot(gb_context* ctx) {
   if (ctx->c.desc_free.empty()) return -1;
   int s = ctx->c.desc_free.back();
@@ -40,6 +30,7 @@ int alloc_slot(gb_context* ctx) {
   return s;
 }
 
+// The descriptor on the device is made by the first kernel that fills it.
 gb_layer* new_arena_layer(gb_context* ctx, int ncell, int g) {
   int s = alloc_slot(ctx);
   if (s < 0) return nullptr;
@@ -51,7 +42,6 @@ gb_layer* new_arena_layer(gb_context* ctx, int ncell, int g) {
   L->binned = 1;
   L->arena_owned = 1;
   L->seq = ++ctx->seq;
-  k_desc_init<<<1, 1, 0, ctx->c.stream>>>(L->d, ncell, g, 1);
   ctx->arena_layers.push_back(L);
   return L;
 }
@@ -107,44 +97,6 @@ DLayer read_desc(gb_context* ctx, gb_layer* L) {
   cudaStreamSynchronize(ctx->c.stream);
   cudaMemcpy(&d, L->d, sizeof(DLayer), cudaMemcpyDeviceToHost);
   return d;
-}
-
-// Frame of an erosion: per cell the cell bbox grown by t (a superset of
-// bbox(P) (+) t is all the construction needs); empty cells get a unit box,
-// which leaves their (empty) result unchanged.
-__global__ void k_make_frame(const DLayer* P, DLayer* F, int ncell, int t, DStatus* st) {
-  if (st->err) return;
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    F->boxes = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * 16, KID_FRAME);
-    F->coff = (long long*)gb_arena_alloc(st, (unsigned long long)(ncell + 1) * 8, KID_FRAME);
-    F->cbox = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * 16, KID_FRAME);
-    F->cell_count = (long long*)gb_arena_alloc(st, (unsigned long long)ncell * 8, KID_FRAME);
-    F->cell_area = (long long*)gb_arena_alloc(st, (unsigned long long)ncell * 8, KID_FRAME);
-    F->nbox = ncell;
-    F->binned = 0;
-    if (F->boxes && F->coff) F->coff[ncell] = ncell;
-  }
-}
-__global__ void k_fill_frame(const DLayer* P, DLayer* F, int ncell, int t, DStatus* st) {
-  if (st->err) return;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ncell; k += gridDim.x * blockDim.x) {
-    const int4 b = P->cbox[k];
-    int4 o = make_int4(0, 0, 1, 1);
-    if (b.x < b.z && b.y < b.w) {
-      const long long x1 = (long long)b.x - t, y1 = (long long)b.y - t;
-      const long long x2 = (long long)b.z + t, y2 = (long long)b.w + t;
-      if (x1 < INT32_MIN || y1 < INT32_MIN || x2 > INT32_MAX || y2 > INT32_MAX) {
-        gb_set_error(st, GB_ERR_INVALID_BOX, KID_FRAME, k);
-      } else {
-        o = make_int4((int)x1, (int)y1, (int)x2, (int)y2);
-      }
-    }
-    F->boxes[k] = o;
-    F->coff[k] = k;
-    F->cbox[k] = o;
-    F->cell_count[k] = 1;
-    F->cell_area[k] = 0;
-  }
 }
 
 __global__ void k_count_tiles(const DLayer* L, long long* per_cell, int ncell, DStatus* st) {
@@ -400,6 +352,7 @@ extern "C" int gb_context_create(int device, unsigned long long arena_bytes, gb_
   s0.arena_cap = arena_bytes;
   cudaMemcpy(c.st, &s0, sizeof(s0), cudaMemcpyHostToDevice);
   if (cudaMalloc(&c.scan_part, (GB_SCAN_BLOCKS + 1) * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
+  cudaMemset(c.scan_part, 0, (GB_SCAN_BLOCKS + 1) * sizeof(long long));
   if (cudaMalloc(&c.dscal, 64 * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
   if (cudaMalloc(&c.tile_counter, 64 * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
   cudaMemset(c.dscal, 0, 64 * sizeof(long long));
@@ -509,22 +462,32 @@ extern "C" void gb_clear_status(gb_context* ctx) {
 // The mark stays on the device, in the stream's order (GB_DMARKS deep; deeper
 // ones, and marks taken during a capture, are read back as numbers).
 #define MARK_ON_DEVICE (~0ull)
-__global__ void k_arena_mark(const DStatus* st, unsigned long long* slot) { *slot = st->arena_off; }
+__global__ void k_arena_mark(DStatus* st, unsigned long long* slot, bool clear) {
+  *slot = st->arena_off;
+  if (clear) {
+    st->err = 0;
+    st->where = 0;
+    st->need = 0;
+  }
+}
 __global__ void k_arena_release(DStatus* st, const unsigned long long* slot) { st->arena_off = *slot; }
 
-extern "C" unsigned long long gb_arena_mark(gb_context* ctx) {
-  if (!ctx) return 0;
+// clear: the status too, as gb_clear_status.
+static unsigned long long arena_mark(gb_context* ctx, bool clear) {
   GbCtx& c = ctx->c;
   const size_t i = ctx->marks.size();
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (i < GB_DMARKS && cudaStreamIsCapturing(c.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
-    k_arena_mark<<<1, 1, 0, c.stream>>>(c.st, c.dmarks + i);
+    k_arena_mark<<<1, 1, 0, c.stream>>>(c.st, c.dmarks + i, clear);
     ctx->marks.push_back({MARK_ON_DEVICE, ctx->seq});
   } else {
+    if (clear) gb_clear_status(ctx);
     ctx->marks.push_back({read_status(ctx).arena_off, ctx->seq});
   }
   return (unsigned long long)i;
 }
+
+extern "C" unsigned long long gb_arena_mark(gb_context* ctx) { return ctx ? arena_mark(ctx, false) : 0; }
 
 extern "C" int gb_arena_release(gb_context* ctx, unsigned long long mark) {
   if (!ctx || mark >= ctx->marks.size()) return GB_ERR_ARG;
@@ -567,15 +530,6 @@ extern "C" int gb_set_tile_scratch(gb_context* ctx, unsigned long long bytes) {
 }
 
 // ======================================================================= layers
-// A raw layer's descriptor; one_cell: its offsets too.
-__global__ void k_raw_desc(DLayer* d, DLayer v, bool one_cell) {
-  *d = v;
-  if (one_cell) {
-    v.coff[0] = 0;
-    v.coff[1] = v.nbox;
-  }
-}
-
 // borrow: boxes is a device pointer used in place (coff then a host pointer).
 static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long long n,
                           const long long* coff, int ncell, bool device_src, gb_layer** out, bool borrow = false) {
@@ -617,7 +571,7 @@ static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long lon
   d.tbase = (long long*)q;
   L->cbox = d.cbox;
   const cudaMemcpyKind kind = device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  k_raw_desc<<<1, 1, 0, c.stream>>>(L->d, d, coff == nullptr);
+  gb_launch_raw_desc(c, L->d, d, coff == nullptr);
   if (n && !borrow) cudaMemcpyAsync(pb, boxes, n * 16, kind, c.stream);
   if (coff) cudaMemcpyAsync(d.coff, coff, (size_t)(ncell + 1) * 8, borrow ? cudaMemcpyHostToDevice : kind, c.stream);
   cudaStreamSynchronize(c.stream);  // the caller's arrays are its own again
@@ -830,9 +784,7 @@ gb_layer* op_erode(gb_context* ctx, gb_layer* P, int t, gb_layer** frame_out, gb
   gb_layer* F = new_arena_layer(ctx, P->ncell, g);
   if (!F) return nullptr;
   F->binned = 0;
-  k_desc_init<<<1, 1, 0, c.stream>>>(F->d, P->ncell, g, 0);
-  k_make_frame<<<1, 1, 0, c.stream>>>(Pb->d, F->d, P->ncell, t, c.st);
-  k_fill_frame<<<(P->ncell + 255) / 256, 256, 0, c.stream>>>(Pb->d, F->d, P->ncell, t, c.st);
+  gb_launch_frame(c, Pb->d, F->d, P->ncell, g, t);
   gb_layer* Q = op_bool(ctx, GB_OP_NOT, F, Pb, 0);
   if (!Q) return nullptr;
   if (frame_out) *frame_out = F;
@@ -868,8 +820,7 @@ template <typename F>
 int run_retry(gb_context* ctx, F&& body) {
   int e = GB_OK;
   for (int attempt = 0; attempt < 6; ++attempt) {
-    gb_clear_status(ctx);
-    const unsigned long long mk = gb_arena_mark(ctx);
+    const unsigned long long mk = arena_mark(ctx, true);
     e = body();
     int where = 0;
     long long need = 0;

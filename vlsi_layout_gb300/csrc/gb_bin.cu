@@ -13,10 +13,49 @@
 #define KID_ALLOC 12
 #define KID_SCAN 13
 #define KID_EXPORT 14
+#define KID_FRAME 50
+
+// Setup kernels of a layer's chain are a few microseconds of launch and memory
+// latency each, so they are few: a binning of raw boxes is five launches
+// (setup, count, two of the scan, scatter; thirteen took 12 us more on an
+// idle chip), a Boolean three beside the tile kernel's, an export three.
 
 // ------------------------------------------------------------------ scans
-__global__ void k_scan1(int* const* inp, const long long* np, long long* part) {
+// What the last block of the first scan launch does with the total.
+enum ScanHook { SCAN_TOTAL, SCAN_BIN, SCAN_EXPORT };
+struct ScanEnd {
+  int hook;
+  long long* total;  // may be null
+  DLayer* out;       // SCAN_BIN: its pieces (elem bytes each) are allocated
+  int elem;
+  const DLayer* src;  // SCAN_EXPORT: its tiles
+  long long* dscal;   // SCAN_EXPORT: [0] box array, [1] offsets, [2] total
+  DStatus* st;
+};
+
+__device__ void scan_end(const ScanEnd& e, long long total) {
+  if (e.total) *e.total = total;
+  if (e.hook == SCAN_BIN) {
+    if (e.st->err) return;
+    DLayer* O = e.out;
+    O->pcs = (unsigned long long*)gb_arena_alloc(e.st, (unsigned long long)(total + 1) * e.elem, KID_ALLOC);
+    O->nused = total;
+    O->ntot = total;
+    if (!O->pcs) O->ntiles = 0;
+  } else if (e.hook == SCAN_EXPORT) {
+    e.dscal[0] = e.dscal[1] = 0;
+    e.dscal[2] = e.st->err ? 0 : total;
+    if (e.st->err) return;
+    e.dscal[1] = (long long)gb_arena_alloc(e.st, (unsigned long long)(e.src->ntiles + 1) * 8, KID_EXPORT);
+    if (e.dscal[1]) e.dscal[0] = (long long)gb_arena_alloc(e.st, (unsigned long long)(total + 1) * 16, KID_EXPORT);
+  }
+}
+
+// Partial sums per block; the last block to finish scans them.  part: the
+// partial sums, then a ticket that is 0 between launches.
+__global__ void k_scan1(int* const* inp, const long long* np, long long* part, ScanEnd e) {
   __shared__ long long tmp[33];
+  __shared__ bool last;
   const int* __restrict__ in = *inp;
   const long long n = in ? *np : 0;
   const long long chunk = (n + gridDim.x - 1) / gridDim.x;
@@ -24,23 +63,29 @@ __global__ void k_scan1(int* const* inp, const long long* np, long long* part) {
   long long s = 0;
   for (long long i = beg + threadIdx.x; i < end; i += blockDim.x) s += in[i];
   s = gb_block_sum(s, tmp);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-__global__ void k_scan2(long long* part, int nb, long long* total) {
-  __shared__ long long tmp[33];
-  long long v = threadIdx.x < nb ? part[threadIdx.x] : 0;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd((unsigned long long*)&part[GB_SCAN_BLOCKS], 1ull) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const long long v = threadIdx.x < gridDim.x ? __ldcg(&part[threadIdx.x]) : 0;
   long long tot;
-  long long ex = gb_block_excl(v, tmp, &tot);
-  if (threadIdx.x < nb) part[threadIdx.x] = ex;
-  if (threadIdx.x == 0 && total) *total = tot;
+  const long long ex = gb_block_excl(v, tmp, &tot);
+  if (threadIdx.x < gridDim.x) part[threadIdx.x] = ex;
+  if (threadIdx.x == 0) {
+    part[GB_SCAN_BLOCKS] = 0;
+    scan_end(e, tot);
+  }
 }
 
-__global__ void k_scan3(int* const* inp, long long* const* outp, const long long* np,
-                        const long long* part) {
+// zero: the counts are cleared once read (a scatter counts them up again).
+__global__ void k_scan2(int* const* inp, long long* const* outp, const long long* np, const long long* part, int zero) {
   __shared__ long long tmp[33];
   constexpr int IT = 8;
-  const int* __restrict__ in = *inp;
+  int* in = *inp;
   long long* __restrict__ out = *outp;
   const long long n = (in && out) ? *np : 0;
   const long long chunk = (n + gridDim.x - 1) / gridDim.x;
@@ -60,18 +105,28 @@ __global__ void k_scan3(int* const* inp, long long* const* outp, const long long
     long long run = carry + ex;
 #pragma unroll
     for (int k = 0; k < IT; ++k) {
-      if (my + k < end) out[my + k] = run;
+      if (my + k < end) {
+        out[my + k] = run;
+        if (zero) in[my + k] = 0;
+      }
       run += v[k];
     }
     carry += tot;
   }
 }
 
+static void launch_scan(GbCtx& c, int* const* in_field, long long* const* out_field, const long long* n_dev,
+                        const ScanEnd& e, int zero) {
+  k_scan1<<<GB_SCAN_BLOCKS, GB_SCAN_THREADS, 0, c.stream>>>(in_field, n_dev, c.scan_part, e);
+  k_scan2<<<GB_SCAN_BLOCKS, GB_SCAN_THREADS, 0, c.stream>>>(in_field, out_field, n_dev, c.scan_part, zero);
+}
+
 void gb_launch_scan_i32(GbCtx& c, int* const* in_field, long long* const* out_field,
                         const long long* n_dev, long long* total_dev) {
-  k_scan1<<<GB_SCAN_BLOCKS, GB_SCAN_THREADS, 0, c.stream>>>(in_field, n_dev, c.scan_part);
-  k_scan2<<<1, GB_SCAN_BLOCKS, 0, c.stream>>>(c.scan_part, GB_SCAN_BLOCKS, total_dev);
-  k_scan3<<<GB_SCAN_BLOCKS, GB_SCAN_THREADS, 0, c.stream>>>(in_field, out_field, n_dev, c.scan_part);
+  ScanEnd e = {};
+  e.hook = SCAN_TOTAL;
+  e.total = total_dev;
+  launch_scan(c, in_field, out_field, n_dev, e, 0);
 }
 
 // ------------------------------------------------------------------ arena
@@ -94,21 +149,50 @@ __device__ __forceinline__ bool grow_box(int4 b, int E, int N, int W, int S, int
   return true;
 }
 
-__global__ void k_cbox_init(DLayer* O, int ncell, DStatus* st) {
-  if (st->err) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && O->cbox == nullptr) {
-    O->cbox = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * sizeof(int4), KID_ALLOC);
-    O->cell_count = (long long*)gb_arena_alloc(st, (unsigned long long)ncell * 8, KID_ALLOC);
-    O->cell_area = (long long*)gb_arena_alloc(st, (unsigned long long)ncell * 8, KID_ALLOC);
-    O->tbase = (long long*)gb_arena_alloc(st, (unsigned long long)(ncell + 1) * 8, KID_ALLOC);
-    O->win = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * sizeof(int4), KID_ALLOC);
+#define BIN_CELLS 16384  // cells that a one-block setup kernel fills itself
+
+// A fresh descriptor with its per-cell arrays (one thread); false when the
+// context has failed or the arena is full (the descriptor is empty then).
+__device__ bool layer_fresh(DLayer* O, int ncell, int g, int binned, DStatus* st) {
+  DLayer z;
+  memset(&z, 0, sizeof(z));
+  z.ncell = ncell;
+  z.g = g;
+  z.binned = binned;
+  const unsigned long long c16 = ((unsigned long long)ncell * 16 + 255) & ~255ull,
+                           c8 = ((unsigned long long)(ncell + 1) * 8 + 255) & ~255ull;
+  char* p = st->err ? nullptr : (char*)gb_arena_alloc(st, 2 * c16 + 3 * c8, KID_ALLOC);
+  if (p) {
+    z.cbox = (int4*)p;
+    z.win = (int4*)(p + c16);
+    z.cell_count = (long long*)(p + 2 * c16);
+    z.cell_area = (long long*)(p + 2 * c16 + c8);
+    z.tbase = (long long*)(p + 2 * c16 + 2 * c8);
+  }
+  *O = z;
+  return p != nullptr;
+}
+
+__device__ __forceinline__ int4 bbox_none() { return make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN); }
+
+// A fresh binned layer with empty bounding boxes (up to BIN_CELLS cells are
+// filled here, more by k_cbox_fill).
+__global__ void k_bin_init(DLayer* O, int ncell, int g, DStatus* st) {
+  __shared__ bool ok;
+  if (threadIdx.x == 0) ok = layer_fresh(O, ncell, g, 1, st);
+  __syncthreads();
+  if (!ok || ncell > BIN_CELLS) return;
+  for (int k = threadIdx.x; k < ncell; k += blockDim.x) {
+    O->cbox[k] = bbox_none();
+    O->cell_count[k] = 0;
+    O->cell_area[k] = 0;
   }
 }
 
 __global__ void k_cbox_fill(DLayer* O, int ncell, DStatus* st) {
   if (st->err) return;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ncell; k += gridDim.x * blockDim.x) {
-    O->cbox[k] = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
+    O->cbox[k] = bbox_none();
     O->cell_count[k] = 0;
     O->cell_area[k] = 0;
   }
@@ -195,7 +279,6 @@ __device__ __forceinline__ void bbox_add(int4* dst, int4 b) {
   if (b.z > cur.z) atomicMax(&dst->z, b.z);
   if (b.w > cur.w) atomicMax(&dst->w, b.w);
 }
-__device__ __forceinline__ int4 bbox_none() { return make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN); }
 __device__ __forceinline__ int4 bbox_join(int4 a, int4 b) {
   return make_int4(min(a.x, b.x), min(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
 }
@@ -212,6 +295,7 @@ __global__ void __launch_bounds__(256) k_bbox_raw(const DLayer* S, DLayer* O, in
   __shared__ int4 wb[8];
   __shared__ int wk[8];
   if (st->err) return;
+  if (S == O && blockIdx.x == 0 && threadIdx.x == 0) O->has_cbox = 1;  // a raw layer's own boxes
   int4* const cb = O->cbox;
   int kc = -1;  // the cell whose bounds the warp holds
   int4 acc = bbox_none();
@@ -219,6 +303,7 @@ __global__ void __launch_bounds__(256) k_bbox_raw(const DLayer* S, DLayer* O, in
     int4 g = bbox_none();
     if (valid_i && !grow_box(box, E, N, W, Sg, g)) {
       gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, i);
+      if (S == O) O->bad = i + 1;
       g = bbox_none();
     }
     const int k0 = __shfl_sync(0xffffffffu, k, 0);
@@ -289,12 +374,13 @@ __global__ void k_bbox_bin(const DLayer* S, DLayer* O, int E, int N, int W, int 
 }
 
 // ------------------------------------------------------------------ windows
-// One block: per-cell tile window from the cell bbox, scan into tbase, and
-// allocate the per-tile arrays.  closed=1 uses closed tile ranges (x2 >> g).
-__global__ void k_window(DLayer* O, int ncell, int g, int closed, DStatus* st) {
+// One block: per-cell tile window from the cell bbox, scan into tbase,
+// allocate the per-tile arrays and clear the counts.  closed=1 uses closed
+// tile ranges (x2 >> g).
+__device__ void window_block(DLayer* O, int ncell, int g, int closed, DStatus* st) {
   __shared__ long long tmp[33];
   __shared__ long long carry;
-  if (st->err) return;
+  __shared__ int* counts;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
   for (int base = 0; base < ncell; base += blockDim.x) {
@@ -321,6 +407,7 @@ __global__ void k_window(DLayer* O, int ncell, int g, int closed, DStatus* st) {
   }
   if (threadIdx.x == 0) {
     const long long total = carry;
+    counts = nullptr;
     O->tbase[ncell] = total;
     O->ntiles = total;
     O->g = g;
@@ -328,30 +415,67 @@ __global__ void k_window(DLayer* O, int ncell, int g, int closed, DStatus* st) {
     if (total > GB_MAX_TILES_PER_OP) {
       gb_set_error(st, GB_ERR_CAPACITY, KID_WINDOW, total);
       O->ntiles = 0;
-      return;
+    } else {
+      const unsigned long long b8 = ((unsigned long long)(total + 1) * 8 + 255) & ~255ull;
+      char* p = (char*)gb_arena_alloc(st, b8 + (unsigned long long)(total + 1) * 4, KID_ALLOC);
+      if (p) {
+        O->tstart = (long long*)p;
+        counts = O->tcount = (int*)(p + b8);
+      } else {
+        O->ntiles = 0;
+      }
     }
-    O->tstart = (long long*)gb_arena_alloc(st, (unsigned long long)(total + 1) * 8, KID_ALLOC);
-    O->tcount = (int*)gb_arena_alloc(st, (unsigned long long)(total + 1) * 4, KID_ALLOC);
-    if (!O->tstart || !O->tcount) O->ntiles = 0;
   }
+  __syncthreads();
+  if (!counts) return;
+  int4* z = reinterpret_cast<int4*>(counts);  // the allocation is whole 256 bytes
+  for (long long i = threadIdx.x; i < (carry + 3) / 4; i += blockDim.x) z[i] = make_int4(0, 0, 0, 0);
 }
 
-__global__ void k_zero_tcount(DLayer* O, DStatus* st) {
+__global__ void __launch_bounds__(1024) k_window(DLayer* O, int ncell, int g, int closed, DStatus* st) {
   if (st->err) return;
-  const long long n = O->ntiles;
-  int* c = O->tcount;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    c[i] = 0;
+  window_block(O, ncell, g, closed, st);
 }
 
-__global__ void k_alloc_pcs(DLayer* O, int elem_bytes, DStatus* st) {
-  if (st->err) return;
-  O->pcs = (unsigned long long*)gb_arena_alloc(st, (unsigned long long)(O->npcs + 1) * elem_bytes,
-                                               KID_ALLOC);
-  O->nused = O->npcs;
-  O->ntot = O->npcs;
-  if (!O->pcs) O->ntiles = 0;
+// One block, raw source, boxes not shrunk, at most BIN_CELLS cells: the cells'
+// bounding boxes are the source's, grown, so the binning needs no pass over
+// the boxes for them.
+__global__ void __launch_bounds__(1024) k_bin_setup(const DLayer* S, DLayer* O, int ncell, int g, int closed, int E, int N,
+                                                    int W, int Sg, DStatus* st) {
+  __shared__ bool ok;
+  if (threadIdx.x == 0) {
+    ok = layer_fresh(O, ncell, g, 1, st);
+    if (ok && S->bad) {  // reported again, as a pass over the boxes would
+      gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, S->bad - 1);
+      ok = false;
+    }
+  }
+  __syncthreads();
+  if (!ok) return;
+  const bool have = S->has_cbox != 0;
+  for (int k = threadIdx.x; k < ncell; k += blockDim.x) {
+    int4 b = have ? S->cbox[k] : bbox_none(), o = bbox_none();
+    if (!have) {  // the layer was made while the context had failed: its boxes one by one
+      for (long long i = S->coff[k]; i < S->coff[k + 1]; ++i) {
+        const int4 q = S->boxes[i];
+        if (!(q.x < q.z && q.y < q.w)) {
+          gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, i);
+          ok = false;
+          break;
+        }
+        b = make_int4(min(b.x, q.x), min(b.y, q.y), max(b.z, q.z), max(b.w, q.w));
+      }
+    }
+    if (b.x <= b.z && !grow_box(b, E, N, W, Sg, o)) {  // past int32: so is a box at that bound
+      gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, S->coff[k]);
+      ok = false;
+    }
+    O->cbox[k] = o;
+    O->cell_count[k] = 0;
+    O->cell_area[k] = 0;
+  }
+  __syncthreads();
+  if (ok) window_block(O, ncell, g, closed, st);
 }
 
 // ------------------------------------------------------------------ count / scatter
@@ -603,21 +727,28 @@ __global__ void k_split_bin(const DLayer* S, DLayer* O, int g, int E, int N, int
 static void launch_bin_common(GbCtx& c, const DLayer* src, int src_binned, DLayer* out, int ncell,
                               int g, int E, int N, int W, int S, int mode) {
   const int wb = c.work_blocks, T = 256;
-  k_cbox_init<<<1, 32, 0, c.stream>>>(out, ncell, c.st);
-  k_cbox_fill<<<(ncell + 255) / 256, 256, 0, c.stream>>>(out, ncell, c.st);
-  if (src_binned) k_bbox_bin<<<wb, T, 0, c.stream>>>(src, out, E, N, W, S, c.st);
-  else k_bbox_raw<<<wb, T, 0, c.stream>>>(src, out, ncell, E, N, W, S, c.st);
-  k_window<<<1, 1024, 0, c.stream>>>(out, ncell, g, mode, c.st);
-  k_zero_tcount<<<wb, T, 0, c.stream>>>(out, c.st);
+  if (!src_binned && ncell <= BIN_CELLS && E >= 0 && N >= 0 && W >= 0 && S >= 0) {
+    k_bin_setup<<<1, 1024, 0, c.stream>>>(src, out, ncell, g, mode, E, N, W, S, c.st);
+  } else {
+    k_bin_init<<<1, 1024, 0, c.stream>>>(out, ncell, g, c.st);
+    if (ncell > BIN_CELLS) k_cbox_fill<<<(ncell + 255) / 256, 256, 0, c.stream>>>(out, ncell, c.st);
+    if (src_binned) k_bbox_bin<<<wb, T, 0, c.stream>>>(src, out, E, N, W, S, c.st);
+    else k_bbox_raw<<<wb, T, 0, c.stream>>>(src, out, ncell, E, N, W, S, c.st);
+    k_window<<<1, 1024, 0, c.stream>>>(out, ncell, g, mode, c.st);
+  }
   if (mode == 0) {
     if (src_binned) k_split_bin<false><<<wb, T, 0, c.stream>>>(src, out, g, E, N, W, S, c.st);
     else k_split_raw<0, false><<<wb, T, 0, c.stream>>>(src, out, ncell, g, E, N, W, S, c.st);
   } else {
     k_split_raw<1, false><<<wb, T, 0, c.stream>>>(src, out, ncell, g, 0, 0, 0, 0, c.st);
   }
-  gb_launch_scan_i32(c, &out->tcount, &out->tstart, &out->ntiles, &out->npcs);
-  k_alloc_pcs<<<1, 1, 0, c.stream>>>(out, mode == 0 ? 8 : 4, c.st);
-  k_zero_tcount<<<wb, T, 0, c.stream>>>(out, c.st);
+  ScanEnd e = {};
+  e.hook = SCAN_BIN;
+  e.total = &out->npcs;
+  e.out = out;
+  e.elem = mode == 0 ? 8 : 4;
+  e.st = c.st;
+  launch_scan(c, &out->tcount, &out->tstart, &out->ntiles, e, 1);
   if (mode == 0) {
     if (src_binned) k_split_bin<true><<<wb, T, 0, c.stream>>>(src, out, g, E, N, W, S, c.st);
     else k_split_raw<0, true><<<wb, T, 0, c.stream>>>(src, out, ncell, g, E, N, W, S, c.st);
@@ -635,11 +766,73 @@ void gb_launch_bin_index(GbCtx& c, const DLayer* src, DLayer* out, int ncell, in
   launch_bin_common(c, src, 0, out, ncell, g, 0, 0, 0, 0, 1);
 }
 
-// Per-cell bounding box of a raw layer (no grow) into its own cbox.
+// Per-cell bounding box of a raw layer (no grow) into its own cbox, which
+// starts empty.
 void gb_launch_cell_bbox_fill(GbCtx& c, DLayer* L, int ncell) {
-  k_cbox_init<<<1, 32, 0, c.stream>>>(L, ncell, c.st);
-  k_cbox_fill<<<(ncell + 255) / 256, 256, 0, c.stream>>>(L, ncell, c.st);
   k_bbox_raw<<<c.work_blocks, 256, 0, c.stream>>>(L, L, ncell, 0, 0, 0, 0, c.st);
+}
+
+// A raw layer's descriptor, per-cell arrays empty; one_cell: its offsets too.
+__global__ void k_raw_desc(DLayer* d, DLayer v, bool one_cell) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0) {
+    *d = v;
+    if (one_cell) {
+      v.coff[0] = 0;
+      v.coff[1] = v.nbox;
+    }
+  }
+  if (k < v.ncell) {
+    v.cbox[k] = bbox_none();
+    v.cell_count[k] = 0;
+    v.cell_area[k] = 0;
+  }
+}
+
+void gb_launch_raw_desc(GbCtx& c, DLayer* d, const DLayer& v, bool one_cell) {
+  k_raw_desc<<<(v.ncell + 255) / 256, 256, 0, c.stream>>>(d, v, one_cell);
+}
+
+// Frame of an erosion: per cell the cell bbox grown by t (a superset of
+// bbox(P) (+) t is all the construction needs); empty cells get a unit box,
+// which leaves their (empty) result unchanged.  A fresh raw layer, one block.
+__global__ void __launch_bounds__(1024) k_frame(const DLayer* P, DLayer* F, int ncell, int g, int t, DStatus* st) {
+  __shared__ bool ok;
+  if (threadIdx.x == 0) {
+    ok = layer_fresh(F, ncell, g, 0, st);
+    if (ok) {
+      F->boxes = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * 16, KID_FRAME);
+      F->coff = (long long*)gb_arena_alloc(st, (unsigned long long)(ncell + 1) * 8, KID_FRAME);
+      F->nbox = ncell;
+      F->has_cbox = 1;
+      ok = F->boxes && F->coff;
+      if (ok) F->coff[ncell] = ncell;
+    }
+  }
+  __syncthreads();
+  if (!ok) return;
+  for (int k = threadIdx.x; k < ncell; k += blockDim.x) {
+    const int4 b = P->cbox[k];
+    int4 o = make_int4(0, 0, 1, 1);
+    if (b.x < b.z && b.y < b.w) {
+      const long long x1 = (long long)b.x - t, y1 = (long long)b.y - t;
+      const long long x2 = (long long)b.z + t, y2 = (long long)b.w + t;
+      if (x1 < INT32_MIN || y1 < INT32_MIN || x2 > INT32_MAX || y2 > INT32_MAX) {
+        gb_set_error(st, GB_ERR_INVALID_BOX, KID_FRAME, k);
+      } else {
+        o = make_int4((int)x1, (int)y1, (int)x2, (int)y2);
+      }
+    }
+    F->boxes[k] = o;
+    F->coff[k] = k;
+    F->cbox[k] = o;
+    F->cell_count[k] = 1;
+    F->cell_area[k] = 0;
+  }
+}
+
+void gb_launch_frame(GbCtx& c, const DLayer* P, DLayer* F, int ncell, int g, int t) {
+  k_frame<<<1, 1024, 0, c.stream>>>(P, F, ncell, g, t, c.st);
 }
 
 // ------------------------------------------------------------------ Boolean op setup
@@ -652,22 +845,27 @@ __device__ __forceinline__ int tile_index_in(const DLayer* L, int k, int tx, int
 }
 
 // Output window per cell: the union of both windows for OR / XOR, A's window
-// otherwise (AND, NOT and MERGE results lie inside A).
-__global__ void k_bool_window(int op, const DLayer* A, const DLayer* B, DLayer* O, int ncell, int g,
-                              DStatus* st) {
+// otherwise (AND, NOT and MERGE results lie inside A).  One block: the fresh
+// result layer, its windows and per-tile arrays, its output pool, and the tile
+// kernel's work counters at zero.
+// Output pool (factor > 0): factor x (pieces of A + pieces of B) plus a
+// little per tile.  Each tile reserves exactly its strip count from the pool
+// cursor (nused) once it knows it, so no per-tile slack is needed; a tile
+// that no longer fits takes its slots from the arena directly (atomically),
+// at an offset relative to the pool base.
+__global__ void __launch_bounds__(1024) k_bool_window(int op, const DLayer* A, const DLayer* B, DLayer* O, int ncell, int g,
+                                                      int factor, long long* counter, DStatus* st) {
   __shared__ long long tmp[33];
   __shared__ long long carry;
-  if (st->err) return;
+  __shared__ bool ok;
   if (threadIdx.x == 0) {
     carry = 0;
-    O->cbox = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * sizeof(int4), KID_ALLOC);
-    O->cell_count = (long long*)gb_arena_alloc(st, (unsigned long long)ncell * 8, KID_ALLOC);
-    O->cell_area = (long long*)gb_arena_alloc(st, (unsigned long long)ncell * 8, KID_ALLOC);
-    O->tbase = (long long*)gb_arena_alloc(st, (unsigned long long)(ncell + 1) * 8, KID_ALLOC);
-    O->win = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * sizeof(int4), KID_ALLOC);
+    counter[0] = 0;
+    counter[2] = 0;
+    ok = layer_fresh(O, ncell, g, 1, st);
   }
   __syncthreads();
-  if (st->err) return;
+  if (!ok) return;
   for (int base = 0; base < ncell; base += blockDim.x) {
     const int k = base + threadIdx.x;
     long long nt = 0;
@@ -701,17 +899,26 @@ __global__ void k_bool_window(int op, const DLayer* A, const DLayer* B, DLayer* 
     const long long total = carry;
     O->tbase[ncell] = total;
     O->ntiles = total;
-    O->g = g;
-    O->binned = 1;
     if (total > GB_MAX_TILES_PER_OP) {
       gb_set_error(st, GB_ERR_CAPACITY, KID_WINDOW, total);
       O->ntiles = 0;
       return;
     }
-    O->tstart = (long long*)gb_arena_alloc(st, (unsigned long long)(total + 1) * 8, KID_ALLOC);
-    O->tcount = (int*)gb_arena_alloc(st, (unsigned long long)(total + 1) * 4, KID_ALLOC);
-    O->tdesc = (TileDesc*)gb_arena_alloc(st, (unsigned long long)(total + 1) * sizeof(TileDesc), KID_ALLOC);
-    if (!O->tstart || !O->tcount || !O->tdesc) O->ntiles = 0;
+    const unsigned long long b8 = ((unsigned long long)(total + 1) * 8 + 255) & ~255ull,
+                             b4 = ((unsigned long long)(total + 1) * 4 + 255) & ~255ull;
+    char* p = (char*)gb_arena_alloc(st, b8 + b4 + (unsigned long long)(total + 1) * sizeof(TileDesc), KID_ALLOC);
+    if (!p) {
+      O->ntiles = 0;
+      return;
+    }
+    O->tstart = (long long*)p;
+    O->tcount = (int*)(p + b8);
+    O->tdesc = (TileDesc*)(p + b8 + b4);
+    if (factor <= 0) return;
+    const long long na = A->ntot, nb = B && op != GB_OP_MERGE ? B->ntot : 0;
+    O->npcs = (na + nb) * factor + 16 * total + 64;
+    O->pcs = (unsigned long long*)gb_arena_alloc(st, (unsigned long long)O->npcs * 8, KID_ALLOC);
+    if (!O->pcs) O->ntiles = 0;
   }
 }
 
@@ -743,40 +950,14 @@ __global__ void k_tile_descs(int op, const DLayer* A, const DLayer* B, DLayer* O
   }
 }
 
-// Output pool of a Boolean op: factor x (pieces of A + pieces of B) plus a
-// little per tile.  Each tile reserves exactly its strip count from the pool
-// cursor (nused) once it knows it, so no per-tile slack is needed; a tile
-// that no longer fits takes its slots from the arena directly (atomically),
-// at an offset relative to the pool base.
-__global__ void k_pool_alloc(const DLayer* A, const DLayer* B, DLayer* O, int factor, DStatus* st) {
-  if (st->err) return;
-  const long long na = A ? A->ntot : 0, nb = B ? B->ntot : 0;
-  O->npcs = (na + nb) * factor + 16 * O->ntiles + 64;
-  O->nused = 0;
-  O->ntot = 0;
-  O->pcs = (unsigned long long*)gb_arena_alloc(st, (unsigned long long)O->npcs * 8, KID_ALLOC);
-  if (!O->pcs) O->ntiles = 0;
-}
-
 void gb_launch_bool_setup(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O, int ncell,
                           int g, int alloc_slots) {
-  k_bool_window<<<1, 1024, 0, c.stream>>>(op, A, B, O, ncell, g, c.st);
+  k_bool_window<<<1, 1024, 0, c.stream>>>(op, A, B, O, ncell, g, alloc_slots ? c.cap_factor : 0, c.tile_counter, c.st);
   k_tile_descs<<<c.work_blocks, 256, 0, c.stream>>>(op, A, B, O, c.st);
-  if (!alloc_slots) return;
-  k_pool_alloc<<<1, 1, 0, c.stream>>>(A, op == GB_OP_MERGE ? nullptr : B, O, c.cap_factor, c.st);
 }
 
 // ------------------------------------------------------------------ export
 // Slots of c.dscal used by the export: [0] = int4* array, [1] = offsets*, [2] = total.
-__global__ void k_export_alloc1(const DLayer* L, long long* dscal, DStatus* st) {
-  if (st->err) { dscal[0] = 0; dscal[1] = 0; dscal[2] = 0; return; }
-  dscal[1] = (long long)gb_arena_alloc(st, (unsigned long long)(L->ntiles + 1) * 8, KID_EXPORT);
-  dscal[3] = L->ntiles;
-}
-__global__ void k_export_alloc2(long long* dscal, DStatus* st) {
-  if (st->err) { dscal[0] = 0; return; }
-  dscal[0] = (long long)gb_arena_alloc(st, (unsigned long long)(dscal[2] + 1) * 16, KID_EXPORT);
-}
 __global__ void k_export(const DLayer* L, const long long* dscal, DStatus* st) {
   if (st->err) return;
   int4* out = (int4*)dscal[0];
@@ -835,9 +1016,11 @@ void gb_launch_digest(GbCtx& c, const DLayer* L, unsigned long long* out, int st
 void gb_launch_export(GbCtx& c, const DLayer* L, int4** out_ptr_dev, long long* total_dev) {
   (void)out_ptr_dev;
   (void)total_dev;
-  k_export_alloc1<<<1, 1, 0, c.stream>>>(L, c.dscal, c.st);
-  gb_launch_scan_i32(c, (int* const*)&L->tcount, (long long* const*)&c.dscal[1], &c.dscal[3],
-                     &c.dscal[2]);
-  k_export_alloc2<<<1, 1, 0, c.stream>>>(c.dscal, c.st);
+  ScanEnd e = {};
+  e.hook = SCAN_EXPORT;
+  e.src = L;
+  e.dscal = c.dscal;
+  e.st = c.st;
+  launch_scan(c, (int* const*)&L->tcount, (long long* const*)&c.dscal[1], &L->ntiles, e, 0);
   k_export<<<c.work_blocks, 256, 0, c.stream>>>(L, c.dscal, c.st);
 }

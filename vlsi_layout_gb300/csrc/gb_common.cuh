@@ -63,13 +63,14 @@ struct DLayer {
   int ncell;
   int g;            // grid log2 (binned form)
   int binned;       // 1 = binned, 0 = raw
-  int pad0;
+  int has_cbox;     // raw: cbox holds the cells' bounding boxes
   long long* cell_count;   // [ncell] boxes (raw) or strips (binned result)
   long long* cell_area;    // [ncell] union area when computed
   // raw form
   int4* boxes;
   long long* coff;         // [ncell+1]
   long long nbox;
+  long long bad;           // raw: 1 + the index of an invalid box (0: none)
   // binned form
   int4* win;               // [ncell]: tx0, ty0, ntx, nty
   long long* tbase;        // [ncell+1]

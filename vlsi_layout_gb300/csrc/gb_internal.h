@@ -164,12 +164,13 @@ void gb_launch_scan_i32(GbCtx& c, int* const* in_field, long long* const* out_fi
                         const long long* n_dev, long long* total_dev);
 void gb_launch_arena_reset(GbCtx& c, unsigned long long mark);
 // Build the binned form of `src` (raw or binned) after growing every box by
-// (E,N,W,S) on grid g.  out must be a descriptor with ncell set by the host.
+// (E,N,W,S) on grid g, into a fresh layer at the descriptor `out`.
 void gb_launch_rebin(GbCtx& c, const DLayer* src, int src_binned, DLayer* out, int ncell, int g,
                      int E, int N, int W, int S);
 // Closed-tile index binning for connectivity (pcs holds int box indices).
 void gb_launch_bin_index(GbCtx& c, const DLayer* src, DLayer* out, int ncell, int g);
-// Output window / slot capacities of a Boolean op.
+// A Boolean op's fresh result layer: output window, tile descriptors, slots;
+// also clears the tile kernel's work counters.
 // alloc_slots = 0: count / area only (no output slots).
 void gb_launch_bool_setup(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O,
                           int ncell, int g, int alloc_slots);
@@ -178,6 +179,9 @@ void gb_launch_bool_setup(GbCtx& c, int op, const DLayer* A, const DLayer* B, DL
 // device pointer to the box array and the total land in *dscal-slots.
 void gb_launch_export(GbCtx& c, const DLayer* L, int4** out_ptr_dev, long long* total_dev);
 void gb_launch_cell_bbox_fill(GbCtx& c, DLayer* L, int ncell);
+void gb_launch_raw_desc(GbCtx& c, DLayer* d, const DLayer& v, bool one_cell);
+// Frame of an erosion by t: a fresh raw layer of one box per cell of P.
+void gb_launch_frame(GbCtx& c, const DLayer* P, DLayer* F, int ncell, int g, int t);
 // Per-cell strip digests of a binned layer, added to out[cell * stride]
 // (out zeroed by the caller).
 void gb_launch_digest(GbCtx& c, const DLayer* L, unsigned long long* out, int stride);

@@ -918,6 +918,22 @@ __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int
   }
 }
 
+// The output pool is sized for the worst case (cap_factor x input pieces) and
+// tiles reserve exactly what they emit.  When nothing was allocated in the
+// arena after the pool (no overflow, no scratch spill), the unused tail goes
+// back to the arena, so a chain of operators keeps only what it produced.  One
+// thread of the kernel's last CTA.
+__device__ void pool_trim(DLayer* O, DStatus* st) {
+  if (*(volatile int*)&st->err || !O->pcs) return;
+  const unsigned long long start = (unsigned long long)((char*)O->pcs - st->arena_base);
+  const unsigned long long end = start + (((unsigned long long)O->npcs * 8ull + 255ull) & ~255ull);
+  const long long nused = (long long)__ldcg((const unsigned long long*)&O->nused);
+  if (__ldcg(&st->arena_off) != end || nused > O->npcs) return;
+  const long long used = nused > 0 ? nused : 0;
+  st->arena_off = start + (((unsigned long long)used * 8ull + 255ull) & ~255ull);
+  O->npcs = used;
+}
+
 // CTAs per tile for a layer of nt tiles when `ctas` CTAs can share (a multiple
 // of 8; 0: never): as many as the chip holds, at least two, else 1.  Sharing
 // repeats the ranking (a quarter of a small tile's time), so it pays while it
@@ -1512,6 +1528,13 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     }
     if (SPLIT) break;
   }
+  if (mode == 0 && tid == 0) {  // the last CTA to finish gives the pool's tail back
+    __threadfence();
+    if (atomicAdd((unsigned long long*)&counter[2], 1ull) == gridDim.x - 1) {
+      __threadfence();
+      pool_trim(O, st);
+    }
+  }
   if (timing && threadIdx.x == 0) {
     atomicAdd((unsigned long long*)&counter[16], (unsigned long long)tA);
     atomicAdd((unsigned long long*)&counter[17], (unsigned long long)tB);
@@ -1553,24 +1576,7 @@ void gb_tile_setup(GbCtx& c) {
   c.split_ctas = std::min(ncl, c.tile_blocks / 8) * 8;
 }
 
-__global__ void k_zero_counter(long long* ctr) { *ctr = 0; }
-
-// The output pool is sized for the worst case (cap_factor x input pieces) and
-// tiles reserve exactly what they emit.  When nothing was allocated in the
-// arena after the pool (no overflow, no scratch spill), the unused tail goes
-// back to the arena, so a chain of operators keeps only what it produced.
-__global__ void k_pool_trim(DLayer* O, DStatus* st) {
-  if (st->err || !O->pcs) return;
-  const unsigned long long start = (unsigned long long)((char*)O->pcs - st->arena_base);
-  const unsigned long long end = start + (((unsigned long long)O->npcs * 8ull + 255ull) & ~255ull);
-  if (st->arena_off != end || O->nused > O->npcs) return;
-  const long long used = O->nused > 0 ? O->nused : 0;
-  st->arena_off = start + (((unsigned long long)used * 8ull + 255ull) & ~255ull);
-  O->npcs = used;
-}
-
 void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode) {
-  k_zero_counter<<<1, 1, 0, c.stream>>>(c.tile_counter);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c.prof) {
     if (c.prof_used + 2 > c.prof_ev.size()) {
@@ -1604,11 +1610,7 @@ void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLa
         op, A, B, O, g, mode, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
   }
   if (c.prof) cudaEventRecordWithFlags(e1, c.stream, c.prof_flags);
-  c.launches += 2;
-  if (mode == 0) {
-    k_pool_trim<<<1, 1, 0, c.stream>>>(O, c.st);
-    ++c.launches;
-  }
+  ++c.launches;
 }
 
 // ===================================================================== no-allocation entry point
