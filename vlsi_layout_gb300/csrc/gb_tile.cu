@@ -43,7 +43,7 @@
 //     (sub-band, column, row) order, so the output of a tile is
 //     deterministic.
 // Layers of few tiles: one tile per CTA would leave most of the chip idle, so a
-// cluster's CTAs then share tiles (k_tile<false, true>): each ranks the whole
+// cluster's CTAs then share tiles (k_tile<false, TILE_SPLIT>): each ranks the whole
 // tile, takes a contiguous share of the sub-bands through phases B to D, and
 // chains that run on into the next CTA's share are followed through a table of
 // that CTA's continuations.  These CTAs meet at two hardware cluster barriers.
@@ -161,6 +161,7 @@ struct TileSmem {
   PieceRec** sbrec;  // strip pieces per sub-band (global piece index = sbinfo.x + local index)
   int* succ;
   int q0, nsbg;  // a shared tile: the CTA's first sub-band, the tile's sub-bands
+  unsigned long long area;  // area mode: the CTA's share of the tile
   int2* cont;    // a shared tile: the CTA's continuations from the CTA before it (ordinal, end)
 };
 
@@ -350,7 +351,13 @@ __device__ __forceinline__ void tile_lookup(int op, const DLayer* A, const DLaye
 // WIDE: the level's larger buffers (level 1..3).  Returns false, with nothing
 // done, when the sub-band needs the next level's buffers; at the last level
 // columns beyond them spill to the scratch.
-template <bool TIMING, bool WIDE, bool SPLIT>
+// FORM: what the kernel does with a tile (below).
+enum TileForm {
+  TILE_WHOLE,  // strips, one tile per CTA
+  TILE_SPLIT,  // strips, CTAs of a cluster share a tile
+  TILE_AREA    // the area alone: no strips, so no chains either, and CTAs share a tile without meeting
+};
+template <bool TIMING, bool WIDE, int FORM>
 __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int nA, char* base,
                              unsigned long long scr, int level, long long* tctr) {
   if (!TIMING) tctr = nullptr;
@@ -376,7 +383,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     }
     return true;
   }
-  const int gsb = SPLIT ? s.q0 + sb : sb;  // of the tile; sb and nsb count the CTA's share
+  const int gsb = FORM != TILE_WHOLE ? s.q0 + sb : sb;  // of the tile; sb and nsb count the CTA's share
   const int rowbase = 63 * gsb - 1;
   const int nwy = ((Ny - 1) >> 5) + 1;
   const int lcn = WIDE ? wide_cols(level) : TK_LCN, mcn = WIDE ? wide_mc(level) : TK_MC;
@@ -580,6 +587,27 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     return true;
   }
   __syncwarp();
+  if (FORM == TILE_AREA) {
+    // per column its height times the width of its runs of rows 1..63 (row 0 is the sub-band before's)
+    const int *Xt = s.Xt, *Yt = s.Yt;
+    long long area = 0;
+    for (int c = c0; c < c1e; ++c) {
+      unsigned long long rr = ca[c] & ~1ull;
+      if (!rr) continue;
+      int w = 0;
+      while (rr) {
+        const int r1 = __ffsll((long long)rr) - 1;
+        const int r2 = r1 + __ffsll((long long)~(rr >> r1)) - 1;  // shifted-in zeros (r1 >= 1) end a run at row 63
+        w += Xt[rowbase + r2] - Xt[rowbase + r1];
+        rr = r2 >= 64 ? 0ull : rr & (~0ull << r2);
+      }
+      area += (long long)w * (Yt[lv[c + 1]] - Yt[lv[c]]);
+    }
+    area = gb_warp_sum(area);
+    if (lane == 0) atomicAdd(&s.area, (unsigned long long)area);
+    __syncwarp();
+    return true;
+  }
   TSTEP(1)
   // ---- run starts S_c = R_c & ~R_{c-1}, transposed to one column bitmap per row
   const bool tr = !WIDE || L <= lcn;
@@ -637,7 +665,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   }
   unsigned long long Fin = __shfl_up_sync(0xffffffffu, IA, 1);
   if (lane == 0) Fin = 0ull;
-  const bool last_sb = gsb == (SPLIT ? s.nsbg : nsb) - 1;
+  const bool last_sb = gsb == (FORM != TILE_WHOLE ? s.nsbg : nsb) - 1;
   TSTEP(2)
 
   // ---- count pieces / opens / heads
@@ -895,7 +923,7 @@ __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* rec
 
 // Levels 1..3 of phase C: the wide sub-bands that the level below listed, by fewer warps with larger buffers.
 // Called by the whole CTA after level 0.  Out of line: its registers stay out of the kernel's narrow path.
-template <bool TIMING, bool SPLIT>
+template <bool TIMING, int FORM>
 __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int nA, char* base,
                                        unsigned long long scr, long long* tctr) {
   for (int level = 1; level <= TK_WLEVELS; ++level) {
@@ -911,7 +939,7 @@ __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int
       k = __shfl_sync(0xffffffffu, k, 0);
       if (k >= todo) break;
       const int sb = TK_WLIST(s, level - 1)[k];
-      if (!tile_subband<TIMING, true, SPLIT>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && gb_lane() == 0)
+      if (!tile_subband<TIMING, true, FORM>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && gb_lane() == 0)
         TK_WLIST(s, level)[atomicAdd(&s.nwide[level], 1)] = sb;
       __syncwarp();
     }
@@ -944,9 +972,12 @@ __device__ __forceinline__ int tile_share(long long nt, int ctas) {
   return nt * 8 <= ctas ? (ctas ? 8 : 1) : nt * 4 <= ctas ? 4 : nt * 2 <= ctas ? 2 : 1;
 }
 
-// SPLIT: clusters of 8 CTAs, groups of `ka` of them share a tile each; every
-// CTA passes two cluster barriers and takes one tile at most.
-template <bool TIMING, bool SPLIT>
+// TILE_SPLIT: clusters of 8 CTAs, groups of `share` of them take a tile each;
+// every CTA passes two cluster barriers and takes one tile at most.
+// TILE_AREA: the work counter hands out (tile, share) pairs.  Klee's measure
+// needs the columns' rows and no strips: without the scans, the records and
+// the stitch, 12M boxes take TODO_AREA and not 2088 us.
+template <bool TIMING, int FORM>
 __global__ void __launch_bounds__(TK_NT, 3)
 k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, char* scratch,
        unsigned long long scr, long long* counter, DStatus* st, int split_ctas) {
@@ -959,10 +990,11 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
   const bool timing = TIMING && (mode & 4) != 0;
   mode &= 3;
   long long tA = 0, tB = 0, tC = 0, tD = 0, t0 = 0;
+  constexpr bool SPLIT = FORM == TILE_SPLIT, AREA = FORM == TILE_AREA;
   const int share = tile_share(O->ntiles, split_ctas);
-  if ((share > 1) != SPLIT) return;  // the other launch takes the layer (the same on every CTA)
+  if (!AREA && (share > 1) != SPLIT) return;  // the other launch takes the layer (the same on every CTA)
   // a shared tile: the CTA's place among the tile's CTAs, the first one's scratch
-  const int me = SPLIT ? (int)blockIdx.x % share : 0;
+  int me = SPLIT ? (int)blockIdx.x % share : 0;
   const char* const pub0 = scratch + (size_t)(blockIdx.x - me) * scr;
   SplitPub* const pub = reinterpret_cast<SplitPub*>(base);
   int ka = 1;  // CTAs that have a part of the tile
@@ -986,6 +1018,11 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       TileRef r;
       if (s.have_nx) r = s.nx;
       else if (SPLIT) tile_lookup(op, A, B, O, blockIdx.x / share, r);
+      else if (AREA) {
+        const long long i = st->err ? (1ll << 61) : (long long)atomicAdd((unsigned long long*)counter, 1ull);
+        tile_lookup(op, A, B, O, i / share, r);
+        r.pad = (int)(i % share);
+      }
       else tile_lookup(op, A, B, O, st->err ? (1ll << 62) : (long long)atomicAdd((unsigned long long*)counter, 1ull), r);
       s.have_nx = 0;
       if (st->err && !SPLIT) r.tile = 1ll << 62;  // an error stops the CTA, a reserved tile too
@@ -999,8 +1036,13 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       s.down = 0;
       s.err = SPLIT && st->err;
       s.rsplit = 0;
+      if (AREA) {
+        s.q0 = r.pad;  // the CTA's place, until its sub-bands are known
+        s.area = 0;
+      }
     }
     __syncthreads();
+    if (AREA) me = s.q0;
     const long long t = s.tile;
     if (!SPLIT && t >= O->ntiles) break;
     const int nA = s.nA, nB = s.nB, P = nA + nB;
@@ -1011,7 +1053,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       break;
     }
     if (P == 0) {
-      if (tid == 0) { O->tcount[t] = 0; O->tstart[t] = 0; }
+      if (!AREA && tid == 0) { O->tcount[t] = 0; O->tstart[t] = 0; }
       continue;
     }
     if (timing) t0 = clock64();
@@ -1129,7 +1171,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     const int nslab = Nx - 1;
     const int nsbg = (nslab + 62) / 63;
     int q0 = 0, q1 = nsbg;  // the CTA's sub-bands
-    if (SPLIT) {
+    if (SPLIT || AREA) {
       ka = min(share, nsbg);
       q0 = (int)((long long)nsbg * min(me, ka) / ka);
       q1 = (int)((long long)nsbg * min(me + 1, ka) / ka);
@@ -1165,7 +1207,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
             const int r1 = bm_rank2(s.xb, s.xp, x1), r2 = bm_rank2(s.xb, s.xp, x2);
             const int lo = max(r1 / 63, q0), hi = min(q1 - 1, r2 / 63);
             int c1 = 0, c2 = 0;
-            if (!SPLIT || lo <= hi) {
+            if (FORM == TILE_WHOLE || lo <= hi) {
               c1 = bm_rank2(s.yb, s.yp, y1);
               c2 = bm_rank2(s.yb, s.yp, y2);
             }
@@ -1271,14 +1313,23 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         if (k >= nsb) break;
         const int sb = lpt ? ord[k] : k;
         if (__any_sync(0xffffffffu, list) ||
-            !tile_subband<TIMING, false, SPLIT>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
+            !tile_subband<TIMING, false, FORM>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
           if (gb_lane() == 0) TK_WLIST(s, 0)[atomicAdd(&s.nwide[0], 1)] = sb;
         }
       }
     }
     __syncthreads();
-    if (s.nwide[0]) tile_wide<TIMING, SPLIT>(s, op, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
+    if (s.nwide[0]) tile_wide<TIMING, FORM>(s, op, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
     if (tid == 0 && !s.err) s.hint = direct ? s.narrow * 4 <= nsb : s.nwide[0] * 4 >= nsb * 3;
+    if (AREA) {
+      __syncthreads();
+      if (tid == 0) {
+        if (s.err) gb_set_error(st, GB_ERR_CAPACITY, KID_TILE, (long long)scr * 2);
+        else atomicAdd((unsigned long long*)&O->cell_area[s.cell], s.area);
+        if (me == 0) atomicAdd((unsigned long long*)&counter[8], (unsigned long long)P * 8ull);
+      }
+      continue;
+    }
     // the bulk copies of phase D (async proxy) read the records written above and overwrite shared
     // memory written in phases A-C (generic proxy)
     asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -1559,17 +1610,18 @@ static cudaLaunchConfig_t split_config(GbCtx& c, cudaLaunchAttribute* at, int ct
 
 void gb_tile_setup(GbCtx& c) {
   c.tile_smem = sizeof(TileSmem);
-  cudaFuncSetAttribute(k_tile<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
-  cudaFuncSetAttribute(k_tile<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
-  cudaFuncSetAttribute(k_tile<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<false, TILE_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<true, TILE_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<false, TILE_SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
+  cudaFuncSetAttribute(k_tile<false, TILE_AREA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.tile_smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<false, false>, TK_NT, c.tile_smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<false, TILE_WHOLE>, TK_NT, c.tile_smem);
   c.tile_blocks = c.nsm * (per_sm > 0 ? per_sm : 1);
   // clusters of 8 CTAs that the chip holds at once
   cudaLaunchAttribute at;
   cudaLaunchConfig_t cfg = split_config(c, &at, c.tile_blocks / 8 * 8);
   int ncl = 0;
-  if (cudaOccupancyMaxActiveClusters(&ncl, k_tile<false, true>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&ncl, k_tile<false, TILE_SPLIT>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     ncl = 0;
   }
@@ -1595,18 +1647,21 @@ void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLa
     cudaEventRecordWithFlags(e0, c.stream, c.prof_flags);
   }
   // which of the two launches takes the layer depends on its tiles, which the device knows
-  if (c.timing) {
-    k_tile<true, false><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
+  if (mode == 1) {
+    k_tile<false, TILE_AREA><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
+        op, A, B, O, g, mode, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.tile_blocks);
+  } else if (c.timing) {
+    k_tile<true, TILE_WHOLE><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
         op, A, B, O, g, mode | 4, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, 0);
   } else {
     if (c.split_ctas) {
       cudaLaunchAttribute at;
       const cudaLaunchConfig_t cfg = split_config(c, &at, c.split_ctas);
-      cudaLaunchKernelEx(&cfg, k_tile<false, true>, op, A, B, O, g, mode, c.tile_scratch,
+      cudaLaunchKernelEx(&cfg, k_tile<false, TILE_SPLIT>, op, A, B, O, g, mode, c.tile_scratch,
                          (unsigned long long)c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
       ++c.launches;
     }
-    k_tile<false, false><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
+    k_tile<false, TILE_WHOLE><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
         op, A, B, O, g, mode, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
   }
   if (c.prof) cudaEventRecordWithFlags(e1, c.stream, c.prof_flags);
@@ -1801,7 +1856,7 @@ extern "C" int gb_bool_tile_noalloc(int op, const int4* d_A, int nA, const int4*
         fprintf(stderr, "gb_bool_tile_noalloc: cudaGetSymbolAddress failed on device %d\n", dev);
         return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
       }
-      if (cudaFuncSetAttribute(k_tile<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)) !=
+      if (cudaFuncSetAttribute(k_tile<false, TILE_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)) !=
           cudaSuccess)
         return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
       g_na_state_ptr[dev] = (NoAllocState*)a;
@@ -1827,7 +1882,7 @@ extern "C" int gb_bool_tile_noalloc(int op, const int4* d_A, int nA, const int4*
     DStatus* st = &S->res.st;
     int split = 0;
     void* args[] = {&op, &la, &lb, &lo, &gg, &mode, &scr, &scr_bytes, &ctr, &st, &split};
-    if (cudaLaunchKernel((const void*)k_tile<false, false>, dim3(1), dim3(TK_NT), args, sizeof(TileSmem), s) != cudaSuccess)
+    if (cudaLaunchKernel((const void*)k_tile<false, TILE_WHOLE>, dim3(1), dim3(TK_NT), args, sizeof(TileSmem), s) != cudaSuccess)
       return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
   }
   {
