@@ -479,81 +479,7 @@ __global__ void __launch_bounds__(1024) k_bin_setup(const DLayer* S, DLayer* O, 
 }
 
 // ------------------------------------------------------------------ count / scatter
-// mode 0: half-open tile ranges, packed pieces; mode 1: closed ranges, int index payload.
-template <int MODE, bool SCATTER>
-__device__ __forceinline__ void emit_box_tiles(DLayer* O, int k, int4 b, long long payload_idx, int g) {
-  const int4 w = O->win[k];
-  const int tx0 = gb_floor_shift(b.x, g), ty0 = gb_floor_shift(b.y, g);
-  const int tx1 = MODE ? gb_floor_shift(b.z, g) : gb_floor_shift(b.z - 1, g);
-  const int ty1 = MODE ? gb_floor_shift(b.w, g) : gb_floor_shift(b.w - 1, g);
-  const long long tb = O->tbase[k];
-  for (int ty = ty0; ty <= ty1; ++ty) {
-    for (int tx = tx0; tx <= tx1; ++tx) {
-      const long long t = tb + (long long)(ty - w.y) * w.z + (tx - w.x);
-      if (!SCATTER) {
-        atomicAdd(&O->tcount[t], 1);
-      } else {
-        const long long pos = O->tstart[t] + atomicAdd(&O->tcount[t], 1);
-        if (MODE == 0) {
-          const int ox = tx << g, oy = ty << g;
-          const int x1 = max(b.x, ox) - ox, y1 = max(b.y, oy) - oy;
-          const int x2 = (int)(min((long long)b.z, (long long)ox + (1ll << g)) - ox);
-          const int y2 = (int)(min((long long)b.w, (long long)oy + (1ll << g)) - oy);
-          O->pcs[pos] = gb_pack(x1, y1, x2, y2);
-        } else {
-          ((int*)O->pcs)[pos] = (int)payload_idx;
-        }
-      }
-    }
-  }
-}
-
-// All 32 lanes call: a box that lies in one tile (nearly all) takes its slot
-// with one atomic per group of lanes that target the same tile (the group's
-// first lane adds the group's size; each lane's slot is its rank in the
-// group), so the pieces of one source tile, which mostly land in one target
-// tile, do not serialise on that tile's counter.  Boxes over several tiles
-// take the per-tile path.  valid = false: the lane places nothing.  Used for
-// binned sources (count 1.71 -> 0.83 ms, scatter 1.93 -> 1.38 ms per two
-// 1024-cell decks); raw sources scatter over many tiles and keep per-lane
-// slots.
-template <int MODE, bool SCATTER>
-__device__ __forceinline__ void emit_warp(DLayer* O, int k, int4 b, long long payload_idx, int g, bool valid) {
-  const int lane = gb_lane();
-  long long t = -1 - lane;  // distinct for lanes without a single tile
-  bool single = false;
-  int tx0 = 0, ty0 = 0;
-  if (valid) {
-    tx0 = gb_floor_shift(b.x, g);
-    ty0 = gb_floor_shift(b.y, g);
-    const int tx1 = MODE ? gb_floor_shift(b.z, g) : gb_floor_shift(b.z - 1, g);
-    const int ty1 = MODE ? gb_floor_shift(b.w, g) : gb_floor_shift(b.w - 1, g);
-    single = tx0 == tx1 && ty0 == ty1;
-    if (single) {
-      const int4 w = O->win[k];
-      t = O->tbase[k] + (long long)(ty0 - w.y) * w.z + (tx0 - w.x);
-    }
-  }
-  const unsigned grp = __match_any_sync(0xffffffffu, t);
-  const int lead = __ffs(grp) - 1;
-  int base = 0;
-  if (single && lane == lead) base = atomicAdd(&O->tcount[t], __popc(grp));
-  base = __shfl_sync(0xffffffffu, base, lead);
-  if (single) {
-    if (SCATTER) {
-      const long long pos = O->tstart[t] + base + __popc(grp & ((1u << lane) - 1u));
-      if (MODE == 0) {
-        const int ox = tx0 << g, oy = ty0 << g;
-        O->pcs[pos] = gb_pack(b.x - ox, b.y - oy, b.z - ox, b.w - oy);
-      } else {
-        ((int*)O->pcs)[pos] = (int)payload_idx;
-      }
-    }
-  } else if (valid) {
-    emit_box_tiles<MODE, SCATTER>(O, k, b, payload_idx, g);
-  }
-}
-
+// MODE 0: half-open tile ranges, packed pieces; MODE 1: closed ranges, int index payload.
 // Raw source, one contiguous chunk of boxes per block.  The tiles of the
 // chunk's cells are counted in shared memory (up to SPLIT_SM tiles; layers of
 // a few hundred tiles had been bound by global atomics on those few counters:
@@ -562,12 +488,12 @@ __device__ __forceinline__ void emit_warp(DLayer* O, int k, int4 b, long long pa
 // its chunk, reserves each tile's slots with one atomic, and places the
 // pieces on a second walk over the chunk.  A chunk over more tiles takes its
 // slots from the global counters, which many tiles spread.  A box over more
-// than SPLIT_WIDE tiles (the one-box frame of an erosion covers them all) is
-// left to the whole block after the walk: one lane had walked its tiles in
-// series (1200 tiles, 280 us).
+// than SPLIT_WIDE tiles (the one-box frames of an erosion's cells cover them
+// all) is left to the whole block after the walk: one lane had walked its tiles
+// in series (1200 tiles, 280 us), and blocks of 512 such frames took 140 us.
 #define SPLIT_SM 8192
 #define SPLIT_SM_MIN 32768  // smaller layers: the counters see few atomics, and the second walk costs more
-#define SPLIT_WIDE 32
+#define SPLIT_WIDE 8
 #define SPLIT_NWIDE 64  // wide boxes of one chunk held for the block; more are walked by their lanes
 
 struct SplitBox {
@@ -611,7 +537,9 @@ __global__ void __launch_bounds__(256) k_split_raw(const DLayer* S, DLayer* O, i
   int* const tcount = O->tcount;
   const long long* const tstart = O->tstart;
   const int nt = blockDim.x, tid = threadIdx.x;
-  const long long ch = max((long long)nt * 2, (((n + gridDim.x - 1) / gridDim.x) + nt - 1) / nt * nt);
+  // few boxes are spread over the blocks (they may all be wide), many in whole warps
+  const long long even = (n + gridDim.x - 1) / gridDim.x;
+  const long long ch = n < SPLIT_SM_MIN ? even : (even + nt - 1) / nt * nt;
   const long long c0 = (long long)blockIdx.x * ch, c1 = min(n, c0 + ch);
   if (c0 >= n) return;
   const int k0 = gb_find_cell(coff, ncell, c0), k1 = gb_find_cell(coff, ncell, c1 - 1);
@@ -695,13 +623,24 @@ __global__ void __launch_bounds__(256) k_split_raw(const DLayer* S, DLayer* O, i
   walk(true);
 }
 
+// Binned source, one warp per source tile.  A grown piece of one tile lies in
+// the tile of the target that the source tile maps to and its eight neighbours
+// (the same grid, grown by less than a tile), so the warp keeps nine counters:
+// count adds them to the layer's at the end; scatter counts its tile, reserves
+// nine ranges and places the pieces in a second walk.  (Global atomics for
+// every group of 32 pieces and target tile, pieces on tile edges one by one:
+// count 247, scatter 378 us per 512 cells of an OP1 deck; now 132 and 260.)  Other pieces take their slots from the layer's counters.
 template <bool SCATTER>
-__global__ void k_split_bin(const DLayer* S, DLayer* O, int g, int E, int N, int W, int Sg,
-                            DStatus* st) {
+__global__ void __launch_bounds__(256) k_split_bin(const DLayer* S, DLayer* O, int g, int E, int N, int W, int Sg,
+                                                   DStatus* st) {
+  __shared__ int near[8][9];
   if (st->err) return;
   const long long nt = S->ntiles;
-  const int sg = S->g;
+  const int sg = S->g, lane = gb_lane();
   const int wpb = blockDim.x >> 5;
+  int* const cn = near[gb_warp()];
+  int* const tcount = O->tcount;
+  const long long* const tstart = O->tstart;
   for (long long t = (long long)blockIdx.x * wpb + gb_warp(); t < nt; t += (long long)gridDim.x * wpb) {
     const int cnt = S->tcount[t];
     if (cnt == 0) continue;
@@ -709,17 +648,41 @@ __global__ void k_split_bin(const DLayer* S, DLayer* O, int g, int E, int N, int
     tile_of_index(S, t, k, tx, ty);
     const unsigned long long* p = S->pcs + S->tstart[t];
     const int ox = tx << sg, oy = ty << sg;
-    for (int j0 = 0; j0 < cnt; j0 += 32) {  // whole warps: emit_warp is a warp collective
-      const int j = j0 + gb_lane();
-      int4 gbx = make_int4(0, 0, 1, 1);
-      bool ok = false;
-      if (j < cnt) {
+    const int4 w = O->win[k];
+    const long long tb = O->tbase[k];
+    const bool same = sg == g;
+    auto index = [&](int x, int y) { return tb + (long long)(y - w.y) * w.z + (x - w.x); };
+    if (lane < 9) cn[lane] = 0;
+    __syncwarp();
+    auto walk = [&](bool place) {
+      for (int j = lane; j < cnt; j += 32) {
         int a, b, c, d;
         gb_unpack(p[j], a, b, c, d);
-        ok = grow_box(make_int4(ox + a, oy + b, ox + c, oy + d), E, N, W, Sg, gbx);
+        int4 o;
+        if (!grow_box(make_int4(ox + a, oy + b, ox + c, oy + d), E, N, W, Sg, o)) continue;
+        const int4 q = box_tiles<0>(o, g);
+        const bool in9 = same && q.x >= tx - 1 && q.z <= tx + 1 && q.y >= ty - 1 && q.w <= ty + 1;
+        for (int y = q.y; y <= q.w; ++y)
+          for (int x = q.x; x <= q.z; ++x) {
+            if (in9) {
+              const int i = (y - ty + 1) * 3 + (x - tx + 1);
+              const int s = atomicAdd(&cn[i], 1);
+              if (place) put_piece<0>(O, tstart[index(x, y)] + s, o, 0, x, y, g);
+            } else if (SCATTER ? place : !place) {
+              const int s = atomicAdd(&tcount[index(x, y)], 1);
+              if (place) put_piece<0>(O, tstart[index(x, y)] + s, o, 0, x, y, g);
+            }
+          }
       }
-      emit_warp<0, SCATTER>(O, k, gbx, 0, g, ok);
+      __syncwarp();
+    };
+    walk(false);
+    if (lane < 9 && cn[lane]) {
+      const int base = atomicAdd(&tcount[index(tx + lane % 3 - 1, ty + lane / 3 - 1)], cn[lane]);
+      if (SCATTER) cn[lane] = base;
     }
+    __syncwarp();
+    if (SCATTER) walk(true);
   }
 }
 
@@ -974,6 +937,7 @@ __global__ void k_export(const DLayer* L, const long long* dscal, DStatus* st) {
     const unsigned long long* p = L->pcs + L->tstart[t];
     const int ox = tx << g, oy = ty << g;
     const long long o = off[t];
+#pragma unroll 4
     for (int j = gb_lane(); j < cnt; j += 32) {
       int a, b, cc, d;
       gb_unpack(p[j], a, b, cc, d);
@@ -998,6 +962,7 @@ __global__ void k_cell_digest(const DLayer* L, unsigned long long* out, int stri
     const unsigned long long* p = L->pcs + L->tstart[t];
     const int ox = tx << g, oy = ty << g;
     unsigned long long h = 0;
+#pragma unroll 4
     for (int j = gb_lane(); j < cnt; j += 32) {
       int a, b, cc, d;
       gb_unpack(p[j], a, b, cc, d);
