@@ -522,9 +522,9 @@ __global__ void k_enc_sizes(const int* __restrict__ bsize, long long nchunks, lo
 // records per chunk, and the guesses cost 14 more each.  A block stages 128
 // segments (32 KB) with the continuation bits of their bytes, so a length is
 // one byte and three words from shared memory and then register work.
-#define SN_SEG 256
-#define SN_WARM 128       // a guess starts this many bytes before its segment
-#define SN_SEGT 128       // segments (threads) per block
+#define SN_SEG 128
+#define SN_WARM 96        // a guess starts this many bytes before its segment
+#define SN_SEGT 256       // segments (threads) per block
 #define SN_SEGB (SN_SEG * SN_SEGT)
 #define SN_LOOK 64        // bytes staged past the block (more than a record's length)
 #define SN_STG (SN_WARM + SN_SEGB + SN_LOOK)
@@ -537,8 +537,8 @@ __device__ __forceinline__ int sn_len(unsigned info, unsigned long long cont) {
   int l = 1;
   bool bad = false;
   auto varint = [&](bool on) {
-    const int k = __ffsll((long long)~cont);
-    const bool ok = k >= 1 && k <= 10;
+    const int k = __ffs(~(unsigned)cont);  // 0 or beyond 10: too long
+    const bool ok = (unsigned)(k - 1) < 10u;
     bad |= on && !ok;
     const int u = on && ok ? k : 0;
     cont >>= u;
@@ -568,19 +568,28 @@ __device__ __forceinline__ long long seg_stage(SegStage& s, const unsigned char*
   // 16-byte groups of the source, so buf[0] lies up to 15 bytes before `first`
   const int sh = (int)((uintptr_t)(base + first) & 15);
   const long long p0 = first - sh;
-  for (int i = threadIdx.x * 16; i < SN_STG + 32; i += SN_SEGT * 16) {
-    const long long p = p0 + i;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (p >= 0 && p + 16 <= L) {
-      v = *reinterpret_cast<const uint4*>(base + p);
-    } else if (p + 16 > 0 && p < L) {
-      unsigned w[4] = {0, 0, 0, 0};
+  constexpr int U = 3;  // groups in flight per thread
+  for (int i0 = threadIdx.x * 16; i0 < SN_STG + 32; i0 += U * SN_SEGT * 16) {
+    uint4 v[U];
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (p + j >= 0 && p + j < L) w[j >> 2] |= (unsigned)base[p + j] << (8 * (j & 3));
-      v = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * SN_SEGT * 16;
+      const long long p = p0 + i;
+      v[u] = make_uint4(0, 0, 0, 0);
+      if (i >= SN_STG + 32) continue;
+      if (p >= 0 && p + 16 <= L) {
+        v[u] = *reinterpret_cast<const uint4*>(base + p);
+      } else if (p + 16 > 0 && p < L) {
+        unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (p + j >= 0 && p + j < L) w[j >> 2] |= (unsigned)base[p + j] << (8 * (j & 3));
+        v[u] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
-    *reinterpret_cast<uint4*>(s.buf + i) = v;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * SN_SEGT * 16 < SN_STG + 32) *reinterpret_cast<uint4*>(s.buf + i0 + u * SN_SEGT * 16) = v[u];
   }
   __syncthreads();
   for (int w = threadIdx.x; w < SN_STG / 32 + 4; w += SN_SEGT) {
@@ -604,19 +613,16 @@ __device__ __forceinline__ int seg_len(const SegStage& s, int b) {
   return sn_len(s.buf[b], cont);
 }
 
-// The chunk of a block: blk[c] is the first block of chunk c.
-__device__ __forceinline__ int seg_chunk(const long long* blk, int nchunks) {
-  return gb_find_cell(blk, nchunks, blockIdx.x);
-}
+// Grid (blocks of the largest chunk, chunks); blk[c] is the number of blocks
+// of the chunks before c, so segment arrays are indexed by blk[c] + blockIdx.x.
 
 __global__ void __launch_bounds__(SN_SEGT)
 k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
-            const long long* __restrict__ raw_len, const long long* __restrict__ blk, int nchunks,
-            unsigned* __restrict__ entry, unsigned* __restrict__ exit_, unsigned* __restrict__ cnt) {
+            const long long* __restrict__ raw_len, const long long* __restrict__ blk, unsigned* __restrict__ entry, unsigned* __restrict__ exit_, unsigned* __restrict__ cnt) {
   __shared__ SegStage s;
-  const int c = seg_chunk(blk, nchunks);
-  const long long L = raw_len[c];
-  const long long start = (blockIdx.x - blk[c]) * SN_SEGB;
+  const int c = blockIdx.y;
+  const long long L = raw_len[c], blk0 = blk[c], start = (long long)blockIdx.x * SN_SEGB;
+  if (blk0 + blockIdx.x >= blk[c + 1]) return;
   const long long p0 = seg_stage(s, raw + raw_off[c], L, start - SN_WARM);
   const int s0 = (int)(start - p0) + (int)threadIdx.x * SN_SEG, s1 = s0 + SN_SEG;
   const int lim = (int)min((long long)s1, L - p0);
@@ -625,7 +631,7 @@ k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__
     b = s0 - SN_WARM;
     while (b < s0) b += max(1, seg_len(s, b));
   }
-  const size_t g = (size_t)blockIdx.x * SN_SEGT + threadIdx.x;
+  const size_t g = (size_t)(blk0 + blockIdx.x) * SN_SEGT + threadIdx.x;
   entry[g] = (unsigned)(p0 + b);
   unsigned n = 0;
   bool bad = false;
@@ -705,17 +711,16 @@ k_seg_settle(const unsigned char* __restrict__ raw, const long long* __restrict_
 // its records' bytes, the block writes the marked offsets in order.
 __global__ void __launch_bounds__(SN_SEGT)
 k_seg_records(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
-              const long long* __restrict__ raw_len, const long long* __restrict__ blk, int nchunks, long long n,
-              const unsigned* __restrict__ entry, const unsigned* __restrict__ first, unsigned* __restrict__ rec,
+              const long long* __restrict__ raw_len, const long long* __restrict__ blk, long long n, const unsigned* __restrict__ entry, const unsigned* __restrict__ first, unsigned* __restrict__ rec,
               DStatus* st) {
   __shared__ SegStage s;
   __shared__ unsigned mark[SN_SEGB / 32];
   __shared__ SumS buf[32];
-  const int c = seg_chunk(blk, nchunks);
+  const int c = blockIdx.y;
   const int nb = (int)min((long long)SN_CHUNK, n - (long long)c * SN_CHUNK);
-  const long long L = raw_len[c];
-  const long long start = (blockIdx.x - blk[c]) * SN_SEGB;
-  const size_t g0 = (size_t)blockIdx.x * SN_SEGT, g = g0 + threadIdx.x;
+  const long long L = raw_len[c], blk0 = blk[c], start = (long long)blockIdx.x * SN_SEGB;
+  if (blk0 + blockIdx.x >= blk[c + 1]) return;
+  const size_t g0 = (size_t)(blk0 + blockIdx.x) * SN_SEGT, g = g0 + threadIdx.x;
   if (first[g0] >= (unsigned)nb) return;  // uniform: the chunk's records end before this block
   for (int i = threadIdx.x; i < SN_SEGB / 32; i += SN_SEGT) mark[i] = 0;
   const long long p0 = seg_stage(s, raw + raw_off[c], L, start - SN_WARM);
@@ -1592,16 +1597,17 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
     ++c.launches;
     raw = d_raw;
   }
-  if (sblk[nch]) {
-    k_seg_guess<<<(unsigned)sblk[nch], SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, (int)nch, d_seg, d_seg + nseg,
-                                                               d_seg + 2 * nseg);
+  long long most = 0;  // blocks of the largest chunk
+  for (long long i = 0; i < nch; ++i) most = std::max(most, sblk[i + 1] - sblk[i]);
+  const dim3 sgrid((unsigned)most, (unsigned)nch);
+  if (most) {
+    k_seg_guess<<<sgrid, SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, d_seg, d_seg + nseg, d_seg + 2 * nseg);
     ++c.launches;
   }
   k_seg_settle<<<(unsigned)nch, SN_T, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, n, d_seg, d_seg + nseg, d_seg + 2 * nseg,
                                                      c.st);
-  if (sblk[nch]) {
-    k_seg_records<<<(unsigned)sblk[nch], SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, (int)nch, n, d_seg,
-                                                                 d_seg + 2 * nseg, d_rec, c.st);
+  if (most) {
+    k_seg_records<<<sgrid, SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, n, d_seg, d_seg + 2 * nseg, d_rec, c.st);
     ++c.launches;
   }
   const unsigned rb = (unsigned)(nch * SN_BPC);
