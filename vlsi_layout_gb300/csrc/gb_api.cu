@@ -489,12 +489,17 @@ static unsigned long long arena_mark(gb_context* ctx, bool clear) {
 
 extern "C" unsigned long long gb_arena_mark(gb_context* ctx) { return ctx ? arena_mark(ctx, false) : 0; }
 
-extern "C" int gb_arena_release(gb_context* ctx, unsigned long long mark) {
-  if (!ctx || mark >= ctx->marks.size()) return GB_ERR_ARG;
+namespace gbi {
+const unsigned long long* mark_word(gb_context* ctx, unsigned long long mark) {
+  return mark < ctx->marks.size() && ctx->marks[mark].first == MARK_ON_DEVICE ? ctx->c.dmarks + mark : nullptr;
+}
+
+void arena_rewind(gb_context* ctx, unsigned long long mark, bool on_device) {
   const auto m = ctx->marks[mark];
-  ctx->marks.resize(mark);
-  if (m.first == MARK_ON_DEVICE) k_arena_release<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st, ctx->c.dmarks + mark);
-  else gb_launch_arena_reset(ctx->c, m.first);
+  if (on_device) {
+    if (m.first == MARK_ON_DEVICE) k_arena_release<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st, ctx->c.dmarks + mark);
+    else gb_launch_arena_reset(ctx->c, m.first);
+  }
   std::vector<gb_layer*> keep;
   for (gb_layer* L : ctx->arena_layers) {
     if (L->seq > m.second) {
@@ -505,6 +510,13 @@ extern "C" int gb_arena_release(gb_context* ctx, unsigned long long mark) {
     }
   }
   ctx->arena_layers.swap(keep);
+}
+}  // namespace gbi
+
+extern "C" int gb_arena_release(gb_context* ctx, unsigned long long mark) {
+  if (!ctx || mark >= ctx->marks.size()) return GB_ERR_ARG;
+  arena_rewind(ctx, mark, true);
+  ctx->marks.resize(mark);
   return GB_OK;
 }
 

@@ -143,6 +143,11 @@ int layer_over_device(gb_context* ctx, const void* d_boxes, long long n, const l
 // The layer's boxes in device memory: a raw layer's array, or a binned layer
 // exported into the work arena.
 int layer_device_boxes(gb_context* ctx, gb_layer* L, const c_box** d_boxes, long long* n);
+// Drops the layers made after a mark, which stays; the arena itself goes back
+// to the mark on the device (unless a kernel of the caller did so).
+void arena_rewind(gb_context* ctx, unsigned long long mark, bool on_device);
+// The device word that holds the arena offset of a mark (null: kept on the host).
+const unsigned long long* mark_word(gb_context* ctx, unsigned long long mark);
 }
 gb_layer* op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, int mode);
 gb_layer* op_grow(gb_context* ctx, gb_layer* A, int E, int N, int W, int S, bool merge);

@@ -21,15 +21,21 @@
 
 using namespace gbi;
 
+// What a request leaves for the host, written to pinned memory by its last
+// kernel: nothing is copied and no stream is waited for when it retires.
+struct gb_served {
+  long long count;  // strips of the result
+  int err;          // GB_* status of the slot's context
+};
+
 struct gb_server_slot {
   gb_context* ctx = nullptr;
   cudaEvent_t done = nullptr;
   int req = -1;
-  unsigned long long mark = 0;
+  unsigned long long mark = 0;  // the slot's empty arena, for its lifetime
   long long est = 0;
   gb_layer* out = nullptr;
-  long long* dcount = nullptr;  // device: strips of the result
-  long long* hcount = nullptr;  // pinned host copy
+  gb_served* back = nullptr;  // pinned
 };
 
 struct gb_server {
@@ -44,8 +50,11 @@ struct gb_server {
 
 namespace {
 
-__global__ void k_copy_count(const DLayer* L, long long* out) {
-  *out = L->cell_count ? L->cell_count[0] : -1;
+// rewind (may be null): the arena goes back there, the result is not needed.
+__global__ void k_served(const DLayer* L, DStatus* st, gb_served* back, const unsigned long long* rewind) {
+  back->count = L->cell_count ? L->cell_count[0] : -1;
+  back->err = st->err;
+  if (rewind) st->arena_off = *rewind;
 }
 
 long long estimate(const gb_server* S, const gb_request& r) {
@@ -94,8 +103,8 @@ extern "C" int gb_serve_create(int device, unsigned long long budget_bytes, int 
     if (!e) e = gb_set_tile_scratch(sl.ctx, 4ull << 20);
     if (e) break;
     cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
-    cudaMalloc(&sl.dcount, 8);
-    cudaMallocHost(&sl.hcount, 8);
+    cudaMallocHost(&sl.back, sizeof(gb_served));
+    sl.mark = gb_arena_mark(sl.ctx);
     S->slots.push_back(sl);
   }
   if (e) { gb_serve_destroy(S); return e; }
@@ -150,10 +159,9 @@ extern "C" int gb_serve_run(gb_server* S, const gb_request* reqs, int nreq, gb_r
     for (gb_server_slot& sl : S->slots) {
       if (sl.req < 0 || cudaEventQuery(sl.done) != cudaSuccess) continue;
       const int i = sl.req;
-      long long need = 0;
-      int e = gb_sync(sl.ctx, &need);
+      const int e = cudaGetLastError() != cudaSuccess ? GB_ERR_CUDA : sl.back->err;  // a failed launch leaves no status
       res[i].status = e;
-      res[i].count = *sl.hcount;
+      res[i].count = sl.back->count;
       if (!e && keep_outputs && sl.out) {
         unsigned long long n = 0;
         gb_layer_to_host(sl.ctx, sl.out, nullptr, 0, &n, nullptr);
@@ -163,7 +171,7 @@ extern "C" int gb_serve_run(gb_server* S, const gb_request* reqs, int nreq, gb_r
       res[i].end_s = now_s();
       res[i].latency_ms = (res[i].end_s - reqs[i].arrival_s) * 1e3;
       if (e) gb_clear_status(sl.ctx);
-      gb_arena_release(sl.ctx, sl.mark);
+      arena_rewind(sl.ctx, sl.mark, keep_outputs != 0);
       inflight -= sl.est;
       sl.req = -1;
       sl.out = nullptr;
@@ -192,19 +200,18 @@ extern "C" int gb_serve_run(gb_server* S, const gb_request* reqs, int nreq, gb_r
       if (!free_slot || inflight + est > (long long)S->budget) break;
       waiting.pop_front();
       gb_server_slot& sl = *free_slot;
-      sl.mark = gb_arena_mark(sl.ctx);
       res[i].start_s = now_s();
       int st = 0;
       sl.out = issue(S, sl, reqs[i], &st);
       if (!sl.out) {
         res[i].status = st;
         res[i].end_s = now_s();
-        gb_arena_release(sl.ctx, sl.mark);
+        arena_rewind(sl.ctx, sl.mark, true);
         ++done;
         continue;
       }
-      k_copy_count<<<1, 1, 0, sl.ctx->c.stream>>>(sl.out->d, sl.dcount);
-      cudaMemcpyAsync(sl.hcount, sl.dcount, 8, cudaMemcpyDeviceToHost, sl.ctx->c.stream);
+      k_served<<<1, 1, 0, sl.ctx->c.stream>>>(sl.out->d, sl.ctx->c.st, sl.back,
+                                              keep_outputs ? nullptr : mark_word(sl.ctx, sl.mark));
       cudaEventRecord(sl.done, sl.ctx->c.stream);
       sl.req = i;
       sl.est = est;
@@ -238,8 +245,7 @@ extern "C" void gb_serve_destroy(gb_server* S) {
   for (gb_server_slot& sl : S->slots) {
     if (sl.ctx) gb_sync(sl.ctx, nullptr);
     if (sl.done) cudaEventDestroy(sl.done);
-    if (sl.dcount) cudaFree(sl.dcount);
-    if (sl.hcount) cudaFreeHost(sl.hcount);
+    if (sl.back) cudaFreeHost(sl.back);
     if (sl.ctx) gb_context_destroy(sl.ctx);
   }
   for (gb_layer* L : S->raw) gb_layer_free(S->home, L);
