@@ -346,6 +346,12 @@ __device__ __forceinline__ void tile_lookup(int op, const DLayer* A, const DLaye
   }
 }
 
+// The 2, 4 or 8 warps of a team of level 1..3 meet (hardware barriers 1..4).
+__device__ __forceinline__ void team_sync(int level) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + (gb_warp() >> level)), "r"(32 << level) : "memory");
+}
+
 // TIMING: the phase counters of gb_tile_timing are compiled in (tctr non-null
 // then); the production instance has none of that code.
 // WIDE: the level's larger buffers (level 1..3).  Returns false, with nothing
@@ -361,11 +367,18 @@ template <bool TIMING, bool WIDE, int FORM>
 __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int nA, char* base,
                              unsigned long long scr, int level, long long* tctr) {
   if (!TIMING) tctr = nullptr;
+  // a wide sub-band's warps (2, 4 or 8: a team) share its members and columns
   const int lane = gb_lane(), wid = gb_warp();
+  const int T = WIDE ? 32 << level : 32, tl = WIDE ? (int)threadIdx.x & (T - 1) : lane;
+  const int wt = WIDE ? tl >> 5 : 0, lead = WIDE ? wid & ~((1 << level) - 1) : 0;
+  auto tsync = [&]() {
+    if (WIDE) team_sync(level);
+    else __syncwarp();
+  };
   long long q0 = tctr ? clock64() : 0;
   const long long qstart = q0;
 #define TSTEP(k)                                                           \
-  if (tctr && lane == 0) {                                                 \
+  if (tctr && tl == 0) {                                                 \
     const long long q1 = clock64();                                        \
     atomicAdd((unsigned long long*)&tctr[k], (unsigned long long)(q1 - q0)); \
     q0 = q1;                                                               \
@@ -374,7 +387,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   const int beg = sb ? s.sbc[sb - 1] : 0, end = s.sbc[sb];
   const int m = end - beg;
   if (m == 0) {
-    if (lane == 0) {
+    if (tl == 0) {
       s.sbinfo[sb] = make_int4(0, 0, 0, 0);
       s.sbh[sb] = 0;
       s.sbct[sb] = 0;
@@ -393,7 +406,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   int* lv;
   const int srw = WIDE ? lcn >> 5 : TK_LCN / 32;  // words per row of srow
   if (WIDE) {
-    ca = reinterpret_cast<unsigned long long*>(s.dbuf + (size_t)wid * (TK_WBUF << level));
+    ca = reinterpret_cast<unsigned long long*>(s.dbuf + (size_t)lead * TK_WBUF);
     cb = ca + lcn;
     mc = cb + lcn;
     lb = reinterpret_cast<unsigned*>(mc + mcn);
@@ -410,18 +423,18 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     srow = s.srow[wid][0];
   }
   const bool cache = m <= mcn;
-  for (int w = lane; w < nwy; w += 32) lb[w] = 0;
-  __syncwarp();
-  for (int j0 = 0; j0 < m; j0 += 32 * TK_MLD) {
+  for (int w = tl; w < nwy; w += T) lb[w] = 0;
+  tsync();
+  for (int j0 = 0; j0 < m; j0 += T * TK_MLD) {
     int4 rr[TK_MLD];
 #pragma unroll
     for (int u = 0; u < TK_MLD; ++u) {
-      const int j = j0 + u * 32 + lane;
+      const int j = j0 + u * T + tl;
       rr[u] = j < m ? s.mem[beg + j] : make_int4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int u = 0; u < TK_MLD; ++u) {
-      const int j = j0 + u * 32 + lane;
+      const int j = j0 + u * T + tl;
       if (j < m) {
         const int4 r = rr[u];
         if (cache) {
@@ -434,40 +447,49 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       }
     }
   }
-  __syncwarp();
+  tsync();
   int nl;
   {
-    const int per = WIDE ? ((nwy + 31) >> 5) | 1 : (nwy + 31) >> 5, w0 = min(nwy, lane * per), w1 = min(nwy, w0 + per);
+    const int per = WIDE ? ((nwy + T - 1) / T) | 1 : (nwy + 31) >> 5, w0 = min(nwy, tl * per), w1 = min(nwy, w0 + per);
     int cnt = 0;
     for (int w = w0; w < w1; ++w) cnt += __popc(lb[w]);
     int tot;
     int ex = gb_warp_excl(cnt, &tot);
+    if (WIDE) {
+      if (lane == 0) s.tmp64[wid] = tot;
+      tsync();
+      tot = 0;
+      for (int i = 0; i < T >> 5; ++i) {
+        const int v = (int)s.tmp64[lead + i];
+        if (i < wt) ex += v;
+        tot += v;
+      }
+    }
     for (int w = w0; w < w1; ++w) { lp[w] = ex; ex += __popc(lb[w]); }
     nl = tot;
   }
   const int L = nl - 1;
   TSTEP(0)
-  if (tctr && lane == 0) {
+  if (tctr && tl == 0) {
     atomicAdd((unsigned long long*)&tctr[6], (unsigned long long)m);
     atomicAdd((unsigned long long*)&tctr[7], (unsigned long long)L);
   }
   if (L > lcn) {
     if (!WIDE || level < TK_WLEVELS) return false;
-    unsigned long long pv = 0, pc = 0;
-    if (lane == 0) {
-      pv = (unsigned long long)sc_up(s, base, half, (unsigned long long)nl * 4);
-      pc = (unsigned long long)sc_up(s, base, half, (unsigned long long)L * 16);
+    if (tl == 0) {
+      s.tmp64[8 + lead] = (long long)sc_up(s, base, half, (unsigned long long)nl * 4);
+      s.tmp64[9 + lead] = (long long)sc_up(s, base, half, (unsigned long long)L * 16);
     }
-    pv = __shfl_sync(0xffffffffu, pv, 0);
-    pc = __shfl_sync(0xffffffffu, pc, 0);
+    tsync();
+    const long long pv = s.tmp64[8 + lead], pc = s.tmp64[9 + lead];
     if (!pv || !pc) return true;  // s.err is set
     lv = (int*)pv;
     ca = (unsigned long long*)pc;
     cb = ca + L;
   }
-  if (WIDE && level == 1 && lane == 0 && L <= TK_LCN && nwy <= TK_LBW) atomicAdd(&s.narrow, 1);
+  if (WIDE && level == 1 && tl == 0 && L <= TK_LCN && nwy <= TK_LBW) atomicAdd(&s.narrow, 1);
   {
-    const int per = WIDE ? ((nwy + 31) >> 5) | 1 : (nwy + 31) >> 5, w0 = min(nwy, lane * per), w1 = min(nwy, w0 + per);
+    const int per = WIDE ? ((nwy + T - 1) / T) | 1 : (nwy + 31) >> 5, w0 = min(nwy, tl * per), w1 = min(nwy, w0 + per);
     for (int w = w0; w < w1; ++w) {
       unsigned bits = lb[w];
       int k = lp[w];
@@ -480,15 +502,15 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   }
   // ---- rasterise: one member per lane; each column word is updated as two
   // 32-bit halves with native shared-memory atomicOr
-  // columns per lane; an odd count keeps the lanes' 8-byte words on different banks (wide ones have 5..33)
-  const int per = WIDE ? ((L + 31) >> 5) | 1 : (L + 31) >> 5, c0 = min(L, lane * per), c1e = min(L, c0 + per);
+  // columns per lane; an odd count keeps the lanes' 8-byte words on different banks
+  const int per = WIDE ? ((L + T - 1) / T) | 1 : (L + 31) >> 5, c0 = min(L, tl * per), c1e = min(L, c0 + per);
   for (int c = c0; c < c1e; ++c) { ca[c] = 0; cb[c] = 0; }
-  __syncwarp();
+  tsync();
   // 32 members at a time: the (member, column) pairs of the group are spread
   // evenly over the lanes (a warp scan of the spans, then a shuffle search for
   // the member of each pair), so one long member does not serialise a lane.
   long long qa = tctr ? clock64() : 0, qsetup = 0, qpaint = 0;
-  for (int jb = 0; jb < m; jb += 32) {
+  for (int jb = 32 * wt; jb < m; jb += T) {
     const int j = jb + lane;
     int lc1 = 0, span = 0, own = 0;
     unsigned long long mk = 0;
@@ -561,8 +583,8 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     }
     if (tctr) { const long long qb = clock64(); qpaint += qb - qa; qa = qb; }
   }
-  __syncwarp();
-  if (tctr && lane == 0) {
+  tsync();
+  if (tctr && tl == 0) {
     atomicAdd((unsigned long long*)&tctr[8], (unsigned long long)qsetup);
     atomicAdd((unsigned long long*)&tctr[9], (unsigned long long)qpaint);
   }
@@ -574,9 +596,15 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   }
   // No region in rows 1..63: the sub-band has no strip pieces (row 0 belongs to
   // the previous sub-band, and its runs matter only to continuations here).
-  if (!__any_sync(0xffffffffu, (rany & ~1ull) != 0ull)) {
+  bool any = __any_sync(0xffffffffu, (rany & ~1ull) != 0ull);
+  if (WIDE) {
+    if (lane == 0) s.tmp64[8 + wid] = any;
+    tsync();
+    for (int i = 0; i < T >> 5; ++i) any |= s.tmp64[8 + lead + i] != 0;
+  }
+  if (!any) {
     TSTEP(1)
-    if (lane == 0) {
+    if (tl == 0) {
       s.sbinfo[sb] = make_int4(0, 0, 0, 0);
       s.sbh[sb] = 0;
       s.sbct[sb] = 0;
@@ -613,7 +641,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   const bool tr = !WIDE || L <= lcn;
   if (tr) {
     const int nb = (L + 31) >> 5;
-    for (int b = 0; b < nb; ++b) {
+    for (int b = wt; b < nb; b += T >> 5) {
       const int c = (b << 5) + lane;
       const unsigned long long Rc = c < L ? ca[c] : 0ull;
       const unsigned long long Rm = (c >= 1 && c - 1 < L) ? ca[c - 1] : 0ull;
@@ -636,7 +664,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       srow[lane * srw + b] = lo;
       srow[(32 + lane) * srw + b] = hi;
     }
-    __syncwarp();
+    if (!WIDE) __syncwarp();  // a team's columns meet at the barriers below
   }
   TSTEP(5)
 
@@ -665,6 +693,18 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   }
   unsigned long long Fin = __shfl_up_sync(0xffffffffu, IA, 1);
   if (lane == 0) Fin = 0ull;
+  if (WIDE) {
+    if (lane == 31) {
+      s.tmp64[wid] = (long long)IA;
+      s.tmp64[16 + wid] = (long long)IB;
+    }
+    tsync();
+    unsigned long long Fw = 0ull;  // into the warp's columns
+    for (int i = 0; i < wt; ++i) Fw = (unsigned long long)s.tmp64[lead + i] | ((unsigned long long)s.tmp64[16 + lead + i] & Fw);
+    unsigned long long Bin = __shfl_up_sync(0xffffffffu, IB, 1);
+    if (lane == 0) Bin = ~0ull;
+    Fin |= Bin & Fw;
+  }
   const bool last_sb = gsb == (FORM != TILE_WHOLE ? s.nsbg : nsb) - 1;
   TSTEP(2)
 
@@ -674,7 +714,8 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   // bitmap words behind it in the wide buffers), dead after the raster.
   const bool packed = !WIDE || L <= 512;
   unsigned long long* const pf = mc;
-  int np = 0, no = 0, nh = 0, ncn = 0, nz = 0;
+  int* const pos = reinterpret_cast<int*>(mc);
+  int np = 0, no = 0, ncn = 0, nz = 0;
   unsigned long long pv = 0;
   {
     unsigned long long Rm1 = R(c0 - 1), fb = ~0ull;
@@ -696,7 +737,6 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       } else {
         np += pc;
         no += open;
-        nh += pc - cont;
         ncn += cont;
         nz += (int)(Ec & 1ull);
       }
@@ -706,26 +746,56 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   int totP, totO, totH, totC, totZ;
   // runs at row 0 are the runs at row 63 of the previous sub-band, both in y
   // order: a continuation's ordinal among them indexes that sub-band's open list
-  int posZ = 0, posP = 0, posO = 0, posH = 0, posC = 0;
+  int posZ = 0, posP = 0, posO = 0, posC = 0;
   if (packed) {
     unsigned long long t;
-    const unsigned long long e = gb_warp_excl(pv, &t);
+    unsigned long long e = gb_warp_excl(pv, &t);
+    if (WIDE) {
+      if (lane == 0) s.tmp64[8 + wid] = (long long)t;
+      tsync();
+      t = 0;
+      for (int i = 0; i < T >> 5; ++i) {
+        const unsigned long long v = (unsigned long long)s.tmp64[8 + lead + i];
+        if (i < wt) e += v;
+        t += v;
+      }
+    }
     for (int c = c0; c < c1e; ++c) pf[c] += e;
     totP = (int)(t & 0xffffu);
     totH = (int)((t >> 16) & 0xffffu);
     totO = (int)((t >> 32) & 0x3ffu);
     totC = (int)((t >> 42) & 0x3ffu);
-    __syncwarp();
+    if (!WIDE) __syncwarp();
   } else {
+    // only in a team: every thread's counts before its columns (pos, in pf's place: the sweeps' words there are
+    // dead), behind the other warps' totals
     posZ = gb_warp_excl(nz, &totZ);
     posP = gb_warp_excl(np, &totP);
     posO = gb_warp_excl(no, &totO);
-    posH = gb_warp_excl(nh, &totH);
     posC = gb_warp_excl(ncn, &totC);
+    if (lane == 0) {
+      s.tmp64[8 + wid] = (long long)totP << 32 | totO;
+      s.tmp64[24 + wid] = (long long)totC << 32 | totZ;
+    }
+    tsync();
+    totP = totO = totC = 0;
+    for (int i = 0; i < T >> 5; ++i) {
+      const long long po = s.tmp64[8 + lead + i], cz = s.tmp64[24 + lead + i];
+      const int vp = (int)(po >> 32), vo = (int)po, vc = (int)(cz >> 32);
+      if (i < wt) { posP += vp; posO += vo; posC += vc; posZ += (int)cz; }
+      totP += vp;
+      totO += vo;
+      totC += vc;
+    }
+    totH = totP - totC;
+    pos[tl] = posP;
+    pos[T + tl] = posO;
+    pos[2 * T + tl] = posC;
+    pos[3 * T + tl] = posZ;
   }
   int pbase = 0;
   unsigned long long obase = 0, rbase = 0;
-  if (lane == 0) {
+  if (tl == 0) {
     pbase = (int)atomicAdd(&s.down, (unsigned long long)totP);
     if (totP > 0) {
       // the record region is the upper half of the scratch, indexed by piece
@@ -746,21 +816,32 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       if (!p) pbase = -1;
     }
   }
-  pbase = __shfl_sync(0xffffffffu, pbase, 0);
-  obase = __shfl_sync(0xffffffffu, obase, 0);
-  rbase = __shfl_sync(0xffffffffu, rbase, 0);
+  if (WIDE) {
+    if (tl == 0) {
+      s.tmp64[lead] = pbase;
+      s.tmp64[lead + 1] = (long long)obase;
+      s.tmp64[16 + lead] = (long long)rbase;
+    }
+    tsync();
+    pbase = (int)s.tmp64[lead];
+    obase = (unsigned long long)s.tmp64[lead + 1];
+    rbase = (unsigned long long)s.tmp64[16 + lead];
+  } else {
+    pbase = __shfl_sync(0xffffffffu, pbase, 0);
+    obase = __shfl_sync(0xffffffffu, obase, 0);
+    rbase = __shfl_sync(0xffffffffu, rbase, 0);
+  }
   if (pbase < 0) return true;
   PieceRec* recs = (PieceRec*)rbase;
   int* olist = (int*)obase;  // open pieces, then continuation pieces, each in y order, then the latter's ordinals
   TSTEP(3)
 
   // ---- write pieces, dealt to the lanes 32 at a time in (column, row) order: piece k's column is found by a
-  // binary search over the columns' packed counts (of more than 512 columns: by a shuffle search over the lanes'
-  // piece counts and a walk over that lane's columns), its row is its rank among the column's piece starts
+  // binary search over the columns' packed counts (of more than 512 columns: over the threads'
+  // counts, and a walk over that thread's columns), its row is its rank among the column's piece starts
   {
-    const int inclP = posP + np;
-    for (int k0 = 0; k0 < totP; k0 += 32) {  // warp-uniform trip count
-      const int k = k0 + lane;
+    for (int k0 = 0; k0 < totP; k0 += T) {  // uniform trip count
+      const int k = k0 + tl;
       int j = 0, o = 0, h = 0, q = 0, z = 0, c = 0;
       if (packed) {
         const unsigned* p32 = reinterpret_cast<const unsigned*>(pf);
@@ -774,17 +855,15 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
         q = (int)((e >> 42) & 0x3ffu);
         z = (int)((e >> 52) & 0x3ffu);
       } else {
-        int ow = 0;  // owner lane: the first lane whose inclusive piece prefix exceeds k
-#pragma unroll
-        for (int st2 = 16; st2 > 0; st2 >>= 1) {
-          const int v = __shfl_sync(0xffffffffu, inclP, ow + st2 - 1);
-          if (v <= k) ow += st2;
-        }
-        j = k - __shfl_sync(0xffffffffu, posP, ow);
-        o = __shfl_sync(0xffffffffu, posO, ow);
-        h = __shfl_sync(0xffffffffu, posH, ow);
-        q = __shfl_sync(0xffffffffu, posC, ow);
-        z = __shfl_sync(0xffffffffu, posZ, ow);
+        int ow = 0;  // owner: the last thread whose columns start at or before piece k
+        for (int st2 = T >> 1; st2 > 0; st2 >>= 1)
+          if (pos[ow + st2] <= k) ow += st2;
+        j = pos[ow];
+        o = pos[T + ow];
+        q = pos[2 * T + ow];
+        z = pos[3 * T + ow];
+        h = j - q;
+        j = k - j;
         c = min(L, ow * per);
       }
       if (k < totP) {
@@ -843,12 +922,12 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     }
   }
   TSTEP(4)
-  if (tctr && lane == 0) {  // wide sub-bands: count and cycles
+  if (tctr && tl == 0) {  // wide sub-bands: count and cycles
     const long long q1 = clock64();
     atomicAdd((unsigned long long*)&tctr[28 + (WIDE ? 0 : 2)], 1ull);
     atomicAdd((unsigned long long*)&tctr[29 + (WIDE ? 0 : 2)], (unsigned long long)(q1 - qstart));
   }
-  if (lane == 0) {
+  if (tl == 0) {
     s.sbinfo[sb] = make_int4(pbase, totP, totO, 0);
     s.sbol[sb] = (int*)obase;
     s.sbrec[sb] = recs;
@@ -921,7 +1000,7 @@ __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* rec
   return area;
 }
 
-// Levels 1..3 of phase C: the wide sub-bands that the level below listed, by fewer warps with larger buffers.
+// Levels 1..3 of phase C: the wide sub-bands that the level below listed, by teams of warps that share a buffer.
 // Called by the whole CTA after level 0.  Out of line: its registers stay out of the kernel's narrow path.
 template <bool TIMING, int FORM>
 __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int nA, char* base,
@@ -932,16 +1011,17 @@ __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int
     if (todo == 0) break;  // uniform: neither changes before the next barrier
     if (threadIdx.x == 0) s.sbnext = 0;
     __syncthreads();
-    if (gb_warp() >= (TK_NW >> level)) continue;
+    const int lead = gb_warp() & ~((1 << level) - 1);
+    const bool first = (threadIdx.x & ((32 << level) - 1)) == 0;  // of the team
     for (;;) {
-      int k = 0;
-      if (gb_lane() == 0) k = atomicAdd(&s.sbnext, 1);
-      k = __shfl_sync(0xffffffffu, k, 0);
+      team_sync(level);  // the sub-band before is done with the team's words
+      if (first) s.tmp64[24 + lead] = atomicAdd(&s.sbnext, 1);
+      team_sync(level);
+      const int k = (int)s.tmp64[24 + lead];
       if (k >= todo) break;
       const int sb = TK_WLIST(s, level - 1)[k];
-      if (!tile_subband<TIMING, true, FORM>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && gb_lane() == 0)
+      if (!tile_subband<TIMING, true, FORM>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && first)
         TK_WLIST(s, level)[atomicAdd(&s.nwide[level], 1)] = sb;
-      __syncwarp();
     }
   }
 }
