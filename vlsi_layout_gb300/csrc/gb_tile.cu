@@ -1357,16 +1357,19 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     if (timing) { const long long t1 = clock64(); tB += t1 - t0; t0 = t1; }
     // ---- C: one warp per sub-band, handed out dynamically, the ones with the most members first
     // (longest processing time first: the phase ends with the last sub-band, so the large ones must
-    // not come last).  The order lives in the value-table region, unused until phase D.
+    // not come last).  The order lives in the value-table region, unused until phase D.  One load a step, four
+    // in flight: 1024 cells 31.45 -> 31.27 ms.
     int* const ord = s.xyv + TK_MD_INTS;
     const bool lpt = !s.err && nsb > TK_NW && nsb <= TK_SBS;
     if (lpt) {
       for (int q = tid; q < nsb; q += TK_NT) {
         const int mq = s.sbc[q] - (q ? s.sbc[q - 1] : 0);
-        int r = 0;
+        int r = 0, before = 0;
+#pragma unroll 4
         for (int j = 0; j < nsb; ++j) {
-          const int mj = s.sbc[j] - (j ? s.sbc[j - 1] : 0);
-          r += (mj > mq) || (mj == mq && j < q);
+          const int e = s.sbc[j], mj = e - before;
+          before = e;
+          r += mj > mq || (mj == mq && j < q);
         }
         ord[r] = q;
       }
