@@ -78,9 +78,10 @@
                     // records 30.88 -> 30.59 ms)
 #define TK_DU 2     // pieces per thread and step of phase D when the records stay in the scratch
 #define TK_LD 2     // independent global loads in flight per thread in the streaming loops
-#define TK_DIRECT 1 // columns of a member painted on its own lane; the rest are spread over the warp
-                    // (measured per 1024-cell deck: 0 / 1 / 2 / 3 / 4 / 8 columns -> 35.16 / 34.78 /
-                    // 34.91 / 34.85 / 35.02 / 38.13 ms)
+// Columns of a member painted on its own lane; the rest are spread over the warp (device time of a 1024-cell deck
+// at 0 / 1 / 2 columns: 30.34 / 30.29 / 30.66 ms; of the wide sub-bands of two 1M-box layers 607 / 592 / 579 us a
+// tile).
+#define TK_DIRECT (WIDE ? 2 : 1)
 #define KID_TILE 20
 
 // A strip piece of one sub-band, 16 bytes, stored downward from the top of
@@ -507,8 +508,11 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   for (int c = c0; c < c1e; ++c) { ca[c] = 0; cb[c] = 0; }
   tsync();
   // 32 members at a time: the (member, column) pairs of the group are spread
-  // evenly over the lanes (a warp scan of the spans, then a shuffle search for
-  // the member of each pair), so one long member does not serialise a lane.
+  // evenly over the lanes (a warp scan of the spans; the member of a pair from
+  // a warp-wide mask of the members' first pairs), so one long member does not
+  // serialise a lane.  A five-step shuffle search in the mask's place: 31.27 ms
+  // a 1024-cell deck and not 30.28; in the wide form it is the faster one (592
+  // against 798 us a tile, the registers).
   long long qa = tctr ? clock64() : 0, qsetup = 0, qpaint = 0;
   for (int jb = 32 * wt; jb < m; jb += T) {
     const int j = jb + lane;
@@ -556,22 +560,39 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     if (__any_sync(0xffffffffu, rest > 0)) {
       const int incl = gb_warp_incl(rest);
       const int total = __shfl_sync(0xffffffffu, incl, 31);
+      const int cm = ((lc1 + TK_DIRECT - (incl - rest)) << 1) | own;  // a pair's column less its index; the operand
+      // the lanes with pairs, in order: lane i keeps the i-th (the bytes lie in srow, unused until the transposition)
+      const unsigned le = 0xffffffffu >> (31 - lane);
+      int src = 0, seen = 0;
+      if (!WIDE) {
+        unsigned char* const order = reinterpret_cast<unsigned char*>(srow);
+        const unsigned has = __ballot_sync(0xffffffffu, rest > 0);
+        if (rest > 0) order[__popc(has & (le >> 1))] = (unsigned char)lane;
+        __syncwarp();
+        src = order[lane];
+        __syncwarp();
+      }
       if (tctr && lane == 0) atomicAdd((unsigned long long*)&tctr[12], (unsigned long long)total);
       for (int k0 = 0; k0 < total; k0 += 32) {  // warp-uniform trip count
         const int k = k0 + lane;
-        int o = 0;  // owner lane: the first lane whose inclusive prefix exceeds k
+        int o = 0;  // owner lane
+        if (WIDE) {  // the first whose inclusive prefix exceeds k
 #pragma unroll
-        for (int st2 = 16; st2 > 0; st2 >>= 1) {
-          const int v = __shfl_sync(0xffffffffu, incl, o + st2 - 1);
-          if (v <= k) o += st2;
+          for (int st2 = 16; st2 > 0; st2 >>= 1) {
+            const int v = __shfl_sync(0xffffffffu, incl, o + st2 - 1);
+            if (v <= k) o += st2;
+          }
+        } else {  // of the lanes with pairs the last that starts at or before k: a bit for each start in [k0, k0 + 32)
+          const unsigned d = (unsigned)(incl - rest - k0);
+          const unsigned starts = __reduce_or_sync(0xffffffffu, rest > 0 && d < 32u ? 1u << d : 0u);
+          o = __shfl_sync(0xffffffffu, src, seen + __popc(starts & le) - 1);
+          seen += __popc(starts);
         }
-        const int ex_o = __shfl_sync(0xffffffffu, incl - rest, o);
-        const int c1_o = __shfl_sync(0xffffffffu, lc1, o);
-        const int own_o = __shfl_sync(0xffffffffu, own, o);
+        const int cm_o = __shfl_sync(0xffffffffu, cm, o);
         const unsigned long long mk_o = __shfl_sync(0xffffffffu, mk, o);
         if (k < total) {
-          unsigned* col = (unsigned*)(own_o ? cb : ca);
-          const int c = c1_o + TK_DIRECT + (k - ex_o);
+          unsigned* col = (unsigned*)((cm_o & 1) ? cb : ca);
+          const int c = (cm_o >> 1) + k;
           if (op == GB_OP_OVERLAP) {
             paint_twice((unsigned*)ca, (unsigned*)cb, c, (unsigned)mk_o, (unsigned)(mk_o >> 32));
           } else {
