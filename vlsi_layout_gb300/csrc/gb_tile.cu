@@ -509,18 +509,6 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     cb = ca + L;
   }
   if (WIDE && level == 1 && tl == 0 && L <= TK_LCN && nwy <= TK_LBW) atomicAdd(&s.narrow, 1);
-  {
-    const int per = WIDE ? ((nwy + T - 1) / T) | 1 : (nwy + 31) >> 5, w0 = min(nwy, tl * per), w1 = min(nwy, w0 + per);
-    for (int w = w0; w < w1; ++w) {
-      unsigned bits = lb[w];
-      int k = lp[w];
-      while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        lv[k++] = (w << 5) + b;
-      }
-    }
-  }
   // ---- rasterise: one member per lane; each column word is updated as two
   // 32-bit halves with native shared-memory atomicOr
   // columns per lane; an odd count keeps the lanes' 8-byte words on different banks
@@ -558,7 +546,10 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       }
       mk = (hi >= 64 ? ~0ull : ((1ull << hi) - 1ull)) & (~0ull << lo);
       lc1 = bm_rank(lb, lp, yz);
-      span = bm_rank(lb, lp, yw) - lc1;
+      const int lc2 = bm_rank(lb, lp, yw);
+      span = lc2 - lc1;
+      lv[lc1] = yz;  // a column's bound comes from every member that has it: the same value
+      lv[lc2] = yw;
     }
     // direct: the first TK_DIRECT columns of every member on its own lane
     {
