@@ -34,7 +34,7 @@
 //     row) order, so a column with many pieces does not hold up the warp; a
 //     piece's 16-byte record goes to the CTA's record region at its index.
 //     A sub-band with more columns or y ranks than a warp's buffer holds is
-//     wide: the tile's wide ones are swept afterwards by fewer warps with
+//     wide: the tile's wide ones are swept afterwards by teams of warps with
 //     larger buffers.
 //  D. Stitch.  The records come into shared memory in one bulk copy.  Each
 //     continuation is linked to the open piece of the previous sub-band with
@@ -111,12 +111,12 @@ struct TileRef {
 };
 
 struct TileSmem {
-  union {  // phases A-B: value bitmaps and their prefix popcounts; phase D: x / y value tables
+  union {  // phases A-B: value bitmaps and their prefix popcounts; then what is below
     struct {
       unsigned xb[TK_WMAX], yb[TK_WMAX];
       unsigned xp[TK_PMAX], yp[TK_PMAX];  // prefix popcount per 2 words
     };
-    int xyv[TK_XYV];  // phase D; after the metadata below when it is here
+    int xyv[TK_XYV];  // sub-band metadata, hand-out order, wide lists, x / y value tables
   };
   int sbc_s[TK_SBS + 2];  // per sub-band member counts / cursors (scratch when more sub-bands)
   union {  // phase C: per-warp sweep buffers; phase D: piece records and chain links
@@ -152,6 +152,7 @@ struct TileSmem {
   // up: bytes allocated from the lower half of the scratch; down: strip pieces so far, whose records sit at
   // their piece index in the upper half (the record region)
   unsigned long long up, down;
+  int t16, t16o;  // the x / y value tables lie in xyv at word t16o, 16 bits a value, t16 x values; t16 0: Xt, Yt
   int* Xt;
   int* Yt;
   int4* rk;
@@ -204,9 +205,24 @@ __device__ __forceinline__ int split_end(const char* pub0, unsigned long long sc
   }
   return 0;  // not reached: the last share has no open pieces
 }
-// Wide lists of phase C, alternating by level, behind the metadata and the hand-out order in xyv.
-#define TK_WLIST(s, level) ((s).xyv + TK_MD_INTS + TK_SBS + ((level) & 1) * (TK_NSBMAX + 2))
+// Wide lists of phase C, alternating by level, behind the metadata and the hand-out order in xyv; then the value
+// tables, when they fit.
+#define TK_WLIST(s, level, nsb) ((s).xyv + TK_MD_INTS + TK_SBS + ((level) & 1) * ((nsb) + 2))
 static_assert(TK_MD_INTS + TK_SBS + 2 * (TK_NSBMAX + 2) <= TK_XYV, "wide lists");
+
+// The values of x and y ranks, as the start or the end of an interval.  16 bits hold 0..65536: no interval ends at 0
+// (stored for 65536) and none starts at 65536.
+struct TileXY {
+  const unsigned short *x16, *y16;
+  const int *x, *y;
+  bool on;
+  __device__ __forceinline__ explicit TileXY(const TileSmem& s)
+      : x16(reinterpret_cast<const unsigned short*>(s.xyv + s.t16o)), y16(x16 + s.t16), x(s.Xt), y(s.Yt), on(s.t16 != 0) {}
+  __device__ __forceinline__ int x0(int r) const { return on ? x16[r] : x[r]; }
+  __device__ __forceinline__ int y0(int r) const { return on ? y16[r] : y[r]; }
+  __device__ __forceinline__ int x1(int r) const { return on ? ((x16[r] + 0xffff) & 0xffff) + 1 : x[r]; }
+  __device__ __forceinline__ int y1(int r) const { return on ? ((y16[r] + 0xffff) & 0xffff) + 1 : y[r]; }
+};
 
 // Sweep buffer of a warp at level 1..3: columns, bitmap words, cached members.
 __device__ __forceinline__ int wide_cols(int level) { return level == 1 ? 288 : level == 2 ? 640 : 1024; }
@@ -229,9 +245,8 @@ static_assert(sizeof(((TileSmem*)0)->lb) + sizeof(((TileSmem*)0)->lp) + sizeof((
 // Bulk asynchronous copies need 16-byte aligned shared-memory addresses, and
 // the staged ranks, piece records and sub-band metadata are read as int4.
 static_assert(offsetof(TileSmem, dbuf) % 16 == 0, "phase C/D region must start on 16 bytes");
-static_assert(offsetof(TileSmem, xyv) % 16 == 0, "value-table region must start on 16 bytes");
+static_assert(offsetof(TileSmem, xyv) % 16 == 0, "bitmaps are cleared 16 bytes at a time");
 static_assert(offsetof(TileSmem, ca) % 16 == 0 && offsetof(TileSmem, srow) % 16 == 0, "per-warp arrays");
-static_assert((TK_MD_INTS * 4) % 16 == 0, "value tables after the metadata start on 16 bytes");
 
 
 __device__ __forceinline__ unsigned long long gb_pred(int op, unsigned long long a, unsigned long long b) {
@@ -649,7 +664,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   __syncwarp();
   if (FORM == TILE_AREA) {
     // per column its height times the width of its runs of rows 1..63 (row 0 is the sub-band before's)
-    const int *Xt = s.Xt, *Yt = s.Yt;
+    const TileXY xy(s);
     long long area = 0;
     for (int c = c0; c < c1e; ++c) {
       unsigned long long rr = ca[c] & ~1ull;
@@ -658,10 +673,10 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
       while (rr) {
         const int r1 = __ffsll((long long)rr) - 1;
         const int r2 = r1 + __ffsll((long long)~(rr >> r1)) - 1;  // shifted-in zeros (r1 >= 1) end a run at row 63
-        w += Xt[rowbase + r2] - Xt[rowbase + r1];
+        w += xy.x1(rowbase + r2) - xy.x0(rowbase + r1);
         rr = r2 >= 64 ? 0ull : rr & (~0ull << r2);
       }
-      area += (long long)w * (Yt[lv[c + 1]] - Yt[lv[c]]);
+      area += (long long)w * (xy.y1(lv[c + 1]) - xy.y0(lv[c]));
     }
     area = gb_warp_sum(area);
     if (lane == 0) atomicAdd(&s.area, (unsigned long long)area);
@@ -975,12 +990,13 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
 // sub-bands as the strip spans, so its links are what bounds the step: on chip (16 bits, sl16) a hop takes an L1
 // latency and not L2's.  Out of line: its registers stay out of the kernel's main path.  Returns the area.
 template <bool SPLIT>
-__device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* recs, int NP, int nsb, const int* Xv,
-                                                    const int* Yv, unsigned long long* outp, bool sl16,
+__device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* recs, int NP, int nsb,
+                                                    unsigned long long* outp, bool sl16,
                                                     const char* pub0, unsigned long long scr, int me, int ka) {
   const PieceRec* rg = reinterpret_cast<const PieceRec*>(recs);
   const unsigned short* s16 = reinterpret_cast<const unsigned short*>(s.dbuf);
   const int* s32 = s.succ;
+  const TileXY xy(s);
   auto rec = [&](int q) -> PieceRec {
     if (!s.rsplit) return rg[q];
     int sb = 0;  // some records lie elsewhere: the sub-band that holds piece q
@@ -1024,7 +1040,7 @@ __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* rec
     for (int u = 0; u < TK_DU; ++u) {
       if (pr_cont(r[u])) continue;
       const int slo = pr_slo(r[u]);
-      const int xs = Xv[slo], xe = Xv[pr_shi(r[u])], ylo = Yv[pr_ylo(r[u])], yhi = Yv[pr_yhi(r[u])];
+      const int xs = xy.x0(slo), xe = xy.x1(pr_shi(r[u])), ylo = xy.y0(pr_ylo(r[u])), yhi = xy.y1(pr_yhi(r[u]));
       if (outp) outp[s.sbh[slo / 63 - (SPLIT ? s.q0 : 0)] + pr_hrank(r[u])] = gb_pack(xs, ylo, xe, yhi);
       area += (long long)(xe - xs) * (long long)(yhi - ylo);
     }
@@ -1051,9 +1067,9 @@ __device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int
       team_sync(level);
       const int k = (int)s.tmp64[24 + lead];
       if (k >= todo) break;
-      const int sb = TK_WLIST(s, level - 1)[k];
+      const int sb = TK_WLIST(s, level - 1, nsb)[k];
       if (!tile_subband<TIMING, true, FORM>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && first)
-        TK_WLIST(s, level)[atomicAdd(&s.nwide[level], 1)] = sb;
+        TK_WLIST(s, level, nsb)[atomicAdd(&s.nwide[level], 1)] = sb;
     }
   }
 }
@@ -1242,7 +1258,11 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       }
     }
     __syncthreads();
-    int Nx, Ny;
+    int Nx, Ny, t16o;
+    // The value tables fit on chip (9136 values less 4 a sub-band): phase B writes them from the pieces' ranks, and
+    // they stay there.  Walking the bitmaps' bits into the scratch and copying the tables back for phase D took 4 us
+    // of a 1024-cell deck's 58 us a tile (28.10 -> 27.22 ms).
+    bool t16;
     {
       // eight words of each bitmap a thread, in registers; the last thread has the word of 65536 too
       const uint4* const x4 = reinterpret_cast<const uint4*>(s.xb) + tid * 2;
@@ -1268,13 +1288,18 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       }
       Nx = (int)(tot & 0xffffffffll);
       Ny = (int)(tot >> 32);
-      // the three allocations by three warps
-      if (tid == 0) s.Xt = (int*)sc_up(s, base, half, (unsigned long long)Nx * 4);
-      if (tid == 32) s.Yt = (int*)sc_up(s, base, half, (unsigned long long)Ny * 4);
+      t16o = TK_MD_INTS + TK_SBS + 2 * ((Nx - 1 + 62) / 63 + 2);
+      t16 = Nx + Ny <= 2 * (TK_XYV - t16o);
+      if (tid == 0) {
+        s.t16 = t16 ? Nx : 0;
+        s.t16o = t16o;
+        if (!t16) s.Xt = (int*)sc_up(s, base, half, (unsigned long long)Nx * 4);
+      }
+      if (tid == 32 && !t16) s.Yt = (int*)sc_up(s, base, half, (unsigned long long)Ny * 4);
       if (tid == 64) s.rk = pst ? srk : (int4*)sc_up(s, base, half, (unsigned long long)P * 16);
       __syncthreads();
-      if (!s.err) {
-        // value tables, one word per thread in turn (set bits are spread, so
+      if (!t16 && !s.err) {
+        // value tables in the scratch, one word per thread in turn (set bits are spread, so
         // the threads stay balanced); the rank of a word's first bit comes
         // from the per-2-word prefix
         int* xt = s.Xt;
@@ -1379,6 +1404,8 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     if (!s.err) {
       const int4* rkp = s.rk;
       int4* memp = s.mem;
+      unsigned short* const x16 = reinterpret_cast<unsigned short*>(s.xyv + t16o);
+      unsigned short* const y16 = x16 + Nx;
       for (int wb = tid & ~31; wb < P; wb += TK_LD * TK_NT) {  // warp-uniform trip count
         const int i0 = wb + gb_lane();
         int4 rr[TK_LD];
@@ -1386,6 +1413,16 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         for (int u = 0; u < TK_LD; ++u) {
           const int i = i0 + u * TK_NT;
           rr[u] = i < P ? rkp[i] : make_int4(0, -1, 0, 0);
+          if (t16 && i < P) {
+            int x1, y1, x2, y2;
+            gb_unpack(i < nA ? pa[i] : pb[i - nA], x1, y1, x2, y2);
+            x16[rr[u].x] = (unsigned short)x1;
+            x16[rr[u].y] = (unsigned short)x2;
+            if (FORM == TILE_WHOLE || max(rr[u].x / 63, q0) <= min(q1 - 1, rr[u].y / 63)) {
+              y16[rr[u].z] = (unsigned short)y1;
+              y16[rr[u].w] = (unsigned short)y2;
+            }
+          }
         }
 #pragma unroll
         for (int u = 0; u < TK_LD; ++u) {
@@ -1403,7 +1440,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     if (timing) { const long long t1 = clock64(); tB += t1 - t0; t0 = t1; }
     // ---- C: one warp per sub-band, handed out dynamically, the ones with the most members first
     // (longest processing time first: the phase ends with the last sub-band, so the large ones must
-    // not come last).  The order lives in the value-table region, unused until phase D.  One load a step, four
+    // not come last).  The order lies behind the metadata.  One load a step, four
     // in flight: 1024 cells 31.45 -> 31.27 ms.
     int* const ord = s.xyv + TK_MD_INTS;
     const bool lpt = !s.err && nsb > TK_NW && nsb <= TK_SBS;
@@ -1443,7 +1480,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         const int sb = lpt ? ord[k] : k;
         if (__any_sync(0xffffffffu, list) ||
             !tile_subband<TIMING, false, FORM>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
-          if (gb_lane() == 0) TK_WLIST(s, 0)[atomicAdd(&s.nwide[0], 1)] = sb;
+          if (gb_lane() == 0) TK_WLIST(s, 0, nsb)[atomicAdd(&s.nwide[0], 1)] = sb;
         }
       }
     }
@@ -1480,9 +1517,6 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     constexpr int DBYTES = (int)(sizeof(s.lb) + sizeof(s.lp) + sizeof(s.lv) + sizeof(s.ca) + sizeof(s.cb) +
                                  sizeof(s.mc) + sizeof(s.srow));
     const bool prs = (long long)NP * 20 <= DBYTES;
-    const int xyoff = nsb <= TK_MDS ? TK_MD_INTS : 0;  // metadata occupies the front of the region
-    const int nx4 = (Nx + 3) & ~3, ny4 = (Ny + 3) & ~3;  // tables start on 16-byte boundaries
-    const bool xys = nx4 + ny4 + xyoff <= TK_XYV;
     // chain links of a tile whose records stay in the scratch: 16 bits each on chip when they fit
     const bool sl16 = !SPLIT && !prs && NP * 2 <= DBYTES;
     if (tid == 0 && !s.err && !prs && !sl16) s.succ = (int*)sc_up(s, base, half, (unsigned long long)NP * 4 + 4);
@@ -1512,25 +1546,19 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     }
     PieceRec* PR = prs ? reinterpret_cast<PieceRec*>(s.dbuf) : nullptr;
     int* succ = prs ? reinterpret_cast<int*>(s.dbuf + (size_t)NP * 16) : s.succ;
-    const int* Xv = xys ? s.xyv + xyoff : s.Xt;
-    const int* Yv = xys ? s.xyv + xyoff + nx4 : s.Yt;
     const int wid = gb_warp(), lane = gb_lane();
-    // piece records of every sub-band and the x / y value tables into shared memory by bulk copies
+    // piece records of every sub-band into shared memory by bulk copies
     // (all 16-byte aligned: records are 16 bytes, scratch allocations are rounded to 16 bytes)
-    if ((prs && NP > 0) || xys) {
+    if (prs && NP > 0) {
       if (tid == 0) {
-        const unsigned bytes = (prs ? (unsigned)NP * 16u : 0u) + (xys ? (unsigned)(nx4 + ny4) * 4u : 0u);
+        const unsigned bytes = (unsigned)NP * 16u;
         asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(mbar),
                      "r"(bytes)
                      : "memory");
-        if (xys) {
-          if (nx4) tk_bulk(s.xyv + xyoff, s.Xt, (unsigned)nx4 * 4u, mbar);
-          if (ny4) tk_bulk(s.xyv + xyoff + nx4, s.Yt, (unsigned)ny4 * 4u, mbar);
-        }
       }
-      if (prs && !s.rsplit) {
-        if (tid == 0 && NP > 0) tk_bulk(PR, base + (half & ~15ull), (unsigned)NP * 16u, mbar);
-      } else if (prs && wid == 0) {
+      if (!s.rsplit) {
+        if (tid == 0) tk_bulk(PR, base + (half & ~15ull), (unsigned)NP * 16u, mbar);
+      } else if (wid == 0) {
         for (int sb = lane; sb < nsb; sb += 32) {
           const int4 inf = s.sbinfo[sb];
           if (inf.y > 0) tk_bulk(PR + inf.x, s.sbrec[sb], (unsigned)inf.y * 16u, mbar);
@@ -1661,6 +1689,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       __syncthreads();
     }
     const long long obase = s.obase;
+    const TileXY xy(s);
     unsigned long long* outp = obase >= 0 ? O->pcs + obase : nullptr;
     long long area = 0;
     if (prs) {
@@ -1674,13 +1703,13 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         int shi = q == p ? pr_shi(pr) : pr_shi(PR[q]);
         if (SPLIT && succ[q] <= -2) shi = split_end(pub0, scr, me, ka, nsbg, -2 - succ[q]);
         const int slo = pr_slo(pr);
-        const int xs = Xv[slo], xe = Xv[shi], ylo = Yv[pr_ylo(pr)], yhi = Yv[pr_yhi(pr)];
+        const int xs = xy.x0(slo), xe = xy.x1(shi), ylo = xy.y0(pr_ylo(pr)), yhi = xy.y1(pr_yhi(pr));
         const int pos = s.sbh[slo / 63 - q0] + pr_hrank(pr);
         if (outp) outp[pos] = gb_pack(xs, ylo, xe, yhi);
         area += (long long)(xe - xs) * (long long)(yhi - ylo);
       }
     } else {
-      area = tile_emit_scratch<SPLIT>(s, base + (half & ~15ull), NP, nsb, Xv, Yv, outp, sl16, pub0, scr, me, ka);
+      area = tile_emit_scratch<SPLIT>(s, base + (half & ~15ull), NP, nsb, outp, sl16, pub0, scr, me, ka);
     }
     {
       long long tot;
