@@ -311,7 +311,7 @@ int realloc_scratch(gb_context* ctx, size_t bytes) {
   cudaStreamSynchronize(c.stream);
   if (c.tile_scratch) cudaFree(c.tile_scratch);
   c.tile_scratch = nullptr;
-  if (cudaMalloc(&c.tile_scratch, bytes * (size_t)c.tile_blocks) != cudaSuccess) {
+  if (gb_dev_alloc(c, (void**)&c.tile_scratch, bytes * (size_t)c.tile_blocks) != cudaSuccess) {
     c.tile_scr_bytes = 0;
     return GB_ERR_OOM;
   }

@@ -249,7 +249,7 @@ static int op1_host_impl(gb_context* ctx, const c_box* boxes, unsigned long long
     if (c.io_buf) cudaFree(c.io_buf);
     c.io_buf = nullptr;
     c.io_cap = 0;
-    if (cudaMalloc(&c.io_buf, bytes) != cudaSuccess) return set_err(ctx, GB_ERR_OOM, "input staging buffer");
+    if (gb_dev_alloc(c, &c.io_buf, bytes) != cudaSuccess) return set_err(ctx, GB_ERR_OOM, "input staging buffer");
     c.io_cap = bytes;
   }
   if (!c.copy_stream && cudaStreamCreateWithFlags(&c.copy_stream, cudaStreamNonBlocking) != cudaSuccess)
@@ -352,7 +352,7 @@ extern "C" int gb_grid_autotune(gb_context* ctx, gb_layer* P, int32_t a, int* be
   if (!ctx || !P || P->dead || !best_g) return GB_ERR_ARG;
   GbCtx& c = ctx->c;
   long long* d_area = nullptr;
-  if (cudaMalloc(&d_area, (size_t)P->ncell * 8) != cudaSuccess) return set_err(ctx, GB_ERR_OOM, "grid tuning buffer");
+  if (gb_dev_alloc(c, (void**)&d_area, (size_t)P->ncell * 8) != cudaSuccess) return set_err(ctx, GB_ERR_OOM, "grid tuning buffer");
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

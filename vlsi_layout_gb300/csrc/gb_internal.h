@@ -66,6 +66,12 @@ struct HostBack {
 // of 20M trackers: 900 of 2000 us).
 #define GB_POOL_KEEP (4ull << 30)
 
+// Waits for the frees in the stream's order; the pool keeps nothing.
+inline void gb_pool_give(GbCtx& c) {
+  cudaStreamSynchronize(c.stream);
+  cudaMemPoolTrimTo(c.pool, 0);
+}
+
 // Temporary device memory of one call or layer, in the order of the context's
 // stream; freed with gb_tmp_free.  Null when there is no memory, or (as
 // cudaMalloc) while the stream is being captured.
@@ -73,11 +79,20 @@ inline void* gb_tmp_alloc(GbCtx& c, size_t bytes) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(c.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
   void* p = nullptr;
-  if (cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, c.pool, c.stream) != cudaSuccess) {
+  for (int t = 0; t < 2; ++t) {
+    if (cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, c.pool, c.stream) == cudaSuccess) return p;
     cudaGetLastError();
-    return nullptr;
+    if (t == 0) gb_pool_give(c);
   }
-  return p;
+  return nullptr;
+}
+// cudaMalloc, with what the pool keeps given back first when memory is short.
+inline cudaError_t gb_dev_alloc(GbCtx& c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  gb_pool_give(c);
+  return cudaMalloc(p, bytes);
 }
 inline void gb_tmp_free(GbCtx& c, void* p) {
   if (p) cudaFreeAsync(p, c.stream);

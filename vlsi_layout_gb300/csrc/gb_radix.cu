@@ -813,7 +813,7 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
     if (S->status) cudaFree(S->status);
     S->status = nullptr;
     S->status_words = 0;
-    if (cudaMalloc(&S->status, want * 8) != cudaSuccess) return -2;
+    if (gb_dev_alloc(c, (void**)&S->status, want * 8) != cudaSuccess) return -2;
     cudaMemsetAsync(S->status, 0, want * 8, c.stream);
     S->status_words = want;
   }
@@ -877,8 +877,8 @@ int gb_radix_tune(GbCtx& c, const unsigned long long* keys, const unsigned* vals
   if (n <= 1 || bits < 1 || bits > 64) return -1;
   unsigned long long *k = nullptr, *kt = nullptr;
   unsigned *v = nullptr, *vt = nullptr;
-  if (cudaMalloc(&k, (size_t)n * 8) != cudaSuccess || cudaMalloc(&kt, (size_t)n * 8) != cudaSuccess ||
-      cudaMalloc(&v, (size_t)n * 4) != cudaSuccess || cudaMalloc(&vt, (size_t)n * 4) != cudaSuccess) {
+  if (gb_dev_alloc(c, (void**)&k, (size_t)n * 8) != cudaSuccess || gb_dev_alloc(c, (void**)&kt, (size_t)n * 8) != cudaSuccess ||
+      gb_dev_alloc(c, (void**)&v, (size_t)n * 4) != cudaSuccess || gb_dev_alloc(c, (void**)&vt, (size_t)n * 4) != cudaSuccess) {
     cudaFree(k);
     cudaFree(kt);
     cudaFree(v);

@@ -1655,7 +1655,7 @@ extern "C" int gb_save_layer_to_snap(gb_context* ctx, const char* path, const c_
   const long long nch = nchunks_of(n);
   std::vector<long long> meta(3 * std::max(nch, 1ll));
   unsigned char* d_out = nullptr;
-  if (n > 0 && cudaMalloc(&d_out, (size_t)cap) != cudaSuccess) return gbi::set_err(ctx, GB_ERR_OOM, "snap output buffer");
+  if (n > 0 && gb_dev_alloc(ctx->c, (void**)&d_out, (size_t)cap) != cudaSuccess) return gbi::set_err(ctx, GB_ERR_OOM, "snap output buffer");
   long long total = 0;
   int e = n > 0 ? gb_compress_boxes_to_stream(ctx, d_boxes, n, method, d_out, cap, meta.data(), &total) : GB_OK;
   if (e == GB_OK && (method != 0 && method != 1)) e = gbi::set_err(ctx, GB_ERR_ARG, "compression method");
@@ -1791,7 +1791,7 @@ extern "C" int gb_restore_snap_to_layer(gb_context* ctx, const char* path, c_box
   }
   if (S.total == 0) return GB_OK;
   unsigned char* d_data = nullptr;
-  if (cudaMalloc(&d_data, std::max<size_t>(S.data.size(), 16)) != cudaSuccess)
+  if (gb_dev_alloc(ctx->c, (void**)&d_data, std::max<size_t>(S.data.size(), 16)) != cudaSuccess)
     return gbi::set_err(ctx, GB_ERR_OOM, "snap data buffer");
   cudaMemcpyAsync(d_data, S.data.data(), S.data.size(), cudaMemcpyHostToDevice, ctx->c.stream);
   e = gb_decompress_stream_to_boxes(ctx, d_data, S.meta.data(), S.nch, S.method, d_boxes);
