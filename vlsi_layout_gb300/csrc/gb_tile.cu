@@ -1365,7 +1365,10 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
               c2 = bm_rank2(s.yb, s.yp, y2);
             }
             s.rk[i] = make_int4(r1, r2, c1, c2);
-            for (int q = lo; q <= hi; ++q) atomicAdd(&s.sbc[q - q0], 1);
+            if (lo <= hi) {  // the changes of the member count along the sub-bands
+              atomicAdd(&s.sbc[lo - q0], 1);
+              atomicSub(&s.sbc[hi - q0 + 1], 1);
+            }
           }
         }
       }
@@ -1373,15 +1376,22 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     __syncthreads();
     int M = 0;
     {
+      // sub-band q starts at the sum of the counts before it, which the changes d_j give as the sum of (q - j) d_j:
+      // one scan of d_j and j d_j (the sums of j d_j in the upper half, a borrow from it for a negative lower half).
+      // Counting every sub-band of a piece: a 1024-cell deck 27.03 ms and not 26.84, phase B of two 1M-box layers 100
+      // us a tile and not 87.
       const int nsbv = s.err ? 0 : nsb;  // after an error the counters are not valid
+      long long carry = 0;
       for (int b0 = 0; b0 < nsbv; b0 += TK_NT) {
         const int q = b0 + tid;
-        int tot;
-        const int ex = tile_excl(q < nsbv ? s.sbc[q] : 0, reinterpret_cast<int*>(s.tmp64 + 8), &tot);
-        if (q < nsbv) s.sbc[q] = M + ex;
-        M += tot;
+        const long long d = q < nsbv ? s.sbc[q] : 0;
+        long long tot;
+        const long long ex = carry + tile_excl((d * q << 32) + d, s.tmp64 + 8, &tot);
+        if (q < nsbv) s.sbc[q] = q * (int)ex - (int)((ex - (int)ex) >> 32);
+        carry += tot;
         if (nsbv > TK_NT) __syncthreads();
       }
+      M = nsbv * (int)carry - (int)((carry - (int)carry) >> 32);
     }
     if (tid == 0) {
       s.mem = (int4*)sc_up(s, base, half, (unsigned long long)M * 16);
