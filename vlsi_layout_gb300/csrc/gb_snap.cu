@@ -31,8 +31,8 @@
 // a shared-memory ring for the copies and long literals copied by the CTA.
 // Decoding the codec.  Record boundaries: a record's length follows from its
 // bytes, so a chain started anywhere falls in with the true one after a few
-// records.  Every 256-byte segment guesses its first record by a chain from
-// 128 bytes before it and walks to its end; one CTA per chunk then redoes the
+// records.  Every 128-byte segment guesses its first record by a chain from
+// 96 bytes before it and walks to its end; one CTA per chunk then redoes the
 // segments whose guess is not where the segment before them ended, until all
 // agree, and the record counts give every segment its first record's number.
 // Boxes: blocks of 1024 records sum their anchor deltas and dictionary
@@ -518,8 +518,8 @@ __global__ void k_enc_sizes(const int* __restrict__ bsize, long long nchunks, lo
 // ---------------------------------------------------------------- codec decoder
 // Record boundaries by guessed segments (see the top).  The walk of a chunk
 // is a serial chain of 65536 lengths (one CTA per chunk with one walking
-// thread: 1774 us for 184 chunks); segments make it 2100 chains of about 30
-// records per chunk, and the guesses cost 14 more each.  A block stages 128
+// thread: 1774 us for 184 chunks); segments make it some 4000 chains of about
+// 15 records per chunk, and the guesses cost 10 more each.  A block stages 256
 // segments (32 KB) with the continuation bits of their bytes, so a length is
 // one byte and three words from shared memory and then register work.
 #define SN_SEG 128
@@ -615,7 +615,6 @@ __device__ __forceinline__ int seg_len(const SegStage& s, int b) {
 
 // Grid (blocks of the largest chunk, chunks); blk[c] is the number of blocks
 // of the chunks before c, so segment arrays are indexed by blk[c] + blockIdx.x.
-
 __global__ void __launch_bounds__(SN_SEGT)
 k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
             const long long* __restrict__ raw_len, const long long* __restrict__ blk, unsigned* __restrict__ entry, unsigned* __restrict__ exit_, unsigned* __restrict__ cnt) {
