@@ -21,7 +21,7 @@
 // Snappy: each 65536-byte fragment of a chunk's codec bytes is compressed by
 // one CTA with the fragment in shared memory.  A position's candidate is the
 // latest earlier position with the same 11-bit hash of its 4 bytes; 32 warps
-// find the candidates of 8192 positions (each warp's last positions per hash,
+// find the candidates of 12288 positions (each warp's last positions per hash,
 // a scan of these over the warps, then every warp through its positions), and
 // mark those whose first 8 bytes match.  One warp takes the greedy parse from
 // mark to mark, extends a match 32 bytes per step and emits Snappy literal /
@@ -979,7 +979,7 @@ __device__ __forceinline__ int sn_copy_piece(unsigned char* o, unsigned off, int
 // elements go to fout + f * SN_FCAP, their count to flout.
 #define SN_CT 1024
 #define SN_CW (SN_CT / 32)
-#define SN_SUB 8192  // positions whose candidates are held at once
+#define SN_SUB 12288  // positions whose candidates are held at once
 struct SnapFrag {
   __align__(16) unsigned char buf[SN_FRAG + 32];  // the fragment at buf[sh], sh = its address modulo 16
   __align__(16) unsigned short tab[SN_CW][2048];  // latest position + 1 per hash (positions with 4 bytes left are < 65533)
@@ -1016,6 +1016,10 @@ k_snappy_compress(const unsigned char* __restrict__ raw, const long long* __rest
     }
     *reinterpret_cast<uint4*>(s.buf + i) = v;
   }
+  // Cleared once: what the tables hold of earlier positions is never above `last`, from which the running maximum
+  // starts, nor at a later position, so it changes nothing.  (Cleared for every 8192 positions, the positions whose
+  // candidates were held at once: 12M boxes encoded in 1320 us, now 1284.)
+  for (int i = t; i < SN_CW * 2048 * 2 / 16; i += SN_CT) reinterpret_cast<uint4*>(s.tab)[i] = make_uint4(0, 0, 0, 0);
   for (int i = t; i < 2048; i += SN_CT) s.last[i] = 0;
   if (t == 0) s.fail = 0;
   __syncthreads();
@@ -1030,7 +1034,6 @@ k_snappy_compress(const unsigned char* __restrict__ raw, const long long* __rest
   for (int h0 = 0; h0 + 4 <= fl; h0 += SN_SUB) {
     const int q0 = h0 + wid * (SN_SUB / SN_CW);
     const int q1 = min(q0 + SN_SUB / SN_CW, fl - 3);  // positions with 4 bytes left
-    for (int i = lane; i < 1024; i += 32) reinterpret_cast<unsigned*>(tab)[i] = 0;
     for (int i = t; i < SN_SUB / 32; i += SN_CT) s.mark[i] = 0;
     __syncwarp();
     for (int b = q0; b < q1; b += 32) {  // the warp's latest position per hash
