@@ -1036,10 +1036,15 @@ k_snappy_compress(const unsigned char* __restrict__ raw, const long long* __rest
     const int q1 = min(q0 + SN_SUB / SN_CW, fl - 3);  // positions with 4 bytes left
     for (int i = t; i < SN_SUB / 32; i += SN_CT) s.mark[i] = 0;
     __syncwarp();
-    for (int b = q0; b < q1; b += 32) {  // the warp's latest position per hash
+    unsigned val[SN_SUB / SN_CT];  // the 4 bytes from each of the lane's positions, for both searches (1277 -> 1239 us)
+#pragma unroll
+    for (int i = 0; i < SN_SUB / SN_CT; ++i) {  // the warp's latest position per hash
+      const int b = q0 + i * 32;
+      if (b >= q1) break;
       const int q = b + lane;
       const bool has = q < q1;
-      const unsigned h = has ? (ld32(q) * 0x9E3779B1u) >> 21 : 0u;
+      val[i] = ld32(min(q, fl - 4));
+      const unsigned h = (val[i] * 0x9E3779B1u) >> 21;
       bool again = has;
       while (__any_sync(0xffffffffu, again)) {  // lanes of one hash: the highest position stays
         if (again) tab[h] = (unsigned short)(q + 1);
@@ -1062,10 +1067,13 @@ k_snappy_compress(const unsigned char* __restrict__ raw, const long long* __rest
       reinterpret_cast<unsigned*>(s.last)[t] = run;
     }
     __syncthreads();
-    for (int b = q0; b < q1; b += 32) {
+#pragma unroll
+    for (int i = 0; i < SN_SUB / SN_CT; ++i) {
+      const int b = q0 + i * 32;
+      if (b >= q1) break;
       const int q = b + lane;
       const bool has = q < q1;
-      const unsigned v = ld32(min(q, fl - 4));
+      const unsigned v = val[i];
       const unsigned h = (v * 0x9E3779B1u) >> 21;
       unsigned cand = has ? tab[h] : 0u;  // 1-based
       __syncwarp();
