@@ -1,7 +1,7 @@
 """The branches of the binning and scanline kernels at the sizes where they
 change over: shared or global tile counters, boxes over many tiles, sub-bands
 of a tile with more columns or y ranks than a warp's buffer holds at each
-level.  Everything bit for bit against the oracle."""
+level, value tables on chip or in the scratch.  Everything bit for bit against the oracle."""
 import numpy as np
 import pytest
 
@@ -77,6 +77,25 @@ def test_many_y_ranks(ctx, oracle, n):
     B = random_layer(500, die=65_000, wmin=20, wmax=3000, seed=n)
     for op in (0, 3):
         assert np.array_equal(run(ctx, lambda: ctx.op(op, ctx.layer(A), ctx.layer(B))), oracle.boolean(A, B, op)), op
+
+
+# distinct x and y values of a tile around what its 16-bit tables hold on chip (4474 of each), and with more
+# sub-bands than on-chip counters (256); the first value is the tile's start, the last its end
+@pytest.mark.parametrize("n", [4473, 4474, 4475, 4476, 16130, 16131, 18000])
+def test_value_tables(ctx, oracle, n):
+    rng = np.random.default_rng(n)
+    v = [np.sort(np.concatenate([[0, 65536], rng.permutation(np.arange(1, 65536))[:n - 2]])) for _ in range(2)]
+    i = np.unique(np.append(np.arange(0, n - 1, 2), n - 2))
+    j = rng.permutation(i)
+    A = np.stack([v[0][i], v[1][j], v[0][i + 1], v[1][j + 1]], 1).astype(np.int32)
+    p, q = np.sort(rng.choice(n, (30, 2)), 1), np.sort(rng.choice(n, (30, 2)), 1)
+    k = (p[:, 0] < p[:, 1]) & (q[:, 0] < q[:, 1])
+    B = np.stack([v[0][p[k, 0]], v[1][q[k, 0]], v[0][p[k, 1]], v[1][q[k, 1]]], 1).astype(np.int32)
+    for op in (0, 3):
+        assert np.array_equal(run(ctx, lambda: ctx.op(op, ctx.layer(A), ctx.layer(B))), oracle.boolean(A, B, op)), op
+    m = ctx.mark()
+    assert int(ctx.area(ctx.layer(A))[0]) == oracle.union_area(A)
+    ctx.release(m)
 
 
 def _snap_cases():
