@@ -128,7 +128,6 @@ __device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin,
 #pragma unroll
     for (int u = 0; u < UF_LB; ++u) {
       const int j = u * 32 + lane;
-      // an inverted box meets nothing
       bb[u] = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
       if (j < k) {
         const int i = ti[j];
@@ -154,6 +153,9 @@ __device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin,
           if (u * 32 < k && closed_overlap(ba, bb[u])) m[u] |= 1u << i;
       }
       m[w] &= (1u << lane) - 1u;  // earlier boxes only
+#pragma unroll
+      for (int u = w; u < UF_LB; ++u)
+        if (u * 32 + lane >= k) m[u] = 0;  // no box: the inverted one held there meets a box that spans all of int32
       unsigned all = 0;
 #pragma unroll
       for (int u = w; u < UF_LB; ++u) {
@@ -257,7 +259,8 @@ __device__ __forceinline__ void cta_tiles(const DLayer* raw, const DLayer* bin, 
       for (int u = 0; u < LB; ++u) {
         if (u * NT + NT - 1 <= a || u * NT >= k) continue;  // uniform
         const int j = u * NT + threadIdx.x;
-        if (j > a && closed_overlap(ba, bb[u])) pair(a, j, s.idx[a], ba, s.idx[j], bb[u]);
+        // a < j < k, in one comparison
+        if ((unsigned)(j - a - 1) < (unsigned)(k - a - 1) && closed_overlap(ba, bb[u])) pair(a, j, s.idx[a], ba, s.idx[j], bb[u]);
       }
     }
     __syncthreads();
