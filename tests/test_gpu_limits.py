@@ -21,3 +21,30 @@ def test_boxes_spanning_int32(ctx, oracle, n):
         assert nc == en and np.array_equal(lab, elab)
         got, exp = ctx.interactions(b), oracle.interactions(b)
         assert got[:2] == exp[:2] and np.array_equal(got[2], exp[2])
+
+
+def _indexed_stream(at, index, height, n=65536):
+    """A valid chunk and one of n records: a new width and height, then records that change nothing, but record `at`,
+    which sets the width (height) to the dictionary's entry `index`."""
+    raw = bytearray([3 | 12, 10, 20]) + bytes(n - 1)
+    rec = bytes([4 if height else 1]) + (index & 0xFFFF).to_bytes(2, "little")
+    bad = bytes(raw[:at + 2]) + rec + bytes(raw[at + 3:])
+    return [(65536, 65538, 65538, bytes(raw[:65538])), (n, len(bad), len(bad), bad)]
+
+
+# records of the first, a middle and the last block of 1024; entries that do not exist, the only one that does
+@pytest.mark.parametrize("at", [1, 1023, 40_000, 65_535])
+@pytest.mark.parametrize("height", [False, True])
+def test_stream_dictionary_index(ctx, oracle, at, height):
+    from vlsi_layout_gb300 import engine
+    ok = _indexed_stream(at, 1, height)
+    b = ctx.decompress_stream_to_boxes(ok, 0)
+    assert np.array_equal(b, np.tile(np.array([[0, 0, 10, 20]], np.int32), (131_072, 1)))
+    for index in (0, 2, 30_000, 32_767, -1, -32_768):
+        bad = _indexed_stream(at, index, height)
+        with pytest.raises(ValueError):
+            oracle.codec_decode_chunk(bad[1][3], 65536)
+        with pytest.raises(engine.GBError) as e:
+            ctx.decompress_stream_to_boxes(bad, 0)
+        assert e.value.code == engine.GB_ERR_CORRUPT, index
+    assert np.array_equal(ctx.decompress_stream_to_boxes(ok, 0), b)

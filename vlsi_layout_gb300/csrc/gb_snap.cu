@@ -837,9 +837,12 @@ k_codec_decode(const unsigned char* __restrict__ raw, const long long* __restric
       pnw[j] = nw + e[2].a - q.nw;
       pnh[j] = nh + e[3].a - q.nh;
       const unsigned mw = __ballot_sync(0xffffffffu, q.lw != 0), mh = __ballot_sync(0xffffffffu, q.lh != 0);
-      // the last block that sets a width (height), its own entries counted from the blocks before it
-      const int aw = q.lw & SN_REL ? (int)pnw[j] + (q.lw & ~SN_REL) : (short)(q.lw & 0xffff);
-      const int ah = q.lh & SN_REL ? (int)pnh[j] + (q.lh & ~SN_REL) : (short)(q.lh & 0xffff);
+      // the last block that sets a width (height), its own entries counted from the blocks before it; an index
+      // outside the entries up to that block sets none (the block reports its record)
+      int aw = q.lw & SN_REL ? (int)pnw[j] + (q.lw & ~SN_REL) : (short)(q.lw & 0xffff);
+      int ah = q.lh & SN_REL ? (int)pnh[j] + (q.lh & ~SN_REL) : (short)(q.lh & 0xffff);
+      if (aw < 1 || aw > (int)(pnw[j] + q.nw)) aw = 0;
+      if (ah < 1 || ah > (int)(pnh[j] + q.nh)) ah = 0;
       const int sw = __shfl_sync(0xffffffffu, aw, mw ? 31 - __clz(mw) : 0);
       const int sh = __shfl_sync(0xffffffffu, ah, mh ? 31 - __clz(mh) : 0);
       if (mw) lw = sw;
