@@ -48,3 +48,30 @@ def test_stream_dictionary_index(ctx, oracle, at, height):
             ctx.decompress_stream_to_boxes(bad, 0)
         assert e.value.code == engine.GB_ERR_CORRUPT, index
     assert np.array_equal(ctx.decompress_stream_to_boxes(ok, 0), b)
+
+
+@pytest.mark.parametrize("nbad", [1, 40, 3000])
+def test_invalid_boxes_on_upload(oracle, nbad):
+    """Invalid boxes that many blocks meet at once are an error, of the layer's every use, and the context goes on."""
+    from vlsi_layout_gb300 import engine
+    A = random_layer(300_000, die=1_500_000, seed=nbad)
+    bad = A.copy()
+    at = np.random.default_rng(nbad).choice(len(A), nbad, replace=False)
+    bad[at, 2] = bad[at, 0]
+    off = np.linspace(0, len(A), 701).astype(np.int64)
+    exp = oracle.union_area(A)
+    with engine.Context(0, 2 << 30) as ctx:
+        good = ctx.layer(A)
+        for cells in (None, off):
+            for _ in range(10):
+                m = ctx.mark()
+                L = ctx.layer(bad, cells)
+                with pytest.raises(engine.GBError) as e:
+                    ctx.sync()
+                assert e.value.code == engine.GB_ERR_INVALID_BOX
+                with pytest.raises(engine.GBError) as e:
+                    ctx.area(L)
+                assert e.value.code == engine.GB_ERR_INVALID_BOX
+                L.free()
+                ctx.release(m)
+            assert int(ctx.area(good)[0]) == exp

@@ -294,7 +294,11 @@ __global__ void __launch_bounds__(256) k_bbox_raw(const DLayer* S, DLayer* O, in
                                                   DStatus* st) {
   __shared__ int4 wb[8];
   __shared__ int wk[8];
-  if (st->err) return;
+  __shared__ bool failed;
+  // other blocks report errors meanwhile: one read for the whole block, whose warps' bounds meet at the end
+  if (threadIdx.x == 0) failed = *(volatile int*)&st->err != 0;
+  __syncthreads();
+  if (failed) return;
   if (S == O && blockIdx.x == 0 && threadIdx.x == 0) O->has_cbox = 1;  // a raw layer's own boxes
   int4* const cb = O->cbox;
   int kc = -1;  // the cell whose bounds the warp holds
