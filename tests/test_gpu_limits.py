@@ -1,6 +1,8 @@
 """Calls at the ends of what the entry points accept, bit for bit against the
 oracle: boxes that span all of int32, malformed streams of several blocks,
 invalid boxes, layers used by another context or made after an error."""
+import time
+
 import numpy as np
 import pytest
 
@@ -75,3 +77,37 @@ def test_invalid_boxes_on_upload(oracle, nbad):
                 L.free()
                 ctx.release(m)
             assert int(ctx.area(good)[0]) == exp
+
+
+def _best(fn, k=4):
+    """Shortest of k times, after a first run."""
+    fn()
+    ts = []
+    for _ in range(k):
+        t = time.perf_counter()
+        fn()
+        ts.append(time.perf_counter() - t)
+    return min(ts)
+
+
+def test_layer_made_after_an_error(ctx, oracle):
+    """A layer uploaded before an error is cleared is as good as another, and as fast."""
+    from vlsi_layout_gb300 import engine
+    A = random_layer(400_000, die=1_700_000, seed=8)
+    m = ctx.mark()
+    before = ctx.layer(A)
+    broken = ctx.layer(np.array([[5, 5, 1, 1]], np.int32))
+    after = ctx.layer(A)
+    with pytest.raises(engine.GBError):
+        ctx.sync()
+    exp = oracle.union_area(A)
+
+    def area(L):
+        k = ctx.mark()
+        assert int(ctx.area(L)[0]) == exp
+        ctx.release(k)
+
+    assert _best(lambda: area(after)) < 20 * _best(lambda: area(before))
+    for L in (before, broken, after):
+        L.free()
+    ctx.release(m)

@@ -295,11 +295,11 @@ __global__ void __launch_bounds__(256) k_bbox_raw(const DLayer* S, DLayer* O, in
   __shared__ int4 wb[8];
   __shared__ int wk[8];
   __shared__ bool failed;
-  // other blocks report errors meanwhile: one read for the whole block, whose warps' bounds meet at the end
-  if (threadIdx.x == 0) failed = *(volatile int*)&st->err != 0;
+  // other blocks report errors meanwhile: one read for the whole block, whose warps' bounds meet at the end.  A raw
+  // layer's own boxes (S == O) are taken whatever the status: the layer may be used after the error is cleared
+  if (threadIdx.x == 0) failed = S != O && *(volatile int*)&st->err != 0;
   __syncthreads();
   if (failed) return;
-  if (S == O && blockIdx.x == 0 && threadIdx.x == 0) O->has_cbox = 1;  // a raw layer's own boxes
   int4* const cb = O->cbox;
   int kc = -1;  // the cell whose bounds the warp holds
   int4 acc = bbox_none();
@@ -473,21 +473,12 @@ __global__ void __launch_bounds__(1024) k_bin_setup(const DLayer* S, DLayer* O, 
     }
   }
   __syncthreads();
-  if (!ok) return;
-  const bool have = S->has_cbox != 0;
+  const bool go = ok;
+  __syncthreads();  // read by all before a thread clears it below
+  if (!go) return;
   for (int k = threadIdx.x; k < ncell; k += blockDim.x) {
-    int4 b = have ? S->cbox[k] : bbox_none(), o = bbox_none();
-    if (!have) {  // the layer was made while the context had failed: its boxes one by one
-      for (long long i = S->coff[k]; i < S->coff[k + 1]; ++i) {
-        const int4 q = S->boxes[i];
-        if (!(q.x < q.z && q.y < q.w)) {
-          gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, i);
-          ok = false;
-          break;
-        }
-        b = make_int4(min(b.x, q.x), min(b.y, q.y), max(b.z, q.z), max(b.w, q.w));
-      }
-    }
+    const int4 b = S->cbox[k];
+    int4 o = bbox_none();
     if (b.x <= b.z && !grow_box(b, E, N, W, Sg, o)) {  // past int32: so is a box at that bound
       gb_set_error(st, GB_ERR_INVALID_BOX, KID_BBOX, S->coff[k]);
       ok = false;
@@ -790,7 +781,6 @@ __global__ void __launch_bounds__(1024) k_frame(const DLayer* P, DLayer* F, int 
       F->boxes = (int4*)gb_arena_alloc(st, (unsigned long long)ncell * 16, KID_FRAME);
       F->coff = (long long*)gb_arena_alloc(st, (unsigned long long)(ncell + 1) * 8, KID_FRAME);
       F->nbox = ncell;
-      F->has_cbox = 1;
       ok = F->boxes && F->coff;
       if (ok) F->coff[ncell] = ncell;
     }

@@ -63,7 +63,7 @@ struct DLayer {
   int ncell;
   int g;            // grid log2 (binned form)
   int binned;       // 1 = binned, 0 = raw
-  int has_cbox;     // raw: cbox holds the cells' bounding boxes
+  int pad0;
   long long* cell_count;   // [ncell] boxes (raw) or strips (binned result)
   long long* cell_area;    // [ncell] union area when computed
   // raw form
