@@ -111,3 +111,19 @@ def test_layer_made_after_an_error(ctx, oracle):
     for L in (before, broken, after):
         L.free()
     ctx.release(m)
+
+
+def test_layer_used_by_another_context(ctx, oracle):
+    """A layer is complete when the call that makes it returns: another context's stream may use it at once."""
+    from vlsi_layout_gb300 import engine
+    A = random_layer(1_500_000, die=3_000_000, seed=6)
+    A = A[np.argsort(A[:, 0], kind="stable")]  # the last boxes widen the bounds
+    exp = oracle.union_area(A)
+    with engine.Context(0, 4 << 30) as other:
+        for _ in range(4):
+            m, k = ctx.mark(), other.mark()
+            L = ctx.layer(A)
+            assert int(other.area(L)[0]) == exp
+            L.free()
+            ctx.release(m)
+            other.release(k)

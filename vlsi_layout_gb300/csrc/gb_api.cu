@@ -543,8 +543,12 @@ extern "C" int gb_set_tile_scratch(gb_context* ctx, unsigned long long bytes) {
 
 // ======================================================================= layers
 // borrow: boxes is a device pointer used in place (coff then a host pointer).
+// internal: the layer is made and freed within one call, on the context's
+// stream alone; any other is complete on return, since other contexts' streams
+// may use it (they take their tile windows from its bounding boxes).
 static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long long n,
-                          const long long* coff, int ncell, bool device_src, gb_layer** out, bool borrow = false) {
+                          const long long* coff, int ncell, bool device_src, gb_layer** out, bool internal = false,
+                          bool borrow = false) {
   if (!ctx || !out || ncell < 1) return GB_ERR_ARG;
   *out = nullptr;
   GbCtx& c = ctx->c;
@@ -555,6 +559,7 @@ static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long lon
   L->d = c.desc + s;
   L->ncell = ncell;
   L->binned = 0;
+  L->internal = internal;
   L->nbox_host = (long long)n;
   // one allocation: boxes (unless borrowed), cell offsets, per-cell arrays
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -586,8 +591,9 @@ static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long lon
   gb_launch_raw_desc(c, L->d, d, coff == nullptr);
   if (n && !borrow) cudaMemcpyAsync(pb, boxes, n * 16, kind, c.stream);
   if (coff) cudaMemcpyAsync(d.coff, coff, (size_t)(ncell + 1) * 8, borrow ? cudaMemcpyHostToDevice : kind, c.stream);
+  if (!internal) gb_launch_cell_bbox_fill(c, L->d, ncell);
   cudaStreamSynchronize(c.stream);  // the caller's arrays are its own again
-  gb_launch_cell_bbox_fill(c, L->d, ncell);
+  if (internal) gb_launch_cell_bbox_fill(c, L->d, ncell);
   *out = L;
   return GB_OK;
 }
@@ -595,7 +601,7 @@ static int make_raw_layer(gb_context* ctx, const c_box* boxes, unsigned long lon
 namespace gbi {
 int layer_over_device(gb_context* ctx, const void* d_boxes, long long n, const long long* h_offsets, int ncell,
                       gb_layer** out) {
-  return make_raw_layer(ctx, (const c_box*)d_boxes, (unsigned long long)n, h_offsets, ncell, true, out, true);
+  return make_raw_layer(ctx, (const c_box*)d_boxes, (unsigned long long)n, h_offsets, ncell, true, out, true, true);
 }
 }  // namespace gbi
 
@@ -883,9 +889,8 @@ extern "C" int gb_components(gb_context* ctx, const c_box* boxes, unsigned long 
   if (n > 0x7fffffffull) return set_err(ctx, GB_ERR_ARG, "too many boxes for int32 indices");
   GbCtx& c = ctx->c;
   gb_layer* L = nullptr;
-  int e = gb_layer_from_host(ctx, boxes, n, nullptr, 1, &L);
+  int e = make_raw_layer(ctx, boxes, n, nullptr, 1, false, &L, true);
   if (e) return e;
-  L->internal = true;
   int g = 0;
   e = pair_grid(ctx, L, (long long)n, &g);
   if (e) { gb_layer_free(ctx, L); return e; }
@@ -927,9 +932,8 @@ extern "C" int gb_interactions(gb_context* ctx, const c_box* boxes, unsigned lon
   }
   GbCtx& c = ctx->c;
   gb_layer* L = nullptr;
-  int e = gb_layer_from_host(ctx, boxes, n, nullptr, 1, &L);
+  int e = make_raw_layer(ctx, boxes, n, nullptr, 1, false, &L, true);
   if (e) return e;
-  L->internal = true;
   int g = 0;
   e = pair_grid(ctx, L, (long long)n, &g);
   if (e) { gb_layer_free(ctx, L); return e; }
@@ -1006,9 +1010,8 @@ extern "C" int gb_component_areas(gb_context* ctx, const c_box* boxes, unsigned 
   }
   GbCtx& c = ctx->c;
   gb_layer* L = nullptr;
-  int e = gb_layer_from_host(ctx, boxes, n, nullptr, 1, &L);
+  int e = make_raw_layer(ctx, boxes, n, nullptr, 1, false, &L, true);
   if (e) return e;
-  L->internal = true;
   int g = 0;
   e = pair_grid(ctx, L, (long long)n, &g);
   if (e) { gb_layer_free(ctx, L); return e; }
@@ -1232,13 +1235,12 @@ static int host_bool(gb_context* ctx, int control, long value, const c_box* A, u
                      const c_box* B, unsigned long BN, std::vector<c_box>& res) {
   gb_layer* LA = nullptr;
   gb_layer* LB = nullptr;
-  int e = gb_layer_from_host(ctx, A, AN, nullptr, 1, &LA);
-  if (!e) e = gb_layer_from_host(ctx, B, BN, nullptr, 1, &LB);
+  int e = make_raw_layer(ctx, A, AN, nullptr, 1, false, &LA, true);
+  if (!e) e = make_raw_layer(ctx, B, BN, nullptr, 1, false, &LB, true);
   if (e) {
     if (LA) gb_layer_free(ctx, LA);
     return e;
   }
-  LA->internal = LB->internal = true;
   e = run_retry(ctx, [&]() -> int {
     gb_layer* O = nullptr;
     int r;

@@ -293,7 +293,6 @@ static int op1_host_impl(gb_context* ctx, const c_box* boxes, unsigned long long
     gb_layer* P = nullptr;
     e = gbi::layer_over_device(ctx, dbox + b0 * 16, off[k1] - b0, goff.data(), k1 - k0, &P);
     if (e) break;
-    P->internal = true;
     const int gn = k1 - k0;
     e = gb_run_retry(ctx, [&]() -> int {
       gb_layer* outs[6];
