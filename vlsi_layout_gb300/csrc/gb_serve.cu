@@ -101,17 +101,25 @@ extern "C" int gb_serve_create(int device, unsigned long long budget_bytes, int 
     gb_server_slot sl;
     e = gb_context_create(device, slot_arena_bytes, &sl.ctx);
     if (!e) e = gb_set_tile_scratch(sl.ctx, 4ull << 20);
-    if (e) break;
+    if (!e && cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) != cudaSuccess) e = GB_ERR_OOM;
+    // written by kernels: without it no request may run
+    if (!e && cudaMallocHost(&sl.back, sizeof(gb_served)) != cudaSuccess) e = GB_ERR_OOM;
+    if (e) {
+      S->slots.push_back(sl);  // what it has is freed with the others
+      break;
+    }
     // Requests of other slots run beside this one's: CTAs that share a tile repeat its ranking, which pays for idle
     // SMs only, so a request counts on half of them (40 requests on 60000 boxes: the whole chip 1555 us, half 1457,
     // no shared tiles 1478; on 2000 boxes 1123, 1123 and 1252 us).
     if (slots > 1) sl.ctx->c.split_ctas = sl.ctx->c.split_ctas / 16 * 8;
-    cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
-    cudaMallocHost(&sl.back, sizeof(gb_served));
     sl.mark = gb_arena_mark(sl.ctx);
     S->slots.push_back(sl);
   }
-  if (e) { gb_serve_destroy(S); return e; }
+  if (e) {
+    cudaGetLastError();
+    gb_serve_destroy(S);
+    return e;
+  }
   *out = S;
   return GB_OK;
 }
