@@ -613,15 +613,16 @@ __device__ __forceinline__ int seg_len(const SegStage& s, int b) {
   return sn_len(s.buf[b], cont);
 }
 
-// Grid (blocks of the largest chunk, chunks); blk[c] is the number of blocks
-// of the chunks before c, so segment arrays are indexed by blk[c] + blockIdx.x.
+// Grid (chunks, blocks of the largest chunk): chunks can be more than a grid's y
+// holds (65535).  blk[c] is the number of blocks of the chunks before c, so
+// segment arrays are indexed by blk[c] + blockIdx.y.
 __global__ void __launch_bounds__(SN_SEGT)
 k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
             const long long* __restrict__ raw_len, const long long* __restrict__ blk, unsigned* __restrict__ entry, unsigned* __restrict__ exit_, unsigned* __restrict__ cnt) {
   __shared__ SegStage s;
-  const int c = blockIdx.y;
-  const long long L = raw_len[c], blk0 = blk[c], start = (long long)blockIdx.x * SN_SEGB;
-  if (blk0 + blockIdx.x >= blk[c + 1]) return;
+  const int c = blockIdx.x;
+  const long long L = raw_len[c], blk0 = blk[c], start = (long long)blockIdx.y * SN_SEGB;
+  if (blk0 + blockIdx.y >= blk[c + 1]) return;
   const long long p0 = seg_stage(s, raw + raw_off[c], L, start - SN_WARM);
   const int s0 = (int)(start - p0) + (int)threadIdx.x * SN_SEG, s1 = s0 + SN_SEG;
   const int lim = (int)min((long long)s1, L - p0);
@@ -630,7 +631,7 @@ k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__
     b = s0 - SN_WARM;
     while (b < s0) b += max(1, seg_len(s, b));
   }
-  const size_t g = (size_t)(blk0 + blockIdx.x) * SN_SEGT + threadIdx.x;
+  const size_t g = (size_t)(blk0 + blockIdx.y) * SN_SEGT + threadIdx.x;
   entry[g] = (unsigned)(p0 + b);
   unsigned n = 0;
   bool bad = false;
@@ -715,11 +716,11 @@ k_seg_records(const unsigned char* __restrict__ raw, const long long* __restrict
   __shared__ SegStage s;
   __shared__ unsigned mark[SN_SEGB / 32];
   __shared__ SumS buf[32];
-  const int c = blockIdx.y;
+  const int c = blockIdx.x;
   const int nb = (int)min((long long)SN_CHUNK, n - (long long)c * SN_CHUNK);
-  const long long L = raw_len[c], blk0 = blk[c], start = (long long)blockIdx.x * SN_SEGB;
-  if (blk0 + blockIdx.x >= blk[c + 1]) return;
-  const size_t g0 = (size_t)(blk0 + blockIdx.x) * SN_SEGT, g = g0 + threadIdx.x;
+  const long long L = raw_len[c], blk0 = blk[c], start = (long long)blockIdx.y * SN_SEGB;
+  if (blk0 + blockIdx.y >= blk[c + 1]) return;
+  const size_t g0 = (size_t)(blk0 + blockIdx.y) * SN_SEGT, g = g0 + threadIdx.x;
   if (first[g0] >= (unsigned)nb) return;  // uniform: the chunk's records end before this block
   for (int i = threadIdx.x; i < SN_SEGB / 32; i += SN_SEGT) mark[i] = 0;
   const long long p0 = seg_stage(s, raw + raw_off[c], L, start - SN_WARM);
@@ -1612,7 +1613,7 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
   }
   long long most = 0;  // blocks of the largest chunk
   for (long long i = 0; i < nch; ++i) most = std::max(most, sblk[i + 1] - sblk[i]);
-  const dim3 sgrid((unsigned)most, (unsigned)nch);
+  const dim3 sgrid((unsigned)nch, (unsigned)most);
   if (most) {
     k_seg_guess<<<sgrid, SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, d_seg, d_seg + nseg, d_seg + 2 * nseg);
     ++c.launches;
