@@ -127,3 +127,46 @@ def test_layer_used_by_another_context(ctx, oracle):
             L.free()
             ctx.release(m)
             other.release(k)
+
+
+def _rows(n, pitch, row, side=100):
+    """Squares in rows, in the order they are drawn: records of one length."""
+    i = np.arange(n, dtype=np.int64)
+    x, y = i % row * pitch, i // row * pitch
+    return np.stack([x, y, x + side, y + side], 1).astype(np.int32)
+
+
+# pitches whose records also parse out of step, over the whole chunk or from row to row; a chain that ends in the middle
+# of a chunk, at its last record and behind it
+@pytest.mark.parametrize("pitch,row", [(240, 256), (240, 70_001), (500, 90), (1008, 1000), (16, 4096), (400, 256)])
+@pytest.mark.parametrize("method", [0, 1])
+def test_stream_out_of_step(ctx, oracle, pitch, row, method):
+    from vlsi_layout_gb300 import engine
+    b = _rows(70_001, pitch, row)
+    chunks = oracle.stream_encode(b, method)
+    assert np.array_equal(ctx.decompress_stream_to_boxes(chunks, method), b)
+    if method == 0:
+        raw, n = chunks[0][3], 65536
+        for cut in (len(raw) - 1, len(raw) // 2, 200):  # the stream, or its last records, end early
+            for tail in (b"", b"\x20" + b"\xff" * 11, b"\x60" * 50):
+                data = raw[:cut] + tail
+                try:
+                    exp = oracle.codec_decode_chunk(data, n)
+                except ValueError:
+                    with pytest.raises(engine.GBError) as e:
+                        ctx.decompress_stream_to_boxes([(n, len(data), len(data), data)], 0)
+                    assert e.value.code == engine.GB_ERR_CORRUPT, (cut, tail)
+                else:
+                    assert np.array_equal(ctx.decompress_stream_to_boxes([(n, len(data), len(data), data)], 0), exp)
+        data = raw + b"\x20" + b"\xff" * 11  # nothing behind the last record is read
+        assert np.array_equal(ctx.decompress_stream_to_boxes([(n, len(data), len(data), data)], 0), b[:n])
+
+
+def test_stream_out_of_step_time(ctx):
+    """Rows whose records also parse out of step decode in the time of others (they took some 3000 times that)."""
+    def seconds(pitch):
+        b = _rows(1_000_000, pitch, 1000)
+        chunks = ctx.compress_boxes_to_stream(b, 0)
+        return _best(lambda: ctx.decompress_stream_to_boxes(chunks, 0, as_tensor=True))
+
+    assert seconds(240) < 5 * seconds(340)

@@ -648,16 +648,96 @@ k_seg_guess(const unsigned char* __restrict__ raw, const long long* __restrict__
   cnt[g] = n;
 }
 
+// The segments from k0 on by table, for chains that do not fall in with the
+// true one by themselves: records of one length whose bytes also parse out of
+// step, as rows of equal boxes at some pitches are (20 e0 03 20 e0 03 ...).
+// Each of SN_TABT threads goes backwards through its segment and leaves, for
+// every byte, the records of a chain from there and where it ends; one thread
+// then follows the chain from segment to segment.  (4M squares in rows at a
+// pitch of 240 decode in 1.2 ms; with rounds of walks alone, each right for one
+// more segment of a chunk, in 704 ms; with one serial walk a chunk in 1.6 ms.)
+#define SN_ROUNDS 2   // rounds of walks before the table: layouts in Morton order need none or one
+#define SN_TABT 256   // segments of a step of the table
+#define SN_TABW 130   // a segment's entries, one word more than its bytes for the banks
+#define SN_TEND 255   // the chain meets a malformed record
+#define SN_TAB_SMEM (SN_TABT * SN_TABW * 2 + (SN_TABT + 1) * 4)
+static_assert(SN_SEG + SN_LMAX < SN_TEND, "an entry's end is a byte");
+
+// 4 bytes from chunk position p (on a word of memory), zeros outside [0, L)
+__device__ __forceinline__ unsigned seg_word(const unsigned char* base, long long L, long long p) {
+  if (p >= 0 && p + 4 <= L) return *reinterpret_cast<const unsigned*>(base + p);
+  unsigned w = 0;
+  for (int j = 0; j < 4; ++j)
+    if (p + j >= 0 && p + j < L) w |= (unsigned)base[p + j] << (8 * j);
+  return w;
+}
+
+__device__ __noinline__ void seg_table(const unsigned char* base, long long L, int k0, int nseg, unsigned* entry,
+                                       const unsigned* exit_, unsigned* cnt, unsigned char* sm) {
+  unsigned short* const tab = reinterpret_cast<unsigned short*>(sm);  // records << 8 | end, from the segment's start
+  int* const ent = reinterpret_cast<int*>(tab + SN_TABT * SN_TABW);   // entries of the step's segments, -1: none
+  const int t = threadIdx.x;
+  if (t == 0) {
+    const unsigned e = exit_[k0 - 1];
+    ent[SN_TABT] = e == SN_DEAD ? -1 : (int)(e - (unsigned)k0 * SN_SEG);
+  }
+  for (; k0 < nseg; k0 += SN_TABT) {
+    const int k = k0 + t, ns = min(SN_TABT, nseg - k0);
+    const long long s0 = (long long)k * SN_SEG;
+    unsigned short* const my = tab + t * SN_TABW;
+    const int lim = (int)min((long long)SN_SEG, L - s0);
+    if (t < ns) {
+      const int mis = (int)((uintptr_t)(base + s0) & 3);
+      unsigned long long cont = 0;  // continuation bits of the bytes behind the current one
+#pragma unroll 4
+      for (int i = (SN_SEG + SN_LMAX + 6) / 4; i >= 0; --i) {
+        const unsigned w = seg_word(base, L, s0 - mis + 4 * i);
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+          const int b = 4 * i + j - mis;
+          const unsigned v = (w >> (8 * j)) & 255u;
+          if (b >= 0 && b < lim) {
+            const int l = sn_len(v, cont), x = b + l;
+            my[b] = (unsigned short)(!l ? SN_TEND : x >= lim ? (1 << 8) + x : (1 << 8) + my[x]);
+          }
+          cont = (cont << 1) | (v >> 7);
+        }
+      }
+    }
+    __syncthreads();
+    if (t == 0) {
+      int e = ent[SN_TABT];
+      for (int q = 0; q < ns; ++q) {
+        ent[q] = e;
+        if (e < 0 || (long long)(k0 + q) * SN_SEG + e >= L) continue;  // the stream ends before the entry: no record
+        const int x = tab[q * SN_TABW + e] & 255;
+        e = x == SN_TEND ? -1 : x - SN_SEG;
+        if (e < 0) e = -1;  // the last segment's: not used
+      }
+      ent[SN_TABT] = e;
+    }
+    __syncthreads();
+    if (t < ns) {
+      const int e = ent[t];
+      entry[k] = e < 0 ? SN_DEAD : (unsigned)(s0 + e);
+      cnt[k] = e < 0 || e >= lim ? 0u : (unsigned)(my[e] >> 8);
+    }
+    __syncthreads();  // the next step writes the table
+  }
+}
+
 // One CTA per chunk: segments whose guess does not follow from the segment
-// before them are walked again until all agree (segment k is right after at
-// most k rounds, so the loop ends), then cnt becomes the number of the
-// segment's first record.  The chunk is malformed when the chain holds fewer
-// records than it has boxes.
+// before them are walked again, a few times, until all agree (segment k is
+// right after at most k rounds); what then still disagrees is settled by table.
+// cnt becomes the number of the segment's first record.  The chunk is malformed
+// when the chain holds fewer records than it has boxes.
 __global__ void __launch_bounds__(SN_T)
 k_seg_settle(const unsigned char* __restrict__ raw, const long long* __restrict__ raw_off,
              const long long* __restrict__ raw_len, const long long* __restrict__ blk, long long n, unsigned* entry,
              unsigned* exit_, unsigned* cnt, DStatus* st) {
+  extern __shared__ __align__(16) unsigned char sm[];
   __shared__ SumS buf[2][32];
+  __shared__ int s_first;
   const int c = blockIdx.x;
   const int nb = (int)min((long long)SN_CHUNK, n - (long long)c * SN_CHUNK);
   const long long L = raw_len[c];
@@ -667,24 +747,35 @@ k_seg_settle(const unsigned char* __restrict__ raw, const long long* __restrict_
   entry += blk[c] * SN_SEGT;
   exit_ += blk[c] * SN_SEGT;
   cnt += blk[c] * SN_SEGT;
-  for (int round = 0; round <= nseg; ++round) {
-    int changed = 0;
+  if (threadIdx.x == 0) s_first = nseg;
+  for (int round = 0;; ++round) {
+    int first = nseg;  // the thread's first segment that does not follow
     for (int k = threadIdx.x; k < nseg; k += SN_T) {
       const unsigned e = k ? *(volatile unsigned*)&exit_[k - 1] : 0u;
       if (entry[k] == e) continue;
-      changed = 1;
+      first = min(first, k);
+      if (round == SN_ROUNDS) break;
       entry[k] = e;
       unsigned m = 0, x = e;
       if (e != SN_DEAD) {
         long long p = e;
         const long long lim = min(L, (long long)(k + 1) * SN_SEG);
         while (p < lim) {
+          // continuation bits of the next bytes: 16 are nearly always enough (a record that needs more is too long
+          // when the others are set), else as many as a record can use
           unsigned long long cont = 0;
-          for (int j = 0; j < SN_LMAX; ++j) {  // as many continuation bits as a record can use
+          for (int j = 0; j < 16; ++j) {
             const long long q = p + 1 + j;
             if (q < L) cont |= (unsigned long long)(base[q] >> 7) << j;
           }
-          const int l = sn_len(base[p], cont);
+          int l = sn_len(base[p], cont | ~0xffffull);
+          if (!l) {
+            for (int j = 16; j < SN_LMAX; ++j) {
+              const long long q = p + 1 + j;
+              if (q < L) cont |= (unsigned long long)(base[q] >> 7) << j;
+            }
+            l = sn_len(base[p], cont);
+          }
           if (!l) break;
           p += l;
           ++m;
@@ -694,7 +785,13 @@ k_seg_settle(const unsigned char* __restrict__ raw, const long long* __restrict_
       cnt[k] = m;
       *(volatile unsigned*)&exit_[k] = x;
     }
-    if (!__syncthreads_or(changed)) break;
+    if (!__syncthreads_or(first < nseg)) break;
+    if (round == SN_ROUNDS) {
+      atomicMin(&s_first, first);
+      __syncthreads();
+      seg_table(base, L, s_first, nseg, entry, exit_, cnt, sm);
+      break;
+    }
   }
   unsigned carry = 0;
   for (int k0 = 0, it = 0; k0 < nseg; k0 += SN_T, ++it) {
@@ -1618,7 +1715,8 @@ int snap_decode(gb_context* ctx, const unsigned char* d_data, const long long* m
     k_seg_guess<<<sgrid, SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, d_seg, d_seg + nseg, d_seg + 2 * nseg);
     ++c.launches;
   }
-  k_seg_settle<<<(unsigned)nch, SN_T, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, n, d_seg, d_seg + nseg, d_seg + 2 * nseg,
+  cudaFuncSetAttribute((const void*)k_seg_settle, cudaFuncAttributeMaxDynamicSharedMemorySize, SN_TAB_SMEM);
+  k_seg_settle<<<(unsigned)nch, SN_T, SN_TAB_SMEM, c.stream>>>(raw, d_roff, d_rlen, d_sblk, n, d_seg, d_seg + nseg, d_seg + 2 * nseg,
                                                      c.st);
   if (most) {
     k_seg_records<<<sgrid, SN_SEGT, 0, c.stream>>>(raw, d_roff, d_rlen, d_sblk, n, d_seg, d_seg + 2 * nseg, d_rec, c.st);
