@@ -170,3 +170,57 @@ def test_stream_out_of_step_time(ctx):
         return _best(lambda: ctx.decompress_stream_to_boxes(chunks, 0, as_tensor=True))
 
     assert seconds(240) < 5 * seconds(340)
+
+
+def _full_arena():
+    """A context, a layer, and how many MERGEs of it its arena holds (3 at least)."""
+    from vlsi_layout_gb300 import engine
+    ctx = engine.Context(0, 96 << 20)
+    L = ctx.layer(random_layer(150_000, die=1_000_000, seed=2))
+    m, k = ctx.mark(), 0
+    try:
+        while True:
+            ctx.op(4, L)
+            ctx.sync()
+            k += 1
+    except engine.GBError as e:
+        assert e.code == engine.GB_ERR_CAPACITY and k >= 3
+    ctx.release(m)
+    return ctx, L, k
+
+
+def test_captured_release():
+    """A release in a graph goes back to its own mark, not to a later one of the same depth."""
+    from vlsi_layout_gb300 import engine
+    ctx, L, k = _full_arena()
+    m = ctx.mark()
+    ctx.op(4, L)
+    ctx.graph_begin()
+    ctx.release(m)
+    g = ctx.graph_end()
+    for _ in range(2):
+        m = ctx.mark()  # behind the first result, where k more do not fit
+        ctx.graph_launch(g)
+        for _ in range(k):
+            ctx.op(4, L)
+        ctx.sync()
+        ctx.release(m)
+    engine.lib().gb_graph_destroy(g)
+    L.free()
+    ctx.close()
+
+
+def test_many_marks():
+    """More marks than are kept on the device, released one by one and in one go."""
+    ctx, L, k = _full_arena()
+    marks = [ctx.mark() for _ in range(200)]
+    ctx.op(4, L)
+    for m in marks[:100:-1]:
+        ctx.release(m)
+    ctx.op(4, L)
+    ctx.release(marks[0])
+    for _ in range(k):
+        ctx.op(4, L)
+    ctx.sync()
+    L.free()
+    ctx.close()

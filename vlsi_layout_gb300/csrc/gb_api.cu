@@ -361,6 +361,7 @@ extern "C" int gb_context_create(int device, unsigned long long arena_bytes, gb_
   cudaMemset(c.desc, 0, GB_NDESC * sizeof(DLayer));
   for (int i = GB_NDESC - 1; i >= 0; --i) c.desc_free.push_back(i);
   if (cudaMalloc(&c.dmarks, GB_DMARKS * 8) != cudaSuccess) return GB_ERR_OOM;
+  for (int i = GB_DMARKS - 1; i >= 0; --i) ctx->dmark_free.push_back(i);
   if (cudaMallocHost(&c.hb, sizeof(HostBack)) != cudaSuccess) return GB_ERR_OOM;
   cudaMemPoolProps pp;
   memset(&pp, 0, sizeof(pp));
@@ -459,9 +460,10 @@ extern "C" void gb_clear_status(gb_context* ctx) {
   if (ctx) k_clear_status<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st);
 }
 
-// The mark stays on the device, in the stream's order (GB_DMARKS deep; deeper
-// ones, and marks taken during a capture, are read back as numbers).
-#define MARK_ON_DEVICE (~0ull)
+// The mark stays on the device, in the stream's order, in one of GB_DMARKS
+// words.  Marks that find none free, and marks taken during a capture, are read
+// back as numbers.  A release that is captured reads the mark's word whenever
+// the graph runs, so that word is not given to a later mark.
 __global__ void k_arena_mark(DStatus* st, unsigned long long* slot, bool clear) {
   *slot = st->arena_off;
   if (clear) {
@@ -472,37 +474,43 @@ __global__ void k_arena_mark(DStatus* st, unsigned long long* slot, bool clear) 
 }
 __global__ void k_arena_release(DStatus* st, const unsigned long long* slot) { st->arena_off = *slot; }
 
+static bool capturing(GbCtx& c) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(c.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
 // clear: the status too, as gb_clear_status.
 static unsigned long long arena_mark(gb_context* ctx, bool clear) {
   GbCtx& c = ctx->c;
-  const size_t i = ctx->marks.size();
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (i < GB_DMARKS && cudaStreamIsCapturing(c.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
-    k_arena_mark<<<1, 1, 0, c.stream>>>(c.st, c.dmarks + i, clear);
-    ctx->marks.push_back({MARK_ON_DEVICE, ctx->seq});
+  ArenaMark m = {0, ctx->seq, -1};
+  if (!ctx->dmark_free.empty() && !capturing(c)) {
+    m.slot = ctx->dmark_free.back();
+    ctx->dmark_free.pop_back();
+    k_arena_mark<<<1, 1, 0, c.stream>>>(c.st, c.dmarks + m.slot, clear);
   } else {
     if (clear) gb_clear_status(ctx);
-    ctx->marks.push_back({read_status(ctx).arena_off, ctx->seq});
+    m.off = read_status(ctx).arena_off;
   }
-  return (unsigned long long)i;
+  ctx->marks.push_back(m);
+  return (unsigned long long)(ctx->marks.size() - 1);
 }
 
 extern "C" unsigned long long gb_arena_mark(gb_context* ctx) { return ctx ? arena_mark(ctx, false) : 0; }
 
 namespace gbi {
 const unsigned long long* mark_word(gb_context* ctx, unsigned long long mark) {
-  return mark < ctx->marks.size() && ctx->marks[mark].first == MARK_ON_DEVICE ? ctx->c.dmarks + mark : nullptr;
+  return mark < ctx->marks.size() && ctx->marks[mark].slot >= 0 ? ctx->c.dmarks + ctx->marks[mark].slot : nullptr;
 }
 
 void arena_rewind(gb_context* ctx, unsigned long long mark, bool on_device) {
-  const auto m = ctx->marks[mark];
+  const ArenaMark m = ctx->marks[mark];
   if (on_device) {
-    if (m.first == MARK_ON_DEVICE) k_arena_release<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st, ctx->c.dmarks + mark);
-    else gb_launch_arena_reset(ctx->c, m.first);
+    if (m.slot >= 0) k_arena_release<<<1, 1, 0, ctx->c.stream>>>(ctx->c.st, ctx->c.dmarks + m.slot);
+    else gb_launch_arena_reset(ctx->c, m.off);
   }
   std::vector<gb_layer*> keep;
   for (gb_layer* L : ctx->arena_layers) {
-    if (L->seq > m.second) {
+    if (L->seq > m.seq) {
       L->dead = true;
       drop_layer(ctx, L);
     } else {
@@ -516,6 +524,9 @@ void arena_rewind(gb_context* ctx, unsigned long long mark, bool on_device) {
 extern "C" int gb_arena_release(gb_context* ctx, unsigned long long mark) {
   if (!ctx || mark >= ctx->marks.size()) return GB_ERR_ARG;
   arena_rewind(ctx, mark, true);
+  const bool kept = capturing(ctx->c);
+  for (size_t i = mark; i < ctx->marks.size(); ++i)
+    if (ctx->marks[i].slot >= 0 && !(kept && i == mark)) ctx->dmark_free.push_back(ctx->marks[i].slot);
   ctx->marks.resize(mark);
   return GB_OK;
 }

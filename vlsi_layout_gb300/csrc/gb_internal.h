@@ -133,13 +133,20 @@ struct gb_layer {
   long long nbox_host = 0;
 };
 
+// An arena mark: its offset is in word `slot` of dmarks, or (slot < 0) here.
+struct ArenaMark {
+  unsigned long long off, seq;
+  int slot;
+};
+
 struct gb_context {
   GbCtx c;
   std::mutex mu;
   std::mutex hb_mu;  // c.hb, for the time of one read_back
   unsigned long long seq = 0;
   std::vector<gb_layer*> arena_layers;
-  std::vector<std::pair<unsigned long long, unsigned long long>> marks;  // (device off, seq)
+  std::vector<ArenaMark> marks;
+  std::vector<int> dmark_free;  // words of c.dmarks that no mark has
   unsigned long long graph_arena_off = 0;
 };
 
