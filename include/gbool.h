@@ -117,11 +117,6 @@ int gb_context_create(int device, unsigned long long arena_bytes, gb_context** o
 int gb_context_destroy(gb_context* ctx);
 /* Run all work of the context on this cudaStream_t (NULL = the context's own). */
 int gb_set_stream(gb_context* ctx, void* stream);
-/* Layers and the temporaries of calls come from a pool that the contexts of a
- * device share.  It keeps up to 4 GiB that is not in use for the next calls;
- * this gives it back to the device, for other users of it.  The engine's own
- * allocations do so by themselves when memory is short. */
-int gb_release_memory(gb_context* ctx);
 const char* gb_last_error(gb_context* ctx);
 /* Synchronise the stream and return the first device-side status (GB_*). */
 int gb_sync(gb_context* ctx, long long* need);

@@ -32,31 +32,3 @@ def test_morton_sort_memory(oracle):
     k = oracle.morton_keys_np(A)
     assert np.array_equal(perm, np.argsort(k, kind="stable"))
     assert np.array_equal(keys, k[perm]) and np.array_equal(b, A[perm])
-
-
-def test_kept_memory_serves_other_contexts():
-    """What a context's calls leave in the pool is there for another context, its layers, and other users."""
-    from vlsi_layout_gb300 import engine
-    A = random_layer(20_000_000, die=3_000_000, seed=1)
-    scratch = 456 * (8 << 20)  # a context's tile scratch
-    with engine.Context(0, 64 << 20) as a:
-        def kept():  # at least 600 MB that is not in use
-            a.morton_sort(A)
-            a.sync()
-
-        kept()
-        ballast = _leave(scratch + (600 << 20))
-        with engine.Context(0, 1 << 30) as b:
-            del ballast
-            torch.cuda.empty_cache()
-            kept()
-            ballast = _leave(100 << 20)
-            L = b.layer(A)
-            assert L.count()[0] == len(A)
-            L.free()
-            del ballast
-            torch.cuda.empty_cache()
-            kept()
-            free = torch.cuda.mem_get_info()[0]
-            a.release_memory()
-            assert torch.cuda.mem_get_info()[0] >= free + (600 << 20)

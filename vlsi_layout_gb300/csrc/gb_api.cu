@@ -7,7 +7,6 @@
 #include <cstring>
 #include <memory>
 #include <functional>
-#include <map>
 #include <mutex>
 #include <vector>
 
@@ -324,49 +323,11 @@ int realloc_scratch(gb_context* ctx, size_t bytes) {
 using namespace gbi;
 
 // ======================================================================= context
-// The pool of each device that has contexts, and their number.
-static std::mutex g_pools_mu;
-static std::map<int, std::pair<cudaMemPool_t, int>> g_pools;
-
-static cudaMemPool_t pool_acquire(int device) {
-  std::lock_guard<std::mutex> lk(g_pools_mu);
-  auto f = g_pools.find(device);
-  if (f != g_pools.end()) {
-    ++f->second.second;
-    return f->second.first;
-  }
-  cudaMemPoolProps pp;
-  memset(&pp, 0, sizeof(pp));
-  pp.allocType = cudaMemAllocationTypePinned;
-  pp.location.type = cudaMemLocationTypeDevice;
-  pp.location.id = device;
-  cudaMemPool_t pool = nullptr;
-  if (cudaMemPoolCreate(&pool, &pp) != cudaSuccess) return nullptr;
-  unsigned long long keep = GB_POOL_KEEP;
-  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  int wait = 0;  // one context's stream is not made to wait for another's
-  cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &wait);
-  g_pools[device] = {pool, 1};
-  return pool;
-}
-
-static void pool_release(int device) {
-  std::lock_guard<std::mutex> lk(g_pools_mu);
-  auto f = g_pools.find(device);
-  if (f == g_pools.end() || --f->second.second > 0) return;
-  cudaMemPoolDestroy(f->second.first);
-  g_pools.erase(f);
-}
-
-struct CtxUndo {
-  void operator()(gb_context* ctx) const { gb_context_destroy(ctx); }
-};
-
 extern "C" int gb_context_create(int device, unsigned long long arena_bytes, gb_context** out) {
   if (!out) return GB_ERR_ARG;
   *out = nullptr;
   if (cudaSetDevice(device) != cudaSuccess) return GB_ERR_CUDA;
-  std::unique_ptr<gb_context, CtxUndo> ctx(new gb_context());  // what a failed creation has made is freed
+  std::unique_ptr<gb_context> ctx(new gb_context());
   GbCtx& c = ctx->c;
   c.device = device;
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess) return GB_ERR_CUDA;
@@ -375,9 +336,6 @@ extern "C" int gb_context_create(int device, unsigned long long arena_bytes, gb_
   cudaGetDeviceProperties(&prop, device);
   c.nsm = prop.multiProcessorCount;
   c.work_blocks = c.nsm * 4;
-  c.pool = pool_acquire(device);
-  if (!c.pool) return GB_ERR_CUDA;
-  if (arena_bytes == 0) gb_pool_give(c);
   size_t freeb = 0, totb = 0;
   cudaMemGetInfo(&freeb, &totb);
   if (arena_bytes == 0) {
@@ -385,26 +343,34 @@ extern "C" int gb_context_create(int device, unsigned long long arena_bytes, gb_
     const unsigned long long lim = 120ull << 30;
     if (arena_bytes > lim) arena_bytes = lim;
   }
-  if (gb_dev_alloc(c, (void**)&c.arena, arena_bytes) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.arena, arena_bytes) != cudaSuccess) return GB_ERR_OOM;
   c.arena_cap = arena_bytes;
-  if (gb_dev_alloc(c, (void**)&c.st, sizeof(DStatus)) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.st, sizeof(DStatus)) != cudaSuccess) return GB_ERR_OOM;
   DStatus s0;
   memset(&s0, 0, sizeof(s0));
   s0.arena_base = c.arena;
   s0.arena_cap = arena_bytes;
   cudaMemcpy(c.st, &s0, sizeof(s0), cudaMemcpyHostToDevice);
-  if (gb_dev_alloc(c, (void**)&c.scan_part, (GB_SCAN_BLOCKS + 1) * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.scan_part, (GB_SCAN_BLOCKS + 1) * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
   cudaMemset(c.scan_part, 0, (GB_SCAN_BLOCKS + 1) * sizeof(long long));
-  if (gb_dev_alloc(c, (void**)&c.dscal, 64 * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
-  if (gb_dev_alloc(c, (void**)&c.tile_counter, 64 * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.dscal, 64 * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.tile_counter, 64 * sizeof(long long)) != cudaSuccess) return GB_ERR_OOM;
   cudaMemset(c.dscal, 0, 64 * sizeof(long long));
   cudaMemset(c.tile_counter, 0, 64 * sizeof(long long));
-  if (gb_dev_alloc(c, (void**)&c.desc, GB_NDESC * sizeof(DLayer)) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.desc, GB_NDESC * sizeof(DLayer)) != cudaSuccess) return GB_ERR_OOM;
   cudaMemset(c.desc, 0, GB_NDESC * sizeof(DLayer));
   for (int i = GB_NDESC - 1; i >= 0; --i) c.desc_free.push_back(i);
-  if (gb_dev_alloc(c, (void**)&c.dmarks, GB_DMARKS * 8) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc(&c.dmarks, GB_DMARKS * 8) != cudaSuccess) return GB_ERR_OOM;
   for (int i = GB_DMARKS - 1; i >= 0; --i) ctx->dmark_free.push_back(i);
   if (cudaMallocHost(&c.hb, sizeof(HostBack)) != cudaSuccess) return GB_ERR_OOM;
+  cudaMemPoolProps pp;
+  memset(&pp, 0, sizeof(pp));
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = device;
+  if (cudaMemPoolCreate(&c.pool, &pp) != cudaSuccess) return GB_ERR_CUDA;
+  unsigned long long keep = GB_POOL_KEEP;
+  cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &keep);
   gb_tile_setup(c);
   if (realloc_scratch(ctx.get(), 8ull << 20) != GB_OK) return GB_ERR_OOM;
   cudaDeviceSynchronize();
@@ -428,7 +394,7 @@ extern "C" int gb_context_destroy(gb_context* ctx) {
   cudaFree(c.tile_scratch);
   cudaFree(c.dmarks);
   if (c.hb) cudaFreeHost(c.hb);
-  if (c.pool) pool_release(c.device);
+  if (c.pool) cudaMemPoolDestroy(c.pool);
   if (c.io_buf) cudaFree(c.io_buf);
   if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
   gb_radix_free(c);
@@ -450,12 +416,6 @@ extern "C" int gb_set_stream(gb_context* ctx, void* stream) {
   if (c.own_stream) cudaStreamDestroy(c.stream);
   c.stream = next;
   c.own_stream = stream == nullptr;
-  return GB_OK;
-}
-
-extern "C" int gb_release_memory(gb_context* ctx) {
-  if (!ctx) return GB_ERR_ARG;
-  gb_pool_give(ctx->c);
   return GB_OK;
 }
 

@@ -171,7 +171,10 @@ int read_snap_layer(Deck& d, const std::string& path, gb_layer** out) {
   }
   if (n == 0) return make_layer(d, d.empty, out);
   c_box* db = nullptr;
-  if (gb_dev_alloc(d.ctx->c, (void**)&db, (size_t)n * sizeof(c_box)) != cudaSuccess) return GB_ERR_OOM;
+  if (cudaMalloc((void**)&db, (size_t)n * sizeof(c_box)) != cudaSuccess) {
+    cudaGetLastError();
+    return GB_ERR_OOM;
+  }
   long long got = 0;
   e = gb_restore_snap_to_layer(d.ctx, path.c_str(), db, n, &got, nullptr);
   if (!e && got != n) e = GB_ERR_CORRUPT;  // diskdesign_impl.f90:104-109: SNAP RESTORATION FAILED

@@ -49,7 +49,7 @@ struct GbCtx {
   void* io_buf = nullptr;            // device staging of host inputs (gb_op1_host), grow-only
   size_t io_cap = 0;
   cudaStream_t copy_stream = nullptr;  // host-to-device copies that overlap the compute stream
-  cudaMemPool_t pool = nullptr;      // layers and call temporaries (gb_tmp_alloc), in the order of the stream; the device's
+  cudaMemPool_t pool = nullptr;      // layers and call temporaries (gb_tmp_alloc), in the order of the stream
   unsigned long long* dmarks = nullptr;  // arena marks kept on the device [GB_DMARKS]
   struct HostBack* hb = nullptr;     // pinned: where read_back's copies land
 };
@@ -60,11 +60,10 @@ struct HostBack {
   long long w[8];
 };
 #define GB_DMARKS 64
-// The contexts of a device share a pool, so that what one has freed is there
-// for the others.  It keeps at most this much memory that is not in use (the
-// rest goes back at the next synchronisation, all of it with the last context
-// or by gb_release_memory): cudaMalloc and cudaFree of the temporaries of a
-// call cost more than its kernels (sort of 20M trackers: 900 of 2000 us).
+// The pool keeps at most this much memory that is not in use (the rest goes
+// back at the next synchronisation, all of it with the context): cudaMalloc
+// and cudaFree of the temporaries of a call cost more than its kernels (sort
+// of 20M trackers: 900 of 2000 us).
 #define GB_POOL_KEEP (4ull << 30)
 
 // Waits for the frees in the stream's order; the pool keeps nothing.
@@ -93,9 +92,7 @@ inline cudaError_t gb_dev_alloc(GbCtx& c, void** p, size_t bytes) {
   if (e != cudaErrorMemoryAllocation) return e;
   cudaGetLastError();
   gb_pool_give(c);
-  e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported by the caller, not by a later call
-  return e;
+  return cudaMalloc(p, bytes);
 }
 inline void gb_tmp_free(GbCtx& c, void* p) {
   if (p) cudaFreeAsync(p, c.stream);

@@ -804,8 +804,8 @@ int gb_radix_sort_pairs(GbCtx& c, unsigned long long* keys, unsigned* vals, long
   const long long ntile = (n + TILE - 1) / TILE;
   RsState* S = state_of(c);
   if (!S->ghist) {
-    if (gb_dev_alloc(c, (void**)&S->ghist, RS_HIST_SLOTS * sizeof(unsigned)) != cudaSuccess ||
-        gb_dev_alloc(c, (void**)&S->ctrs, (RS_MAXPASS + 1) * sizeof(long long)) != cudaSuccess)
+    if (cudaMalloc(&S->ghist, RS_HIST_SLOTS * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&S->ctrs, (RS_MAXPASS + 1) * sizeof(long long)) != cudaSuccess)
       return -2;
   }
   const size_t want = (size_t)(ntile + 1024) * maxradix;

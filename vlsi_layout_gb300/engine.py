@@ -57,7 +57,6 @@ def lib():
         "gb_context_create": (ctypes.c_int, [ctypes.c_int, u64, pp]),
         "gb_context_destroy": (ctypes.c_int, [P]),
         "gb_set_stream": (ctypes.c_int, [P, P]),
-        "gb_release_memory": (ctypes.c_int, [P]),
         "gb_last_error": (ctypes.c_char_p, [P]),
         "gb_sync": (ctypes.c_int, [P, P]),
         "gb_clear_status": (None, [P]),
@@ -211,10 +210,6 @@ class Context:
 
     def set_stream(self, stream_handle):
         self._chk(lib().gb_set_stream(self.h, ctypes.c_void_p(stream_handle)))
-
-    def release_memory(self):
-        """Give back the device memory that the engine keeps for its next calls."""
-        self._chk(lib().gb_release_memory(self.h))
 
     def set_grid(self, g):
         """Tile grid of the operators: slab height 2^g dbu (10..16, default 16)."""
