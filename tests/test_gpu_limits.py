@@ -224,3 +224,29 @@ def test_many_marks():
     ctx.sync()
     L.free()
     ctx.close()
+
+
+# empty tiles between, before and behind the others: fewer and many more tiles than the kernel has CTAs
+@pytest.mark.parametrize("tiles,n", [(3, 2), (40, 7), (60, 900), (300, 2), (300, 5000), (1000, 400)])
+def test_sparse_layers(ctx, oracle, tiles, n):
+    rng = np.random.default_rng(tiles + n)
+    side = tiles * 65536
+
+    def layer(k):
+        p = rng.integers(-side // 2, side // 2 - 70_000, (k, 2))
+        b = np.concatenate([p, p + rng.integers(20, 60_000, (k, 2))], 1)
+        b[:2] = [[-side // 2, -side // 2, -side // 2 + 9, -side // 2 + 5], [side // 2 - 9, side // 2 - 5, side // 2, side // 2]]
+        return b.astype(np.int32)
+
+    A, B = layer(n), layer(n)
+    for op in (0, 2, 3, 4):
+        m = ctx.mark()
+        got = ctx.op(op, ctx.layer(A), ctx.layer(B) if op != 4 else None).to_numpy()
+        ctx.release(m)
+        exp = oracle.boolean(A, B, op) if op != 4 else oracle.merge(A)
+        assert np.array_equal(got[np.lexsort((got[:, 3], got[:, 2], got[:, 1], got[:, 0]))], exp), op
+    m = ctx.mark()
+    assert int(ctx.area(ctx.layer(A))[0]) == oracle.union_area(A)
+    both = ctx.area(ctx.layer(np.concatenate([A, B]), [0, len(A), len(A), 2 * len(A)]))
+    assert [int(a) for a in both] == [oracle.union_area(A), 0, oracle.union_area(B)]
+    ctx.release(m)
