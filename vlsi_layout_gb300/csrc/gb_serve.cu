@@ -63,6 +63,14 @@ long long estimate(const gb_server* S, const gb_request& r) {
   return 48ll * n + (4ll << 20);
 }
 
+// CTAs that a request's operators may share tiles with when k requests are in flight or waiting for a slot.  CTAs that
+// share a tile repeat its ranking, which pays on idle SMs only: all of them for one request, fewer the more run beside
+// it.  40 requests (us; 8 slots with a burst / 3 slots with a burst / one at a time) by this rule, with half of the
+// chip whatever k, the whole chip, none: on 20000 boxes 731 / 1276 / 3082, 749 / 1275 / 3242, 1028 / 1386 / 3095, 677 /
+// 1390 / 3836; on 60000 1062 / 1599 / 3734, 1113 / 1610 / 3975, 1332 / 1730 / 3782, 1027 / 1527 / 3967; on 2000 all but
+// none (1278 us with 3 slots, 3553 one at a time) within 3% of 637 / 1157 / 2950.
+int shared_ctas(int full, int k) { return full * 2 / (k + 1) / 8 * 8; }
+
 gb_layer* issue(gb_server* S, gb_server_slot& sl, const gb_request& r, int* status) {
   gb_layer* O = nullptr;
   int e = GB_ERR_ARG;
@@ -108,10 +116,6 @@ extern "C" int gb_serve_create(int device, unsigned long long budget_bytes, int 
       S->slots.push_back(sl);  // what it has is freed with the others
       break;
     }
-    // Requests of other slots run beside this one's: CTAs that share a tile repeat its ranking, which pays for idle
-    // SMs only, so a request counts on half of them (40 requests on 60000 boxes: the whole chip 1555 us, half 1457,
-    // no shared tiles 1478; on 2000 boxes 1123, 1123 and 1252 us).
-    if (slots > 1) sl.ctx->c.split_ctas = sl.ctx->c.split_ctas / 16 * 8;
     sl.mark = gb_arena_mark(sl.ctx);
     S->slots.push_back(sl);
   }
@@ -214,6 +218,9 @@ extern "C" int gb_serve_run(gb_server* S, const gb_request* reqs, int nreq, gb_r
       gb_server_slot& sl = *free_slot;
       res[i].start_s = now_s();
       int st = 0;
+      int k = 1 + (int)waiting.size();
+      for (const gb_server_slot& o : S->slots) k += o.req >= 0;
+      sl.ctx->c.split_ctas = shared_ctas(S->home->c.split_ctas, std::min(k, (int)S->slots.size()));
       sl.out = issue(S, sl, reqs[i], &st);
       if (!sl.out) {
         res[i].status = st;
