@@ -406,7 +406,10 @@ long long gb_launch_count(gb_context* ctx);
  * per sub-band-count bucket (1, 2-3, 4-7, 8-15, 16-31, 32+) the tiles and
  * their phase-C cycles; the wide sub-bands (more columns or y ranks than one
  * warp's buffer holds) and their cycles, the others and theirs; all since
- * gb_tile_timing(ctx, 1). */
+ * gb_tile_timing(ctx, 1).  While on, operators run the timed form of the
+ * kernel, one tile per CTA: layers of few tiles, whose tiles CTAs share
+ * otherwise, run another kernel than the one that is timed.  gb_op_area is
+ * not timed. */
 int gb_tile_timing(gb_context* ctx, int on);
 /* Diagnostics: runs one radix pass whose only CTA waits for a predecessor
  * tile that never publishes; returns the status it reports (GB_ERR_TIMEOUT

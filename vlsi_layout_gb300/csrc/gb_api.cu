@@ -762,7 +762,9 @@ extern "C" void gb_layer_free(gb_context* ctx, gb_layer* L) {
 }
 
 // ======================================================================= operators
-gb_layer* op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, int mode) {
+// area: the result has its cells' areas only, no strips and no counts, and is
+// for the caller's own use.
+gb_layer* op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, bool area) {
   GbCtx& c = ctx->c;
   const int g = c.grid;
   gb_layer* Ab = binned_of(ctx, A, g);
@@ -771,9 +773,10 @@ gb_layer* op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, int mode) {
   if (!Ab || (B && !single && !Bb)) return nullptr;
   gb_layer* O = new_arena_layer(ctx, A->ncell, g);
   if (!O) return nullptr;
-  gb_launch_bool_setup(c, op, Ab->d, Bb ? Bb->d : nullptr, O->d, A->ncell, g, mode == 0);
-  gb_launch_tile_bool(c, op, Ab->d, Bb ? Bb->d : nullptr, O->d, g, mode);
-  O->counted = 1;
+  gb_launch_bool_setup(c, op, Ab->d, Bb ? Bb->d : nullptr, O->d, A->ncell, g, !area);
+  gb_launch_tile_bool(c, op, Ab->d, Bb ? Bb->d : nullptr, O->d, g, area);
+  O->counted = !area;
+  O->dead = area;  // no entry point takes it
   return O;
 }
 
@@ -784,7 +787,7 @@ extern "C" int gb_op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, gb_
   if (!single && !B) return GB_ERR_ARG;
   if (single) B = nullptr;
   if (B && B->ncell != A->ncell) return set_err(ctx, GB_ERR_ARG, "operands differ in cell count");
-  *out = op_bool(ctx, op, A, B, 0);
+  *out = op_bool(ctx, op, A, B);
   return *out ? GB_OK : set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
 }
 
@@ -794,7 +797,7 @@ gb_layer* op_grow(gb_context* ctx, gb_layer* A, int E, int N, int W, int S, bool
   if (!R) return nullptr;
   gb_launch_rebin(ctx->c, A->d, A->binned, R->d, A->ncell, g, E, N, W, S);
   if (!merge) return R;
-  return op_bool(ctx, GB_OP_MERGE, R, nullptr, 0);
+  return op_bool(ctx, GB_OP_MERGE, R, nullptr);
 }
 
 extern "C" int gb_op_grow(gb_context* ctx, gb_layer* A, int32_t E, int32_t N, int32_t W, int32_t S,
@@ -814,26 +817,26 @@ gb_layer* op_erode(gb_context* ctx, gb_layer* P, int t, gb_layer** frame_out, gb
   if (!F) return nullptr;
   F->binned = 0;
   gb_launch_frame(c, Pb->d, F->d, P->ncell, g, t);
-  gb_layer* Q = op_bool(ctx, GB_OP_NOT, F, Pb, 0);
+  gb_layer* Q = op_bool(ctx, GB_OP_NOT, F, Pb);
   if (!Q) return nullptr;
   if (frame_out) *frame_out = F;
   if (comp_out) *comp_out = Q;
   gb_layer* D = op_grow(ctx, Q, t, t, t, t, false);
   if (!D) return nullptr;
-  return op_bool(ctx, GB_OP_NOT, Pb, D, 0);
+  return op_bool(ctx, GB_OP_NOT, Pb, D);
 }
 
 extern "C" int gb_op_size(gb_context* ctx, gb_layer* A, int32_t s, gb_layer** out) {
   if (!ctx || !A || !out || A->dead) return GB_ERR_ARG;
   if (s > 0) *out = op_grow(ctx, A, s, s, s, s, true);
-  else if (s == 0) *out = op_bool(ctx, GB_OP_MERGE, A, nullptr, 0);
+  else if (s == 0) *out = op_bool(ctx, GB_OP_MERGE, A, nullptr);
   else *out = op_erode(ctx, A, -s);
   return *out ? GB_OK : set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
 }
 
 extern "C" int gb_op_area(gb_context* ctx, gb_layer* A, long long* area_per_cell) {
   if (!ctx || !A || A->dead || !area_per_cell) return GB_ERR_ARG;
-  gb_layer* O = op_bool(ctx, GB_OP_MERGE, A, nullptr, 1);
+  gb_layer* O = op_bool(ctx, GB_OP_MERGE, A, nullptr, true);
   if (!O) return set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
   int e = gb_sync(ctx, nullptr);
   if (e) return e;

@@ -78,8 +78,9 @@ extern "C" int gb_profile_read(gb_context* ctx, double* ms_total, long long* lau
 // enables them; gb_tile_timing_read returns [cycA, cycB, cycC, cycD, tiles,
 // pieces, sub-bands, strip pieces] summed over CTAs since enabling, the
 // sub-band step counters, per sub-band-count bucket the tiles and their
-// phase-C cycles, and the sub-bands with and without spilled column words and
-// their cycles (40 values).
+// phase-C cycles, and the wide and the other sub-bands and their cycles (40
+// values).  While on, strips are made by the timed form of the kernel, one
+// tile per CTA whatever their number; areas are not timed.
 __global__ void k_zero_timing(long long* ctr) {
   for (int i = 16; i < 56; ++i) ctr[i] = 0;
 }
@@ -159,13 +160,13 @@ extern "C" void gb_graph_destroy(gb_graph* G) {
 static int op1_chain(gb_context* ctx, gb_layer* P, int32_t a, gb_layer** outs, gb_layer** F, gb_layer** Q) {
   gb_layer* p1 = a >= 0 ? op_grow(ctx, P, a, a, a, a, true) : op_erode(ctx, P, -a);
   gb_layer* p2 = a > 0 ? op_erode(ctx, P, a, F, Q)
-                       : (a == 0 ? op_bool(ctx, GB_OP_MERGE, P, nullptr, 0) : op_grow(ctx, P, -a, -a, -a, -a, true));
+                       : (a == 0 ? op_bool(ctx, GB_OP_MERGE, P, nullptr) : op_grow(ctx, P, -a, -a, -a, -a, true));
   if (!p1 || !p2) return set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
-  gb_layer* outer = op_bool(ctx, GB_OP_NOT, p1, P, 0);
-  gb_layer* inner = op_bool(ctx, GB_OP_NOT, P, p2, 0);
+  gb_layer* outer = op_bool(ctx, GB_OP_NOT, p1, P);
+  gb_layer* inner = op_bool(ctx, GB_OP_NOT, P, p2);
   if (!outer || !inner) return set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
-  gb_layer* and1 = op_bool(ctx, GB_OP_AND, outer, P, 0);
-  gb_layer* inter = op_bool(ctx, GB_OP_AND, outer, inner, 0);
+  gb_layer* and1 = op_bool(ctx, GB_OP_AND, outer, P);
+  gb_layer* inter = op_bool(ctx, GB_OP_AND, outer, inner);
   if (!and1 || !inter) return set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
   outs[0] = p1; outs[1] = p2; outs[2] = outer; outs[3] = inner; outs[4] = and1; outs[5] = inter;
   return GB_OK;
@@ -194,7 +195,7 @@ __global__ void k_copy_area(const DLayer* A, long long* out, int ncell, DStatus*
 
 // The OP1 chain plus the union area of P per cell into d_area (device, ncell
 // entries).  With a > 0 the area falls out of the erosion (no extra pass over
-// P); otherwise it is a count-mode union of P.  Asynchronous, capturable.
+// P); otherwise it is an area pass over P.  Asynchronous, capturable.
 extern "C" int gb_op1_area(gb_context* ctx, gb_layer* P, int32_t a, gb_layer** outs, long long* d_area) {
   if (!ctx || !P || !outs || !d_area || P->dead) return GB_ERR_ARG;
   GbCtx& c = ctx->c;
@@ -206,7 +207,7 @@ extern "C" int gb_op1_area(gb_context* ctx, gb_layer* P, int32_t a, gb_layer** o
   if (F && Q) {
     k_area_from_frame<<<nb, 256, 0, c.stream>>>(F->d, Q->d, d_area, P->ncell, c.st);
   } else {
-    gb_layer* M = op_bool(ctx, GB_OP_MERGE, P, nullptr, 1);
+    gb_layer* M = op_bool(ctx, GB_OP_MERGE, P, nullptr, true);
     if (!M) return set_err(ctx, GB_ERR_CAPACITY, "descriptor pool exhausted");
     k_copy_area<<<nb, 256, 0, c.stream>>>(M->d, d_area, P->ncell, c.st);
   }

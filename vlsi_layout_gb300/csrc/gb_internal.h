@@ -171,7 +171,7 @@ void arena_rewind(gb_context* ctx, unsigned long long mark, bool on_device);
 // The device word that holds the arena offset of a mark (null: kept on the host).
 const unsigned long long* mark_word(gb_context* ctx, unsigned long long mark);
 }
-gb_layer* op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, int mode);
+gb_layer* op_bool(gb_context* ctx, int op, gb_layer* A, gb_layer* B, bool area = false);
 gb_layer* op_grow(gb_context* ctx, gb_layer* A, int E, int N, int W, int S, bool merge);
 // Erosion of P by the square [-t,t]^2.  frame_out / comp_out (optional)
 // receive the frame F (bbox of each cell grown by t, one box per cell) and
@@ -198,7 +198,7 @@ void gb_launch_rebin(GbCtx& c, const DLayer* src, int src_binned, DLayer* out, i
 void gb_launch_bin_index(GbCtx& c, const DLayer* src, DLayer* out, int ncell, int g);
 // A Boolean op's fresh result layer: output window, tile descriptors, slots;
 // also clears the tile kernel's work counters.
-// alloc_slots = 0: count / area only (no output slots).
+// alloc_slots = 0: areas only (no output slots).
 void gb_launch_bool_setup(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O,
                           int ncell, int g, int alloc_slots);
 // Export a binned layer to global-coordinate int4 boxes (tile order).
@@ -215,9 +215,9 @@ void gb_launch_digest(GbCtx& c, const DLayer* L, unsigned long long* out, int st
 
 // ---- tile kernel (gb_tile.cu)
 void gb_tile_setup(GbCtx& c);
-// mode: 0 = emit strips, 1 = count + area only
+// area: the cells' areas only, else strips
 void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O, int g,
-                         int mode);
+                         bool area);
 
 // ---- connectivity (gb_uf.cu)
 void gb_launch_components(GbCtx& c, const DLayer* raw, DLayer* binidx, int* parent,

@@ -1117,7 +1117,7 @@ __device__ __forceinline__ int tile_share(long long nt, int ctas) {
 // since).
 template <bool TIMING, int FORM>
 __global__ void __launch_bounds__(TK_NT, 3)
-k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, char* scratch,
+k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch,
        unsigned long long scr, long long* counter, DStatus* st, int split_ctas) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TileSmem& s = *reinterpret_cast<TileSmem*>(smraw);
@@ -1125,8 +1125,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
   char* base = scratch + (size_t)blockIdx.x * scr;
   const unsigned long long half = scr >> 1;
   const int W = ((1 << g) >> 5) + 1;
-  const bool timing = TIMING && (mode & 4) != 0;
-  mode &= 3;
+  constexpr bool timing = TIMING;
   long long tA = 0, tB = 0, tC = 0, tD = 0, t0 = 0;
   constexpr bool SPLIT = FORM == TILE_SPLIT, AREA = FORM == TILE_AREA;
   const int share = tile_share(O->ntiles, split_ctas);
@@ -1652,7 +1651,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     if (nsb <= 0) __syncthreads();  // else the scan's barrier: the links are cleared
     if (!SPLIT && tid == TK_NT - 32) {  // read after the links' barrier
       s.obase = -1;
-      if (mode == 0 && H > 0) {
+      if (H > 0) {
         atomicAdd((unsigned long long*)&O->ntot, (unsigned long long)H);
         const long long o = (long long)atomicAdd((unsigned long long*)&O->nused, (unsigned long long)H);
         if (o + H <= O->npcs) {
@@ -1725,7 +1724,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
       }
       if (me == 0 && tid == 0) {
         long long o = -1;
-        if (mode == 0 && total > 0 && !bad) {
+        if (total > 0 && !bad) {
           atomicAdd((unsigned long long*)&O->ntot, (unsigned long long)total);
           o = (long long)atomicAdd((unsigned long long*)&O->nused, (unsigned long long)total);
           if (o + total > O->npcs) {
@@ -1779,12 +1778,8 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
     }
     if (SPLIT && tid == 0 && me > 0) atomicAdd((unsigned long long*)&O->cell_area[s.cell], (unsigned long long)area);
     if (tid == 0 && me == 0) {
-      if (mode == 0) {
-        O->tcount[t] = obase >= 0 ? H : 0;
-        O->tstart[t] = obase >= 0 ? obase : 0;
-      } else {
-        O->tcount[t] = H;
-      }
+      O->tcount[t] = obase >= 0 ? H : 0;
+      O->tstart[t] = obase >= 0 ? obase : 0;
       atomicAdd((unsigned long long*)&O->cell_area[s.cell], (unsigned long long)area);
       atomicAdd((unsigned long long*)&O->cell_count[s.cell], (unsigned long long)H);
       if (timing) {
@@ -1796,11 +1791,11 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode, cha
         atomicAdd((unsigned long long*)&counter[23], (unsigned long long)NP);
       }
       atomicAdd((unsigned long long*)&counter[8], (unsigned long long)P * 8ull);
-      atomicAdd((unsigned long long*)&counter[9], (unsigned long long)(mode == 0 ? H : 0) * 8ull);
+      atomicAdd((unsigned long long*)&counter[9], (unsigned long long)H * 8ull);
     }
     if (SPLIT) break;
   }
-  if (mode == 0 && tid == 0) {  // the last CTA to finish gives the pool's tail back
+  if (!AREA && tid == 0) {  // the last CTA to finish gives the pool's tail back
     __threadfence();
     if (atomicAdd((unsigned long long*)&counter[2], 1ull) == gridDim.x - 1) {
       __threadfence();
@@ -1849,7 +1844,7 @@ void gb_tile_setup(GbCtx& c) {
   c.split_ctas = std::min(ncl, c.tile_blocks / 8) * 8;
 }
 
-void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O, int g, int mode) {
+void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLayer* O, int g, bool area) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c.prof) {
     if (c.prof_used + 2 > c.prof_ev.size()) {
@@ -1868,22 +1863,22 @@ void gb_launch_tile_bool(GbCtx& c, int op, const DLayer* A, const DLayer* B, DLa
     cudaEventRecordWithFlags(e0, c.stream, c.prof_flags);
   }
   // which of the two launches takes the layer depends on its tiles, which the device knows
-  if (mode == 1) {
+  if (area) {
     k_tile<false, TILE_AREA><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
-        op, A, B, O, g, mode, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.tile_blocks);
+        op, A, B, O, g, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.tile_blocks);
   } else if (c.timing) {
     k_tile<true, TILE_WHOLE><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
-        op, A, B, O, g, mode | 4, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, 0);
+        op, A, B, O, g, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, 0);
   } else {
     if (c.split_ctas) {
       cudaLaunchAttribute at;
       const cudaLaunchConfig_t cfg = split_config(c, &at, c.split_ctas);
-      cudaLaunchKernelEx(&cfg, k_tile<false, TILE_SPLIT>, op, A, B, O, g, mode, c.tile_scratch,
+      cudaLaunchKernelEx(&cfg, k_tile<false, TILE_SPLIT>, op, A, B, O, g, c.tile_scratch,
                          (unsigned long long)c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
       ++c.launches;
     }
     k_tile<false, TILE_WHOLE><<<c.tile_blocks, TK_NT, c.tile_smem, c.stream>>>(
-        op, A, B, O, g, mode, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
+        op, A, B, O, g, c.tile_scratch, c.tile_scr_bytes, c.tile_counter, c.st, c.split_ctas);
   }
   if (c.prof) cudaEventRecordWithFlags(e1, c.stream, c.prof_flags);
   ++c.launches;
@@ -2097,12 +2092,12 @@ extern "C" int gb_bool_tile_noalloc(int op, const int4* d_A, int nA, const int4*
     DLayer* la = &S->L[0];
     DLayer* lb = &S->L[1];
     DLayer* lo = &S->L[2];
-    int gg = g, mode = 0;
+    int gg = g;
     unsigned long long scr_bytes = GB_NA_SCRATCH;
     long long* ctr = S->ctr;
     DStatus* st = &S->res.st;
     int split = 0;
-    void* args[] = {&op, &la, &lb, &lo, &gg, &mode, &scr, &scr_bytes, &ctr, &st, &split};
+    void* args[] = {&op, &la, &lb, &lo, &gg, &scr, &scr_bytes, &ctr, &st, &split};
     if (cudaLaunchKernel((const void*)k_tile<false, TILE_WHOLE>, dim3(1), dim3(TK_NT), args, sizeof(TileSmem), s) != cudaSuccess)
       return na_refuse(GB_ERR_CUDA, d_count, d_area, s);
   }
