@@ -250,3 +250,20 @@ def test_sparse_layers(ctx, oracle, tiles, n):
     both = ctx.area(ctx.layer(np.concatenate([A, B]), [0, len(A), len(A), 2 * len(A)]))
     assert [int(a) for a in both] == [oracle.union_area(A), 0, oracle.union_area(B)]
     ctx.release(m)
+
+
+# y ranks of a tile around what the buffers of one warp (188 words, wide form 420), two, four and eight warps hold (844,
+# 1724, 2052 words); few columns a sub-band and many
+@pytest.mark.parametrize("n", [3008, 3009, 6720, 6721, 13504, 13505, 27584, 27585, 32000])
+def test_y_rank_limits(ctx, oracle, n):
+    rng = np.random.default_rng(n)
+    y = rng.permutation(32_000)[:n] * 2
+    for width in (40, 900):
+        x = rng.integers(0, 65_536 - width, n)
+        A = np.stack([x, y, x + rng.integers(1, width, n), y + 1], 1).astype(np.int32)
+        m = ctx.mark()
+        L = ctx.layer(A)
+        got = ctx.op(4, L).to_numpy()
+        assert np.array_equal(got[np.lexsort((got[:, 3], got[:, 2], got[:, 1], got[:, 0]))], oracle.merge(A))
+        assert int(ctx.area(L)[0]) == oracle.union_area(A)
+        ctx.release(m)

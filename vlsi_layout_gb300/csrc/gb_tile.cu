@@ -67,10 +67,15 @@
 #define TK_MDS 128   // sub-bands whose metadata fits in the bitmap region after phase B
 #define TK_MD_INTS (TK_MDS * 4 + (TK_MDS + 2) * 2 + TK_MDS * 2 * 2)  // sbinfo, sbh, sbct, sbol, sbrec
 // Per-warp sweep buffers of phase C (6 KB a warp): bitmap words over the tile's y ranks, columns.  A sub-band
-// that needs more is wide; the wide ones of a tile are swept after the others by 4, 2 or 1 warps with 2, 4 or 8
-// times the buffer (levels 1..3), so their words stay in shared memory too.  Standard-cell tiles (2700 boxes of
+// that needs more is wide; the wide ones of a tile are swept after the others by teams of 2, 4 or 8 warps with their
+// buffers together (levels 1..3), so their words stay in shared memory too.  Standard-cell tiles (2700 boxes of
 // each layer) have 160..290 columns in nearly every sub-band: with their words in the global scratch, and a walk
 // back over them for every piece, XOR of two 1M-box layers took 2337 us, now 1898 us.
+// The wide buffers keep a bitmap's prefix popcounts per 64-bit word and the run starts in the bitmap's place, so they
+// hold more y ranks.  A tile whose y ranks are too many for level 0 though its sub-bands have few columns (3000 small
+// random boxes and more) has them swept by single warps with such a buffer (level 0 of the wide form): one CTA, XOR of
+// 3000 and 3000 boxes of one tile 704 us by teams, now 381; 484 such tiles 1737 and 1047.  In the common form the 64-bit
+// ranks cost 3% of an OP1 deck.
 #define TK_LBW 188
 #define TK_LVN 132
 #define TK_LCN 128
@@ -144,11 +149,11 @@ struct TileSmem {
     int4 dbuf_align;  // the region starts on 16 bytes: bulk copies and int4 records land in it
   };
   int sbnext;                            // next sub-band to hand to a warp
-  int nwide[TK_WLEVELS + 1];             // wide sub-bands found at each level of phase C (listed in xyv)
+  int nwide[TK_WLEVELS + 2];             // sub-bands that the wide form takes at each level (listed in xyv)
   int narrow;                            // sub-bands swept at level 1 that level 0 could have held
   int hint;                              // the previous tile was mostly wide: start at level 1
   unsigned long long mbar;               // completion of phase D's bulk copies (one phase per tile)
-  long long tmp64[33];
+  long long tmp64[40];
   long long tile;
   const unsigned long long* pa;
   const unsigned long long* pb;
@@ -233,16 +238,25 @@ struct TileXY {
   __device__ __forceinline__ int y1(int r) const { return on ? ((y16[r] + 0xffff) & 0xffff) + 1 : y[r]; }
 };
 
-// Sweep buffer of a warp at level 1..3: columns, bitmap words, cached members.
-__device__ __forceinline__ int wide_cols(int level) { return level == 1 ? 288 : level == 2 ? 640 : 1024; }
-__device__ __forceinline__ int wide_lbw(int level) { return level == 1 ? 320 : level == 2 ? 640 : 2052; }
-__device__ __forceinline__ int wide_mc(int level) { return level == 1 ? 176 : level == 2 ? 168 : 488; }
-constexpr int wide_bytes(int cols, int lbw, int mc) {
-  return cols * 16 + mc * 8 + lbw * 8 + (cols + 4) * 4 + 64 * (cols / 32) * 4;
+// Sweep buffer of the wide form at level 0..3: columns, bitmap words, cached members.
+__host__ __device__ constexpr int wide_cols(int level) {
+  return level == 0 ? TK_LCN : level == 1 ? 288 : level == 2 ? 640 : 1024;
+}
+__host__ __device__ constexpr int wide_lbw(int level) { return level == 0 ? 420 : level == 1 ? 844 : level == 2 ? 1724 : 2052; }
+__host__ __device__ constexpr int wide_mc(int level) { return level == 0 ? TK_MC : level == 1 ? 176 : level == 2 ? 168 : 488; }
+constexpr int wide_bytes(int level) {
+  return wide_cols(level) * 16 + wide_mc(level) * 8 + wide_lbw(level) * 6 + (wide_cols(level) + 4) * 4;
+}
+// The bitmap and its prefixes are dead after the raster: the run starts lie at the end of their place, and the packed
+// counts (pf) of up to 512 columns reach from the member cache into its start.
+constexpr bool wide_fits(int level) {
+  const int cols = wide_cols(level), packed = cols < 512 ? cols : 512;
+  return (packed - wide_mc(level)) * 8 + 64 * (cols / 32) * 4 <= wide_lbw(level) * 6;
 }
 constexpr int TK_WBUF = 6128;  // level 0's bytes per warp; 2, 4 or 8 warps' buffers together at the levels above
-static_assert(wide_bytes(288, 320, 176) <= 2 * TK_WBUF && wide_bytes(640, 640, 168) <= 4 * TK_WBUF &&
-                  wide_bytes(1024, 2052, 488) <= 8 * TK_WBUF,
+static_assert(wide_bytes(0) <= TK_WBUF && wide_bytes(1) <= 2 * TK_WBUF && wide_bytes(2) <= 4 * TK_WBUF &&
+                  wide_bytes(3) <= 8 * TK_WBUF && wide_fits(0) && wide_fits(1) && wide_fits(2) && wide_fits(3) &&
+                  TK_WBUF % 16 == 0,
               "wide sweep buffers");
 static_assert(sizeof(((TileSmem*)0)->lb) + sizeof(((TileSmem*)0)->lp) + sizeof(((TileSmem*)0)->lv) +
                       sizeof(((TileSmem*)0)->ca) + sizeof(((TileSmem*)0)->cb) + sizeof(((TileSmem*)0)->mc) +
@@ -391,15 +405,16 @@ __device__ __forceinline__ void tile_lookup(int op, const DLayer* A, const DLaye
   }
 }
 
-// The 2, 4 or 8 warps of a team of level 1..3 meet (hardware barriers 1..4).
+// The 2, 4 or 8 warps of a team of level 1..3 meet (hardware barriers 1..4); at level 0 a team is a warp.
 __device__ __forceinline__ void team_sync(int level) {
   __syncwarp();
+  if (level == 0) return;
   asm volatile("bar.sync %0, %1;" ::"r"(1 + (gb_warp() >> level)), "r"(32 << level) : "memory");
 }
 
 // TIMING: the phase counters of gb_tile_timing are compiled in (tctr non-null
 // then); the production instance has none of that code.
-// WIDE: the level's larger buffers (level 1..3).  Returns false, with nothing
+// WIDE: the level's larger buffers (level 0..3).  Returns false, with nothing
 // done, when the sub-band needs the next level's buffers; at the last level
 // columns beyond them spill to the scratch.
 // FORM: what the kernel does with a tile (below).
@@ -412,7 +427,7 @@ template <bool TIMING, bool WIDE, int FORM>
 __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int nsb, int Ny, int nA, char* base,
                              unsigned long long scr, int level, long long* tctr) {
   if (!TIMING) tctr = nullptr;
-  // a wide sub-band's warps (2, 4 or 8: a team) share its members and columns
+  // a wide sub-band's warps (1, 2, 4 or 8: a team) share its members and columns
   const int lane = gb_lane(), wid = gb_warp();
   const int T = WIDE ? 32 << level : 32, tl = WIDE ? (int)threadIdx.x & (T - 1) : lane;
   const int wt = WIDE ? tl >> 5 : 0, lead = WIDE ? wid & ~((1 << level) - 1) : 0;
@@ -456,8 +471,8 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     mc = cb + lcn;
     lb = reinterpret_cast<unsigned*>(mc + mcn);
     lp = lb + wide_lbw(level);
-    lv = reinterpret_cast<int*>(lp + wide_lbw(level));
-    srow = reinterpret_cast<unsigned*>(lv + lcn + 4);
+    lv = reinterpret_cast<int*>(lp + wide_lbw(level) / 2);
+    srow = reinterpret_cast<unsigned*>(lv) - 64 * srw;
   } else {
     ca = s.ca[wid];
     cb = s.cb[wid];
@@ -468,7 +483,12 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     srow = s.srow[wid][0];
   }
   const bool cache = m <= mcn;
-  for (int w = tl; w < nwy; w += T) lb[w] = 0;
+  unsigned long long* const lb64 = reinterpret_cast<unsigned long long*>(lb);
+  const int nw = WIDE ? (nwy + 1) >> 1 : nwy;  // words with a prefix: of 64 ranks in the wide form, else of 32
+  for (int w = tl; w < nw; w += T) {
+    if (WIDE) lb64[w] = 0;
+    else lb[w] = 0;
+  }
   tsync();
   for (int j0 = 0; j0 < m; j0 += T * TK_MLD) {
     int4 rr[TK_MLD];
@@ -495,9 +515,9 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   tsync();
   int nl;
   {
-    const int per = WIDE ? ((nwy + T - 1) / T) | 1 : (nwy + 31) >> 5, w0 = min(nwy, tl * per), w1 = min(nwy, w0 + per);
+    const int per = WIDE ? ((nw + T - 1) / T) | 1 : (nw + 31) >> 5, w0 = min(nw, tl * per), w1 = min(nw, w0 + per);
     int cnt = 0;
-    for (int w = w0; w < w1; ++w) cnt += __popc(lb[w]);
+    for (int w = w0; w < w1; ++w) cnt += WIDE ? __popcll(lb64[w]) : __popc(lb[w]);
     int tot;
     int ex = gb_warp_excl(cnt, &tot);
     if (WIDE) {
@@ -510,7 +530,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
         tot += v;
       }
     }
-    for (int w = w0; w < w1; ++w) { lp[w] = ex; ex += __popc(lb[w]); }
+    for (int w = w0; w < w1; ++w) { lp[w] = ex; ex += WIDE ? __popcll(lb64[w]) : __popc(lb[w]); }
     nl = tot;
   }
   const int L = nl - 1;
@@ -532,7 +552,7 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
     ca = (unsigned long long*)pc;
     cb = ca + L;
   }
-  if (WIDE && level == 1 && tl == 0 && L <= TK_LCN && nwy <= TK_LBW) atomicAdd(&s.narrow, 1);
+  if (WIDE && level == 1 && tl == 0 && L <= TK_LCN && nwy <= wide_lbw(0)) atomicAdd(&s.narrow, 1);
   // ---- rasterise: one member per lane; each column word is updated as two
   // 32-bit halves with native shared-memory atomicOr
   // columns per lane; an odd count keeps the lanes' 8-byte words on different banks
@@ -569,8 +589,8 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
         yw = r.w;
       }
       mk = (hi >= 64 ? ~0ull : ((1ull << hi) - 1ull)) & (~0ull << lo);
-      lc1 = bm_rank(lb, lp, yz);
-      const int lc2 = bm_rank(lb, lp, yw);
+      lc1 = WIDE ? bm_rank2(lb, lp, yz) : bm_rank(lb, lp, yz);
+      const int lc2 = WIDE ? bm_rank2(lb, lp, yw) : bm_rank(lb, lp, yw);
       span = lc2 - lc1;
       lv[lc1] = yz;  // a column's bound comes from every member that has it: the same value
       lv[lc2] = yw;
@@ -875,12 +895,12 @@ __device__ __forceinline__ bool tile_subband(TileSmem& s, int op, int sb, int ns
   if (WIDE) {
     if (tl == 0) {
       s.tmp64[lead] = pbase;
-      s.tmp64[lead + 1] = (long long)obase;
+      s.tmp64[32 + lead] = (long long)obase;
       s.tmp64[16 + lead] = (long long)rbase;
     }
     tsync();
     pbase = (int)s.tmp64[lead];
-    obase = (unsigned long long)s.tmp64[lead + 1];
+    obase = (unsigned long long)s.tmp64[32 + lead];
     rbase = (unsigned long long)s.tmp64[16 + lead];
   } else {
     pbase = __shfl_sync(0xffffffffu, pbase, 0);
@@ -1057,28 +1077,33 @@ __device__ __noinline__ long long tile_emit_scratch(TileSmem& s, const char* rec
   return area;
 }
 
-// Levels 1..3 of phase C: the wide sub-bands that the level below listed, by teams of warps that share a buffer.
-// Called by the whole CTA after level 0.  Out of line: its registers stay out of the kernel's narrow path.
+// Levels first..3 of phase C: the wide sub-bands that were listed for the level, by teams of warps that share a
+// buffer.  Called by the whole CTA after level 0.  Out of line: its registers stay out of the kernel's narrow path.
 template <bool TIMING, int FORM>
-__device__ __noinline__ void tile_wide(TileSmem& s, int op, int nsb, int Ny, int nA, char* base,
+__device__ __noinline__ void tile_wide(TileSmem& s, int op, int first, int nsb, int Ny, int nA, char* base,
                                        unsigned long long scr, long long* tctr) {
-  for (int level = 1; level <= TK_WLEVELS; ++level) {
+  for (int level = first; level <= TK_WLEVELS; ++level) {
     __syncthreads();
-    const int todo = s.err ? 0 : s.nwide[level - 1];
+    const int todo = s.err ? 0 : s.nwide[level];
     if (todo == 0) break;  // uniform: neither changes before the next barrier
     if (threadIdx.x == 0) s.sbnext = 0;
     __syncthreads();
     const int lead = gb_warp() & ~((1 << level) - 1);
-    const bool first = (threadIdx.x & ((32 << level) - 1)) == 0;  // of the team
+    const bool one = (threadIdx.x & ((32 << level) - 1)) == 0;  // of the team
     for (;;) {
       team_sync(level);  // the sub-band before is done with the team's words
-      if (first) s.tmp64[24 + lead] = atomicAdd(&s.sbnext, 1);
+      if (one) {
+        const int k = atomicAdd(&s.sbnext, 1), w = *(volatile int*)&s.nwide[level + 1];
+        // once three of four were too wide for the level, the rest are listed for the next without a try
+        s.tmp64[24 + lead] = k | (w >= TK_NW && w * 4 >= k * 3 ? 1ll << 32 : 0ll);
+      }
       team_sync(level);
-      const int k = (int)s.tmp64[24 + lead];
+      const long long e = s.tmp64[24 + lead];
+      const int k = (int)e;
       if (k >= todo) break;
-      const int sb = TK_WLIST(s, level - 1, nsb)[k];
-      if (!tile_subband<TIMING, true, FORM>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr) && first)
-        TK_WLIST(s, level, nsb)[atomicAdd(&s.nwide[level], 1)] = sb;
+      const int sb = TK_WLIST(s, level, nsb)[k];
+      if ((e >> 32 || !tile_subband<TIMING, true, FORM>(s, op, sb, nsb, Ny, nA, base, scr, level, tctr)) && one)
+        TK_WLIST(s, level + 1, nsb)[atomicAdd(&s.nwide[level + 1], 1)] = sb;
     }
   }
 }
@@ -1517,22 +1542,25 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
         if (q < nsb && (tid & 7) == 0) ord[r] = q;
       }
     }
-    if (tid <= TK_WLEVELS) s.nwide[tid] = 0;
+    if (tid < TK_WLEVELS + 2) s.nwide[tid] = 0;
     if (tid == 0) {
       s.sbnext = 0;
       s.narrow = 0;
     }
     __syncthreads();
     // level 0: every warp with its own buffer.  Wide sub-bands are listed for level 1; once three of four have
-    // been wide (or when the previous tile's were), the rest are listed without a try.
-    const bool direct = s.hint != 0;
+    // been wide (or when the previous tile's were), the rest are listed without a try.  Those of a tile with more y
+    // ranks than the buffer holds are listed for the wide form's level 0 while its buffer holds them.
+    const int nwy = ((Ny - 1) >> 5) + 1;
+    const bool mostly = s.hint != 0, tall = nwy > TK_LBW && nwy <= wide_lbw(0);
+    const int first = tall && !mostly ? 0 : 1;  // level of the listed ones
     if (!s.err) {
       for (;;) {
         int k = 0;
-        bool list = direct;
+        bool list = mostly || tall;
         if (gb_lane() == 0) {
           k = atomicAdd(&s.sbnext, 1);
-          const int w = *(volatile int*)&s.nwide[0];
+          const int w = *(volatile int*)&s.nwide[1];
           list |= w >= TK_NW && w * 4 >= k * 3;
         }
         k = __shfl_sync(0xffffffffu, k, 0);
@@ -1540,13 +1568,13 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
         const int sb = lpt ? ord[k] : k;
         if (__any_sync(0xffffffffu, list) ||
             !tile_subband<TIMING, false, FORM>(s, op, sb, nsb, Ny, nA, base, scr, 0, timing ? counter + 24 : nullptr)) {
-          if (gb_lane() == 0) TK_WLIST(s, 0, nsb)[atomicAdd(&s.nwide[0], 1)] = sb;
+          if (gb_lane() == 0) TK_WLIST(s, first, nsb)[atomicAdd(&s.nwide[first], 1)] = sb;
         }
       }
     }
     __syncthreads();
-    if (s.nwide[0]) tile_wide<TIMING, FORM>(s, op, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
-    if (tid == 0 && !s.err) s.hint = direct ? s.narrow * 4 <= nsb : s.nwide[0] * 4 >= nsb * 3;
+    if (s.nwide[first]) tile_wide<TIMING, FORM>(s, op, first, nsb, Ny, nA, base, scr, timing ? counter + 24 : nullptr);
+    if (tid == 0 && !s.err) s.hint = mostly ? s.narrow * 4 <= nsb : s.nwide[1] * 4 >= nsb * 3;
     if (AREA) {
       __syncthreads();
       if (tid == 0) {
