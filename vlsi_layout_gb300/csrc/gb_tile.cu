@@ -161,6 +161,7 @@ struct TileSmem {
   int rsplit;  // some sub-band's piece records did not fit the record region (allocated below instead)
   TileRef nx;   // the next tile, reserved and looked up during this tile's phase D
   int have_nx;
+  long long nxi;  // a work item reserved but not looked up yet (-1: none)
   long long obase;
   DStatus* st;
   // up: bytes allocated from the lower half of the scratch; down: strip pieces so far, whose records sit at
@@ -1170,6 +1171,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s.have_nx = 0;
+    s.nxi = -1;
     s.hint = 0;
   }
   for (;;) {
@@ -1193,7 +1195,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
         // reserved before one is looked up (1000 boxes on 2^24 tiles: 51.6 ms with the block's barriers for every
         // tile); not at the end, where a tile reserved behind another would keep other CTAs idle.
         auto reserve = [&]() { return (long long)atomicAdd((unsigned long long*)counter, 1ull); };
-        long long i = reserve(), j = -1;
+        long long i = s.nxi >= 0 ? s.nxi : reserve(), j = -1;
         for (;;) {
           item(i, r);
           if (r.tile >= O->ntiles || r.nA + r.nB) break;
@@ -1201,10 +1203,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
           i = j >= 0 ? j : reserve();
           j = r.tile + 4ll * gridDim.x < O->ntiles ? reserve() : -1;
         }
-        if (j >= 0) {
-          item(j, s.nx);
-          s.have_nx = 1;
-        }
+        s.nxi = j;
       }
       if (st->err && !SPLIT) r.tile = 1ll << 62;  // an error stops the CTA, a reserved tile too
       s.tile = r.tile;
@@ -1628,8 +1627,9 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
     }
     // the next tile's reservation (the work counter) and its descriptor load run on the last thread while
     // the bulk copies below land
-    if (!SPLIT && tid == TK_NT - 1 && !s.have_nx && !st->err) {
-      tile_lookup(op, A, B, O, (long long)atomicAdd((unsigned long long*)counter, 1ull), s.nx);
+    if (!SPLIT && tid == TK_NT - 1 && !st->err) {
+      tile_lookup(op, A, B, O, s.nxi >= 0 ? s.nxi : (long long)atomicAdd((unsigned long long*)counter, 1ull), s.nx);
+      s.nxi = -1;
       s.have_nx = 1;
     }
     PieceRec* PR = prs ? reinterpret_cast<PieceRec*>(s.dbuf) : nullptr;
