@@ -153,13 +153,11 @@ __device__ __forceinline__ void warp_tiles(const DLayer* raw, const DLayer* bin,
           if (u * 32 < k && closed_overlap(ba, bb[u])) m[u] |= 1u << i;
       }
       m[w] &= (1u << lane) - 1u;  // earlier boxes only
-#pragma unroll
-      for (int u = w; u < UF_LB; ++u)
-        if (u * 32 + lane >= k) m[u] = 0;  // no box: the inverted one held there meets a box that spans all of int32
       unsigned all = 0;
 #pragma unroll
       for (int u = w; u < UF_LB; ++u) {
         if (u * 32 >= k) break;
+        if (u * 32 + lane >= k) m[u] = 0;  // no box: the inverted one held there meets a box that spans all of int32
         if (m[u]) {
           hit |= 1u << u;
           met(u * 32 + lane, w * 32, m[u]);
