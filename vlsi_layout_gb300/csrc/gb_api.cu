@@ -1133,9 +1133,14 @@ static int morton_sort_impl(gb_context* ctx, c_box* boxes, long long n, int sort
                             bool dev_io) {
   GbCtx& c = ctx->c;
   if (n <= 0) return GB_OK;
+  // Up to 2^20 boxes one allocation for all (two less: 1000 boxes 112 us and not 119); above, the output arrays once
+  // the sort's own buffers are free again: 44 bytes a box at most, not 64.
+  const bool one = n <= 1 << 20;
+  const size_t nb2 = sort_boxes ? (size_t)n * 16 : 0, np = perm_out && !dev_io ? (size_t)n * 8 : 0;
   GbTmp M(c);
   // keys, then one word for their span
-  const size_t o_k = M.add((size_t)(n + 1) * 8), o_v = M.add((size_t)n * 4), o_b = M.add(dev_io ? 0 : (size_t)n * 16);
+  const size_t o_k = M.add((size_t)(n + 1) * 8), o_v = M.add((size_t)n * 4), o_b = M.add(dev_io ? 0 : (size_t)n * 16),
+               o_b2 = M.add(one ? nb2 : 0), o_p = M.add(one ? np : 0);
   if (!M.get()) return GB_ERR_OOM;
   int4* db = dev_io ? (int4*)boxes : M.ptr<int4>(o_b);
   unsigned long long* dk = M.ptr<unsigned long long>(o_k);
@@ -1146,12 +1151,11 @@ static int morton_sort_impl(gb_context* ctx, c_box* boxes, long long n, int sort
   const int e = sort_keys_perm(ctx, dk, dv, n, dk + n);
   if (e) return e;
   if (keys_out) cudaMemcpy(keys_out, dk, (size_t)n * 8, dev_io ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost);
-  // the outputs' arrays once the sort's own are free again: 44 bytes a box at most, not 64
   if (perm_out) {
     GbTmp P(c);
-    P.add(dev_io ? 0 : (size_t)n * 8);
-    if (!dev_io && !P.get()) return GB_ERR_OOM;
-    long long* dp = dev_io ? perm_out : P.ptr<long long>(0);
+    P.add(np);
+    if (!one && np && !P.get()) return GB_ERR_OOM;
+    long long* dp = dev_io ? perm_out : one ? M.ptr<long long>(o_p) : P.ptr<long long>(0);
     k_perm_out<<<c.work_blocks, 256, 0, c.stream>>>(dv, dp, n, perm_add);
     if (!dev_io) {
       cudaMemcpyAsync(perm_out, dp, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream);
@@ -1160,9 +1164,9 @@ static int morton_sort_impl(gb_context* ctx, c_box* boxes, long long n, int sort
   }
   if (sort_boxes) {
     GbTmp B(c);
-    B.add((size_t)n * 16);
-    if (!B.get()) return GB_ERR_OOM;
-    int4* db2 = B.ptr<int4>(0);
+    B.add(nb2);
+    if (!one && !B.get()) return GB_ERR_OOM;
+    int4* db2 = one ? M.ptr<int4>(o_b2) : B.ptr<int4>(0);
     k_gather_boxes<<<c.work_blocks, 256, 0, c.stream>>>(db, dv, db2, n);
     cudaMemcpyAsync(boxes, db2, (size_t)n * 16, dev_io ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                     c.stream);
