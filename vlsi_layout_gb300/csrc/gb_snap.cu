@@ -1074,7 +1074,7 @@ __device__ __forceinline__ int sn_copy_piece(unsigned char* o, unsigned off, int
 
 // One CTA per fragment (see the top; one warp per fragment, 2048 steps of 32
 // positions behind one another and bytes copied singly, took 1950 us for 1600
-// fragments, this 706 us: bound by shared memory, 74% of its wavefronts, the
+// fragments, this 620 us: bound by shared memory, 74% of its wavefronts, the
 // hash tables' random 2-byte accesses most of them; match_any in every step
 // cost 1097 us, the scan one hash at a time 838 us).  fsrc / flen: the fragment's bytes in raw; the compressed
 // elements go to fout + f * SN_FCAP, their count to flout.

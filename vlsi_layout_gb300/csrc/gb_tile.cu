@@ -34,8 +34,9 @@
 //     row) order, so a column with many pieces does not hold up the warp; a
 //     piece's 16-byte record goes to the CTA's record region at its index.
 //     A sub-band with more columns or y ranks than a warp's buffer holds is
-//     wide: the tile's wide ones are swept afterwards by teams of warps with
-//     larger buffers.
+//     wide: the tile's wide ones are swept afterwards, tall ones of few columns
+//     by single warps with a layout for more y ranks, the others by teams of
+//     warps with larger buffers.
 //  D. Stitch.  The records come into shared memory in one bulk copy.  Each
 //     continuation is linked to the open piece of the previous sub-band with
 //     the same y-interval; every chain head becomes one strip.  The output
@@ -1316,7 +1317,7 @@ k_tile(int op, const DLayer* A, const DLayer* B, DLayer* O, int g, char* scratch
     else mark(piece_g);
     __syncthreads();
     int Nx, Ny, t16o;
-    // The value tables fit on chip (9136 values less 4 a sub-band): phase B writes them from the pieces' ranks, and
+    // The value tables fit on chip (9232 values less 4 a sub-band): phase B writes them from the pieces' ranks, and
     // they stay there.  Walking the bitmaps' bits into the scratch and copying the tables back for phase D took 4 us
     // of a 1024-cell deck's 58 us a tile (28.10 -> 27.22 ms).
     bool t16;
